@@ -8,29 +8,23 @@
 // pivot t lives in physical row prow[t].
 //
 // One window of 256 columns (4 words) at a time:
-//   window_factor   one CTA.  Walks the list of active rows in chunks of 320.
-//                   Each row's window part is reduced by the basis found so
-//                   far (reduced row echelon, lowest set bit leading) through
-//                   64 tables of the 16 combinations of 4 basis vectors; the
-//                   rows left nonzero are eliminated among themselves by a
-//                   CTA-wide Gauss-Jordan (a thread per row, one barrier per
-//                   pivot: the next pivot is the row with the lowest leading
-//                   bit, found by a warp min-reduction and a shared-memory
-//                   atomicMin); the older basis vectors are then reduced by the
-//                   new ones.  Every basis vector carries its combination
-//                   ("tag") over the rows P_j that entered the basis, so
-//                   R_window = T * A[P, window].  The walk stops as soon as the
-//                   basis spans every column of the window.  The walked part of
-//                   the list is then compacted in place (pivot rows and rows
-//                   found zero from the window on are dropped, order kept).
-//   window_combine  R_t = sum_j T[t][j] A[P_j] over the words from the window
+//   window_factor   one CTA.  Walks the list of active rows in chunks of 320
+//                   and brings the window part to reduced row echelon form
+//                   (lowest set bit leading), 32 columns at a time.  Every
+//                   basis vector carries its combination ("tag") over the rows
+//                   P_b that entered the basis, so R_window = tag * A[P, window].
+//                   The walk stops as soon as the basis spans every column of
+//                   the window.  The walked part of the list is then compacted
+//                   in place (pivot rows and rows found zero from the window on
+//                   are dropped, order kept).
+//   window_combine  R_b = sum_j tag[b][j] A[P_j] over the words from the window
 //                   on, into the panel buffer (a block per 4 words, 4-bit
 //                   tables over the P rows).
 //   window_coef     every other row to update (rank: the active rows; RREF: all
 //                   rows) whose bits at the window's pivot columns are not all
 //                   zero gets a slot; those bits become a row of 0/1 bytes.
-//   window_rt       R transposed as 0/1 bytes, Rt8[j][t] = bit j of R_t, and
-//                   R_t written over row P_t.
+//   window_rt       R transposed as 0/1 bytes, Rt8[j][b] = bit j of R_b, and
+//                   R_b written over row P_b.
 //   tc_update       A[row(slot), w..] ^= parity(X8[slot] . Rt8^T): tcgen05
 //                   kind::i8 128 x 256 tiles with K = 256.  A persistent CTA
 //                   keeps a 256-column strip of Rt8 in shared memory and
@@ -38,8 +32,8 @@
 //                   TMEM accumulators; sixteen epilogue warps XOR the parity
 //                   bits into the packed rows while the next tile is
 //                   multiplied, and flag the rows that are still nonzero.
-// Since the basis is reduced, a row's coefficient for R_t is its own bit at
-// pivot column t, and XORing sum_t x_t R_t clears every pivot column of the
+// Since the basis is reduced, a row's coefficient for R_b is its own bit at
+// pivot column b, and XORing sum_b x_b R_b clears every pivot column of the
 // window; a row whose window part lies in the basis' span (every active row,
 // once the scan has ended) is then zero across the window.
 #include <climits>
@@ -62,50 +56,63 @@ constexpr int WW = 4;         // words per window
 constexpr int WBITS = 256;    // columns per window
 constexpr int WF_THREADS = 320;  // a chunk of rows; 320 random rows span 256 columns but with probability 2^-64
 
+// Everything that belongs to a pivot of a window is indexed by its column in
+// the window (0..255), so the coefficient of a row is its window part masked
+// by `have`.
 struct WinState {
     long long rank;         // pivots so far (every window)
     int rt;                 // pivots of the current window
     int nu;                 // rows to update in the current window
     int na;                 // rows in the active-row list
     int lbase;              // the list is list[lbase .. lbase + na)
-    u64 have[WW];           // window-relative pivot columns
-    int prow[WBITS];        // physical row of P-index j
-    u64 tag[WBITS][WW];     // pivot t (ascending column): R_t = sum_j bit j * A[prow[j]]
+    u64 have[WW];           // pivot columns of the window
+    int prow[WBITS];        // physical row P_b of pivot column b (-1: none)
+    u64 tag[WBITS][WW];     // R_b = sum_j bit j * A[P_j]
 };
 
+constexpr int WF_CAND = 64;  // rows one selection round eliminates among themselves
+
 struct WfSmem {
-    u64 bd[WBITS][WW];        // basis vector whose leading bit is b
-    u64 bt[WBITS][WW];        // its tag
-    u64 tab[64][16][WW];      // nibble tables of the basis
-    u64 tabt[64][16][WW];     // the same over the tags
-    u64 cx[WF_THREADS][WW];   // rows of the current chunk (residual)
-    u64 ct[WF_THREADS][WW];   //   and their tags
-    int newslot[WBITS];       // chunk slot of the k-th new basis vector
-    int newlead[WBITS];       //   and its leading bit
-    int prow[WBITS];          // physical row of P-index j
-    u64 have[WW];
-    unsigned keys[3];         // smallest key, rotating by iteration
-    int nb, cnt;
+    uint4 basis[WBITS][2];    // vector of pivot column b (in-place form)
+    uint4 tab[2][64][16];     // 4-bit tables of the basis, a plane per 16-byte half
+    uint4 vt[2][8][16];       // 4-bit tables of a round's pivot rows
+    uint4 cv[WF_CAND][2];     // the candidates' vectors
+    u32 tt[8][16];            // 4-bit tables of T
+    u32 cand[WF_CAND];        // the candidates' data bits in the half word
+    u32 T[32];                // row of T of the pivot in column c of the half word
+    int ci[32];               // its candidate (-1: no pivot)
+    int pcol[WF_CAND];        // column of a candidate's pivot (-1: none)
+    u32 C;                    // the round's pivot columns
+    int prow[WBITS];          // physical row of pivot column b
+    int cnt;
+    int wcnt[2][32];          // candidates per warp, alternating
     int wsum[32];
 };
 
 __device__ __forceinline__ int ctz64w(u64 x) { return __ffsll((long long)x) - 1; }
 
-// Word q of a 4-word vector held in registers (selects, no local memory).
-__device__ __forceinline__ u64 sel4(const u64 (&v)[WW], int q)
+// Half word h of an 8-word vector held in registers (selects, no local memory).
+__device__ __forceinline__ u32 sel8(const u32 (&v)[8], int h)
 {
-    return q == 0 ? v[0] : (q == 1 ? v[1] : (q == 2 ? v[2] : v[3]));
+    const u32 a = (h & 1) ? v[1] : v[0], b = (h & 1) ? v[3] : v[2];
+    const u32 c = (h & 1) ? v[5] : v[4], d = (h & 1) ? v[7] : v[6];
+    const u32 e = (h & 2) ? b : a, f = (h & 2) ? d : c;
+    return (h & 4) ? f : e;
 }
-__device__ __forceinline__ bool bit_of(const u64 (&v)[WW], int b) { return (sel4(v, b >> 6) >> (b & 63)) & 1; }
-__device__ __forceinline__ void or_word(u64 (&v)[WW], int q, u64 x)
+__device__ __forceinline__ void xor8(u32 (&v)[8], const uint4 &a, const uint4 &b)
 {
-#pragma unroll
-    for (int i = 0; i < WW; ++i) v[i] |= (i == q) ? x : 0ull;
+    v[0] ^= a.x;
+    v[1] ^= a.y;
+    v[2] ^= a.z;
+    v[3] ^= a.w;
+    v[4] ^= b.x;
+    v[5] ^= b.y;
+    v[6] ^= b.z;
+    v[7] ^= b.w;
 }
-__device__ __forceinline__ void xor4s(u64 (&a)[WW], const u64 *b)
+__device__ __forceinline__ uint4 xor4u(const uint4 &a, const uint4 &b)
 {
-#pragma unroll
-    for (int q = 0; q < WW; ++q) a[q] ^= b[q];
+    return make_uint4(a.x ^ b.x, a.y ^ b.y, a.z ^ b.z, a.w ^ b.w);
 }
 __device__ __forceinline__ bool any4(const u64 (&v)[WW]) { return (v[0] | v[1] | v[2] | v[3]) != 0; }
 
@@ -137,6 +144,89 @@ __device__ __forceinline__ int block_slot(bool flag, int *wsum, int &total)
 }  // namespace
 
 // ---------------------------------------------------------------- window_factor
+namespace {
+
+// Gauss-Jordan of up to 64 candidate rows over the 32 columns of a half word,
+// by one warp, columns in lanes: lane c's mask holds column c of the rows (bit
+// r = row r).  A step broadcasts column c, takes its lowest unused row p as
+// the pivot and, in every other lane whose column has bit p, XORs in the rows
+// that hold bit c.  The rows stay in in-place form: lane c's own mask is left
+// alone, its bits now meaning "contains pivot row p".  Column c + 1 is fetched
+// while the step before it runs and brought up to date in registers, so a
+// step's chain is a few logical operations and no shuffle latency.
+__device__ __forceinline__ void wf_select(WfSmem &S, int ncand)
+{
+    const int lane = threadIdx.x & 31;
+    const u32 lo = lane < ncand ? S.cand[lane] : 0u;
+    const u32 hi = lane + 32 < ncand ? S.cand[lane + 32] : 0u;
+    u64 col = (u64)transpose32_warp(lo) | ((u64)transpose32_warp(hi) << 32);
+    u64 unused = ~0ull, mypb = 0;
+    u64 cur = __shfl_sync(0xffffffffu, col, 0);
+#pragma unroll
+    for (int c = 0; c < 32; ++c) {
+        u64 nx = __shfl_sync(0xffffffffu, col, (c + 1) & 31);
+        const u64 av = cur & unused;
+        const u64 pb = av & (~av + 1);
+        const u64 rs = cur ^ pb;
+        unused ^= pb;
+        if (lane == c)
+            mypb = pb;
+        else if (col & pb)
+            col ^= rs;
+        if (nx & pb) nx ^= rs;
+        cur = nx;
+    }
+    const u32 C = __ballot_sync(0xffffffffu, mypb != 0);
+    const u32 wlo = transpose32_warp((u32)col), whi = transpose32_warp((u32)(col >> 32));
+    const int ci = mypb ? ctz64w(mypb) : -1;
+    const u32 t0 = __shfl_sync(0xffffffffu, wlo, ci & 31), t1 = __shfl_sync(0xffffffffu, whi, ci & 31);
+    S.T[lane] = ci < 0 ? 0u : ((ci < 32 ? t0 : t1) & C);
+    S.ci[lane] = ci;
+    if (ci >= 0) S.pcol[ci] = lane;
+    if (lane == 0) S.C = C;
+}
+
+// A row's vector v after a round with pivot columns C of half word h: its
+// bits y at C select sum_k y_k T_k = z, the combination of the round's
+// original pivot rows to add; z itself takes the place of the bits at C.
+__device__ __forceinline__ void wf_apply(const WfSmem &S, u32 (&v)[8], int h, u32 C, u32 z)
+{
+#pragma unroll
+    for (int q = 0; q < 8; ++q) v[q] &= q == h ? ~C : ~0u;
+#pragma unroll
+    for (int g = 0; g < 8; ++g) {
+        const int e = (int)((z >> (4 * g)) & 15);
+        xor8(v, S.vt[0][g][e], S.vt[1][g][e]);
+    }
+#pragma unroll
+    for (int q = 0; q < 8; ++q) v[q] |= q == h ? z : 0u;
+}
+__device__ __forceinline__ u32 wf_times_T(const WfSmem &S, u32 y)
+{
+    u32 z = 0;
+#pragma unroll
+    for (int g = 0; g < 8; ++g) z ^= S.tt[g][(y >> (4 * g)) & 15];
+    return z;
+}
+
+}  // namespace
+
+// Blocked Gauss-Jordan of the window, in place: a row is 256 bits, which at
+// the pivot columns found so far hold its combination over the pivot rows P_b
+// and elsewhere its data (a row with bit c set gets v ^= v_p without bit c, so
+// its bit c stays set and becomes the coefficient of P_c).  One CTA walks the
+// active rows in chunks of a row per thread; the columns go 32 at a time (half
+// words): up to 64 rows with data left there are eliminated by one warp
+// (wf_select), and every row of the chunk then takes the round's pivots in
+// through 4-bit tables; rounds repeat until no unused row has data left in
+// the half word.
+// Bound by the serial chain, not by throughput (one CTA): a step costs about
+// 45 cycles in wf_select and a round of up to 32 pivots four barriers and 16
+// 16-byte table reads a row, against a barrier and about 800 cycles for each
+// pivot when the rows are eliminated one pivot at a time (whole rank of a
+// 3000 x 5000 matrix of rank 2200: 605 against 1418 us; rank and null space
+// of 16384 x 32768, rank 12000: 7.1 against 8.9 ms, the update then setting
+// the pace).
 __global__ void __launch_bounds__(WF_THREADS, 1)
 window_factor_kernel(const u64 *__restrict__ M, i64 ld, i64 m, i64 n, i64 w, int *list, const unsigned char *live,
                      unsigned char *state, int *stamp, int wid, const WinState *prev, WinState *ws, long long *piv,
@@ -144,223 +234,176 @@ window_factor_kernel(const u64 *__restrict__ M, i64 ld, i64 m, i64 n, i64 w, int
 {
     extern __shared__ __align__(16) unsigned char wf_raw[];
     WfSmem &S = *reinterpret_cast<WfSmem *>(wf_raw);
-    const int tid = threadIdx.x, lane = tid & 31;
+    constexpr int NW = WF_THREADS / 32;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const i64 wc = words_of(n);
     const int wn = (wc - w) < WW ? (int)(wc - w) : WW;
     const i64 vb = n - 64 * w;
     const int valid = vb < WBITS ? (int)vb : WBITS;  // columns of this window inside the matrix
     const int na = prev->na;
     int *L0 = list + prev->lbase;
-    constexpr unsigned NOKEY = 0xFFFFFFFFu;
 
-    for (int e = tid; e < 64 * 16 * WW; e += WF_THREADS) {
-        (&S.tab[0][0][0])[e] = 0;
-        (&S.tabt[0][0][0])[e] = 0;
-    }
-    if (tid < WW) S.have[tid] = 0;
-    if (tid == 0) S.nb = 0;
-    __syncthreads();
-
-    int walked = 0;
-    for (int base = 0; base < na; base += WF_THREADS) {
-        if (S.nb >= valid) break;
+    u32 H[8] = {};  // pivot columns so far (the same in every thread)
+    int nb = 0;     // their number
+    int walked = 0, par = 0;
+    for (int base = 0; base < na && nb < valid; base += WF_THREADS) {
         walked = base + WF_THREADS < na ? base + WF_THREADS : na;
-        const int nb0 = S.nb;
-        u64 hv[WW];
+        const bool older = nb > 0;  // basis vectors of earlier chunks
+        u32 H0[8];
 #pragma unroll
-        for (int q = 0; q < WW; ++q) hv[q] = S.have[q];
+        for (int q = 0; q < 8; ++q) H0[q] = H[q];
+        const bool obasis = older && tid < WBITS && ((sel8(H0, (tid >> 5) & 7) >> (tid & 31)) & 1);
+        if (older) {
+            // tables of the 16 combinations of basis vectors 4g..4g+3
+            for (int e = tid; e < 2 * 64 * 16; e += WF_THREADS) {
+                const int half = e >> 10, g = (e >> 4) & 63, v = e & 15;
+                uint4 a = make_uint4(0, 0, 0, 0);
+#pragma unroll
+                for (int b = 0; b < 4; ++b)
+                    if (((v >> b) & 1) && ((sel8(H0, g >> 3) >> ((4 * g + b) & 31)) & 1))
+                        a = xor4u(a, S.basis[4 * g + b][half]);
+                S.tab[half][g][v] = a;
+            }
+            __syncthreads();
+        }
         const int k = base + tid;
         int row = -1;
-        u64 x[WW] = {0, 0, 0, 0};
+        u32 v[8] = {};
         if (k < na) {
             row = L0[k];
 #pragma unroll
             for (int q = 0; q < WW; ++q)
-                if (q < wn) x[q] = M[(i64)row * ld + w + q];
+                if (q < wn) {
+                    const u64 x = M[(i64)row * ld + w + q];
+                    v[2 * q] = (u32)x;
+                    v[2 * q + 1] = (u32)(x >> 32);
+                }
         }
-        u64 cx[WW] = {x[0], x[1], x[2], x[3]}, ct[WW] = {0, 0, 0, 0};
-        if (any4(x) && nb0) {
+        if (older) {
+            u32 y[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                y[q] = v[q] & H0[q];
+                v[q] &= ~H0[q];
+            }
 #pragma unroll
             for (int g = 0; g < 64; ++g) {
-                const int q = g >> 4, sh = 4 * (g & 15);
-                const u64 hn = (hv[q] >> sh) & 15;
-                if (hn) {
-                    const int nib = (int)((x[q] >> sh) & hn);
-                    if (nib) xor4s(cx, S.tab[g][nib]);
-                }
-            }
-            if (any4(cx)) {
-#pragma unroll
-                for (int g = 0; g < 64; ++g) {
-                    const int q = g >> 4, sh = 4 * (g & 15);
-                    const u64 hn = (hv[q] >> sh) & 15;
-                    if (hn) {
-                        const int nib = (int)((x[q] >> sh) & hn);
-                        if (nib) xor4s(ct, S.tabt[g][nib]);
-                    }
-                }
+                const int e = (int)((y[g >> 3] >> (4 * (g & 7))) & 15);
+                if (e) xor8(v, S.tab[0][g][e], S.tab[1][g][e]);
             }
         }
-        // Gauss-Jordan among the chunk's residual rows, a pivot per barrier,
-        // one 64-column word of the window at a time.  A row's key is
-        // (leading bit, slot); the next pivot is the smallest key.  Inside
-        // word q every unused row is zero in the words before q, so its key
-        // comes from word q alone and a pivot row is XORed in from word q on;
-        // word q is done once no unused row has a bit left there.  Only the
-        // row holding its warp's smallest key publishes itself to shared
-        // memory, its tag already carrying the P-index it would enter as, so
-        // the pivot is always published.
-        bool used = false;
-        int myj = -1;
-        unsigned key = NOKEY;
-        auto publish = [&](unsigned *kslot, int jn) {
-            const unsigned mk = __reduce_min_sync(0xffffffffu, key);
-            if (key == mk && key != NOKEY) {
-                ulonglong2 *dv = reinterpret_cast<ulonglong2 *>(S.cx[tid]);
-                ulonglong2 *dt = reinterpret_cast<ulonglong2 *>(S.ct[tid]);
-                const u64 e = 1ull << (jn & 63);
-                const int jq = jn >> 6;
-                dv[0] = make_ulonglong2(cx[0], cx[1]);
-                dv[1] = make_ulonglong2(cx[2], cx[3]);
-                dt[0] = make_ulonglong2(ct[0] ^ (jq == 0 ? e : 0ull), ct[1] ^ (jq == 1 ? e : 0ull));
-                dt[1] = make_ulonglong2(ct[2] ^ (jq == 2 ? e : 0ull), ct[3] ^ (jq == 3 ? e : 0ull));
-            }
-            if (lane == 0 && mk != NOKEY) atomicMin(kslot, mk);
-        };
-        int nnew = 0;
-#pragma unroll
-        for (int q = 0; q < WW; ++q) {
-            if (nb0 + nnew >= valid) break;  // uniform
-            key = (!used && cx[q]) ? ((unsigned)(64 * q + ctz64w(cx[q])) << 10 | (unsigned)tid) : NOKEY;
-            __syncthreads();  // the previous word's last keys have been read
-            if (tid < 3) S.keys[tid] = NOKEY;
-            __syncthreads();
-            publish(&S.keys[0], nb0 + nnew);
-            __syncthreads();
-            int kr = 0;  // slot holding this iteration's key
-            for (;;) {
-                const unsigned kk = S.keys[kr];
-                if (kk == NOKEY || nb0 + nnew >= valid) break;
-                const int kn = kr == 2 ? 0 : kr + 1, kz = kn == 2 ? 0 : kn + 1;
-                if (tid == 0) S.keys[kz] = NOKEY;  // read last in the previous iteration
-                const int p = (int)(kk & 1023u), L = (int)(kk >> 10);
-                if (tid == p) {
-                    used = true;
-                    myj = nb0 + nnew;
-                    key = NOKEY;
-                    S.newslot[nnew] = p;
-                    S.newlead[nnew] = L;
-                    S.prow[myj] = row;
-                } else if ((cx[q] >> (L & 63)) & 1) {
-                    const u64 *pv = S.cx[p];
-                    const ulonglong2 *pt = reinterpret_cast<const ulonglong2 *>(S.ct[p]);
-                    const ulonglong2 t0 = pt[0], t1 = pt[1];
-#pragma unroll
-                    for (int qq = q; qq < WW; ++qq) cx[qq] ^= pv[qq];
-                    ct[0] ^= t0.x;
-                    ct[1] ^= t0.y;
-                    ct[2] ^= t1.x;
-                    ct[3] ^= t1.y;
-                    if (!used) key = cx[q] ? ((unsigned)(64 * q + ctz64w(cx[q])) << 10 | (unsigned)tid) : NOKEY;
-                }
-                ++nnew;
-                publish(&S.keys[kn], nb0 + nnew);
-                kr = kn;
+        int mycol = -1;  // this row's pivot column
+        for (int h = 0; h < 8 && nb < valid; ++h) {
+            u32 Hh = sel8(H, h);
+            while (Hh != 0xffffffffu && nb < valid) {
+                const u32 d = mycol < 0 ? sel8(v, h) & ~Hh : 0u;
+                const unsigned bal = __ballot_sync(0xffffffffu, d != 0);
+                par ^= 1;
+                if (lane == 0) S.wcnt[par][warp] = __popc(bal);
                 __syncthreads();
-            }
-        }
-        __syncthreads();  // every key is read before the next chunk publishes
-        if (nnew == 0) continue;  // uniform
-        if (used) {
-            ct[0] ^= (myj >> 6) == 0 ? (1ull << (myj & 63)) : 0ull;
-            ct[1] ^= (myj >> 6) == 1 ? (1ull << (myj & 63)) : 0ull;
-            ct[2] ^= (myj >> 6) == 2 ? (1ull << (myj & 63)) : 0ull;
-            ct[3] ^= (myj >> 6) == 3 ? (1ull << (myj & 63)) : 0ull;
-#pragma unroll
-            for (int q = 0; q < WW; ++q) {
-                S.cx[tid][q] = cx[q];
-                S.ct[tid][q] = ct[q];
-            }
-        }
-        __syncthreads();
-        // older basis vectors: clear the new leading bits (the new vectors are
-        // reduced among themselves and zero at the older leads)
-        if (nb0 && tid < WBITS && ((S.have[tid >> 6] >> (tid & 63)) & 1)) {
-            u64 v[WW], t[WW];
-#pragma unroll
-            for (int q = 0; q < WW; ++q) {
-                v[q] = S.bd[tid][q];
-                t[q] = S.bt[tid][q];
-            }
-            const u64 ov[WW] = {v[0], v[1], v[2], v[3]};
-            for (int e = 0; e < nnew; ++e) {
-                if (bit_of(ov, S.newlead[e])) {
-                    xor4s(v, S.cx[S.newslot[e]]);
-                    xor4s(t, S.ct[S.newslot[e]]);
+                const int wv = lane < NW ? S.wcnt[par][lane] : 0;
+                const int total = __reduce_add_sync(0xffffffffu, wv);
+                if (total == 0) break;
+                int idx = __reduce_add_sync(0xffffffffu, lane < warp ? wv : 0) + __popc(bal & ((1u << lane) - 1));
+                if (d == 0 || idx >= WF_CAND) idx = -1;
+                if (idx >= 0) {
+                    S.cand[idx] = d;
+                    S.cv[idx][0] = make_uint4(v[0], v[1], v[2], v[3]);
+                    S.cv[idx][1] = make_uint4(v[4], v[5], v[6], v[7]);
+                    S.pcol[idx] = -1;
                 }
-            }
+                __syncthreads();
+                if (warp == 0) wf_select(S, total < WF_CAND ? total : WF_CAND);
+                __syncthreads();
+                const u32 C = S.C;
+                // tables over the round's pivots: their original rows (without
+                // the bits at C) and the rows of T
+                if (tid < 256) {
+                    const int half = tid >> 7, g = (tid >> 4) & 7, e = tid & 15;
+                    uint4 a = make_uint4(0, 0, 0, 0);
 #pragma unroll
-            for (int q = 0; q < WW; ++q) {
-                S.bd[tid][q] = v[q];
-                S.bt[tid][q] = t[q];
-            }
-        }
-        __syncthreads();
-        if (tid < nnew) {
-            const int Ld = S.newlead[tid], sl = S.newslot[tid];
+                    for (int b = 0; b < 4; ++b) {
+                        const int ci = S.ci[4 * g + b];
+                        if (((e >> b) & 1) && ci >= 0) a = xor4u(a, S.cv[ci][half]);
+                    }
+                    if (half == (h >> 2)) {
+                        const int q = h & 3;
+                        a.x &= q == 0 ? ~C : ~0u;
+                        a.y &= q == 1 ? ~C : ~0u;
+                        a.z &= q == 2 ? ~C : ~0u;
+                        a.w &= q == 3 ? ~C : ~0u;
+                    }
+                    S.vt[half][g][e] = a;
+                }
+                for (int x = WF_THREADS - 1 - tid; x < 128; x += WF_THREADS) {
+                    const int g = x >> 4, e = x & 15;
+                    u32 a = 0;
 #pragma unroll
-            for (int q = 0; q < WW; ++q) {
-                S.bd[Ld][q] = S.cx[sl][q];
-                S.bt[Ld][q] = S.ct[sl][q];
-            }
-        }
-        if (tid == 0) {
-            for (int e = 0; e < nnew; ++e) S.have[S.newlead[e] >> 6] |= 1ull << (S.newlead[e] & 63);
-            S.nb = nb0 + nnew;
-        }
-        __syncthreads();
-        if (S.nb < valid && base + WF_THREADS < na) {
-            // tables of the 16 combinations of basis vectors 4g..4g+3
-            for (int e = tid; e < 64 * 16; e += WF_THREADS) {
-                const int g = e >> 4, v = e & 15;
-                u64 a[WW] = {0, 0, 0, 0}, b[WW] = {0, 0, 0, 0};
+                    for (int b = 0; b < 4; ++b) a ^= ((e >> b) & 1) ? S.T[4 * g + b] : 0u;
+                    S.tt[g][e] = a;
+                }
+                const int pc = idx >= 0 ? S.pcol[idx] : -1;
+                __syncthreads();
+                if (pc >= 0) {
+                    mycol = 32 * h + pc;
+                    S.prow[mycol] = row;
 #pragma unroll
-                for (int h = 0; h < 4; ++h) {
-                    const int bb = 4 * g + h;
-                    if (((v >> h) & 1) && ((S.have[bb >> 6] >> (bb & 63)) & 1)) {
-                        xor4s(a, S.bd[bb]);
-                        xor4s(b, S.bt[bb]);
+                    for (int q = 0; q < 8; ++q) v[q] = 0;
+                    wf_apply(S, v, h, C, S.T[pc]);
+                } else {
+                    const u32 y = sel8(v, h) & C;
+                    if (y) wf_apply(S, v, h, C, wf_times_T(S, y));
+                }
+                if (obasis) {
+                    uint4 a = S.basis[tid][0], b = S.basis[tid][1];
+                    u32 o[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+                    const u32 y = sel8(o, h) & C;
+                    if (y) {
+                        wf_apply(S, o, h, C, wf_times_T(S, y));
+                        S.basis[tid][0] = make_uint4(o[0], o[1], o[2], o[3]);
+                        S.basis[tid][1] = make_uint4(o[4], o[5], o[6], o[7]);
                     }
                 }
+                nb += __popc(C);
+                Hh |= C;
 #pragma unroll
-                for (int q = 0; q < WW; ++q) {
-                    S.tab[g][v][q] = a[q];
-                    S.tabt[g][v][q] = b[q];
-                }
+                for (int q = 0; q < 8; ++q) H[q] |= q == h ? C : 0u;
             }
-            __syncthreads();
         }
+        if (mycol >= 0) {
+            S.basis[mycol][0] = make_uint4(v[0], v[1], v[2], v[3]);
+            S.basis[mycol][1] = make_uint4(v[4], v[5], v[6], v[7]);
+        }
+        __syncthreads();
     }
 
-    // results: pivot t = t-th leading bit; P-index t is its physical row
-    const int nb = S.nb;
+    // results, by column; pivot t of the window is its t-th pivot column
     const long long r0 = prev->rank;
-    if (tid < WBITS && ((S.have[tid >> 6] >> (tid & 63)) & 1)) {
-        int t = 0;
-        for (int q = 0; q < (tid >> 6); ++q) t += __popcll(S.have[q]);
-        t += __popcll(S.have[tid >> 6] & ((1ull << (tid & 63)) - 1));
+    if (tid < WBITS) {
+        const u32 hq = sel8(H, tid >> 5);
+        int r = -1;
+        if ((hq >> (tid & 31)) & 1) {
+            int t = __popc(hq & ((1u << (tid & 31)) - 1));
 #pragma unroll
-        for (int q = 0; q < WW; ++q) ws->tag[t][q] = S.bt[tid][q];
-        piv[r0 + t] = 64 * w + tid;
-    }
-    if (tid < nb) {
-        const int r = S.prow[tid];
+            for (int q = 0; q < 8; ++q) t += q < (tid >> 5) ? __popc(H[q]) : 0;
+            const uint4 a = S.basis[tid][0], b = S.basis[tid][1];
+            ws->tag[tid][0] = (u64)(a.x & H[0]) | ((u64)(a.y & H[1]) << 32);
+            ws->tag[tid][1] = (u64)(a.z & H[2]) | ((u64)(a.w & H[3]) << 32);
+            ws->tag[tid][2] = (u64)(b.x & H[4]) | ((u64)(b.y & H[5]) << 32);
+            ws->tag[tid][3] = (u64)(b.z & H[6]) | ((u64)(b.w & H[7]) << 32);
+            r = S.prow[tid];
+            piv[r0 + t] = 64 * w + tid;
+            prow[r0 + t] = r;
+            state[r] = 0;
+            stamp[r] = wid;
+        }
         ws->prow[tid] = r;
-        prow[r0 + tid] = r;
-        state[r] = 0;
-        stamp[r] = wid;
     }
-    if (tid < WW) ws->have[tid] = S.have[tid];
+    if (tid < WW) {
+        const u32 a = tid == 0 ? H[0] : tid == 1 ? H[2] : tid == 2 ? H[4] : H[6];
+        const u32 b = tid == 0 ? H[1] : tid == 1 ? H[3] : tid == 2 ? H[5] : H[7];
+        ws->have[tid] = (u64)a | ((u64)b << 32);
+    }
     if (tid == 0) S.cnt = walked;
     __syncthreads();
     // compact the walked part [0, walked) of the list to its right end, in
@@ -390,9 +433,9 @@ window_factor_kernel(const u64 *__restrict__ M, i64 ld, i64 m, i64 n, i64 w, int
 }
 
 // ---------------------------------------------------------------- window_combine
-// Block: CB_W words x every pivot.  R_t = XOR_j T[t][j] A[P_j] is evaluated
-// four P-indices at a time from 64 tables of the 16 combinations of P rows
-// 4g..4g+3 (restricted to the block's words).
+// Block: CB_W words x every pivot.  R_b = XOR_j tag[b][j] A[P_j] is evaluated
+// four columns j at a time from 64 tables of the 16 combinations of the pivot
+// rows of columns 4g..4g+3 (restricted to the block's words).
 namespace {
 constexpr int CB_W = 4;
 struct CbSmem {
@@ -408,15 +451,15 @@ window_combine_kernel(const u64 *__restrict__ M, i64 ld, i64 wc, i64 w, const Wi
 {
     extern __shared__ __align__(16) unsigned char cb_raw[];
     CbSmem &S = *reinterpret_cast<CbSmem *>(cb_raw);
-    const int rt = ws->rt;
-    if (rt == 0) return;
+    if (ws->rt == 0) return;
     const int tid = threadIdx.x;
     const i64 w0 = w + (i64)blockIdx.x * CB_W;
     {
-        const int j = tid;  // 256 threads: one P row each
+        const int j = tid;  // 256 threads: a column each
+        const int pr = ws->prow[j];
         u64 v[CB_W];
-        if (j < rt) {
-            const u64 *src = M + (i64)ws->prow[j] * ld + w0;
+        if (pr >= 0) {
+            const u64 *src = M + (i64)pr * ld + w0;
 #pragma unroll
             for (int q = 0; q < CB_W; ++q) v[q] = (w0 + q < wc) ? src[q] : 0ull;
         } else {
@@ -426,7 +469,7 @@ window_combine_kernel(const u64 *__restrict__ M, i64 ld, i64 wc, i64 w, const Wi
 #pragma unroll
         for (int q = 0; q < CB_W; ++q) S.rows[j][q] = v[q];
 #pragma unroll
-        for (int q = 0; q < WW; ++q) S.tag[j][q] = j < rt ? ws->tag[j][q] : 0ull;
+        for (int q = 0; q < WW; ++q) S.tag[j][q] = pr >= 0 ? ws->tag[j][q] : 0ull;
     }
     __syncthreads();
     for (int e = tid; e < 64 * 16; e += 256) {
@@ -442,17 +485,18 @@ window_combine_kernel(const u64 *__restrict__ M, i64 ld, i64 wc, i64 w, const Wi
         for (int q = 0; q < CB_W; ++q) S.tab[g][v][q] = a[q];
     }
     __syncthreads();
-    // thread: word q = tid % CB_W, pivots t = tid / CB_W + 64 i
+    // thread: word q = tid % CB_W, columns b = tid / CB_W + 64 i (zero where
+    // there is no pivot)
     const int q = tid % CB_W;
-    for (int t = tid / CB_W; t < rt; t += 256 / CB_W) {
+    for (int b = tid / CB_W; b < WBITS; b += 256 / CB_W) {
         u64 acc = 0;
 #pragma unroll
         for (int qq = 0; qq < WW; ++qq) {
-            const u64 tg = S.tag[t][qq];
+            const u64 tg = S.tag[b][qq];
 #pragma unroll
             for (int g = 0; g < 16; ++g) acc ^= S.tab[16 * qq + g][(tg >> (4 * g)) & 15][q];
         }
-        if (w0 + q < wc) Rbuf[(i64)t * ldr + (w0 + q - w)] = acc;
+        if (w0 + q < wc) Rbuf[(i64)b * ldr + (w0 + q - w)] = acc;
     }
 }
 
@@ -485,33 +529,9 @@ window_coef_kernel(const u64 *__restrict__ M, i64 ld, i64 m, i64 wc, i64 w, cons
         }
         u64 xc[WW] = {0, 0, 0, 0};
         if (row >= 0) {
-            int pos = 0;
 #pragma unroll
-            for (int q = 0; q < WW; ++q) {
-                const u64 h = hv[q];
-                if (q >= wn || !h) continue;
-                const u64 x = M[row * ld + w + q];
-                u64 e;
-                int c;
-                if (h == ~0ull) {
-                    e = x;
-                    c = 64;
-                } else {
-                    e = 0;
-                    c = 0;
-                    u64 hh = h;
-                    while (hh) {
-                        const u64 lb = hh & (~hh + 1);
-                        if (x & lb) e |= 1ull << c;
-                        ++c;
-                        hh ^= lb;
-                    }
-                }
-                const int wq = pos >> 6, sb = pos & 63;
-                or_word(xc, wq, e << sb);
-                if (sb && sb + c > 64) or_word(xc, wq + 1, e >> (64 - sb));
-                pos += c;
-            }
+            for (int q = 0; q < WW; ++q)
+                if (q < wn && hv[q]) xc[q] = M[row * ld + w + q] & hv[q];
         }
         const bool nz = any4(xc);
         const unsigned b = __ballot_sync(0xffffffffu, nz);
@@ -535,19 +555,19 @@ window_coef_kernel(const u64 *__restrict__ M, i64 ld, i64 m, i64 wc, i64 w, cons
 }
 
 // ---------------------------------------------------------------- window_rt
-// Block W (word w + W): Rt8 rows 64W..64W+63 and word w + W of every row P_t.
+// Block W (word w + W): Rt8 rows 64W..64W+63 and word w + W of every row P_b.
 __global__ void __launch_bounds__(256)
 window_rt_kernel(u64 *__restrict__ M, i64 ld, i64 w, const u64 *__restrict__ Rbuf, i64 ldr, const WinState *ws,
                  unsigned char *Rt8)
 {
     __shared__ u64 col[WBITS];
-    const int rt = ws->rt;
-    if (rt == 0) return;
+    if (ws->rt == 0) return;
     const int tid = threadIdx.x;
     const i64 W = blockIdx.x;
-    const u64 v = tid < rt ? Rbuf[(i64)tid * ldr + W] : 0ull;
+    const u64 v = Rbuf[(i64)tid * ldr + W];  // zero where the column has no pivot
     col[tid] = v;
-    if (tid < rt) M[(i64)ws->prow[tid] * ld + w + W] = v;
+    const int pr = ws->prow[tid];
+    if (pr >= 0) M[(i64)pr * ld + w + W] = v;
     __syncthreads();
     for (int e = tid; e < 64 * 16; e += 256) {
         const int jl = e >> 4, c = e & 15;
