@@ -93,7 +93,8 @@ typedef enum {
  *   MELA_TUNE_K(k)     MELA_ELIM_M4RI: table width k in {4, 6, 7, 8, 9, 10}
  *                      (MELA_ELIM_M4RI_K4 takes only 4; MELA_GEMM_M4RI only 8).
  *   MELA_TUNE_TILE(t)  MELA_ELIM_M4RI / _K4: rows per update CTA, t = 1: 256,
- *                      2: 1024 (default), 3: 4096.
+ *                      2: 1024, 3: 4096 (default: 256, or 1024 for
+ *                      panels with many column tiles).
  *                      MELA_GEMM_TC / _TC_FP4: t = 1: one CTA per 128 x 256
  *                      tile; 2: CTA pairs per 256 x 256 tile (the default
  *                      where the padded row count allows).

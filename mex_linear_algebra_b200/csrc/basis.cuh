@@ -1,142 +1,94 @@
-// basis.cuh -- warp-level XOR bases of 64-bit panel words, shared by the
-// blocked elimination of single matrices (elim.cu) and of batches (batch.cu).
+// basis.cuh -- Gauss-Jordan elimination of a few rows over a 32-column half
+// word by one warp: the pivot search of the blocked eliminations (elim.cu,
+// elim_tc.cu).
 //
-// A basis holds at most 64 vectors, each stored under its lowest set bit
-// ("leading bit"); the set of leading bits of any such basis of a space is
-// the space's set of greedy pivot columns.  Alongside each reduced vector
-// the basis keeps the ORIGINAL word and the row it came from, so the rows
-// that entered a basis are original rows spanning the same space.
+// Rows are kept in in-place form: at the pivot columns found so far a row
+// holds its combination over the pivot rows (bit c: contains the original row
+// of pivot column c), elsewhere its data.  Eliminating with pivot row p of
+// column c is v ^= v_p without bit c for every other row with bit c set, whose
+// bit c thereby turns from data into the coefficient of that pivot row.
 #pragma once
 
 #include "mela_common.cuh"
 
 namespace mela {
 
-struct WarpBasis {
-    u64 B[64];  // reduced vector with leading bit b
-    u64 O[64];  // original word of the row that entered at b
-    int R[64];  // that row
-};
-
 __device__ __forceinline__ int ctz64_(u64 x) { return __ffsll((long long)x) - 1; }
 
-// Insert the 32 lane values x (original word o, row r) into `wb`, whose
-// occupied leading bits are `have` (warp-uniform).  Lanes reduce their value
-// by the basis from the lowest bit up; among lanes left with a new leading
-// bit the lowest lane enters first, then the others reduce by it, until no
-// lane holds a nonzero value.
-__device__ inline void warp_basis_insert(WarpBasis &wb, u64 x, u64 o, int r, u64 &have)
+constexpr int kHalfCand = 64;  // rows one selection round eliminates among themselves
+
+// One round's shared state.
+struct HalfRound {
+    u32 tt[8][16];         // 4-bit tables of T
+    u32 cand[kHalfCand];   // the candidates' data bits in the half word
+    u32 T[32];             // row of T of the pivot in column c of the half word
+    int ci[32];            // its candidate (-1: no pivot)
+    int pcol[kHalfCand];   // column of a candidate's pivot (-1: none)
+    u32 C;                 // the round's pivot columns
+};
+
+// Gauss-Jordan of the first ncand candidates by one warp, columns in lanes:
+// lane c's mask (bit r = row r, two registers) holds column c.  A step
+// broadcasts column c, takes its lowest unused row p as the pivot and, in
+// every other lane whose column has bit p, XORs in the rows that hold bit c.
+// Lane c's own mask is left alone: it becomes column c of the combinations.
+// Column c + 1 is fetched while the step before it runs and brought up to
+// date in registers, so a step's chain has no shuffle latency; selects, no
+// branches (64 cycles a step against 115 with a branch on the own column).
+__device__ __forceinline__ void half_word_select(HalfRound &S, int ncand)
 {
     const int lane = threadIdx.x & 31;
-    while (true) {
-        while (x) {
-            const u64 lb = x & (~x + 1);
-            if (!(lb & have)) break;
-            x ^= wb.B[ctz64_(lb)];
-        }
-        const unsigned bal = __ballot_sync(0xffffffffu, x != 0);
-        if (!bal) break;
-        const int src = __ffs(bal) - 1;
-        const u64 xb = __shfl_sync(0xffffffffu, x, src);
-        const u64 ob = __shfl_sync(0xffffffffu, o, src);
-        const int rb = __shfl_sync(0xffffffffu, r, src);
-        const int b = ctz64_(xb);
-        if (lane == 0) {
-            wb.B[b] = xb;
-            wb.O[b] = ob;
-            wb.R[b] = rb;
-        }
-        have |= 1ull << b;
-        if (lane == src) x = 0;
-        __syncwarp();
+    u32 lo = transpose32_warp(lane < ncand ? S.cand[lane] : 0u);
+    u32 hi = transpose32_warp(lane + 32 < ncand ? S.cand[lane + 32] : 0u);
+    u32 ulo = ~0u, uhi = ~0u;    // unused rows
+    u32 mlo = 0, mhi = 0;        // this column's pivot row
+    u32 xlo = __shfl_sync(0xffffffffu, lo, 0), xhi = __shfl_sync(0xffffffffu, hi, 0);
+#pragma unroll
+    for (int c = 0; c < 32; ++c) {
+        const u32 nlo = __shfl_sync(0xffffffffu, lo, (c + 1) & 31);
+        const u32 nhi = __shfl_sync(0xffffffffu, hi, (c + 1) & 31);
+        const u32 alo = xlo & ulo, ahi = xhi & uhi;
+        const u32 plo = alo & (0u - alo), phi = alo ? 0u : ahi & (0u - ahi);
+        const u32 rlo = xlo ^ plo, rhi = xhi ^ phi;
+        ulo ^= plo;
+        uhi ^= phi;
+        const bool own = lane == c;
+        mlo = own ? plo : mlo;
+        mhi = own ? phi : mhi;
+        const bool hit = ((lo & plo) | (hi & phi)) != 0 && !own;
+        lo ^= hit ? rlo : 0u;
+        hi ^= hit ? rhi : 0u;
+        const bool nhit = ((nlo & plo) | (nhi & phi)) != 0;
+        xlo = nhit ? nlo ^ rlo : nlo;
+        xhi = nhit ? nhi ^ rhi : nhi;
     }
+    const u32 C = __ballot_sync(0xffffffffu, (mlo | mhi) != 0);
+    const u32 wlo = transpose32_warp(lo), whi = transpose32_warp(hi);
+    const int ci = mlo ? __ffs(mlo) - 1 : mhi ? 31 + __ffs(mhi) : -1;
+    const u32 t0 = __shfl_sync(0xffffffffu, wlo, ci & 31), t1 = __shfl_sync(0xffffffffu, whi, ci & 31);
+    S.T[lane] = ci < 0 ? 0u : ((ci < 32 ? t0 : t1) & C);
+    S.ci[lane] = ci;
+    if (ci >= 0) S.pcol[ci] = lane;
+    if (lane == 0) S.C = C;
 }
 
-// Insert every vector of basis `src` (occupied bits `src_have`) into `dst`
-// by its original word.
-__device__ inline void warp_basis_merge(WarpBasis &dst, u64 &have, const WarpBasis &src, u64 src_have)
+// Entry x = 16 g + e of the tables of T.
+__device__ __forceinline__ void half_word_tt(HalfRound &S, int x)
 {
-    const int lane = threadIdx.x & 31;
-    for (int half = 0; half < 2; ++half) {
-        const int b = half * 32 + lane;
-        u64 o = 0;
-        int r = 0;
-        if ((src_have >> b) & 1) {
-            o = src.O[b];
-            r = src.R[b];
-        }
-        warp_basis_insert(dst, o, o, r, have);
-    }
+    const int g = x >> 4, e = x & 15;
+    u32 a = 0;
+#pragma unroll
+    for (int b = 0; b < 4; ++b) a ^= ((e >> b) & 1) ? S.T[4 * g + b] : 0u;
+    S.tt[g][e] = a;
 }
-
-// Gauss-Jordan on the final basis (one warp).  With the p = popc(pm) entered
-// rows S_k (k in order of increasing leading bit), finds for each pivot bit
-// b_t (t-th set bit of pm, increasing) the combination coef[t] (bit k set:
-// S_k included) whose restriction to the pivot bits is the unit vector of
-// b_t.  Writes bits[t] = b_t, coef[t], srow[t] (the S row that receives
-// the reduced row t) and sel[k] = S_k.  Returns p.
-__device__ inline int warp_panel_gauss_jordan(const WarpBasis &wb, u64 pm, int *bits, u64 *coef,
-                                              int *srow, int *sel)
+// sum_k y_k T_k: the combination of the round's original pivot rows that
+// clears the bits y at its pivot columns.
+__device__ __forceinline__ u32 half_word_times_T(const HalfRound &S, u32 y)
 {
-    const int lane = threadIdx.x & 31;
-    const int p = __popcll(pm);
-    u64 q[2], a[2];
-    int rowk[2], step[2] = {-1, -1};
-    bool used[2] = {false, false};
+    u32 z = 0;
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const int k = lane + 32 * h;
-        q[h] = 0;
-        a[h] = 0;
-        rowk[h] = -1;
-        if (k < p) {
-            u64 t = pm;
-            for (int i = 0; i < k; ++i) t &= t - 1;
-            const int b = ctz64_(t);
-            q[h] = wb.O[b] & pm;
-            a[h] = 1ull << k;
-            rowk[h] = wb.R[b];
-        }
-    }
-    // The row chosen at step t keeps being reduced by later steps, so its
-    // combination is final only after the loop.
-    u64 rest = pm;
-    for (int t = 0; t < p; ++t) {
-        const int b = ctz64_(rest);
-        rest &= rest - 1;
-        const u64 bit = 1ull << b;
-        const unsigned c0 = __ballot_sync(0xffffffffu, !used[0] && (q[0] & bit));
-        const unsigned c1 = __ballot_sync(0xffffffffu, !used[1] && (q[1] & bit));
-        const int src = c0 ? (__ffs(c0) - 1) : (__ffs(c1) - 1);
-        const int sh = c0 ? 0 : 1;
-        const u64 qs = __shfl_sync(0xffffffffu, sh ? q[1] : q[0], src);
-        const u64 as = __shfl_sync(0xffffffffu, sh ? a[1] : a[0], src);
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const bool me = (lane == src && h == sh);
-            if (!me && (q[h] & bit)) {
-                q[h] ^= qs;
-                a[h] ^= as;
-            }
-            if (me) {
-                used[h] = true;
-                step[h] = t;
-            }
-        }
-        if (lane == 0) bits[t] = b;
-    }
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const int k = lane + 32 * h;
-        if (k < p) {
-            const int t = step[h];
-            sel[k] = rowk[h];
-            coef[t] = a[h];
-            srow[t] = rowk[h];
-        }
-    }
-    __syncwarp();
-    return p;
+    for (int g = 0; g < 8; ++g) z ^= S.tt[g][(y >> (4 * g)) & 15];
+    return z;
 }
 
 }  // namespace mela

@@ -24,14 +24,14 @@ bool decode_elim_variant(int32_t v, Tuning *t)
     Tuning r{};
     r.base = base;
     r.k = 0;
-    r.row_tile = 1024;
+    r.row_tile = 0;
     r.tc_tile = 0;
     if (base == MELA_ELIM_M4RI || base == MELA_ELIM_M4RI_K4) {
         const int dflt = base == MELA_ELIM_M4RI ? 8 : 4;
         r.k = k ? k : dflt;
         if (base == MELA_ELIM_M4RI_K4 && r.k != 4) return false;
         if (r.k != 4 && (r.k < 6 || r.k > 10)) return false;
-        static const int tiles[4] = {1024, 256, 1024, 4096};
+        static const int tiles[4] = {0, 256, 1024, 4096};
         if (tile > 3) return false;
         r.row_tile = tiles[tile];
     } else if (k || tile) {
@@ -68,7 +68,7 @@ bool decode_gemm_variant(int32_t v, Tuning *t)
 
 // ---------------------------------------------------------------- configurations
 // Model output order per op.  Elimination: the plain form, the blocked form
-// over M4RI k = 4, 6, 7, 8 (with 1024-row update tiles), k = 8 with 256-row
+// over M4RI k = 4, 6, 7, 8 (update tiles by the panel's size), k = 8 with 256-row
 // tiles (more CTAs for short matrices), k = 9 and 10 with 4096-row tiles
 // (their larger tables pay off over more rows), the single-CTA form and the
 // tensor-core windows.  Products: plain, Four-Russians (16 warps of 32 rows

@@ -14,21 +14,19 @@
 //
 // Blocked form (the Four-Russians / PLE form), one 64-column panel (one
 // word column w) at a time:
-//   panel_select  one CTA.  Each warp inserts its rows' panel words into a
-//                 warp-local XOR basis (lowest set bit leading, warp ballots
-//                 resolve who inserts next); the 32 warp bases are merged by
-//                 re-inserting their ORIGINAL words, so the final basis is
-//                 spanned by p original active rows S.  Its leading bits are
-//                 the panel's greedy pivot columns.  A warp Gauss-Jordan on
-//                 Q = S restricted to the pivot columns gives, for each
-//                 pivot k, the combination coef[k] of S rows whose panel part
-//                 is the unit vector of that pivot column.
-//   panel_rows    R_k = XOR of the S rows in coef[k] (full width from word
-//                 w on), written to a panel buffer and over the S rows.
+//   panel_select  one CTA.  Brings the active rows' panel words to reduced row
+//                   echelon form (lowest set bit leading) in chunks of a row
+//                   per thread, 32 columns at a time (basis.cuh); the walk ends
+//                   once the basis spans the panel.  Gives the panel's greedy
+//                   pivot columns b, the row S_b that entered the basis at
+//                   each, and the combination coef[b] of the S rows whose panel
+//                   part is the unit vector of column b.
+//   panel_rows    R_b = XOR of the S rows in coef[b] (full width from word
+//                   w on), written to a panel buffer and over row S_b.
 //   panel_update  every other row j (active rows for rank; all rows for
 //                 RREF) XORs sum_k bit(c_k of row j) * R_k, looked up 8 pivot
 //                 bits at a time in shared-memory tables of the 256
-//                 combinations of 8 R rows (built level by level).
+//                 combinations of 8 R rows.
 // Plain form: one cooperative persistent kernel, one grid barrier per
 // column: every CTA searches its rows for the first active row holding the
 // column's bit (atomicMin over the grid), then every CTA XORs that pivot row
@@ -47,122 +45,199 @@ namespace mela {
 // ---------------------------------------------------------------- helpers
 __device__ __forceinline__ int ctz64(u64 x) { return ctz64_(x); }
 
-// Panel bookkeeping shared by the three blocked kernels (device memory).
+// Panel bookkeeping shared by the blocked kernels (device memory); everything
+// of a pivot is indexed by its column in the panel.
 struct PanelState {
     long long rank;  // pivots found so far
     int p;           // pivots in the current panel
     int pad;
-    u64 pivmask;     // pivot bit positions of the current panel
-    int srow[64];    // physical row that receives R_k
-    int sel[64];     // original S rows (index i of coef)
-    u64 coef[64];    // R_k = XOR_{i in coef[k]} row sel[i]
+    u64 pivmask;     // pivot columns of the current panel
+    int srow[64];    // physical row S_b of pivot column b (-1: none), which receives R_b
+    u64 coef[64];    // R_b = XOR_{j in coef[b]} row S_j
 };
 
 // ---------------------------------------------------------------- panel_select
+// Word 0 of every row: the first panel's words.
+__global__ void panel_words_kernel(const u64 *__restrict__ M, i64 ld, i64 m, u64 *__restrict__ y)
+{
+    for (i64 j = blockIdx.x * (i64)blockDim.x + threadIdx.x; j < m; j += (i64)gridDim.x * blockDim.x)
+        y[j] = M[j * ld];
+}
+
 namespace {
-constexpr int SEL_WARPS = 32;
+constexpr int SEL_THREADS = 512;
 struct SelSmem {
-    WarpBasis wb[SEL_WARPS];
-    u64 have[SEL_WARPS];
-    int bits[64];
+    u64 basis[64];     // in-place vector of pivot column b
+    u64 tab[16][16];   // 4-bit tables of the basis
+    u64 vt[8][16];     // 4-bit tables of a round's pivot rows
+    u64 cv[kHalfCand]; // the candidates' vectors
+    int prow[64];
+    int wcnt[2][32];
+    HalfRound r;
 };
+
+// A row's vector after a round with pivot columns C of half word h and the
+// combination z of the round's pivot rows.
+__device__ __forceinline__ u64 sel_apply(const SelSmem &S, u64 v, int h, u32 C, u32 z)
+{
+    v &= ~((u64)C << (32 * h));
+#pragma unroll
+    for (int g = 0; g < 8; ++g) v ^= S.vt[g][(z >> (4 * g)) & 15];
+    return v | ((u64)z << (32 * h));
+}
 }  // namespace
 
-__global__ void __launch_bounds__(1024, 1)
-panel_select_kernel(const u64 *__restrict__ M, i64 ld, i64 m, i64 w, unsigned char *state,
-                    int *stamp, int panel, PanelState *ps, long long *piv, long long *prow,
-                    u64 *__restrict__ ysnap)
+// The panel words y come packed (the update of the panel before writes them),
+// so a chunk is one coalesced read; on dense matrices the first chunk fills
+// the basis.  Bound by its serial chain (one CTA): half_word_select and four
+// barriers a round of up to 32 pivots, 7.8 us for a full panel of 64 against
+// 44 us with warp-local XOR bases merged pairwise.  Whole calls with the rows
+// and update kernels below: rank of 1501 x 2900 760 us, of 16384 x 32768 (rank
+// 12000) 28.0 ms, before 3.0 and 56.7 ms.
+__global__ void __launch_bounds__(SEL_THREADS, 1)
+panel_select_kernel(const u64 *__restrict__ y, i64 m, i64 n, i64 w, unsigned char *state, int *stamp, int panel,
+                    PanelState *ps, long long *piv, long long *prow)
 {
-    extern __shared__ __align__(16) unsigned char sel_raw[];
-    SelSmem &sm = *reinterpret_cast<SelSmem *>(sel_raw);
-    const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
-    u64 have = 0;
-    for (i64 chunk = wi; chunk * 32 < m; chunk += SEL_WARPS) {
-        const i64 j = chunk * 32 + lane;
-        u64 x = 0;
-        if (j < m) {
-            // the update kernel reads every row's panel word from this snapshot,
-            // because the CTA owning word w rewrites it while the others read it
-            const u64 word = M[j * ld + w];
-            ysnap[j] = word;
-            if (state[j]) x = word;
+    __shared__ SelSmem S;
+    constexpr int NW = SEL_THREADS / 32;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int valid = n - 64 * w < 64 ? (int)(n - 64 * w) : 64;
+    u64 H = 0;  // pivot columns so far
+    int nb = 0, par = 0;
+    for (i64 base = 0; base < m && nb < valid; base += SEL_THREADS) {
+        const u64 H0 = H;  // basis vectors of earlier chunks
+        if (H0) {
+            for (int e = tid; e < 256; e += SEL_THREADS) {
+                const int g = e >> 4, v = e & 15;
+                u64 a = 0;
+#pragma unroll
+                for (int b = 0; b < 4; ++b)
+                    if (((v >> b) & 1) && ((H0 >> (4 * g + b)) & 1)) a ^= S.basis[4 * g + b];
+                S.tab[g][v] = a;
+            }
+            __syncthreads();
         }
-        warp_basis_insert(sm.wb[wi], x, x, (int)j, have);
-    }
-    if (lane == 0) sm.have[wi] = have;
-    for (int step = 1; step < SEL_WARPS; step <<= 1) {
+        const i64 j = base + tid;
+        u64 v = (j < m && state[j]) ? y[j] : 0ull;
+        const u64 yb = v & H0;
+        if (yb) {
+            v ^= yb;
+#pragma unroll
+            for (int g = 0; g < 16; ++g) v ^= S.tab[g][(yb >> (4 * g)) & 15];
+        }
+        int mycol = -1;
+        for (int h = 0; h < 2 && nb < valid; ++h) {
+            u32 Hh = (u32)(H >> (32 * h));
+            while (Hh != 0xffffffffu && nb < valid) {
+                const u32 d = mycol < 0 ? (u32)(v >> (32 * h)) & ~Hh : 0u;
+                const unsigned bal = __ballot_sync(0xffffffffu, d != 0);
+                par ^= 1;
+                if (lane == 0) S.wcnt[par][warp] = __popc(bal);
+                __syncthreads();
+                const int wv = lane < NW ? S.wcnt[par][lane] : 0;
+                const int total = __reduce_add_sync(0xffffffffu, wv);
+                if (total == 0) break;
+                int idx = __reduce_add_sync(0xffffffffu, lane < warp ? wv : 0) + __popc(bal & ((1u << lane) - 1));
+                if (d == 0 || idx >= kHalfCand) idx = -1;
+                if (idx >= 0) {
+                    S.r.cand[idx] = d;
+                    S.cv[idx] = v;
+                    S.r.pcol[idx] = -1;
+                }
+                __syncthreads();
+                if (warp == 0) half_word_select(S.r, total < kHalfCand ? total : kHalfCand);
+                __syncthreads();
+                const u32 C = S.r.C;
+                if (tid < 128) {
+                    const int g = tid >> 4, e = tid & 15;
+                    u64 a = 0;
+#pragma unroll
+                    for (int b = 0; b < 4; ++b) {
+                        const int ci = S.r.ci[4 * g + b];
+                        if (((e >> b) & 1) && ci >= 0) a ^= S.cv[ci];
+                    }
+                    S.vt[g][e] = a & ~((u64)C << (32 * h));
+                } else if (tid < 256) {
+                    half_word_tt(S.r, tid - 128);
+                }
+                const int pc = idx >= 0 ? S.r.pcol[idx] : -1;
+                __syncthreads();
+                if (pc >= 0) {
+                    mycol = 32 * h + pc;
+                    S.prow[mycol] = (int)j;
+                    v = sel_apply(S, 0, h, C, S.r.T[pc]);
+                } else {
+                    const u32 yr = (u32)(v >> (32 * h)) & C;
+                    if (yr) v = sel_apply(S, v, h, C, half_word_times_T(S.r, yr));
+                }
+                if (tid < 64 && ((H0 >> tid) & 1)) {
+                    const u64 o = S.basis[tid];
+                    const u32 yr = (u32)(o >> (32 * h)) & C;
+                    if (yr) S.basis[tid] = sel_apply(S, o, h, C, half_word_times_T(S.r, yr));
+                }
+                nb += __popc(C);
+                Hh |= C;
+                H |= (u64)C << (32 * h);
+            }
+        }
+        if (mycol >= 0) S.basis[mycol] = v;
         __syncthreads();
-        if ((wi % (2 * step)) == 0 && wi + step < SEL_WARPS) {
-            warp_basis_merge(sm.wb[wi], have, sm.wb[wi + step], sm.have[wi + step]);
-            if (lane == 0) sm.have[wi] = have;
-        }
     }
-    __syncthreads();
-    if (wi != 0) return;
-
-    const u64 pm = have;
     const long long r0 = ps->rank;
-    const int p = warp_panel_gauss_jordan(sm.wb[0], pm, sm.bits, ps->coef, ps->srow, ps->sel);
-    for (int t = lane; t < p; t += 32) {
-        const int rs = ps->srow[t];
-        piv[r0 + t] = 64 * w + sm.bits[t];
-        prow[r0 + t] = rs;
-        state[rs] = 0;
-        stamp[rs] = panel;
+    __syncthreads();  // every thread has read the rank before it is advanced
+    if (tid < 64) {
+        int r = -1;
+        if ((H >> tid) & 1) {
+            const int t = __popcll(H & ((1ull << tid) - 1));
+            r = S.prow[tid];
+            ps->coef[tid] = S.basis[tid] & H;
+            piv[r0 + t] = 64 * w + tid;
+            prow[r0 + t] = r;
+            state[r] = 0;
+            stamp[r] = panel;
+        }
+        ps->srow[tid] = r;
     }
-    if (lane == 0) {
-        ps->p = p;
-        ps->pivmask = pm;
-        ps->rank = r0 + p;
+    if (tid == 0) {
+        ps->p = nb;
+        ps->pivmask = H;
+        ps->rank = r0 + nb;
     }
 }
 
 // ---------------------------------------------------------------- panel_rows
-// Block: 32 words x all p rows.  Loads S rows' words into shared memory,
-// forms R_k, writes R_k to the panel buffer and over row srow[k].
+// Block: 4 words x every pivot, a thread per (column, word).  R_b is looked
+// up four columns at a time in 16 tables of the 16 combinations of the S rows
+// of columns 4g..4g+3; every S row is read before any is overwritten.
 __global__ void __launch_bounds__(256)
 panel_rows_kernel(u64 *__restrict__ M, i64 ld, i64 wc, i64 w, const PanelState *ps,
                   u64 *__restrict__ Rbuf)
 {
-    __shared__ u64 S[64][33];
-    __shared__ u64 coef[64];
-    __shared__ int srow[64];
-    const int p = ps->p;
-    if (p == 0) return;
-    const i64 w0 = w + (i64)blockIdx.x * 32;
-    const int tid = threadIdx.x;
-    for (int e = tid; e < p * 32; e += 256) {
-        const int i = e >> 5, t = e & 31;
-        const i64 word = w0 + t;
-        S[i][t] = word < wc ? M[(i64)ps->sel[i] * ld + word] : 0ull;
-    }
-    if (tid < p) {
-        coef[tid] = ps->coef[tid];
-        srow[tid] = ps->srow[tid];
+    __shared__ u64 rows[64][4];
+    __shared__ u64 tab[16][16][4];
+    if (ps->p == 0) return;
+    const int tid = threadIdx.x, b = tid >> 2, q = tid & 3;
+    const i64 word = w + (i64)blockIdx.x * 4 + q;
+    const int sr = ps->srow[b];
+    const u64 coef = sr >= 0 ? ps->coef[b] : 0ull;
+    const bool ok = sr >= 0 && word < wc;
+    rows[b][q] = ok ? M[(i64)sr * ld + word] : 0ull;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int e = (tid >> 2) + 64 * i, g = e >> 4, v = e & 15;
+        u64 a = 0;
+#pragma unroll
+        for (int h = 0; h < 4; ++h) a ^= ((v >> h) & 1) ? rows[4 * g + h][q] : 0ull;
+        tab[g][v][q] = a;
     }
     __syncthreads();
-    u64 out[8];
-    int cnt = 0;
-    for (int e = tid; e < p * 32; e += 256) {
-        const int k = e >> 5, t = e & 31;
-        u64 c = coef[k], v = 0;
-        while (c) {
-            const int i = ctz64(c);
-            c &= c - 1;
-            v ^= S[i][t];
-        }
-        out[cnt++] = v;
-    }
-    __syncthreads();  // every S row is read before any is overwritten
-    cnt = 0;
-    for (int e = tid; e < p * 32; e += 256) {
-        const int k = e >> 5, t = e & 31;
-        const i64 word = w0 + t;
-        const u64 v = out[cnt++];
-        if (word < wc) {
-            M[(i64)srow[k] * ld + word] = v;
-            Rbuf[(i64)k * wc + word] = v;
-        }
+    u64 acc = 0;
+#pragma unroll
+    for (int g = 0; g < 16; ++g) acc ^= tab[g][(coef >> (4 * g)) & 15][q];
+    if (ok) {
+        M[(i64)sr * ld + word] = acc;
+        Rbuf[(i64)b * wc + word] = acc;
     }
 }
 
@@ -171,8 +246,9 @@ panel_rows_kernel(u64 *__restrict__ M, i64 ld, i64 wc, i64 w, const PanelState *
 // 64 bit positions are cut into G = ceil(64/K) groups of consecutive
 // positions (the last one shorter when K does not divide 64); group g's table
 // holds the 2^bits(g) XOR combinations of the reduced rows R of its positions
-// (zero rows where a position holds no pivot), built level by level: entry v
-// = entry (v - 2^h) ^ entry 2^h for v in (2^h, 2^(h+1)).  Every other row j
+// (zero rows where a position holds no pivot), built in two steps: the
+// combinations of the low and of the high half of the group's bits from the
+// rows, then every other entry from one of each.  Every other row j
 // (active rows for the rank; all rows for the RREF) then XORs, per word,
 // one entry per group, indexed by its panel bits at the pivot positions.
 // Each CTA covers TW words (columns) and `rt` rows; the table build is paid
@@ -190,57 +266,72 @@ template <int K, int TW>
 __global__ void __launch_bounds__(256)
 panel_update_kernel(u64 *__restrict__ M, i64 ld, i64 m, i64 wc, i64 w, const PanelState *ps,
                     const u64 *__restrict__ Rbuf, const unsigned char *state, const int *stamp,
-                    int panel, int rref, const u64 *__restrict__ ysnap, int rt)
+                    int panel, int rref, const u64 *__restrict__ y, u64 *__restrict__ ynext, int rt)
 {
     using Gr = M4riGroups<K>;
     extern __shared__ __align__(16) unsigned char upd_raw[];
     u64 *T = reinterpret_cast<u64 *>(upd_raw);  // entry e of group g: T[((g << K) + e) * TW + t]
     const int p = ps->p;
-    if (p == 0) return;
+    const int tid = threadIdx.x;
+    const i64 row0 = (i64)blockIdx.y * rt;
+    // the next panel's words (word w + 1, in the first column tile) also go,
+    // packed, to ynext
+    if (p == 0) {
+        if (blockIdx.x == 0 && w + 1 < wc)
+            for (i64 j = row0 + tid; j < row0 + rt && j < m; j += 256) ynext[j] = M[j * ld + w + 1];
+        return;
+    }
     const u64 pm = ps->pivmask;
     const i64 w0 = w + (i64)blockIdx.x * TW;
-    const int tid = threadIdx.x;
 
-    // level 0: entry 0 of every group is zero, entry 2^h of group g is R'(gK + h)
+    // entry 0 of every group is zero, entry 2^h of group g is R_(gK + h)
     for (int e = tid; e < Gr::G * TW; e += 256) T[(((e / TW) << K)) * TW + e % TW] = 0;
     for (int e = tid; e < 64 * TW; e += 256) {
         const int t = e % TW, b = e / TW, g = b / K, h = b - g * K;
         const i64 word = w0 + t;
-        u64 v = 0;
-        if (((pm >> b) & 1) && word < wc) {
-            const int k = __popcll(pm & ((1ull << b) - 1));
-            v = Rbuf[(i64)k * wc + word];
-        }
-        T[((g << K) + (1 << h)) * TW + t] = v;
+        T[((g << K) + (1 << h)) * TW + t] = (((pm >> b) & 1) && word < wc) ? Rbuf[(i64)b * wc + word] : 0ull;
     }
     __syncthreads();
-#pragma unroll 1
-    for (int h = 1; h < K; ++h) {
-        const int cnt = (1 << h) - 1;
-        for (int e = tid; e < Gr::G * cnt * TW; e += 256) {
-            const int t = e % TW, rest = e / TW, g = rest / cnt, v = (1 << h) + 1 + rest % cnt;
-            if (h < Gr::bits(g)) {
-                u64 *Tg = T + ((size_t)g << K) * TW;
-                Tg[v * TW + t] = Tg[(v - (1 << h)) * TW + t] ^ Tg[(1 << h) * TW + t];
-            }
-        }
-        __syncthreads();
+    // combinations of the low LB bits (entries x) and of the others (x << LB)
+    constexpr int LB = K / 2, HB = K - LB, NX = (1 << LB) + (1 << HB);
+    for (int e = tid; e < Gr::G * NX * TW; e += 256) {
+        const int t = e % TW, rest = e / TW, g = rest / NX, i = rest % NX;
+        const int x = i < (1 << LB) ? i : (i - (1 << LB)) << LB;
+        if (x >= (1 << Gr::bits(g)) || (x & (x - 1)) == 0) continue;
+        const u64 *Tg = T + ((size_t)g << K) * TW;
+        u64 a = 0;
+#pragma unroll
+        for (int h = 0; h < K; ++h) a ^= ((x >> h) & 1) ? Tg[(1 << h) * TW + t] : 0ull;
+        T[(((size_t)g << K) + x) * TW + t] = a;
     }
+    __syncthreads();
+    for (int e = tid; e < Gr::entries * TW; e += 256) {
+        const int t = e % TW, ge = e / TW, g = ge >> K, x = ge & ((1 << K) - 1);
+        const int lo = x & ((1 << LB) - 1), hi = x ^ lo;
+        if (!lo || !hi) continue;
+        const u64 *Tg = T + ((size_t)g << K) * TW;
+        T[(size_t)e] = Tg[lo * TW + t] ^ Tg[hi * TW + t];
+    }
+    __syncthreads();
 
-    const i64 row0 = (i64)blockIdx.y * rt;
     const int t = tid % TW;
     const i64 word = w0 + t;
+    const bool next = word == w + 1;
+    if (word >= wc) return;
     for (int rr = tid / TW; rr < rt; rr += 256 / TW) {
         const i64 j = row0 + rr;
         if (j >= m) break;
-        if (rref ? (stamp[j] == panel) : (state[j] == 0)) continue;
-        const u64 y = ysnap[j] & pm;
-        if (!y || word >= wc) continue;
-        u64 acc = 0;
+        const u64 yj = (rref ? (stamp[j] == panel) : (state[j] == 0)) ? 0ull : y[j] & pm;
+        if (!yj) {
+            if (next) ynext[j] = M[j * ld + word];
+            continue;
+        }
+        u64 acc = M[j * ld + word];
 #pragma unroll
         for (int g = 0; g < Gr::G; ++g)
-            acc ^= T[((g << K) + (int)((y >> (g * K)) & ((1ull << Gr::bits(g)) - 1))) * TW + t];
-        M[j * ld + word] ^= acc;
+            acc ^= T[((g << K) + (int)((yj >> (g * K)) & ((1ull << Gr::bits(g)) - 1))) * TW + t];
+        M[j * ld + word] = acc;
+        if (next) ynext[j] = acc;
     }
 }
 
@@ -258,8 +349,8 @@ template <> struct M4riTile<10> { static constexpr int TW = 2; };
 template <int K>
 static mela_status launch_panel_update(u64 *M, i64 ld, i64 m, i64 wc, i64 w, const PanelState *ps,
                                        const u64 *Rbuf, const unsigned char *state, const int *stamp,
-                                       int panel, int rref, const u64 *ysnap, int rt, cudaStream_t s,
-                                       bool configure)
+                                       int panel, int rref, const u64 *y, u64 *ynext, int rt,
+                                       cudaStream_t s, bool configure)
 {
     constexpr int TW = M4riTile<K>::TW;
     constexpr size_t smem = (size_t)M4riGroups<K>::entries * TW * 8;
@@ -271,13 +362,13 @@ static mela_status launch_panel_update(u64 *M, i64 ld, i64 m, i64 wc, i64 w, con
     const i64 rem = wc - w;
     const i64 rtiles = (m + rt - 1) / rt;
     panel_update_kernel<K, TW><<<dim3((unsigned)((rem + TW - 1) / TW), (unsigned)rtiles), 256, smem, s>>>(
-        M, ld, m, wc, w, ps, Rbuf, state, stamp, panel, rref, ysnap, rt);
+        M, ld, m, wc, w, ps, Rbuf, state, stamp, panel, rref, y, ynext, rt);
     return MELA_OK;
 }
 
 using PanelUpdateFn = mela_status (*)(u64 *, i64, i64, i64, i64, const PanelState *, const u64 *,
-                                      const unsigned char *, const int *, int, int, const u64 *, int,
-                                      cudaStream_t, bool);
+                                      const unsigned char *, const int *, int, int, const u64 *, u64 *,
+                                      int, cudaStream_t, bool);
 
 static PanelUpdateFn panel_update_for(int k)
 {
@@ -538,7 +629,7 @@ ElimLayout elim_layout(i64 m, i64 n)
     L.rbuf = off;   off += al256((size_t)64 * (size_t)(wc ? wc : 1) * 8);
     L.cand = off;   off += al256(3 * sizeof(int));
     L.gb = off;     off += al256(sizeof(GridBar));
-    L.ysnap = off;  off += al256((size_t)m * 8);
+    L.ysnap = off;  off += 2 * al256((size_t)m * 8);  // this and the next panel's words
     L.total = off;
     return L;
 }
@@ -584,7 +675,7 @@ mela_status elim_device(int variant_arg, u64 *M, i64 ld, i64 m, i64 n, int rref,
     u64 *rbuf = (u64 *)(w + L.rbuf);
     int *cand = (int *)(w + L.cand);
     GridBar *gb = (GridBar *)(w + L.gb);
-    u64 *ysnap = (u64 *)(w + L.ysnap);
+    u64 *ysnap[2] = {(u64 *)(w + L.ysnap), (u64 *)(w + L.ysnap + al256((size_t)m * 8))};
     const i64 wc = words_of(n);
 
     MELA_CUDA_TRY(cudaMemsetAsync(state, 1, (size_t)m, s));
@@ -624,26 +715,34 @@ mela_status elim_device(int variant_arg, u64 *M, i64 ld, i64 m, i64 n, int rref,
     }
     MELA_CUDA_TRY(cudaMemsetAsync(stamp, 0xff, (size_t)m * 4, s));
     MELA_CUDA_TRY(cudaMemsetAsync(ps, 0, sizeof(PanelState), s));
-    const size_t sel_smem = sizeof(SelSmem);
-    MELA_CUDA_TRY(cudaFuncSetAttribute(panel_select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)sel_smem));
     const PanelUpdateFn update = panel_update_for(tune.k);
     if (!update) {
         set_error("blocked elimination: M4RI k = %d (4 or 6..10 supported)", tune.k);
         return MELA_ERR_INVALID;
     }
-    const int rt = tune.row_tile;
-    if (mela_status st = check_grid_yz((m + rt - 1) / rt, 1, "blocked elimination update"); st != MELA_OK)
+    // Rows per update CTA, unless the variant names them: 256 while those CTAs
+    // make at most two waves of three per SM, else 1024.  A CTA's table build
+    // is a fixed cost that 256 rows pay back worse, but smaller matrices need
+    // the CTAs (rank, k = 8: 2048 x 4096 1150 us with 256 rows, 1385 with 1024;
+    // 4096 x 8192 2853 / 3226; 16384 x 32768 35.7 / 28.0 ms).
+    const int col_tile = tune.k <= 6 ? 8 : tune.k <= 8 ? 4 : 2;
+    auto rows_per_cta = [&](i64 rem) -> int {
+        if (tune.row_tile) return tune.row_tile;
+        return (rem + col_tile - 1) / col_tile * ((m + 255) / 256) <= 6ll * sm_count() ? 256 : 1024;
+    };
+    const int rt_min = rows_per_cta(1);
+    if (mela_status st = check_grid_yz((m + rt_min - 1) / rt_min, 1, "blocked elimination update"); st != MELA_OK)
         return st;
-    if (mela_status st = update(M, ld, m, wc, 0, ps, rbuf, state, stamp, 0, rref, ysnap, rt, s, true);
+    if (mela_status st = update(M, ld, m, wc, 0, ps, rbuf, state, stamp, 0, rref, nullptr, nullptr, 0, s, true);
         st != MELA_OK)
         return st;
+    panel_words_kernel<<<grid_cap(m, 256), 256, 0, s>>>(M, ld, m, ysnap[0]);
     for (i64 pw = 0; pw < wc; ++pw) {  // every word column is one panel
-        panel_select_kernel<<<1, 1024, sel_smem, s>>>(M, ld, m, pw, state, stamp, (int)pw, ps,
-                                                       d_piv, d_prow, ysnap);
-        const i64 rem = wc - pw;
-        panel_rows_kernel<<<(unsigned)((rem + 31) / 32), 256, 0, s>>>(M, ld, wc, pw, ps, rbuf);
-        update(M, ld, m, wc, pw, ps, rbuf, state, stamp, (int)pw, rref, ysnap, rt, s, false);
+        const u64 *y = ysnap[pw & 1];
+        panel_select_kernel<<<1, SEL_THREADS, 0, s>>>(y, m, n, pw, state, stamp, (int)pw, ps, d_piv, d_prow);
+        panel_rows_kernel<<<(unsigned)((wc - pw + 3) / 4), 256, 0, s>>>(M, ld, wc, pw, ps, rbuf);
+        update(M, ld, m, wc, pw, ps, rbuf, state, stamp, (int)pw, rref, y, ysnap[(pw + 1) & 1], rows_per_cta(wc - pw), s,
+               false);
     }
     MELA_LAUNCH_CHECK("panel elimination");
     MELA_CUDA_TRY(cudaMemcpyAsync(d_rank, &ps->rank, sizeof(long long), cudaMemcpyDeviceToDevice, s));

@@ -46,6 +46,7 @@
 #include "mela_internal.h"
 #include "mela_host.h"
 #include "elim.h"
+#include "basis.cuh"
 #include "tc_ptx.cuh"
 
 namespace mela {
@@ -54,7 +55,8 @@ namespace {
 
 constexpr int WW = 4;         // words per window
 constexpr int WBITS = 256;    // columns per window
-constexpr int WF_THREADS = 320;  // a chunk of rows; 320 random rows span 256 columns but with probability 2^-64
+constexpr int WF_ROWS = 320;     // a chunk of rows; 320 random rows span 256 columns but with probability 2^-64
+constexpr int WF_THREADS = WF_ROWS + 32;  // a thread per row and the selecting warp
 
 // Everything that belongs to a pivot of a window is indexed by its column in
 // the window (0..255), so the coefficient of a row is its window part masked
@@ -70,26 +72,17 @@ struct WinState {
     u64 tag[WBITS][WW];     // R_b = sum_j bit j * A[P_j]
 };
 
-constexpr int WF_CAND = 64;  // rows one selection round eliminates among themselves
-
 struct WfSmem {
     uint4 basis[WBITS][2];    // vector of pivot column b (in-place form)
     uint4 tab[2][64][16];     // 4-bit tables of the basis, a plane per 16-byte half
     uint4 vt[2][8][16];       // 4-bit tables of a round's pivot rows
-    uint4 cv[WF_CAND][2];     // the candidates' vectors
-    u32 tt[8][16];            // 4-bit tables of T
-    u32 cand[WF_CAND];        // the candidates' data bits in the half word
-    u32 T[32];                // row of T of the pivot in column c of the half word
-    int ci[32];               // its candidate (-1: no pivot)
-    int pcol[WF_CAND];        // column of a candidate's pivot (-1: none)
-    u32 C;                    // the round's pivot columns
+    uint4 cv[kHalfCand][2];   // the candidates' vectors
+    HalfRound r;
     int prow[WBITS];          // physical row of pivot column b
     int cnt;
     int wcnt[2][32];          // candidates per warp, alternating
     int wsum[32];
 };
-
-__device__ __forceinline__ int ctz64w(u64 x) { return __ffsll((long long)x) - 1; }
 
 // Half word h of an 8-word vector held in registers (selects, no local memory).
 __device__ __forceinline__ u32 sel8(const u32 (&v)[8], int h)
@@ -146,46 +139,6 @@ __device__ __forceinline__ int block_slot(bool flag, int *wsum, int &total)
 // ---------------------------------------------------------------- window_factor
 namespace {
 
-// Gauss-Jordan of up to 64 candidate rows over the 32 columns of a half word,
-// by one warp, columns in lanes: lane c's mask holds column c of the rows (bit
-// r = row r).  A step broadcasts column c, takes its lowest unused row p as
-// the pivot and, in every other lane whose column has bit p, XORs in the rows
-// that hold bit c.  The rows stay in in-place form: lane c's own mask is left
-// alone, its bits now meaning "contains pivot row p".  Column c + 1 is fetched
-// while the step before it runs and brought up to date in registers, so a
-// step's chain is a few logical operations and no shuffle latency.
-__device__ __forceinline__ void wf_select(WfSmem &S, int ncand)
-{
-    const int lane = threadIdx.x & 31;
-    const u32 lo = lane < ncand ? S.cand[lane] : 0u;
-    const u32 hi = lane + 32 < ncand ? S.cand[lane + 32] : 0u;
-    u64 col = (u64)transpose32_warp(lo) | ((u64)transpose32_warp(hi) << 32);
-    u64 unused = ~0ull, mypb = 0;
-    u64 cur = __shfl_sync(0xffffffffu, col, 0);
-#pragma unroll
-    for (int c = 0; c < 32; ++c) {
-        u64 nx = __shfl_sync(0xffffffffu, col, (c + 1) & 31);
-        const u64 av = cur & unused;
-        const u64 pb = av & (~av + 1);
-        const u64 rs = cur ^ pb;
-        unused ^= pb;
-        if (lane == c)
-            mypb = pb;
-        else if (col & pb)
-            col ^= rs;
-        if (nx & pb) nx ^= rs;
-        cur = nx;
-    }
-    const u32 C = __ballot_sync(0xffffffffu, mypb != 0);
-    const u32 wlo = transpose32_warp((u32)col), whi = transpose32_warp((u32)(col >> 32));
-    const int ci = mypb ? ctz64w(mypb) : -1;
-    const u32 t0 = __shfl_sync(0xffffffffu, wlo, ci & 31), t1 = __shfl_sync(0xffffffffu, whi, ci & 31);
-    S.T[lane] = ci < 0 ? 0u : ((ci < 32 ? t0 : t1) & C);
-    S.ci[lane] = ci;
-    if (ci >= 0) S.pcol[ci] = lane;
-    if (lane == 0) S.C = C;
-}
-
 // A row's vector v after a round with pivot columns C of half word h: its
 // bits y at C select sum_k y_k T_k = z, the combination of the round's
 // original pivot rows to add; z itself takes the place of the bits at C.
@@ -201,12 +154,18 @@ __device__ __forceinline__ void wf_apply(const WfSmem &S, u32 (&v)[8], int h, u3
 #pragma unroll
     for (int q = 0; q < 8; ++q) v[q] |= q == h ? z : 0u;
 }
-__device__ __forceinline__ u32 wf_times_T(const WfSmem &S, u32 y)
+// Half word ht of what wf_apply makes of v.
+__device__ __forceinline__ u32 wf_half(const WfSmem &S, const u32 (&v)[8], int h, int ht, u32 C, u32 z)
 {
-    u32 z = 0;
+    u32 x = sel8(v, ht);
+    if (z) {
+        if (ht == h) x &= ~C;
+        const u32 *t = reinterpret_cast<const u32 *>(&S.vt[ht >> 2][0][0]) + (ht & 3);
 #pragma unroll
-    for (int g = 0; g < 8; ++g) z ^= S.tt[g][(y >> (4 * g)) & 15];
-    return z;
+        for (int g = 0; g < 8; ++g) x ^= t[4 * (16 * g + ((z >> (4 * g)) & 15))];
+        if (ht == h) x |= z;
+    }
+    return x;
 }
 
 }  // namespace
@@ -217,16 +176,16 @@ __device__ __forceinline__ u32 wf_times_T(const WfSmem &S, u32 y)
 // its bit c stays set and becomes the coefficient of P_c).  One CTA walks the
 // active rows in chunks of a row per thread; the columns go 32 at a time (half
 // words): up to 64 rows with data left there are eliminated by one warp
-// (wf_select), and every row of the chunk then takes the round's pivots in
-// through 4-bit tables; rounds repeat until no unused row has data left in
-// the half word.
-// Bound by the serial chain, not by throughput (one CTA): a step costs about
-// 45 cycles in wf_select and a round of up to 32 pivots four barriers and 16
-// 16-byte table reads a row, against a barrier and about 800 cycles for each
-// pivot when the rows are eliminated one pivot at a time (whole rank of a
-// 3000 x 5000 matrix of rank 2200: 605 against 1418 us; rank and null space
-// of 16384 x 32768, rank 12000: 7.1 against 8.9 ms, the update then setting
-// the pace).
+// (half_word_select), and every row of the chunk then takes the round's pivots
+// in through 4-bit tables; rounds repeat until no unused row has data left in
+// the half word.  Where a round fills its half word, the rows first bring only
+// the next half word up to date, so that the next round's selection runs in a
+// warp of its own beside the rest of the row updates.
+// Bound by the serial chain, not by throughput (one CTA): a round of up to 32
+// pivots costs about 2600 cycles in half_word_select, four barriers, the
+// tables and one half word of every row: about 29 us for a full window, against
+// 133 us when the rows are eliminated one pivot and one barrier at a time.
+// Whole rank of 3000 x 5000 (rank 2200): 532 against 1415 us.
 __global__ void __launch_bounds__(WF_THREADS, 1)
 window_factor_kernel(const u64 *__restrict__ M, i64 ld, i64 m, i64 n, i64 w, int *list, const unsigned char *live,
                      unsigned char *state, int *stamp, int wid, const WinState *prev, WinState *ws, long long *piv,
@@ -246,8 +205,8 @@ window_factor_kernel(const u64 *__restrict__ M, i64 ld, i64 m, i64 n, i64 w, int
     u32 H[8] = {};  // pivot columns so far (the same in every thread)
     int nb = 0;     // their number
     int walked = 0, par = 0;
-    for (int base = 0; base < na && nb < valid; base += WF_THREADS) {
-        walked = base + WF_THREADS < na ? base + WF_THREADS : na;
+    for (int base = 0; base < na && nb < valid; base += WF_ROWS) {
+        walked = base + WF_ROWS < na ? base + WF_ROWS : na;
         const bool older = nb > 0;  // basis vectors of earlier chunks
         u32 H0[8];
 #pragma unroll
@@ -269,7 +228,7 @@ window_factor_kernel(const u64 *__restrict__ M, i64 ld, i64 m, i64 n, i64 w, int
         const int k = base + tid;
         int row = -1;
         u32 v[8] = {};
-        if (k < na) {
+        if (tid < WF_ROWS && k < na) {
             row = L0[k];
 #pragma unroll
             for (int q = 0; q < WW; ++q)
@@ -293,83 +252,100 @@ window_factor_kernel(const u64 *__restrict__ M, i64 ld, i64 m, i64 n, i64 w, int
             }
         }
         int mycol = -1;  // this row's pivot column
-        for (int h = 0; h < 8 && nb < valid; ++h) {
-            u32 Hh = sel8(H, h);
-            while (Hh != 0xffffffffu && nb < valid) {
-                const u32 d = mycol < 0 ? sel8(v, h) & ~Hh : 0u;
-                const unsigned bal = __ballot_sync(0xffffffffu, d != 0);
-                par ^= 1;
-                if (lane == 0) S.wcnt[par][warp] = __popc(bal);
-                __syncthreads();
-                const int wv = lane < NW ? S.wcnt[par][lane] : 0;
-                const int total = __reduce_add_sync(0xffffffffu, wv);
-                if (total == 0) break;
-                int idx = __reduce_add_sync(0xffffffffu, lane < warp ? wv : 0) + __popc(bal & ((1u << lane) - 1));
-                if (d == 0 || idx >= WF_CAND) idx = -1;
+        // the last round, while its pivots are not in v yet: half word h,
+        // columns C, combination z of this row
+        bool pend = false;
+        int h = 0;
+        u32 C = 0, z = 0;
+        auto take_in = [&]() {
+            if (!pend) return;
+            if (z) wf_apply(S, v, h, C, z);
+            if (obasis) {
+                const uint4 a = S.basis[tid][0], b = S.basis[tid][1];
+                u32 o[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+                const u32 y = sel8(o, h) & C;
+                if (y) {
+                    wf_apply(S, o, h, C, half_word_times_T(S.r, y));
+                    S.basis[tid][0] = make_uint4(o[0], o[1], o[2], o[3]);
+                    S.basis[tid][1] = make_uint4(o[4], o[5], o[6], o[7]);
+                }
+            }
+            pend = false;
+        };
+        while (h < 8 && nb < valid) {
+            int ht = h;  // the half word of the next round
+            if (pend && sel8(H, h) == 0xffffffffu && ++ht == 8) break;
+            const u32 Ht = sel8(H, ht);
+            const u32 x = pend ? wf_half(S, v, h, ht, C, z) : sel8(v, ht);
+            const u32 d = mycol < 0 ? x & ~Ht : 0u;
+            const unsigned bal = __ballot_sync(0xffffffffu, d != 0);
+            par ^= 1;
+            if (lane == 0) S.wcnt[par][warp] = __popc(bal);
+            __syncthreads();
+            const int wv = lane < NW ? S.wcnt[par][lane] : 0;
+            const int total = __reduce_add_sync(0xffffffffu, wv);
+            if (total == 0) {  // no unused row has data left in half word ht
+                take_in();
+                h = ht + 1;
+                continue;
+            }
+            int idx = __reduce_add_sync(0xffffffffu, lane < warp ? wv : 0) + __popc(bal & ((1u << lane) - 1));
+            if (d == 0 || idx >= kHalfCand) idx = -1;
+            if (idx >= 0) {
+                S.r.cand[idx] = d;
+                S.r.pcol[idx] = -1;
+            }
+            __syncthreads();
+            if (warp == NW - 1) {
+                half_word_select(S.r, total < kHalfCand ? total : kHalfCand);
+            } else {
+                take_in();
                 if (idx >= 0) {
-                    S.cand[idx] = d;
                     S.cv[idx][0] = make_uint4(v[0], v[1], v[2], v[3]);
                     S.cv[idx][1] = make_uint4(v[4], v[5], v[6], v[7]);
-                    S.pcol[idx] = -1;
                 }
-                __syncthreads();
-                if (warp == 0) wf_select(S, total < WF_CAND ? total : WF_CAND);
-                __syncthreads();
-                const u32 C = S.C;
-                // tables over the round's pivots: their original rows (without
-                // the bits at C) and the rows of T
-                if (tid < 256) {
-                    const int half = tid >> 7, g = (tid >> 4) & 7, e = tid & 15;
-                    uint4 a = make_uint4(0, 0, 0, 0);
-#pragma unroll
-                    for (int b = 0; b < 4; ++b) {
-                        const int ci = S.ci[4 * g + b];
-                        if (((e >> b) & 1) && ci >= 0) a = xor4u(a, S.cv[ci][half]);
-                    }
-                    if (half == (h >> 2)) {
-                        const int q = h & 3;
-                        a.x &= q == 0 ? ~C : ~0u;
-                        a.y &= q == 1 ? ~C : ~0u;
-                        a.z &= q == 2 ? ~C : ~0u;
-                        a.w &= q == 3 ? ~C : ~0u;
-                    }
-                    S.vt[half][g][e] = a;
-                }
-                for (int x = WF_THREADS - 1 - tid; x < 128; x += WF_THREADS) {
-                    const int g = x >> 4, e = x & 15;
-                    u32 a = 0;
-#pragma unroll
-                    for (int b = 0; b < 4; ++b) a ^= ((e >> b) & 1) ? S.T[4 * g + b] : 0u;
-                    S.tt[g][e] = a;
-                }
-                const int pc = idx >= 0 ? S.pcol[idx] : -1;
-                __syncthreads();
-                if (pc >= 0) {
-                    mycol = 32 * h + pc;
-                    S.prow[mycol] = row;
-#pragma unroll
-                    for (int q = 0; q < 8; ++q) v[q] = 0;
-                    wf_apply(S, v, h, C, S.T[pc]);
-                } else {
-                    const u32 y = sel8(v, h) & C;
-                    if (y) wf_apply(S, v, h, C, wf_times_T(S, y));
-                }
-                if (obasis) {
-                    uint4 a = S.basis[tid][0], b = S.basis[tid][1];
-                    u32 o[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-                    const u32 y = sel8(o, h) & C;
-                    if (y) {
-                        wf_apply(S, o, h, C, wf_times_T(S, y));
-                        S.basis[tid][0] = make_uint4(o[0], o[1], o[2], o[3]);
-                        S.basis[tid][1] = make_uint4(o[4], o[5], o[6], o[7]);
-                    }
-                }
-                nb += __popc(C);
-                Hh |= C;
-#pragma unroll
-                for (int q = 0; q < 8; ++q) H[q] |= q == h ? C : 0u;
             }
+            __syncthreads();
+            C = S.r.C;
+            // tables over the round's pivots: their original rows (without
+            // the bits at C) and the rows of T
+            if (tid < 256) {
+                const int half = tid >> 7, g = (tid >> 4) & 7, e = tid & 15;
+                uint4 a = make_uint4(0, 0, 0, 0);
+#pragma unroll
+                for (int b = 0; b < 4; ++b) {
+                    const int ci = S.r.ci[4 * g + b];
+                    if (((e >> b) & 1) && ci >= 0) a = xor4u(a, S.cv[ci][half]);
+                }
+                if (half == (ht >> 2)) {
+                    const int q = ht & 3;
+                    a.x &= q == 0 ? ~C : ~0u;
+                    a.y &= q == 1 ? ~C : ~0u;
+                    a.z &= q == 2 ? ~C : ~0u;
+                    a.w &= q == 3 ? ~C : ~0u;
+                }
+                S.vt[half][g][e] = a;
+            }
+            for (int e = WF_THREADS - 1 - tid; e < 128; e += WF_THREADS) half_word_tt(S.r, e);
+            const int pc = idx >= 0 ? S.r.pcol[idx] : -1;
+            __syncthreads();
+            if (pc >= 0) {
+                mycol = 32 * ht + pc;
+                S.prow[mycol] = row;
+#pragma unroll
+                for (int q = 0; q < 8; ++q) v[q] = 0;
+                z = S.r.T[pc];
+            } else {
+                const u32 y = x & C;
+                z = y ? half_word_times_T(S.r, y) : 0u;
+            }
+            pend = true;
+            h = ht;
+            nb += __popc(C);
+#pragma unroll
+            for (int q = 0; q < 8; ++q) H[q] |= q == ht ? C : 0u;
         }
+        take_in();
         if (mycol >= 0) {
             S.basis[mycol][0] = make_uint4(v[0], v[1], v[2], v[3]);
             S.basis[mycol][1] = make_uint4(v[4], v[5], v[6], v[7]);
@@ -410,10 +386,10 @@ window_factor_kernel(const u64 *__restrict__ M, i64 ld, i64 m, i64 n, i64 w, int
     // order, dropping this window's pivot rows and rows known to be zero from
     // the window on; chunks go from the last to the first, so every write lands
     // at or after the chunk being read
-    for (int c0 = ((walked - 1) / WF_THREADS) * WF_THREADS; walked > 0 && c0 >= 0; c0 -= WF_THREADS) {
+    for (int c0 = ((walked - 1) / WF_ROWS) * WF_ROWS; walked > 0 && c0 >= 0; c0 -= WF_ROWS) {
         const int k = c0 + tid;
         int row = -1;
-        if (k < walked) row = L0[k];
+        if (tid < WF_ROWS && k < walked) row = L0[k];
         const bool keep = row >= 0 && state[row] && live[row];
         int total;
         const int slot = block_slot(keep, S.wsum, total);

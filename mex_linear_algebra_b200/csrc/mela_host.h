@@ -38,7 +38,7 @@ i64 even_words(i64 bits);
 struct Tuning {
     int base;      // mela_gemm_variant or mela_elim_variant
     int k;         // Four-Russians table width (M4RI forms)
-    int row_tile;  // rows per update CTA (blocked elimination)
+    int row_tile;  // rows per update CTA (blocked elimination; 0: by the panel's size)
     int tc_tile;   // tensor-core products: 0 default, 1 single CTAs, 2 CTA pairs
 };
 // false when a field is out of range for the base variant

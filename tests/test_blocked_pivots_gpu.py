@@ -1,0 +1,44 @@
+"""Pivot search of the blocked eliminations at the edges of its blocking:
+32-column half words and 64 candidate rows a round in both forms, 320 rows a
+chunk and 256 columns a window on the tensor cores, 512 rows a chunk and 64
+columns a panel in the Four-Russians form (whose update tiles change from 1024
+to 256 rows).  Bit-exact against the oracle (rank, pivot columns, RREF rows,
+null basis)."""
+import numpy as np
+import pytest
+
+from mex_linear_algebra_b200 import gen
+from test_elim_gpu import check_all
+
+pytestmark = pytest.mark.gpu
+
+
+def repeated(m, n, seed):
+    """The first 70 rows equal: the first round's 64 candidates span one
+    dimension, the other pivots come in later rounds."""
+    P = gen.dense_packed(seed, 0, m, n)
+    P[: min(70, m)] = P[0]
+    return P
+
+
+def late_pivots(m, n, seed):
+    """The first 512 rows are zero in every even column: the even pivot columns
+    come from a later chunk, below and between the first chunk's."""
+    P = gen.dense_packed(seed, 0, m, n)
+    P[: min(512, m)] &= np.uint64(0xAAAAAAAAAAAAAAAA)
+    return P
+
+
+def low_rank(m, n, seed):
+    """Rank 40: every later row reduces to zero through the basis tables."""
+    import oracle as O
+    L, R = gen.dense_packed(seed, 0, m, 40), gen.dense_packed(seed, 1, 40, n)
+    return O.matmul(L, R, m, 40, n)
+
+
+@pytest.mark.parametrize("make", [repeated, late_pivots, low_rank])
+@pytest.mark.parametrize("form,m,n", [("tc", 31, 33), ("tc", 65, 64), ("tc", 319, 255), ("tc", 321, 257),
+                                      ("tc", 641, 545), ("tc", 900, 288), ("m4ri", 33, 31), ("m4ri", 511, 65),
+                                      ("m4ri", 513, 96), ("m4ri", 1100, 161), ("m4ri", 300, 20000)])
+def test_pivot_search_edges(cuda, make, form, m, n):
+    check_all(make(m, n, 1000 * m + n), m, n, form)
