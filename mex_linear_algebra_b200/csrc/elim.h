@@ -9,8 +9,8 @@ struct ElimLayout {
     size_t state, stamp, ps, rbuf, cand, gb, ysnap, total;
 };
 struct NullLayout {
-    size_t pm, pbase, free, rc, rt, total;
-    i64 ldr;
+    size_t mask, before, mv, x, total;
+    i64 ldx;
 };
 
 ElimLayout elim_layout(i64 m, i64 n);
