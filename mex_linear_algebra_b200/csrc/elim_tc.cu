@@ -17,15 +17,17 @@
 //                   the window.  The walked part of the list is then compacted
 //                   in place (pivot rows and rows found zero from the window on
 //                   are dropped, order kept).
+//   window_near     the next window's words of every other row to update (rank:
+//                   the active rows; RREF: all rows), all that the next
+//                   factorization reads, by tables over the tags and the P
+//                   rows; a row whose bits at the window's pivot columns are
+//                   not all zero gets a slot, those bits as a row of 0/1 bytes.
 //   window_combine  R_b = sum_j tag[b][j] A[P_j] over the words from the window
 //                   on, into the panel buffer (a block per 4 words, 4-bit
 //                   tables over the P rows).
-//   window_coef     every other row to update (rank: the active rows; RREF: all
-//                   rows) whose bits at the window's pivot columns are not all
-//                   zero gets a slot; those bits become a row of 0/1 bytes.
 //   window_rt       R transposed as 0/1 bytes, Rt8[j][b] = bit j of R_b, and
 //                   R_b written over row P_b.
-//   tc_update       A[row(slot), w..] ^= parity(X8[slot] . Rt8^T): tcgen05
+//   tc_update       the other words: A[row(slot)] ^= parity(X8[slot] . Rt8^T): tcgen05
 //                   kind::i8 128 x 256 tiles with K = 256.  A persistent CTA
 //                   keeps a 256-column strip of Rt8 in shared memory and
 //                   streams 128-row tiles of X8 through a 4-stage ring into two
@@ -36,6 +38,7 @@
 // pivot column b, and XORing sum_b x_b R_b clears every pivot column of the
 // window; a row whose window part lies in the basis' span (every active row,
 // once the scan has ended) is then zero across the window.
+#include <algorithm>
 #include <climits>
 #include <cstdlib>
 #include <cstring>
@@ -69,7 +72,7 @@ struct WinState {
     int lbase;              // the list is list[lbase .. lbase + na)
     u64 have[WW];           // pivot columns of the window
     int prow[WBITS];        // physical row P_b of pivot column b (-1: none)
-    u64 tag[WBITS][WW];     // R_b = sum_j bit j * A[P_j]
+    alignas(16) u64 tag[WBITS][WW];  // R_b = sum_j bit j * A[P_j]
 };
 
 struct WfSmem {
@@ -107,7 +110,6 @@ __device__ __forceinline__ uint4 xor4u(const uint4 &a, const uint4 &b)
 {
     return make_uint4(a.x ^ b.x, a.y ^ b.y, a.z ^ b.z, a.w ^ b.w);
 }
-__device__ __forceinline__ bool any4(const u64 (&v)[WW]) { return (v[0] | v[1] | v[2] | v[3]) != 0; }
 
 
 // Exclusive position of this thread's flag among the block's flags (thread
@@ -185,11 +187,10 @@ __device__ __forceinline__ u32 wf_half(const WfSmem &S, const u32 (&v)[8], int h
 // pivots costs about 2600 cycles in half_word_select, four barriers, the
 // tables and one half word of every row: about 29 us for a full window, against
 // 133 us when the rows are eliminated one pivot and one barrier at a time.
-// Whole rank of 3000 x 5000 (rank 2200): 532 against 1415 us.
 __global__ void __launch_bounds__(WF_THREADS, 1)
 window_factor_kernel(const u64 *__restrict__ M, i64 ld, i64 m, i64 n, i64 w, int *list, const unsigned char *live,
                      unsigned char *state, int *stamp, int wid, const WinState *prev, WinState *ws, long long *piv,
-                     long long *prow)
+                     long long *prow, long long *rank)
 {
     extern __shared__ __align__(16) unsigned char wf_raw[];
     WfSmem &S = *reinterpret_cast<WfSmem *>(wf_raw);
@@ -200,6 +201,14 @@ window_factor_kernel(const u64 *__restrict__ M, i64 ld, i64 m, i64 n, i64 w, int
     const i64 vb = n - 64 * w;
     const int valid = vb < WBITS ? (int)vb : WBITS;  // columns of this window inside the matrix
     const int na = prev->na;
+    if (na == 0) {  // every row is a pivot or zero: nothing in any later window
+        if (tid == 0) {
+            ws->rt = 0;
+            ws->na = 0;
+            ws->rank = prev->rank;
+        }
+        return;
+    }
     int *L0 = list + prev->lbase;
 
     u32 H[8] = {};  // pivot columns so far (the same in every thread)
@@ -405,6 +414,7 @@ window_factor_kernel(const u64 *__restrict__ M, i64 ld, i64 m, i64 n, i64 w, int
         ws->lbase = prev->lbase + S.cnt;  // S.cnt = entries dropped
         ws->na = na - S.cnt;
         ws->rank = r0 + nb;
+        *rank = r0 + nb;
     }
 }
 
@@ -476,57 +486,151 @@ window_combine_kernel(const u64 *__restrict__ M, i64 ld, i64 wc, i64 w, const Wi
     }
 }
 
-// ---------------------------------------------------------------- window_coef
 // 4 bits -> 4 bytes of 0/1.
 __device__ __forceinline__ u32 nib_bytes(u32 v) { return ((v & 15u) * 0x00204081u) & 0x01010101u; }
 
-// Rows to update: rank form, the list of active rows (pivot rows of this
-// window already removed); RREF form, every row except this window's pivots.
-__global__ void __launch_bounds__(256)
-window_coef_kernel(const u64 *__restrict__ M, i64 ld, i64 m, i64 wc, i64 w, const int *__restrict__ list,
-                   const int *stamp, int wid, int rref, WinState *ws, int *ulist, unsigned char *X8,
-                   unsigned char *live)
+// ---------------------------------------------------------------- window_near
+namespace {
+struct NrSmem {
+    uint4 tag[2][16][64];   // 4-bit tables of the tags, entry-major: [16-byte half][entry][group]
+    uint4 prow[2][16][64];  // the same of the pivot rows' words of the next window
+    int cnt[8];
+    int base;
+};
+
+// Half words 0..7 in a group of 8 lanes, one a lane -> nibble s of half word k
+// in bits 4k .. 4k + 3 (s: the lane's place in its group).
+__device__ __forceinline__ u32 gather_nibbles(u32 v, int lane)
 {
-    if (ws->rt == 0) return;
-    u64 hv[WW];
+    const int s = lane & 7;
+    u32 r = 0;
 #pragma unroll
-    for (int q = 0; q < WW; ++q) hv[q] = ws->have[q];
+    for (int k = 0; k < 8; ++k)
+        r |= ((__shfl_sync(0xffffffffu, v, (lane & 24) + k) >> (4 * s)) & 15u) << (4 * k);
+    return r;
+}
+// XOR over a group of 8 lanes of an 8-word vector, word s left in lane s.
+__device__ __forceinline__ u32 xor_scatter(const u32 (&a)[8], int lane)
+{
+    u32 b[4], c[2];
+    const bool h4 = lane & 4, h2 = lane & 2, h1 = lane & 1;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const u32 send = h4 ? a[i] : a[4 + i], keep = h4 ? a[4 + i] : a[i];
+        b[i] = keep ^ __shfl_xor_sync(0xffffffffu, send, 4);
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const u32 send = h2 ? b[i] : b[2 + i], keep = h2 ? b[2 + i] : b[i];
+        c[i] = keep ^ __shfl_xor_sync(0xffffffffu, send, 2);
+    }
+    return (h1 ? c[1] : c[0]) ^ __shfl_xor_sync(0xffffffffu, h1 ? c[0] : c[1], 1);
+}
+// sum over the lane's groups s, s + 8, .. of table entries, XORed over the 8
+// lanes: the lanes of a row read 8 different 16-byte bank groups.
+__device__ __forceinline__ u32 near_lookup(const uint4 (&t)[2][16][64], u32 nib, int lane)
+{
+    u32 a[8] = {};
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const int e = (int)((nib >> (4 * k)) & 15), g = (lane & 7) + 8 * k;
+        xor8(a, t[0][e][g], t[1][e][g]);
+    }
+    return xor_scatter(a, lane);
+}
+}  // namespace
+
+// The next window's words of every row to update (rank: the active rows;
+// RREF: every row but this window's pivots), which is all that the next
+// factorization reads, and the coefficients of the tensor-core update.  A
+// group of 8 lanes per row, a half word each: the row's bits y at the window's
+// pivot columns give z = sum_b y_b tag[b], the combination of the original
+// pivot rows, and the words change by sum_j z_j A[P_j] -- 64 table reads each,
+// without waiting for the reduced rows R.  Rows with y != 0 get a slot of
+// ulist and their coefficients as 0/1 bytes in X8; live says whether the
+// row's words of the next window are nonzero (the update adds the others).
+// Latency-bound: about 2 us of table building and dependent loads, then
+// 1000 cycles per 32 rows.  It takes the place, on the critical path, of the
+// combine, transpose and one-strip tensor-core launches (15 us a window):
+// rank of 3000 x 5000 (rank 2200) 422 against 516 us, 8192 x 8192 1.22 ms.
+__global__ void __launch_bounds__(256)
+window_near_kernel(u64 *__restrict__ M, i64 ld, i64 m, i64 wc, i64 w, const int *__restrict__ list, const int *stamp,
+                   int wid, int rref, WinState *ws, int *ulist, unsigned char *X8, unsigned char *live)
+{
+    extern __shared__ __align__(16) unsigned char nr_raw[];
+    NrSmem &S = *reinterpret_cast<NrSmem *>(nr_raw);
+    if (ws->rt == 0) return;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, s = lane & 7;
+    {
+        // a thread per (table, 16-byte half, group): its 16 entries in Gray-code order
+        const int half = (tid >> 6) & 1, g = tid & 63;
+        const i64 pw = w + WW + 2 * half;
+        uint4 v[4];
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const int pr = ws->prow[4 * g + b];
+            v[b] = make_uint4(0, 0, 0, 0);
+            if (pr >= 0 && tid < 128) v[b] = reinterpret_cast<const uint4 *>(ws->tag[4 * g + b])[half];
+            if (pr >= 0 && tid >= 128) {
+                const u64 *src = M + (i64)pr * ld + pw;
+                const u64 x0 = pw < wc ? src[0] : 0ull, x1 = pw + 1 < wc ? src[1] : 0ull;
+                v[b] = make_uint4((u32)x0, (u32)(x0 >> 32), (u32)x1, (u32)(x1 >> 32));
+            }
+        }
+        uint4 *T = tid < 128 ? &S.tag[half][0][g] : &S.prow[half][0][g];
+        uint4 a = make_uint4(0, 0, 0, 0);
+        T[0] = a;
+#pragma unroll
+        for (int i = 1; i < 16; ++i) {
+            a = xor4u(a, v[(i & 1) ? 0 : (i & 2) ? 1 : (i & 4) ? 2 : 3]);
+            T[(i ^ (i >> 1)) * 64] = a;
+        }
+    }
+    const u32 have = reinterpret_cast<const u32 *>(ws->have)[s];
     const i64 cnt = rref ? m : (i64)ws->na;
     list += ws->lbase;
-    const int wn = (wc - w) < WW ? (int)(wc - w) : WW;
-    const int lane = threadIdx.x & 31;
-    const i64 stride = (i64)gridDim.x * blockDim.x;
-    for (i64 i0 = (i64)blockIdx.x * blockDim.x; i0 < cnt; i0 += stride) {
-        const i64 idx = i0 + threadIdx.x;
+    __syncthreads();
+    for (i64 i0 = (i64)blockIdx.x * 32; i0 < cnt; i0 += (i64)gridDim.x * 32) {
+        const i64 idx = i0 + (tid >> 3);
         i64 row = -1;
         if (idx < cnt) {
             row = rref ? idx : (i64)list[idx];
             if (rref && stamp[row] == wid) row = -1;
         }
-        u64 xc[WW] = {0, 0, 0, 0};
-        if (row >= 0) {
+        u32 *p = reinterpret_cast<u32 *>(M + row * ld + w) + s;
+        const bool in_y = row >= 0 && w + (s >> 1) < wc, in_v = row >= 0 && w + WW + (s >> 1) < wc;
+        const u32 y = in_y ? p[0] & have : 0u;
+        u32 v = in_v ? p[2 * WW] : 0u;
+        const unsigned nzl = __ballot_sync(0xffffffffu, y != 0);
+        const unsigned nz4 = ((nzl & 0xffu) != 0) | ((nzl & 0xff00u) != 0) << 1 | ((nzl & 0xff0000u) != 0) << 2 |
+                             ((nzl & 0xff000000u) != 0) << 3;  // the warp's four rows
+        if (lane == 0) S.cnt[warp] = __popc(nz4);
+        __syncthreads();
+        if (tid == 0) {
+            int t = 0;
 #pragma unroll
-            for (int q = 0; q < WW; ++q)
-                if (q < wn && hv[q]) xc[q] = M[row * ld + w + q] & hv[q];
+            for (int q = 0; q < 8; ++q) t += S.cnt[q];
+            S.base = t ? atomicAdd(&ws->nu, t) : 0;
         }
-        const bool nz = any4(xc);
-        const unsigned b = __ballot_sync(0xffffffffu, nz);
-        int basepos = 0;
-        if (b) {
-            if (lane == 0) basepos = atomicAdd(&ws->nu, __popc(b));
-            basepos = __shfl_sync(0xffffffffu, basepos, 0);
+        const bool nz = (nz4 >> (lane >> 3)) & 1;
+        if (nz4) {
+            const u32 z = near_lookup(S.tag, gather_nibbles(y, lane), lane);
+            v ^= near_lookup(S.prow, gather_nibbles(z, lane), lane);
+            if (nz && in_v) p[2 * WW] = v;
+            const unsigned vl = __ballot_sync(0xffffffffu, in_v && v != 0);
+            if (nz && s == 0) live[row] = ((vl >> (lane & 24)) & 0xffu) != 0;
         }
+        __syncthreads();
         if (nz) {
-            const int slot = basepos + __popc(b & ((1u << lane) - 1));
-            ulist[slot] = (int)row;
-            live[row] = 0;  // set again by the update if the row stays nonzero
-            uint4 *dst = reinterpret_cast<uint4 *>(X8 + (size_t)slot * WBITS);
+            int slot = S.base + __popc(nz4 & ((1u << (lane >> 3)) - 1));
 #pragma unroll
-            for (int c = 0; c < 16; ++c) {
-                const u32 bits = (u32)(xc[c >> 2] >> (16 * (c & 3))) & 0xFFFFu;
-                dst[c] = make_uint4(nib_bytes(bits), nib_bytes(bits >> 4), nib_bytes(bits >> 8), nib_bytes(bits >> 12));
-            }
+            for (int q = 0; q < 8; ++q) slot += q < warp ? S.cnt[q] : 0;
+            if (s == 0) ulist[slot] = (int)row;
+            uint4 *dst = reinterpret_cast<uint4 *>(X8 + (size_t)slot * WBITS + 32 * s);
+            dst[0] = make_uint4(nib_bytes(y), nib_bytes(y >> 4), nib_bytes(y >> 8), nib_bytes(y >> 12));
+            dst[1] = make_uint4(nib_bytes(y >> 16), nib_bytes(y >> 20), nib_bytes(y >> 24), nib_bytes(y >> 28));
         }
+        __syncthreads();  // cnt and base are read before the next rows write them
     }
 }
 
@@ -881,14 +985,25 @@ tc_update_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
 // ---------------------------------------------------------------- host side
 static size_t al256(size_t x) { return (x + 255) & ~(size_t)255; }
 
-// The first window's list: every row, in order.
-__global__ void list_init_kernel(int *list, i64 m, WinState *ws)
+// The state before the first window: every row active, possibly nonzero and
+// in the list, in order; no pivots.
+__global__ void window_init_kernel(i64 m, int *list, unsigned char *state, int *stamp, unsigned char *live0,
+                                   unsigned char *live1, WinState *prev, long long *rank)
 {
-    for (i64 i = blockIdx.x * (i64)blockDim.x + threadIdx.x; i < m; i += (i64)gridDim.x * blockDim.x)
+    for (i64 i = blockIdx.x * (i64)blockDim.x + threadIdx.x; i < m; i += (i64)gridDim.x * blockDim.x) {
         list[i] = (int)i;
+        state[i] = 1;
+        stamp[i] = -1;
+        live0[i] = 1;
+        live1[i] = 1;
+    }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        ws->na = (int)m;
-        ws->lbase = 0;
+        prev->rank = 0;
+        prev->rt = 0;
+        prev->nu = 0;
+        prev->na = (int)m;
+        prev->lbase = 0;
+        *rank = 0;
     }
 }
 
@@ -1026,8 +1141,6 @@ mela_status elim_tc_device(u64 *M, i64 ld, i64 m, i64 n, int rref, long long *d_
     if (st != MELA_OK) return st;
     cudaStream_t s2;
     if ((st = side_stream(&s2)) != MELA_OK) return st;
-    cudaStream_t s3;  // the coefficient pass, beside the combine and transpose
-    if ((st = aux_stream(&s3)) != MELA_OK) return st;
 
     const size_t wf_smem = sizeof(WfSmem);
     MELA_CUDA_TRY(cudaFuncSetAttribute(window_factor_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1036,39 +1149,32 @@ mela_status elim_tc_device(u64 *M, i64 ld, i64 m, i64 n, int rref, long long *d_
     const int cb_smem = (int)sizeof(CbSmem);
     MELA_CUDA_TRY(cudaFuncSetAttribute(window_combine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, cb_smem));
     const int sms = sm_count();
-    const i64 coef_blocks_full = (m + 255) / 256;
-    const int coef_blocks = (int)(coef_blocks_full < (i64)sms * 8 ? coef_blocks_full : (i64)sms * 8);
+    const int nr_smem = (int)sizeof(NrSmem);
+    MELA_CUDA_TRY(cudaFuncSetAttribute(window_near_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, nr_smem));
+    const int near_blocks = (int)std::min<i64>((m + 31) / 32, 2 * sms);
     const i64 tiles_max = L.mpad / UM, chunks_max = (tiles_max + U_MCH - 1) / U_MCH;
     u32 *err = device_error_word();
 
-    // Look-ahead: the update of window w is split into its second strip
-    // (window w+1's columns), run on the caller's stream before window w+1 is
-    // factored, and the rest, forked to the side stream so that it runs while
-    // window w+1 is factored (on an SM the fork leaves free).
-    // Window w+1's combine waits for it: it reads the pivot rows' later words,
-    // and its coefficient and R buffers are the ones the rest still reads.
-    // Window states and row flags alternate by window parity so that the
-    // factorization of w+1 never writes what the update of w reads.
-    // The coefficient pass of a window reads only rows that are not its pivot
-    // rows, which the transpose kernel overwrites, so it runs on a third
-    // stream beside the combine and the transpose and rejoins before the
-    // update.
-    cudaEvent_t evs[4] = {};
-    for (int i = 0; i < 4; ++i) {
+    // Look-ahead: window_near brings window w + 1's columns of every row up to
+    // date, so the next factorization follows it at once; the reduced rows and
+    // the update of the other columns are forked to the side stream and run
+    // beside it (on SMs the fork leaves free).  window_near of window w + 1
+    // waits for them: it reads the pivot rows' later words, and the coefficient
+    // and R buffers are the ones the update still reads.  Window states and row
+    // flags alternate by window parity so that the factorization of w + 1 never
+    // writes what the update of w reads.
+    cudaEvent_t evs[2] = {};
+    for (int i = 0; i < 2; ++i) {
         if (cudaEventCreateWithFlags(&evs[i], cudaEventDisableTiming) != cudaSuccess) {
             for (int j = 0; j < i; ++j) cudaEventDestroy(evs[j]);
             set_error("cudaEventCreate failed");
             return MELA_ERR_CUDA;
         }
     }
-    cudaEvent_t ev_fork = evs[0], ev_join = evs[1], ev_cfork = evs[2], ev_cjoin = evs[3];
+    cudaEvent_t ev_fork = evs[0], ev_join = evs[1];
     cudaStream_t sx = s;  // the stream the launches go to (a capture stream while capturing)
     auto run = [&]() -> mela_status {
-        MELA_CUDA_TRY(cudaMemsetAsync(state, 1, (size_t)m, sx));
-        MELA_CUDA_TRY(cudaMemsetAsync(stamp, 0xff, (size_t)m * 4, sx));
-        MELA_CUDA_TRY(cudaMemsetAsync(b + L.live, 1, 2 * al256((size_t)m), sx));
-        MELA_CUDA_TRY(cudaMemsetAsync(b + L.ws, 0, 2 * al256(sizeof(WinState)), sx));
-        list_init_kernel<<<grid_for(m), 256, 0, sx>>>(list, m, wsv[1]);  // the state "before" window 0
+        window_init_kernel<<<grid_for(m), 256, 0, sx>>>(m, list, state, stamp, livev[0], livev[1], wsv[1], d_rank);
         bool forked = false;
         int wid = 0;
         for (i64 w = 0; w < wc; w += WW, ++wid) {
@@ -1076,49 +1182,36 @@ mela_status elim_tc_device(u64 *M, i64 ld, i64 m, i64 n, int rref, long long *d_
             WinState *cur = wsv[wid & 1], *prev = wsv[(wid + 1) & 1];
             unsigned char *live = livev[wid & 1];  // flags of window wid-2 (complete); then this window's
             window_factor_kernel<<<1, WF_THREADS, wf_smem, sx>>>(M, ld, m, n, w, list, live, state, stamp, wid, prev,
-                                                                cur, d_piv, d_prow);
+                                                                cur, d_piv, d_prow, d_rank);
             if (forked) {
                 MELA_CUDA_TRY(cudaStreamWaitEvent(sx, ev_join, 0));
                 forked = false;
             }
-            MELA_CUDA_TRY(cudaEventRecord(ev_cfork, sx));
-            MELA_CUDA_TRY(cudaStreamWaitEvent(s3, ev_cfork, 0));
-            window_coef_kernel<<<coef_blocks, 256, 0, s3>>>(M, ld, m, wc, w, list, stamp, wid, rref, cur, ulist, X8,
-                                                           live);
-            MELA_CUDA_TRY(cudaEventRecord(ev_cjoin, s3));
-            window_combine_kernel<<<(unsigned)((lw + CB_W - 1) / CB_W), 256, cb_smem, sx>>>(M, ld, wc, w, cur, Rbuf,
+            window_near_kernel<<<near_blocks, 256, nr_smem, sx>>>(M, ld, m, wc, w, list, stamp, wid, rref, cur, ulist,
+                                                                 X8, live);
+            MELA_CUDA_TRY(cudaEventRecord(ev_fork, sx));
+            MELA_CUDA_TRY(cudaStreamWaitEvent(s2, ev_fork, 0));
+            window_combine_kernel<<<(unsigned)((lw + CB_W - 1) / CB_W), 256, cb_smem, s2>>>(M, ld, wc, w, cur, Rbuf,
                                                                                            wc);
-            window_rt_kernel<<<(unsigned)lw, 256, 0, sx>>>(M, ld, w, Rbuf, wc, cur, Rt8);
-            MELA_CUDA_TRY(cudaStreamWaitEvent(sx, ev_cjoin, 0));
-            // near: strip 1 (the next window's columns, all the next
-            // factorization reads), one row tile per CTA; far: strip 0 (the
-            // window's own columns: only the RREF needs them -- for the rank
-            // every updated row is in the window basis' span and its window
-            // part becomes zero) and strips 2.., on the side stream
+            window_rt_kernel<<<(unsigned)lw, 256, 0, s2>>>(M, ld, w, Rbuf, wc, cur, Rt8);
+            // strips 2.. and, for the RREF, strip 0 (the window's own columns;
+            // for the rank every updated row is in the window basis' span and
+            // its window part becomes zero)
             const i64 strips = (lw + 3) / 4;
-            if (strips >= 2) {
-                const int grid_near = (int)(tiles_max < sms ? tiles_max : sms);
-                tc_update_kernel<<<grid_near, U_THREADS, U_SMEM, sx>>>(mx, mr, M, ld, wc, w, cur, ulist, live, 1, 2,
-                                                                      -1, 1, err);
-            }
             const int far_lo = rref ? 0 : 2, far_skip = (rref && strips >= 2) ? 1 : -1;
             const i64 far_strips = (strips > far_lo ? strips - far_lo : 0) - (far_skip >= 0 ? 1 : 0);
             if (far_strips > 0) {
                 const i64 units = far_strips * chunks_max;
                 const int cap = sms > 4 ? sms - 2 : sms;  // SMs left for the next factorization
                 const int grid_far = (int)(units < cap ? units : cap);
-                MELA_CUDA_TRY(cudaEventRecord(ev_fork, sx));
-                MELA_CUDA_TRY(cudaStreamWaitEvent(s2, ev_fork, 0));
                 tc_update_kernel<<<grid_far, U_THREADS, U_SMEM, s2>>>(mx, mr, M, ld, wc, w, cur, ulist, live, far_lo,
                                                                      (int)strips, far_skip, U_MCH, err);
-                MELA_CUDA_TRY(cudaEventRecord(ev_join, s2));
-                forked = true;
             }
+            MELA_CUDA_TRY(cudaEventRecord(ev_join, s2));
+            forked = true;
         }
         if (forked) MELA_CUDA_TRY(cudaStreamWaitEvent(sx, ev_join, 0));
         MELA_LAUNCH_CHECK("tensor-core elimination");
-        WinState *last = wsv[(wid + 1) & 1];  // the state written by the last window (wid-1)
-        MELA_CUDA_TRY(cudaMemcpyAsync(d_rank, &last->rank, sizeof(long long), cudaMemcpyDeviceToDevice, sx));
         return MELA_OK;
     };
     // The launch sequence depends only on the shape and the buffers, so from

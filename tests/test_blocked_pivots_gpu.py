@@ -42,3 +42,17 @@ def low_rank(m, n, seed):
                                       ("m4ri", 513, 96), ("m4ri", 1100, 161), ("m4ri", 300, 20000)])
 def test_pivot_search_edges(cuda, make, form, m, n):
     check_all(make(m, n, 1000 * m + n), m, n, form)
+
+
+@pytest.mark.parametrize("m,n", [(33, 513), (70, 700), (300, 1100)])
+def test_rows_that_leave_the_list(cuda, m, n):
+    """Zero rows, rows that become zero in the first window and rows whose first
+    ones come two windows later: the lists, flags and coefficient slots of the
+    later windows, up to windows with no row left."""
+    P = gen.dense_packed(m + n, 0, m, n)
+    P[::5] = 0
+    P[1::5] = P[min(2, m - 1)]
+    P[3::5, : (n // 64) // 2] = 0
+    check_all(P, m, n, "tc")
+    P[:, 4:] = 0  # no pivots past the first window
+    check_all(P, m, n, "tc")
