@@ -25,15 +25,16 @@
 //   window_combine  R_b = sum_j tag[b][j] A[P_j] over the words from the window
 //                   on, into the panel buffer (a block per 4 words, 4-bit
 //                   tables over the P rows).
-//   window_rt       R transposed as 0/1 bytes, Rt8[j][b] = bit j of R_b, and
-//                   R_b written over row P_b.
+//   window_rt       R transposed as 0/1 bytes, Rt8[j][b] = bit j of R_b (the
+//                   columns of each 32 in the order the update's epilogue
+//                   gathers them), and R_b written over row P_b.
 //   tc_update       the other words: A[row(slot)] ^= parity(X8[slot] . Rt8^T): tcgen05
 //                   kind::i8 128 x 256 tiles with K = 256.  A persistent CTA
 //                   keeps a 256-column strip of Rt8 in shared memory and
 //                   streams 128-row tiles of X8 through a 4-stage ring into two
-//                   TMEM accumulators; sixteen epilogue warps XOR the parity
-//                   bits into the packed rows while the next tile is
-//                   multiplied, and flag the rows that are still nonzero.
+//                   TMEM accumulators; four groups of four epilogue warps XOR
+//                   the parity bits into the packed rows while the next tiles
+//                   are multiplied, and flag the rows that are still nonzero.
 // Since the basis is reduced, a row's coefficient for R_b is its own bit at
 // pivot column b, and XORing sum_b x_b R_b clears every pivot column of the
 // window; a row whose window part lies in the basis' span (every active row,
@@ -634,8 +635,22 @@ window_near_kernel(u64 *__restrict__ M, i64 ld, i64 m, i64 wc, i64 w, const int 
     }
 }
 
+// The parity bits of 32 columns from 16 registers of column pairs (low 16 bits
+// of columns 2i and 2i + 1): columns 2i in bits 0..15, 2i + 1 in bits 16..31.
+__device__ __forceinline__ u32 parity_pairs(const u32 *r)
+{
+    u32 b = r[0] & 0x00010001u;
+#pragma unroll
+    for (int i = 1; i < 16; ++i) b |= (r[i] << i) & (0x00010001u << i);
+    return b;
+}
+// Place of column bit b of a 32-column group in the strip, so that
+// parity_pairs leaves it in bit b.
+__device__ __forceinline__ int pair_place(int b) { return b < 16 ? 2 * b : 2 * (b - 16) + 1; }
+
 // ---------------------------------------------------------------- window_rt
-// Block W (word w + W): Rt8 rows 64W..64W+63 and word w + W of every row P_b.
+// Block W (word w + W): Rt8 rows 64W..64W+63 (in pair_place order) and word
+// w + W of every row P_b.
 __global__ void __launch_bounds__(256)
 window_rt_kernel(u64 *__restrict__ M, i64 ld, i64 w, const u64 *__restrict__ Rbuf, i64 ldr, const WinState *ws,
                  unsigned char *Rt8)
@@ -659,7 +674,9 @@ window_rt_kernel(u64 *__restrict__ M, i64 ld, i64 w, const u64 *__restrict__ Rbu
             for (int b = 0; b < 4; ++b) x |= (u32)((col[16 * c + 4 * r + b] >> jl) & 1) << (8 * b);
             o[r] = x;
         }
-        *reinterpret_cast<uint4 *>(Rt8 + ((size_t)(W * 64 + jl)) * WBITS + 16 * c) = make_uint4(o[0], o[1], o[2], o[3]);
+        const int place = (jl & 32) + pair_place(jl & 31);
+        *reinterpret_cast<uint4 *>(Rt8 + ((size_t)(W * 64 + place)) * WBITS + 16 * c) =
+            make_uint4(o[0], o[1], o[2], o[3]);
     }
 }
 
@@ -673,24 +690,17 @@ constexpr int UA_BYTES = 2 * UA_BOX;          // K = 256
 constexpr int UB_BYTES = 2 * UB_BOX;
 constexpr int U_STAGES = 4;                   // X8 tiles in flight
 constexpr int U_BSTAGES = 1;                  // Rt8 strips in shared memory
-constexpr int U_STAGE_BYTES = 2 * 2 * UM * 4 * 8;  // per accumulator, two 128-row x 4-word stages
+constexpr int U_GROUPS = 4;                   // epilogue groups, tile t to group t % 4
+constexpr int U_STAGE_BYTES = U_GROUPS * UM * 4 * 8;  // per group, 128 rows x 4 words
 constexpr int U_SMEM = U_BSTAGES * UB_BYTES + U_STAGES * UA_BYTES + U_STAGE_BYTES + 1024 + 256;
 constexpr int U_MCH = 8;                      // row tiles per work unit (far part)
-constexpr int U_EPI_THREADS = 256;           // warps draining one accumulator: 2 per TMEM lane quarter
-constexpr int U_THREADS = 64 + 2 * U_EPI_THREADS;  // and the same for the other accumulator
-
-// bit `pos` of base := bit 0 of src
-__device__ __forceinline__ u32 bfi1(u32 src, u32 base, u32 pos)
-{
-    u32 d;
-    asm("bfi.b32 %0, %1, %2, %3, 1;" : "=r"(d) : "r"(src), "r"(base), "r"(pos));
-    return d;
-}
+constexpr int U_EPI_THREADS = 128;           // a group: one warp per TMEM lane quarter
+constexpr int U_THREADS = 64 + U_GROUPS * U_EPI_THREADS;
 
 struct UCtl {
     u64 bfull[U_BSTAGES], bempty[U_BSTAGES];
     u64 afull[U_STAGES], aempty[U_STAGES];
-    u64 accfull[2], accempty[2];
+    u64 accfull[U_GROUPS], accempty[2];
     u64 drain;
     u32 tmem;
     int abort;
@@ -698,6 +708,12 @@ struct UCtl {
 
 }  // namespace
 
+// Bound by the matrix instructions (M = 128 kind::i8 reads 12 KB of shared
+// memory an instruction: 87 us of the 100 us that a launch over 16384 rows x
+// 32256 columns takes without any epilogue work).  Before, 134 us: the parity
+// bits one by one (two logical operations an element against one for a pair
+// of columns read together), and each epilogue warp waiting for the row
+// numbers of its own tile.
 __global__ void __launch_bounds__(U_THREADS, 1)
 tc_update_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmR,
                  u64 *__restrict__ M, i64 ld, i64 wc, i64 w, const WinState *ws, const int *__restrict__ ulist,
@@ -726,7 +742,7 @@ tc_update_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(u_raw) + 1023) & ~(uintptr_t)1023);
     unsigned char *sB = smem;
     unsigned char *sA = smem + U_BSTAGES * UB_BYTES;
-    u64 *stage = reinterpret_cast<u64 *>(sA + U_STAGES * UA_BYTES);  // [acc][2][UM][4]
+    u64 *stage = reinterpret_cast<u64 *>(sA + U_STAGES * UA_BYTES);  // [group][UM][4]
     UCtl *ctl = reinterpret_cast<UCtl *>(sA + U_STAGES * UA_BYTES + U_STAGE_BYTES);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
@@ -739,10 +755,8 @@ tc_update_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
             ptx::mbar_init(&ctl->afull[s], 1);
             ptx::mbar_init(&ctl->aempty[s], 1);
         }
-        for (int a = 0; a < 2; ++a) {
-            ptx::mbar_init(&ctl->accfull[a], 1);
-            ptx::mbar_init(&ctl->accempty[a], U_EPI_THREADS);
-        }
+        for (int q = 0; q < U_GROUPS; ++q) ptx::mbar_init(&ctl->accfull[q], 1);
+        for (int a = 0; a < 2; ++a) ptx::mbar_init(&ctl->accempty[a], U_EPI_THREADS);
         ptx::mbar_init(&ctl->drain, 1);
         ctl->abort = 0;
         ptx::fence_barrier_init();
@@ -854,7 +868,7 @@ tc_update_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
                             ptx::umma_i8(d, ptx::desc_k_sw128(a0 + kb * UA_BOX + kk * 32),
                                          ptx::desc_k_sw128(b0 + kb * UB_BOX + kk * 32), idesc, (kb | kk) != 0);
                     ptx::umma_commit(&ctl->aempty[s]);
-                    ptx::umma_commit(&ctl->accfull[acc]);
+                    ptx::umma_commit(&ctl->accfull[it % U_GROUPS]);
                 }
                 if (!ok) break;
                 // the strip's buffer is free once this unit's products are done
@@ -869,108 +883,104 @@ tc_update_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         }
         __syncwarp();
     } else {
-        // Sixteen warps: for each of the two accumulators (tiles with
-        // it % 2 == g), two warps per TMEM lane quarter, one per 128-column
-        // half.  A tile's packed parity words go through shared memory, so
-        // that the read-modify-write of the rows is done with 32 contiguous
-        // bytes per row (4 lanes a row, 8 rows a warp instruction).  The
-        // rows' current words for a tile are fetched before the previous
-        // tile is drained.
-        const int e = warp - 2;
+        // Four groups of four warps take the tiles in turn, a warp per TMEM
+        // lane quarter (32 rows): a group has four tiles' time for the memory
+        // latencies of its own.  A tile's packed parity words go through
+        // shared memory, within the warp, so that the read-modify-write of the
+        // rows is done with 32 contiguous bytes per row (4 lanes a row, 8 rows a
+        // warp instruction).  The rows' numbers are fetched a tile ahead of
+        // their words, and the words before the previous tile is drained.
         const int ew = warp & 3;          // TMEM lane quarter of this warp
-        const int g = (e >> 2) & 1;       // accumulator
-        const int half = e >> 3;          // columns 128*half .. +127 (words 2*half, 2*half+1)
-        const int gt = ((e >> 3) << 7) | ((e & 3) << 5) | lane;  // 0..255 within the group
-        u64 *gstage = stage + (size_t)g * 2 * UM * 4;
-        int it = 0, k = 0;
+        const int g = (warp - 2) >> 2;    // group: tiles 4k + g of the CTA
+        const int r8 = lane >> 2, q = lane & 3;  // item c: row r8 + 8c of the quarter, word q
+        u64 *wstage = stage + (size_t)(g * UM + ew * 32) * 4;
+        int k = 0;  // own tiles so far
         bool ok = true;
         // previous own tile
-        int p_it = 0;
-        i64 p_w0 = 0;
-        int p_nw = 0;
-        int p_row[2] = {-1, -1};
-        u64 p_old[2] = {0, 0};
-        // Every warp of the group reaches the group barrier once per tile, on
-        // the error path too (a failed wait skips the work, not the barrier).
+        i64 p_w = 0;
+        int p_row[4] = {-1, -1, -1, -1};
+        u64 p_old[4] = {0, 0, 0, 0};
+        bool p_in = false;
         auto drain_and_write = [&]() -> bool {
-            const int acc = p_it & 1;
-            const bool good = !*abort_flag && ptx::mbar_wait(&ctl->accfull[acc], (p_it >> 1) & 1, err);
-            if (!good) *abort_flag = 1;
-            u32 pb0 = 0, pb1 = 0, pb2 = 0, pb3 = 0;
-            if (good) {
-                ptx::tc_fence_after();
-                const u32 tbase = tmem + ((u32)(ew * 32) << 16) + (u32)(acc * UN + half * 128);
-#pragma unroll 1
-                for (int h = 0; h < 4; ++h) {
-                    u32 r[32];
-                    ptx::tmem_ld_32x32b_x32(tbase + (u32)(h * 32), r);
-                    ptx::tmem_ld_wait();
-                    u32 b = r[0] & 1u;
-#pragma unroll
-                    for (int j = 1; j < 32; ++j) b = bfi1(r[j], b, (u32)j);
-                    pb0 = h == 0 ? b : pb0;
-                    pb1 = h == 1 ? b : pb1;
-                    pb2 = h == 2 ? b : pb2;
-                    pb3 = h == 3 ? b : pb3;
-                }
-                ptx::tc_fence_before();
-                ptx::mbar_arrive(&ctl->accempty[acc]);
+            const bool good = !*abort_flag && ptx::mbar_wait(&ctl->accfull[g], (k - 1) & 1, err);
+            if (!good) {
+                *abort_flag = 1;
+                return false;
             }
-            // stage row (ew*32 + lane), words 2*half, 2*half+1
-            u64 *st = gstage + (size_t)((k - 1) & 1) * UM * 4 + (size_t)(ew * 32 + lane) * 4 + 2 * half;
-            *reinterpret_cast<ulonglong2 *>(st) =
-                make_ulonglong2((u64)pb0 | ((u64)pb1 << 32), (u64)pb2 | ((u64)pb3 << 32));
-            asm volatile("bar.sync %0, %1;" ::"r"(1 + g), "r"(U_EPI_THREADS) : "memory");
-            // items gt and gt + 256: row = item / 4, word = item % 4
-            const u64 *sb = gstage + (size_t)((k - 1) & 1) * UM * 4;
+            ptx::tc_fence_after();
+            const u32 tbase = tmem + ((u32)(ew * 32) << 16) + (u32)((g & 1) * UN);
+            u32 pb[8];
 #pragma unroll
-            for (int c = 0; c < 2; ++c) {
-                const int item = gt + 256 * c;
-                const int q = item & 3;
+            for (int h = 0; h < 4; ++h) {
+                u32 r[32];
+                ptx::tmem_ld_32x32b_x32_pack16(tbase + 64 * h, r);
+                ptx::tmem_ld_wait();
+                pb[2 * h] = parity_pairs(r);
+                pb[2 * h + 1] = parity_pairs(r + 16);
+            }
+            ptx::tc_fence_before();
+            ptx::mbar_arrive(&ctl->accempty[g & 1]);
+            __syncwarp();  // the previous tile's words have been read
+            uint4 *st = reinterpret_cast<uint4 *>(wstage + 4 * lane);
+            st[0] = make_uint4(pb[0], pb[1], pb[2], pb[3]);
+            st[1] = make_uint4(pb[4], pb[5], pb[6], pb[7]);
+            __syncwarp();
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
                 u64 v = 0;
-                if (good && p_row[c] >= 0 && q < p_nw) {
-                    v = p_old[c] ^ sb[item];
-                    M[(i64)p_row[c] * ld + p_w0 + q] = v;
+                if (p_row[c] >= 0 && p_in) {
+                    v = p_old[c] ^ wstage[lane + 32 * c];
+                    M[(i64)p_row[c] * ld + p_w] = v;
                 }
                 // one flag per row: the four lanes of a row combine their words
-                v |= __shfl_xor_sync(0xffffffffu, v, 1);
-                v |= __shfl_xor_sync(0xffffffffu, v, 2);
-                if (q == 0 && p_row[c] >= 0 && v) live[p_row[c]] = 1;
+                const unsigned nz = __ballot_sync(0xffffffffu, v != 0);
+                if (q == 0 && p_row[c] >= 0 && ((nz >> (4 * r8)) & 15u)) live[p_row[c]] = 1;
             }
-            return good;
+            return true;
         };
-        for (long long u = ub; u < ue; ++u) {
-            const int strip = strip_of(u / chunks), chunk = (int)(u % chunks);
-            const i64 w0 = w + (i64)strip * 4;
-            const int nw = (wc - w0) < 4 ? (int)(wc - w0) : 4;
-            const int t1 = (chunk + 1) * mch < mt ? (chunk + 1) * mch : mt;
-            for (int tile = chunk * mch; tile < t1; ++tile, ++it) {
-                if ((it & 1) != g) continue;
-                // fetch this tile's words (coalesced layout), then finish the previous tile
-                int row[2] = {-1, -1};
-                u64 old[2] = {0, 0};
+        // the CTA's tiles in order
+        long long at = ub;
+        int vs = (int)(ub / chunks), chunk = (int)(ub % chunks), tile = chunk * mch;
+        auto step = [&]() {
+            if (++tile < mt && tile < (chunk + 1) * mch) return;
+            ++at;
+            if (++chunk == chunks) {
+                chunk = 0;
+                ++vs;
+            }
+            tile = chunk * mch;
+        };
+        auto rows_of = [&](int (&row)[4]) {
 #pragma unroll
-                for (int c = 0; c < 2; ++c) {
-                    const int item = gt + 256 * c;
-                    const int slot = tile * UM + (item >> 2), q = item & 3;
-                    if (slot < nu) {
-                        row[c] = ulist[slot];
-                        if (q < nw) old[c] = M[(i64)row[c] * ld + w0 + q];
-                    }
-                }
-                if (k > 0 && !drain_and_write()) ok = false;
-                ++k;
-                p_it = it;
-                p_w0 = w0;
-                p_nw = nw;
+            for (int c = 0; c < 4; ++c) {
+                const int slot = tile * UM + 32 * ew + r8 + 8 * c;
+                row[c] = at < ue && slot < nu ? ulist[slot] : -1;
+            }
+        };
+        int n_row[4];  // rows of the next own tile
+        for (int i = 0; i < g && at < ue; ++i) step();
+        rows_of(n_row);
+        while (at < ue && ok) {
+            const i64 pw = w + (i64)strip_of(vs) * 4 + q;
+            const bool in = pw < wc;
+            const int row[4] = {n_row[0], n_row[1], n_row[2], n_row[3]};
+            u64 old[4] = {0, 0, 0, 0};
 #pragma unroll
-                for (int c = 0; c < 2; ++c) {
-                    p_row[c] = row[c];
-                    p_old[c] = old[c];
-                }
+            for (int c = 0; c < 4; ++c)
+                if (row[c] >= 0 && in) old[c] = M[(i64)row[c] * ld + pw];
+            for (int i = 0; i < U_GROUPS && at < ue; ++i) step();
+            rows_of(n_row);
+            if (k > 0 && !drain_and_write()) ok = false;
+            ++k;
+            p_w = pw;
+            p_in = in;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                p_row[c] = row[c];
+                p_old[c] = old[c];
             }
         }
-        if (k > 0 && !drain_and_write()) ok = false;
+        if (ok && k > 0 && !drain_and_write()) ok = false;
         if (!ok) *abort_flag = 1;
     }
 

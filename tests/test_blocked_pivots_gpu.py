@@ -56,3 +56,12 @@ def test_rows_that_leave_the_list(cuda, m, n):
     check_all(P, m, n, "tc")
     P[:, 4:] = 0  # no pivots past the first window
     check_all(P, m, n, "tc")
+
+
+@pytest.mark.parametrize("m,n", [(300, 5000), (1400, 1500), (129, 4161)])
+def test_update_tiles(cuda, m, n):
+    """The tensor-core update over one, a few and many row tiles per strip:
+    fewer tiles than epilogue groups, strips split between CTAs, a last strip of
+    one word."""
+    P = gen.dense_packed(m, 0, m, n)
+    check_all(P, m, n, "tc")
