@@ -27,8 +27,7 @@ mela_status rank_of_packed(u64 *P, i64 ld, i64 m, i64 n, int variant, cudaStream
     st = elim_device(variant, P, ld, m, n, 0, d, d + 1, d + 1 + mn, ws.p, wsb, s);
     if (st != MELA_OK) return st;
     long long r = 0;
-    MELA_CUDA_TRY(cudaMemcpyAsync(&r, d, sizeof r, cudaMemcpyDeviceToHost, s));
-    if ((st = finish(s)) != MELA_OK) return st;
+    if ((st = read_value(&r, d, s, true)) != MELA_OK) return st;
     *rank = (double)r;
     return MELA_OK;
 }
@@ -54,8 +53,7 @@ mela_status null_of_packed(u64 *P, i64 ld, i64 m, i64 n, int variant, mela_alloc
         if ((st = ws.alloc(wsb, s)) != MELA_OK) return st;
         st = elim_device(variant, P, ld, m, n, 1, d, d + 1, d + 1 + mn, ws.p, wsb, s);
         if (st != MELA_OK) return st;
-        MELA_CUDA_TRY(cudaMemcpyAsync(&r, d, sizeof r, cudaMemcpyDeviceToHost, s));
-        MELA_CUDA_TRY(cudaStreamSynchronize(s));
+        if ((st = read_value(&r, d, s, false)) != MELA_OK) return st;
     }
     const i64 f = n - r;
     uint8_t *Z = alloc(ctx, n, f);
@@ -75,8 +73,7 @@ mela_status null_of_packed(u64 *P, i64 ld, i64 m, i64 n, int variant, mela_alloc
     if ((st = bytes.alloc((size_t)f * n, s)) != MELA_OK) return st;
     if ((st = launch_unpack_rows((const u64 *)Zt.p, ldz, f, n, (unsigned char *)bytes.p, s)) != MELA_OK)
         return st;
-    MELA_CUDA_TRY(cudaMemcpyAsync(Z, bytes.p, (size_t)f * n, cudaMemcpyDeviceToHost, s));
-    return finish(s);
+    return download_finish(Z, bytes.p, (size_t)f * n, s);
 }
 
 mela_status host_rank(const mela_host_matrix *A, int variant, double *rank)

@@ -27,6 +27,10 @@ mela_status side_stream(cudaStream_t *s);
 mela_status capture_stream(cudaStream_t *s);
 // Synchronise `s` and turn a device-side wait timeout into MELA_ERR_TIMEOUT.
 mela_status finish(cudaStream_t s);
+// A device value read back to the host; last: this ends the call (finish).
+mela_status read_value(long long *value, const long long *d, cudaStream_t s, bool last);
+// Device bytes copied to a host array of the caller, ending the call (finish).
+mela_status download_finish(void *dst, const void *src, size_t bytes, cudaStream_t s);
 
 // Row pitch in words, rounded up to an even count (16-byte rows).
 i64 even_words(i64 bits);
