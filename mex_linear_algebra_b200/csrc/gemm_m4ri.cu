@@ -22,12 +22,16 @@
 // tile load per stage into a double-buffered 4 KB tile, issued one stage
 // ahead by one thread and counted on an mbarrier (bounded wait), zeros past
 // the matrix edges.  The table builders read their 8 rows from that tile.
+// Few blocks of C leave most of the chip idle (3001 x 1777: six), so K is then
+// split over gridDim.z: each CTA multiplies its slice of the stages and XORs
+// its block into C, which starts as zero -- GF(2) sums need no order.
 // Where TMA cannot address B (a row pitch that is not a multiple of 16 bytes,
 // or an unaligned base) the rows are read with ordinary loads instead.
 #include "mela_common.cuh"
 #include "mela_internal.h"
 #include "tc_ptx.cuh"
 
+#include <algorithm>
 #include <cstring>
 
 namespace mela {
@@ -59,8 +63,8 @@ constexpr int M4_BTILE_WORDS = 16 * M4_CTA_WORDS;  // one stage's rows of B (4 K
 template <int WARPS, bool kTma>
 __global__ void __launch_bounds__(WARPS * 32, 1)
 gemm_m4ri_kernel(const u64 *__restrict__ A, i64 lda, const u64 *__restrict__ B, i64 ldb,
-                 u64 *__restrict__ C, i64 ldc, i64 m, i64 k, i64 n, const __grid_constant__ CUtensorMap bmap,
-                 u32 *err)
+                 u64 *__restrict__ C, i64 ldc, i64 m, i64 k, i64 n, i64 stages_per_split,
+                 const __grid_constant__ CUtensorMap bmap, u32 *err)
 {
     extern __shared__ __align__(128) u64 T[];  // [M4_STRIPS][256][32], then [2][16][32] rows of B
     u64 *Bt = T + M4_STRIPS * 256 * M4_CTA_WORDS;
@@ -81,7 +85,9 @@ gemm_m4ri_kernel(const u64 *__restrict__ A, i64 lda, const u64 *__restrict__ B, 
 #pragma unroll
     for (int r = 0; r < M4_ROWS_PER_WARP; ++r) acc[r] = 0;
 
-    const i64 nstages = (k + 15) / 16;
+    // this CTA's stages: st0 .. nstages-1 (st0 a multiple of 4, whole words of A)
+    const i64 st0 = (i64)blockIdx.z * stages_per_split;
+    const i64 all = (k + 15) / 16, nstages = st0 + stages_per_split < all ? st0 + stages_per_split : all;
 
     // B: the 8 rows of this warp's strip in stage st, this lane's word
     auto load_b = [&](i64 st, u64 (&bv)[8]) {
@@ -94,7 +100,7 @@ gemm_m4ri_kernel(const u64 *__restrict__ A, i64 lda, const u64 *__restrict__ B, 
     // TMA: rows 16*st .. 16*st+15, words cw0 .. cw0+31 into tile buffer st & 1
     const int cw0 = (int)((i64)blockIdx.x * M4_CTA_WORDS);
     auto issue_b = [&](i64 st) {
-        const int buf = (int)(st & 1);
+        const int buf = (int)(st & 1);  // st0 is even
         ptx::mbar_arrive_expect_tx(&bfull[buf], M4_BTILE_WORDS * 8);
         ptx::tma_load_2d(Bt + buf * M4_BTILE_WORDS, &bmap, &bfull[buf], cw0, (int)(st * 16));
     };
@@ -114,25 +120,25 @@ gemm_m4ri_kernel(const u64 *__restrict__ A, i64 lda, const u64 *__restrict__ B, 
             ptx::mbar_init(&bfull[0], 1);
             ptx::mbar_init(&bfull[1], 1);
             ptx::fence_barrier_init();
-            issue_b(0);
+            issue_b(st0);
         }
         __syncthreads();
     } else {
-        load_b(0, bv);
+        load_b(st0, bv);
     }
-    load_a(0, av);
-    load_a(1, av_next);
+    load_a(st0 / 4, av);
+    load_a(st0 / 4 + 1, av_next);
 
-    for (i64 st = 0; st < nstages; ++st) {
+    for (i64 st = st0; st < nstages; ++st) {
         const int sub = (int)(st & 3);  // 16-bit slice of the current A word
         if constexpr (kTma) {
             // this stage's rows of B have landed (every thread waits, bounded);
             // the barrier after it also ends the previous stage's lookups
-            const bool ok = ptx::mbar_wait(&bfull[st & 1], (u32)((st >> 1) & 1), err);
+            const bool ok = ptx::mbar_wait(&bfull[st & 1], (u32)(((st - st0) >> 1) & 1), err);
             if (__syncthreads_or(!ok)) {
                 // a wait ran out (timeout bit set): give the copy in flight one
                 // more bounded wait, then leave without writing C
-                if (threadIdx.x == 0) ptx::mbar_wait(&bfull[st & 1], (u32)((st >> 1) & 1), nullptr);
+                if (threadIdx.x == 0) ptx::mbar_wait(&bfull[st & 1], (u32)(((st - st0) >> 1) & 1), nullptr);
                 return;
             }
             // the other tile was last read by the previous stage's builders
@@ -179,7 +185,12 @@ gemm_m4ri_kernel(const u64 *__restrict__ A, i64 lda, const u64 *__restrict__ B, 
 #pragma unroll
         for (int r = 0; r < M4_ROWS_PER_WARP; ++r) {
             const i64 row = row0 + r;
-            if (row < m) C[row * ldc + cw] = acc[r];
+            if (row < m) {
+                if (gridDim.z == 1)
+                    C[row * ldc + cw] = acc[r];
+                else
+                    atomicXor(&C[row * ldc + cw], acc[r]);
+            }
         }
     }
 }
@@ -206,11 +217,24 @@ mela_status launch_gemm_m4ri(const u64 *A, i64 lda, const u64 *B, i64 ldb, u64 *
     const bool tma = (((uintptr_t)B & 15) == 0) && (ldb % 2 == 0) &&
                      make_u64_rows_map(&bmap, B, k, words_of(n), ldb, M4_CTA_WORDS, 16) == MELA_OK;
     u32 *err = device_error_word();
-    const dim3 grid((unsigned)gx, (unsigned)gy);
+    // K slices: as many as one wave of CTAs takes (one per SM), each of at least
+    // 4 stages (one word of A; a stage takes 2.3 us, the launch, first loads and
+    // the atomic writes of a block about 6).  3001 x 2500 x 1777: 25.5 us in 20
+    // slices, 367 us unsplit; 8192^3 in two 0.64 ms, 1.21 ms unsplit.
+    const i64 nstages = (k + 15) / 16;
+    i64 splits = std::min<i64>(sm_count() / (gx * gy), (nstages + 3) / 4);
+    i64 per = nstages;
+    if (splits > 1) {
+        per = ((nstages + splits - 1) / splits + 3) / 4 * 4;
+        splits = (nstages + per - 1) / per;
+    }
+    if (splits < 1) splits = 1;
+    if (splits > 1) MELA_CUDA_TRY(cudaMemset2DAsync(C, (size_t)ldc * 8, 0, (size_t)words_of(n) * 8, (size_t)m, s));
+    const dim3 grid((unsigned)gx, (unsigned)gy, (unsigned)splits);
     if (!tma) cudaGetLastError();
     auto launch = [&](auto kernel, int threads) -> mela_status {
         MELA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        kernel<<<grid, threads, smem, s>>>(A, lda, B, ldb, C, ldc, m, k, n, bmap, err);
+        kernel<<<grid, threads, smem, s>>>(A, lda, B, ldb, C, ldc, m, k, n, per, bmap, err);
         return MELA_OK;
     };
     mela_status st;
