@@ -858,7 +858,7 @@ def run_mela(args, ws, rank, local):
                              "sample": f"reference mela_matmul_gf2 ({isa}) on A * B[:, :{ns_}] "
                                        f"({ms_}x{ks_} * {ks_}x{ns_} logical), one call"},
             "e2e": e2e,
-            "gpu_launches": 3 * args.steps,  # expand A, transposing expand of B, product
+            "gpu_launches": 2 * args.steps,  # expansion of both operands, product
             "forms": forms,
             "clocks": clk,
             "device_error_flags": flags,

@@ -314,14 +314,8 @@ mela_status gemm_prepare(int variant, const u64 *A, i64 lda, const u64 *B, i64 l
             MELA_CUDA_TRY(cudaMemset2DAsync(b.Bt + words_of(k), (size_t)p.ldbt * 8, 0, 8, (size_t)n, s));
         }
     }
-    if (p.variant == MELA_GEMM_TC) {
-        if ((st = launch_expand_u8(A, lda, m, k, p.mp, p.kp, b.A8, s)) != MELA_OK) return st;
-        if ((st = launch_expand_t(B, ldb, k, n, p.np, p.kp, b.B8, false, s)) != MELA_OK) return st;
-    }
-    if (p.variant == MELA_GEMM_TC_FP4) {
-        if ((st = launch_expand_f4(A, lda, m, k, p.mp, p.kp, b.A8, s)) != MELA_OK) return st;
-        if ((st = launch_expand_t(B, ldb, k, n, p.np, p.kp, b.B8, true, s)) != MELA_OK) return st;
-    }
+    if (p.variant == MELA_GEMM_TC || p.variant == MELA_GEMM_TC_FP4)
+        return launch_expand(A, lda, m, p.mp, b.A8, B, ldb, n, p.np, b.B8, k, p.kp, p.variant == MELA_GEMM_TC_FP4, s);
     return MELA_OK;
 }
 
@@ -847,10 +841,8 @@ static mela_status matmul_packed_host_pipelined(const uint64_t *A, int64_t lda, 
             if (r < bm) {
                 const i64 r0 = r * mb, rows = rows_of(r);
                 MELA_CUDA_TRY(cudaStreamWaitEvent(s, ev_a(r), 0));
-                e = fp4 ? launch_expand_f4(a + r0 * wk, wk, rows, k, round_up(rows, 256), p.kp,
-                                           b.A8 + (size_t)r0 * p.kp, s)
-                        : launch_expand_u8(a + r0 * wk, wk, rows, k, round_up(rows, 256), p.kp,
-                                           b.A8 + (size_t)r0 * p.kp, s);
+                e = launch_expand(a + r0 * wk, wk, rows, round_up(rows, 256), b.A8 + (size_t)r0 * p.kp, nullptr, 0, 0, 0,
+                                  nullptr, k, p.kp, fp4, s);
                 if (e != MELA_OK) return e;
                 for (int j = 0; j < r && j < bn; ++j)
                     if ((e = product(r, j)) != MELA_OK) return e;
@@ -858,8 +850,8 @@ static mela_status matmul_packed_host_pipelined(const uint64_t *A, int64_t lda, 
             if (r < bn) {
                 const i64 c0 = r * nb, cols = cols_of(r);
                 MELA_CUDA_TRY(cudaStreamWaitEvent(s, ev_b(r), 0));
-                e = launch_expand_t(bb + c0 / 64, wn, k, cols, round_up(cols, 256), p.kp, b.B8 + (size_t)c0 * p.kp,
-                                    fp4, s);
+                e = launch_expand(nullptr, 0, 0, 0, nullptr, bb + c0 / 64, wn, cols, round_up(cols, 256),
+                                  b.B8 + (size_t)c0 * p.kp, k, p.kp, fp4, s);
                 if (e != MELA_OK) return e;
                 for (int i = 0; i <= r && i < bm; ++i)
                     if ((e = product(i, r)) != MELA_OK) return e;

@@ -21,15 +21,12 @@ mela_status launch_pack_words(int kind, i64 m, i64 n, const void *in, u64 *out, 
 mela_status launch_unpack(const u64 *in, i64 ld, i64 m, i64 n, unsigned char *out, cudaStream_t s);
 mela_status launch_transpose(const u64 *in, i64 ld_in, i64 rows, i64 cols, u64 *out, i64 ld_out,
                              cudaStream_t s);
-mela_status launch_expand_f4(const u64 *in, i64 ld, i64 rows, i64 kbits, i64 rows_pad, i64 kpad_bytes,
-                             unsigned char *out, cudaStream_t s);
-// Column j of the packed kbits x cols matrix `in` as row j of a K-major
-// tensor-core operand (cols_pad rows, a multiple of 256; kpad bytes per row:
-// 0/1 bytes, or e2m1 pairs when fp4), zero past kbits and cols.
-mela_status launch_expand_t(const u64 *in, i64 ld, i64 kbits, i64 cols, i64 cols_pad, i64 kpad,
-                            unsigned char *out, bool fp4, cudaStream_t s);
-mela_status launch_expand_u8(const u64 *in, i64 ld, i64 rows, i64 kbits, i64 rows_pad, i64 kpad,
-                             unsigned char *out, cudaStream_t s);
+// Tensor-core operands, both K-major with kp bytes per row (0/1 bytes, or e2m1
+// pairs when fp4), zero past the matrices' edges: A8 (mp rows) from the packed
+// m x k matrix A, B8 (np rows, a multiple of 256) from the columns of the packed
+// k x n matrix B.  mp or np 0: that operand is left out.
+mela_status launch_expand(const u64 *A, i64 lda, i64 m, i64 mp, unsigned char *A8, const u64 *B, i64 ldb, i64 n,
+                          i64 np, unsigned char *B8, i64 k, i64 kp, bool fp4, cudaStream_t s);
 
 // ---- products (packed, device)
 // Plain AND+popcount product: C (m x n) = A (m x k) * B (k x n), with the
