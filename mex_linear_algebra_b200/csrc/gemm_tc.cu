@@ -1,7 +1,7 @@
 // gemm_tc.cu -- GF(2) product on the sm_100a tensor cores (tcgen05, kind::i8).
 //
 // Both operands are 0/1 bytes (expanded from the packed bits by
-// expand_u8_kernel), K-major: A8 is m x k, Bt8 is n x k (B transposed).  The
+// expand_kernel), K-major: A8 is m x k, Bt8 is n x k (B transposed).  The
 // tensor cores accumulate the integer dot products in 32-bit TMEM cells;
 // bit (i,j) of the GF(2) product is the low bit of the sum.  The sum is at
 // most k < 2^31, and the low bit of a 32-bit two's-complement sum is exact
@@ -15,6 +15,9 @@
 //   warps 2..5     : epilogue; each reads its 32 TMEM lanes (= 32 output
 //                    rows) x 256 columns, keeps the parity bit and writes 4
 //                    packed words per row.
+// Where the tiles leave most of the chip idle, K is split over gridDim.y: each
+// CTA multiplies its slice of the stages and XORs its parity bits into C, which
+// starts as zero.
 // Tiles are rasterised in bands of 16 tile-rows so that the CTAs resident
 // at one time share A and B tiles in L2.
 //
@@ -60,10 +63,13 @@ struct Ctl {
 template <bool F4>
 __global__ void __launch_bounds__(192, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-               u64 *__restrict__ C, i64 ldc, i64 m, i64 n, int tiles_m, int tiles_n, int kstages,
-               u32 *err)
+               u64 *__restrict__ C, i64 ldc, i64 m, i64 n, int tiles_m, int tiles_n, int all_stages,
+               int split_stages, u32 *err)
 {
     constexpr u32 TMEM_COLS = F4 ? 512 : 256;
+    // this CTA's stages of K: ks0 .. ks0 + kstages - 1
+    const int ks0 = (int)blockIdx.y * split_stages;
+    const int kstages = all_stages - ks0 < split_stages ? all_stages - ks0 : split_stages;
     extern __shared__ unsigned char smem_raw[];
     unsigned char *smem =
         reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -130,8 +136,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 if (*abort_flag) break;
                 unsigned char *sa = smem + s * STAGE_BYTES;
                 ptx::mbar_arrive_expect_tx(&ctl->full[s], STAGE_BYTES);
-                ptx::tma_load_2d(sa, &tmA, &ctl->full[s], ks * BK, tm * BM);
-                ptx::tma_load_2d(sa + A_BYTES, &tmB, &ctl->full[s], ks * BK, tn * BN);
+                ptx::tma_load_2d(sa, &tmA, &ctl->full[s], (ks0 + ks) * BK, tm * BM);
+                ptx::tma_load_2d(sa + A_BYTES, &tmB, &ctl->full[s], (ks0 + ks) * BK, tn * BN);
                 last_round[s] = round;
             }
             if (*abort_flag) {
@@ -201,7 +207,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 #pragma unroll
                 for (int q = 0; q < BN / 64; ++q) {
                     const i64 w = (i64)tn * (BN / 64) + q;
-                    if (w < nw) C[row * ldc + w] = (u64)bits[2 * q] | ((u64)bits[2 * q + 1] << 32);
+                    const u64 v = (u64)bits[2 * q] | ((u64)bits[2 * q + 1] << 32);
+                    if (w >= nw) continue;
+                    if (gridDim.y == 1)
+                        C[row * ldc + w] = v;
+                    else
+                        atomicXor(&C[row * ldc + w], v);
                 }
             }
         }
@@ -555,17 +566,24 @@ mela_status launch_gemm_tc(const unsigned char *A8, const unsigned char *Bt8, i6
     if (st != MELA_OK) return st;
     st = make_map(&mb, Bt8, np, kp, BN);
     if (st != MELA_OK) return st;
-    if (fp4) {
-        MELA_CUDA_TRY(cudaFuncSetAttribute(gemm_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           SMEM_BYTES));
-        gemm_tc_kernel<true><<<(unsigned)(tiles_m * tiles_n), 192, SMEM_BYTES, s>>>(
-            ma, mb, C, ldc, m, n, (int)tiles_m, (int)tiles_n, (int)kst, device_error_word());
+    // Slices of K: as many as fill one wave (a CTA takes an SM), each of at least
+    // 4 stages, and only past 16 stages, where the time saved (0.2 us a stage)
+    // passes the clearing of C (200 x 20000 x 300 in FP4: 12.4 us in 19 slices,
+    // 34.3 us in one).
+    i64 splits = kst >= 16 ? sm_count() / (tiles_m * tiles_n) : 1, per = kst;
+    if (splits > kst / 4) splits = kst / 4;
+    if (splits > 1) {
+        per = (kst + splits - 1) / splits;
+        splits = (kst + per - 1) / per;
+        MELA_CUDA_TRY(cudaMemset2DAsync(C, (size_t)ldc * 8, 0, (size_t)words_of(n) * 8, (size_t)m, s));
     } else {
-        MELA_CUDA_TRY(cudaFuncSetAttribute(gemm_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           SMEM_BYTES));
-        gemm_tc_kernel<false><<<(unsigned)(tiles_m * tiles_n), 192, SMEM_BYTES, s>>>(
-            ma, mb, C, ldc, m, n, (int)tiles_m, (int)tiles_n, (int)kst, device_error_word());
+        splits = 1;
     }
+    const dim3 grid((unsigned)(tiles_m * tiles_n), (unsigned)splits);
+    const auto kernel = fp4 ? gemm_tc_kernel<true> : gemm_tc_kernel<false>;
+    MELA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+    kernel<<<grid, 192, SMEM_BYTES, s>>>(ma, mb, C, ldc, m, n, (int)tiles_m, (int)tiles_n, (int)kst, (int)per,
+                                         device_error_word());
     MELA_LAUNCH_CHECK("gemm_tc_kernel");
     return MELA_OK;
 }
