@@ -201,7 +201,9 @@ def heuristic(op: str, m: int, n: int, p: int, density: float, rule: str | None 
         if m >= 1024 and n >= 1024 and p >= 1024:
             return "tc_fp4_pair" if n < (1 << 23) else "tc_pair"
         return "plain"
-    return "fused" if m * n < 8192 else "tc"
+    wc = (n + 63) // 64  # the single-CTA form holds the matrix and its tables in 192 KB
+    fits = n <= 64 * 256 and (m * (wc | 1) + 128 * wc) * 8 <= 192 * 1024
+    return "fused" if m <= 256 and fits else "tc"
 
 
 def evaluate(params: np.ndarray, records):

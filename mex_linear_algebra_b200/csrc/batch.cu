@@ -11,8 +11,8 @@
 //          (256 threads)    not fit, the CTA's L2-resident global scratch;
 //                           blocked by 64-column panels (process_big_blocked)
 //
-// (two CTAs per SM; the single-matrix fused mode runs the same engines in
-// one CTA of 512 threads with 220 KB)
+// (two CTAs per SM; the single-matrix fused mode runs the big engine in one
+// CTA of 512 threads with 220 KB)
 //
 // The host sorts the matrices into the three classes (largest first inside
 // each class); every CTA drains the big queue, then the mid queue (2 groups),
@@ -100,7 +100,7 @@ __device__ __forceinline__ int ctz64b(u64 x) { return __ffsll((long long)x) - 1;
 template <int G>
 __device__ void process_matrix(const BatchDevItem &it, const u64 *__restrict__ in, u64 *__restrict__ zt,
                                long long *ranks, int item, unsigned char *region, u64 *gmat, int gtid,
-                               int bar_id, const FusedOut *fo = nullptr)
+                               int bar_id)
 {
     const int m = it.m, n = it.n, wc = (n + 63) >> 6, mn = m < n ? m : n;
     const bool in_smem = it.flags & 1;
@@ -165,20 +165,6 @@ __device__ void process_matrix(const BatchDevItem &it, const u64 *__restrict__ i
         }
         search(c + 1);
         group_sync(G, bar_id);
-    }
-    if (fo) {
-        // single-matrix mode: RREF rows back to the caller, pivot lists, rank
-        for (long long e = gtid; e < (long long)m * wc; e += G) {
-            const int rr = (int)(e / wc), x = (int)(e - (long long)rr * wc);
-            fo->M[(long long)rr * fo->ldm + x] = A[(size_t)rr * ld + x];
-        }
-        for (int t = gtid; t < r; t += G) {
-            fo->piv[t] = piv[t];
-            fo->prow[t] = prow[t];
-        }
-        if (gtid == 0) *fo->rank = r;
-        group_sync(G, bar_id);
-        return;
     }
     if (gtid == 0) ranks[item] = r;
 
@@ -1418,18 +1404,15 @@ __global__ void __launch_bounds__(256) batch_unpack_kernel(const BatchDevItem *_
 }
 
 // ---------------------------------------------------------------- single matrix
-// RREF of one matrix by one CTA in one launch: in shared memory by the
-// column-by-column engine when it fits, else by the blocked engine over
-// global scratch.  Reads the packed matrix M (row pitch ldm, any pitch >=
-// ceil(n/64)) and writes the RREF rows back over it.
+// RREF of one matrix too large for shared memory (elim_small.cu) by one CTA in
+// one launch: the blocked engine over global scratch.  Reads the packed matrix
+// from a compact copy and writes the RREF rows over the caller's matrix (row
+// pitch ldm, any pitch >= ceil(n/64)).
 __global__ void __launch_bounds__(kThreads, 1)
 fused_elim_kernel(BatchDevItem it, const u64 *__restrict__ in_compact, FusedOut fo, u64 *scratch)
 {
     extern __shared__ __align__(16) unsigned char smem[];
-    if (it.flags & 1)
-        process_matrix<kThreads>(it, in_compact, nullptr, nullptr, 0, smem, nullptr, threadIdx.x, 0, &fo);
-    else
-        process_big_blocked<kThreads, kSmemTotal>(it, in_compact, nullptr, nullptr, 0, smem, scratch, &fo);
+    process_big_blocked<kThreads, kSmemTotal>(it, in_compact, nullptr, nullptr, 0, smem, scratch, &fo);
 }
 
 size_t fused_workspace(i64 m, i64 n)
@@ -1451,6 +1434,7 @@ mela_status launch_fused_elim(u64 *M, i64 ld, i64 m, i64 n, long long *d_rank, l
         set_error("fused elimination workspace of %zu bytes needed, %zu given", need, ws_bytes);
         return MELA_ERR_INVALID;
     }
+    if (small_elim_fits(m, n)) return launch_small_elim(M, ld, m, n, d_rank, d_piv, d_prow, s);
     const i64 wc = words_of(n);
     u64 *compact = (u64 *)ws;
     u64 *scratch = compact + m * wc;
@@ -1461,9 +1445,6 @@ mela_status launch_fused_elim(u64 *M, i64 ld, i64 m, i64 n, long long *d_rank, l
     it.n = (int)n;
     it.in_off = 0;
     it.z_off = 0;
-    const size_t aux = aux_bytes((int)m, (int)n);
-    const size_t mat = (size_t)m * smem_ld((int)n) * 8;
-    it.flags = (aux + mat <= (size_t)kSmemTotal) ? 1 : 0;
     FusedOut fo{M, ld, d_rank, d_piv, d_prow};
     MELA_CUDA_TRY(cudaFuncSetAttribute(fused_elim_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        kSmemTotal));

@@ -330,8 +330,9 @@ int32_t resolve_elim_variant(int32_t variant, const u64 *M, i64 ld, i64 m, i64 n
 
 int32_t fixed_elim_variant(i64 m, i64 n)
 {
-    // one CTA for small matrices, tensor-core windows otherwise
-    return (double)m * (double)n < 8192.0 ? MELA_ELIM_FUSED : MELA_ELIM_TC;
+    // one CTA in shared memory for small matrices, tensor-core windows
+    // otherwise (256 x 512 36 us against 43, 400 x 800 92 against 80)
+    return m <= 256 && small_elim_fits(m, n) ? MELA_ELIM_FUSED : MELA_ELIM_TC;
 }
 
 }  // namespace mela

@@ -53,7 +53,12 @@ mela_status make_u64_rows_map(CUtensorMap *map, const u64 *base, i64 rows, i64 w
 mela_status launch_gemm_m4ri(const u64 *A, i64 lda, const u64 *B, i64 ldb, u64 *C, i64 ldc,
                              i64 m, i64 k, i64 n, cudaStream_t s, int tile = 0);
 
-// Whole RREF of one matrix in one single-CTA launch (batch.cu).
+// Whole RREF of one matrix by one CTA in one launch: in shared memory where it
+// fits (elim_small.cu: up to 512 rows, 192 KB with its tables), else by the
+// batch engine for big matrices over the workspace (batch.cu).
+bool small_elim_fits(i64 m, i64 n);
+mela_status launch_small_elim(u64 *M, i64 ld, i64 m, i64 n, long long *d_rank, long long *d_piv,
+                              long long *d_prow, cudaStream_t s);
 size_t fused_workspace(i64 m, i64 n);
 mela_status launch_fused_elim(u64 *M, i64 ld, i64 m, i64 n, long long *d_rank, long long *d_piv,
                               long long *d_prow, void *ws, size_t ws_bytes, cudaStream_t s);

@@ -2,7 +2,7 @@
 32-column half words and 64 candidate rows a round in both forms, 320 rows a
 chunk and 256 columns a window on the tensor cores, 512 rows a chunk and 64
 columns a panel in the Four-Russians form (whose update tiles change from 1024
-to 256 rows).  Bit-exact against the oracle (rank, pivot columns, RREF rows,
+to 256 rows), 1 to 16 lanes a row and up to 512 rows in the single-CTA form.  Bit-exact against the oracle (rank, pivot columns, RREF rows,
 null basis)."""
 import numpy as np
 import pytest
@@ -39,7 +39,10 @@ def low_rank(m, n, seed):
 @pytest.mark.parametrize("make", [repeated, late_pivots, low_rank])
 @pytest.mark.parametrize("form,m,n", [("tc", 31, 33), ("tc", 65, 64), ("tc", 319, 255), ("tc", 321, 257),
                                       ("tc", 641, 545), ("tc", 900, 288), ("m4ri", 33, 31), ("m4ri", 511, 65),
-                                      ("m4ri", 513, 96), ("m4ri", 1100, 161), ("m4ri", 300, 20000)])
+                                      ("m4ri", 513, 96), ("m4ri", 1100, 161), ("m4ri", 300, 20000),
+                                      ("fused", 1, 1), ("fused", 33, 31), ("fused", 65, 129), ("fused", 100, 255),
+                                      ("fused", 130, 513), ("fused", 511, 320), ("fused", 512, 2047),
+                                      ("fused", 513, 65), ("fused", 90, 7000), ("fused", 200, 8000)])
 def test_pivot_search_edges(cuda, make, form, m, n):
     check_all(make(m, n, 1000 * m + n), m, n, form)
 
