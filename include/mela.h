@@ -78,7 +78,8 @@ typedef enum {
 typedef enum {
     MELA_ELIM_AUTO = 0,
     MELA_ELIM_PLAIN = 1,  /* per-pivot warp-ballot search + broadcast-XOR sweep */
-    MELA_ELIM_M4RI = 2,   /* 64-column panels, Four-Russians tables in shared memory (k = 8 unless tuned) */
+    MELA_ELIM_M4RI = 2,   /* Four-Russians tables in shared memory: 256-column windows with 4-bit tables, or
+                             64-column panels when a tuning field names k or the tile (k = 8 by default) */
     MELA_ELIM_M4RI_K4 = 3, /* the same panels with 4-bit tables (M4RI k = 4) */
     MELA_ELIM_FUSED = 4,   /* the whole elimination by one CTA in one launch */
     MELA_ELIM_TC = 5       /* 256-column windows, trailing update on the tensor cores (tcgen05 kind::i8) */

@@ -735,7 +735,10 @@ mela_status elim_device(int variant_arg, u64 *M, i64 ld, i64 m, i64 n, int rref,
     }
     if (variant == MELA_ELIM_FUSED)
         return launch_fused_elim(M, ld, m, n, d_rank, d_piv, d_prow, ws, ws_bytes, s);
-    if (variant == MELA_ELIM_TC) return elim_tc_device(M, ld, m, n, rref, d_rank, d_piv, d_prow, ws, ws_bytes, s);
+    // the Four-Russians form without tuning fields also goes by windows
+    const bool tables = variant_arg == MELA_ELIM_M4RI;
+    if (variant == MELA_ELIM_TC || tables)
+        return elim_windows_device(M, ld, m, n, rref, tables, d_rank, d_piv, d_prow, ws, ws_bytes, s);
     ElimLayout L = elim_layout(m, n);
     if (ws_bytes < L.total || !ws) {
         set_error("elimination workspace of %zu bytes needed, %zu given", elim_workspace(m, n), ws_bytes);

@@ -1,5 +1,6 @@
-// elim_tc.cu -- blocked GF(2) elimination whose trailing (Schur) update runs
-// on the sm_100a tensor cores.
+// elim_tc.cu -- blocked GF(2) elimination by 256-column windows, the trailing
+// (Schur) update on the sm_100a tensor cores or, in the Four-Russians form, by
+// tables on the CUDA cores.
 //
 // Results are those of the other forms (elim.cu): the rank of
 // bitrank_packed / rank_m4ri (src/mela_rank_gf2.c:27-121,
@@ -548,7 +549,8 @@ __device__ __forceinline__ u32 near_lookup(const uint4 (&t)[2][16][64], u32 nib,
 // pivot columns give z = sum_b y_b tag[b], the combination of the original
 // pivot rows, and the words change by sum_j z_j A[P_j] -- 64 table reads each,
 // without waiting for the reduced rows R.  Rows with y != 0 get a slot of
-// ulist and their coefficients as 0/1 bytes in X8; live says whether the
+// ulist and their coefficients in X8 (256 0/1 bytes, or the 32 bytes of y as
+// they are, for table_update); live says whether the
 // row's words of the next window are nonzero (the update adds the others).
 // Latency-bound: about 2 us of table building and dependent loads, then
 // 1000 cycles per 32 rows.  It takes the place, on the critical path, of the
@@ -556,7 +558,7 @@ __device__ __forceinline__ u32 near_lookup(const uint4 (&t)[2][16][64], u32 nib,
 // rank of 3000 x 5000 (rank 2200) 422 against 516 us, 8192 x 8192 1.22 ms.
 __global__ void __launch_bounds__(256)
 window_near_kernel(u64 *__restrict__ M, i64 ld, i64 m, i64 wc, i64 w, const int *__restrict__ list, const int *stamp,
-                   int wid, int rref, WinState *ws, int *ulist, unsigned char *X8, unsigned char *live)
+                   int wid, int rref, WinState *ws, int *ulist, unsigned char *X8, int bytes, unsigned char *live)
 {
     extern __shared__ __align__(16) unsigned char nr_raw[];
     NrSmem &S = *reinterpret_cast<NrSmem *>(nr_raw);
@@ -627,9 +629,13 @@ window_near_kernel(u64 *__restrict__ M, i64 ld, i64 m, i64 wc, i64 w, const int 
 #pragma unroll
             for (int q = 0; q < 8; ++q) slot += q < warp ? S.cnt[q] : 0;
             if (s == 0) ulist[slot] = (int)row;
-            uint4 *dst = reinterpret_cast<uint4 *>(X8 + (size_t)slot * WBITS + 32 * s);
-            dst[0] = make_uint4(nib_bytes(y), nib_bytes(y >> 4), nib_bytes(y >> 8), nib_bytes(y >> 12));
-            dst[1] = make_uint4(nib_bytes(y >> 16), nib_bytes(y >> 20), nib_bytes(y >> 24), nib_bytes(y >> 28));
+            if (bytes) {
+                uint4 *dst = reinterpret_cast<uint4 *>(X8 + (size_t)slot * WBITS + 32 * s);
+                dst[0] = make_uint4(nib_bytes(y), nib_bytes(y >> 4), nib_bytes(y >> 8), nib_bytes(y >> 12));
+                dst[1] = make_uint4(nib_bytes(y >> 16), nib_bytes(y >> 20), nib_bytes(y >> 24), nib_bytes(y >> 28));
+            } else {
+                reinterpret_cast<u32 *>(X8)[(size_t)slot * 8 + s] = y;
+            }
         }
         __syncthreads();  // cnt and base are read before the next rows write them
     }
@@ -992,6 +998,81 @@ tc_update_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
     }
 }
 
+// ---------------------------------------------------------------- table_update
+// The update of the words that window_near leaves, on the CUDA cores (the
+// Four-Russians form): strip q is words w + 4q .. w + 4q + 3.  A CTA builds the
+// 4-bit tables of the reduced rows' words of its strip (32 KB) and takes every
+// gridDim.y-th group of 32 listed rows, 8 lanes a row and a half word each as
+// in window_near: 64 conflict-free table reads a row.  For the RREF the CTAs of
+// the first row group also write the reduced rows over the pivot rows, in
+// strip `skip` (whose listed rows window_near has done) nothing else.
+// Bound by the shared-memory reads, 4 cycles a row word and SM, where the
+// matrix is large; up to 4096 x 8192 it hides behind the next factorization
+// and costs the window fewer launches than the tensor cores (rank of 2048 x
+// 4096, rank 1800: 308 us, 331 on the tensor cores, 1074 in 64-column panels;
+// 16384 x 32768, rank 12000: 7.8, 5.5 and 27.9 ms).
+namespace {
+struct TuSmem {
+    uint4 t[2][16][64];
+};
+}  // namespace
+
+__global__ void __launch_bounds__(256)
+table_update_kernel(u64 *__restrict__ M, i64 ld, i64 wc, i64 w, const WinState *ws, const u64 *__restrict__ Rbuf,
+                    i64 ldr, const int *__restrict__ ulist, const u32 *__restrict__ Y, unsigned char *live,
+                    int strip_lo, int skip, int rref)
+{
+    extern __shared__ __align__(16) unsigned char tu_raw[];
+    TuSmem &S = *reinterpret_cast<TuSmem *>(tu_raw);
+    if (ws->rt == 0) return;
+    const int nu = ws->nu;
+    const int strip = strip_lo + (int)blockIdx.x;
+    if (strip == skip && blockIdx.y > 0) return;
+    const i64 w0 = 4 * (i64)strip;            // from the window's first word
+    const int tid = threadIdx.x, lane = tid & 31, s = lane & 7;
+    const int nwords = wc - w - w0 < 4 ? (int)(wc - w - w0) : 4;
+    if (tid < 128) {
+        const int half = tid >> 6, g = tid & 63;
+        uint4 v[4];
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const u64 *src = Rbuf + (i64)(4 * g + b) * ldr + w0 + 2 * half;
+            const u64 x0 = 2 * half < nwords ? src[0] : 0ull, x1 = 2 * half + 1 < nwords ? src[1] : 0ull;
+            v[b] = make_uint4((u32)x0, (u32)(x0 >> 32), (u32)x1, (u32)(x1 >> 32));
+        }
+        uint4 a = make_uint4(0, 0, 0, 0);
+        S.t[half][0][g] = a;
+#pragma unroll
+        for (int i = 1; i < 16; ++i) {
+            a = xor4u(a, v[(i & 1) ? 0 : (i & 2) ? 1 : (i & 4) ? 2 : 3]);
+            S.t[half][i ^ (i >> 1)][g] = a;
+        }
+    }
+    __syncthreads();
+    const bool in = (s >> 1) < nwords;
+    if (rref && blockIdx.y == 0) {
+        for (int b = tid >> 3; b < WBITS; b += 32) {
+            const int pr = ws->prow[b];
+            if (pr >= 0 && in)
+                reinterpret_cast<u32 *>(M + (i64)pr * ld + w + w0)[s] =
+                    reinterpret_cast<const u32 *>(Rbuf + (i64)b * ldr + w0)[s];
+        }
+    }
+    if (strip == skip) return;  // its listed rows are up to date (window_near)
+    for (int i0 = 32 * (int)blockIdx.y; i0 < nu; i0 += 32 * (int)gridDim.y) {
+        const int slot = i0 + (tid >> 3);
+        const bool ok = slot < nu;
+        const int row = ok ? ulist[slot] : 0;
+        const u32 y = ok ? Y[(size_t)slot * 8 + s] : 0u;
+        u32 *p = reinterpret_cast<u32 *>(M + (i64)row * ld + w + w0) + s;
+        u32 v = ok && in ? *p : 0u;
+        v ^= near_lookup(S.t, gather_nibbles(y, lane), lane);
+        if (ok && in) *p = v;
+        const unsigned vl = __ballot_sync(0xffffffffu, ok && in && v != 0);
+        if (ok && s == 0 && ((vl >> (lane & 24)) & 0xffu)) live[row] = 1;
+    }
+}
+
 // ---------------------------------------------------------------- host side
 static size_t al256(size_t x) { return (x + 255) & ~(size_t)255; }
 
@@ -1120,8 +1201,8 @@ void elim_graph_store(const ElimGraphKey &k, cudaGraphExec_t exec)
 }
 }  // namespace
 
-mela_status elim_tc_device(u64 *M, i64 ld, i64 m, i64 n, int rref, long long *d_rank, long long *d_piv,
-                           long long *d_prow, void *wsp, size_t ws_bytes, cudaStream_t s)
+mela_status elim_windows_device(u64 *M, i64 ld, i64 m, i64 n, int rref, bool tables, long long *d_rank,
+                                long long *d_piv, long long *d_prow, void *wsp, size_t ws_bytes, cudaStream_t s)
 {
     const TcLayout L = tc_layout(m, n);
     if (!wsp || ws_bytes < L.total) {
@@ -1159,6 +1240,8 @@ mela_status elim_tc_device(u64 *M, i64 ld, i64 m, i64 n, int rref, long long *d_
     const int cb_smem = (int)sizeof(CbSmem);
     MELA_CUDA_TRY(cudaFuncSetAttribute(window_combine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, cb_smem));
     const int sms = sm_count();
+    const int tu_smem = (int)sizeof(TuSmem);
+    MELA_CUDA_TRY(cudaFuncSetAttribute(table_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tu_smem));
     const int nr_smem = (int)sizeof(NrSmem);
     MELA_CUDA_TRY(cudaFuncSetAttribute(window_near_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, nr_smem));
     const int near_blocks = (int)std::min<i64>((m + 31) / 32, 2 * sms);
@@ -1198,19 +1281,27 @@ mela_status elim_tc_device(u64 *M, i64 ld, i64 m, i64 n, int rref, long long *d_
                 forked = false;
             }
             window_near_kernel<<<near_blocks, 256, nr_smem, sx>>>(M, ld, m, wc, w, list, stamp, wid, rref, cur, ulist,
-                                                                 X8, live);
+                                                                 X8, tables ? 0 : 1, live);
             MELA_CUDA_TRY(cudaEventRecord(ev_fork, sx));
             MELA_CUDA_TRY(cudaStreamWaitEvent(s2, ev_fork, 0));
             window_combine_kernel<<<(unsigned)((lw + CB_W - 1) / CB_W), 256, cb_smem, s2>>>(M, ld, wc, w, cur, Rbuf,
                                                                                            wc);
-            window_rt_kernel<<<(unsigned)lw, 256, 0, s2>>>(M, ld, w, Rbuf, wc, cur, Rt8);
+            if (!tables) window_rt_kernel<<<(unsigned)lw, 256, 0, s2>>>(M, ld, w, Rbuf, wc, cur, Rt8);
             // strips 2.. and, for the RREF, strip 0 (the window's own columns;
             // for the rank every updated row is in the window basis' span and
             // its window part becomes zero)
             const i64 strips = (lw + 3) / 4;
             const int far_lo = rref ? 0 : 2, far_skip = (rref && strips >= 2) ? 1 : -1;
             const i64 far_strips = (strips > far_lo ? strips - far_lo : 0) - (far_skip >= 0 ? 1 : 0);
-            if (far_strips > 0) {
+            if (tables) {
+                const i64 all = strips > far_lo ? strips - far_lo : 0;
+                if (all > 0) {
+                    const i64 groups = (m + 31) / 32, want = (4 * sms + all - 1) / all;
+                    table_update_kernel<<<dim3((unsigned)all, (unsigned)(groups < want ? groups : want)), 256, tu_smem,
+                                          s2>>>(M, ld, wc, w, cur, Rbuf, wc, ulist, (const u32 *)X8, live, far_lo,
+                                                far_skip, rref);
+                }
+            } else if (far_strips > 0) {
                 const i64 units = far_strips * chunks_max;
                 const int cap = sms > 4 ? sms - 2 : sms;  // SMs left for the next factorization
                 const int grid_far = (int)(units < cap ? units : cap);
@@ -1242,7 +1333,7 @@ mela_status elim_tc_device(u64 *M, i64 ld, i64 m, i64 n, int rref, long long *d_
     key.v[0] = ld;
     key.v[1] = m;
     key.v[2] = n;
-    key.v[3] = rref;
+    key.v[3] = rref + (tables ? 2 : 0);
     cudaGraphExec_t exec = elim_graph_lookup(key);
     cudaStream_t cap = nullptr;
     if (exec) {

@@ -1,8 +1,8 @@
 """Pivot search of the blocked eliminations at the edges of its blocking:
-32-column half words and 64 candidate rows a round in both forms, 320 rows a
-chunk and 256 columns a window on the tensor cores, 512 rows a chunk and 64
-columns a panel in the Four-Russians form (whose update tiles change from 1024
-to 256 rows), 1 to 16 lanes a row and up to 512 rows in the single-CTA form.  Bit-exact against the oracle (rank, pivot columns, RREF rows,
+32-column half words and 64 candidate rows a round in every form, 320 rows a
+chunk and 256 columns a window in the forms by windows (tensor cores and
+Four-Russians tables), 512 rows a chunk and 64 columns a panel in the tuned
+Four-Russians form (whose update tiles change from 1024 to 256 rows), 1 to 16 lanes a row and up to 512 rows in the single-CTA form.  Bit-exact against the oracle (rank, pivot columns, RREF rows,
 null basis)."""
 import numpy as np
 import pytest
@@ -38,8 +38,9 @@ def low_rank(m, n, seed):
 
 @pytest.mark.parametrize("make", [repeated, late_pivots, low_rank])
 @pytest.mark.parametrize("form,m,n", [("tc", 31, 33), ("tc", 65, 64), ("tc", 319, 255), ("tc", 321, 257),
-                                      ("tc", 641, 545), ("tc", 900, 288), ("m4ri", 33, 31), ("m4ri", 511, 65),
-                                      ("m4ri", 513, 96), ("m4ri", 1100, 161), ("m4ri", 300, 20000),
+                                      ("tc", 641, 545), ("tc", 900, 288), ("m4ri_k8", 33, 31), ("m4ri_k8", 511, 65),
+                                      ("m4ri_k8", 513, 96), ("m4ri_k8", 1100, 161), ("m4ri_k8", 300, 20000),
+                                      ("m4ri", 65, 64), ("m4ri", 321, 257), ("m4ri", 641, 545), ("m4ri", 900, 288),
                                       ("fused", 1, 1), ("fused", 33, 31), ("fused", 65, 129), ("fused", 100, 255),
                                       ("fused", 130, 513), ("fused", 511, 320), ("fused", 512, 2047),
                                       ("fused", 513, 65), ("fused", 90, 7000), ("fused", 200, 8000)])
@@ -47,8 +48,9 @@ def test_pivot_search_edges(cuda, make, form, m, n):
     check_all(make(m, n, 1000 * m + n), m, n, form)
 
 
+@pytest.mark.parametrize("form", ["tc", "m4ri"])
 @pytest.mark.parametrize("m,n", [(33, 513), (70, 700), (300, 1100)])
-def test_rows_that_leave_the_list(cuda, m, n):
+def test_rows_that_leave_the_list(cuda, form, m, n):
     """Zero rows, rows that become zero in the first window and rows whose first
     ones come two windows later: the lists, flags and coefficient slots of the
     later windows, up to windows with no row left."""
@@ -56,15 +58,16 @@ def test_rows_that_leave_the_list(cuda, m, n):
     P[::5] = 0
     P[1::5] = P[min(2, m - 1)]
     P[3::5, : (n // 64) // 2] = 0
-    check_all(P, m, n, "tc")
+    check_all(P, m, n, form)
     P[:, 4:] = 0  # no pivots past the first window
-    check_all(P, m, n, "tc")
+    check_all(P, m, n, form)
 
 
+@pytest.mark.parametrize("form", ["tc", "m4ri"])
 @pytest.mark.parametrize("m,n", [(300, 5000), (1400, 1500), (129, 4161)])
-def test_update_tiles(cuda, m, n):
-    """The tensor-core update over one, a few and many row tiles per strip:
+def test_update_tiles(cuda, form, m, n):
+    """The update of the far columns over one, a few and many row tiles per strip:
     fewer tiles than epilogue groups, strips split between CTAs, a last strip of
     one word."""
     P = gen.dense_packed(m, 0, m, n)
-    check_all(P, m, n, "tc")
+    check_all(P, m, n, form)
