@@ -61,7 +61,12 @@ namespace {
 constexpr int WW = 4;         // words per window
 constexpr int WBITS = 256;    // columns per window
 constexpr int WF_ROWS = 320;     // a chunk of rows; 320 random rows span 256 columns but with probability 2^-64
-constexpr int WF_THREADS = WF_ROWS + 32;  // a thread per row and the selecting warp
+// Warps 3, 7, 11 share one scheduler: warp 3 selects, the other two only help
+// with the tables; the rest hold the rows, a thread each.
+constexpr int WF_WARPS = WF_ROWS / 32 + 3;
+constexpr int WF_THREADS = 32 * WF_WARPS;
+constexpr int WF_SELECTOR = 3;
+static_assert(WF_ROWS == 320, "ten row warps on three schedulers");
 
 // Everything that belongs to a pivot of a window is indexed by its column in
 // the window (0..255), so the coefficient of a row is its window part masked
@@ -196,8 +201,11 @@ window_factor_kernel(const u64 *__restrict__ M, i64 ld, i64 m, i64 n, i64 w, int
 {
     extern __shared__ __align__(16) unsigned char wf_raw[];
     WfSmem &S = *reinterpret_cast<WfSmem *>(wf_raw);
-    constexpr int NW = WF_THREADS / 32;
+    constexpr int NW = WF_ROWS / 32;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const bool holds = (warp & 3) != 3;            // this warp holds rows:
+    const int rw = holds ? warp - (warp >> 2) : NW;  // 32 rw .. of the chunk
+    const int ri = 32 * rw + lane;
     const i64 wc = words_of(n);
     const int wn = (wc - w) < WW ? (int)(wc - w) : WW;
     const i64 vb = n - 64 * w;
@@ -222,7 +230,7 @@ window_factor_kernel(const u64 *__restrict__ M, i64 ld, i64 m, i64 n, i64 w, int
         u32 H0[8];
 #pragma unroll
         for (int q = 0; q < 8; ++q) H0[q] = H[q];
-        const bool obasis = older && tid < WBITS && ((sel8(H0, (tid >> 5) & 7) >> (tid & 31)) & 1);
+        const bool obasis = older && holds && ri < WBITS && ((sel8(H0, (ri >> 5) & 7) >> (ri & 31)) & 1);
         if (older) {
             // tables of the 16 combinations of basis vectors 4g..4g+3
             for (int e = tid; e < 2 * 64 * 16; e += WF_THREADS) {
@@ -236,10 +244,10 @@ window_factor_kernel(const u64 *__restrict__ M, i64 ld, i64 m, i64 n, i64 w, int
             }
             __syncthreads();
         }
-        const int k = base + tid;
+        const int k = base + ri;
         int row = -1;
         u32 v[8] = {};
-        if (tid < WF_ROWS && k < na) {
+        if (holds && k < na) {
             row = L0[k];
 #pragma unroll
             for (int q = 0; q < WW; ++q)
@@ -269,48 +277,50 @@ window_factor_kernel(const u64 *__restrict__ M, i64 ld, i64 m, i64 n, i64 w, int
         int h = 0;
         u32 C = 0, z = 0;
         auto take_in = [&]() {
-            if (!pend) return;
             if (z) wf_apply(S, v, h, C, z);
             if (obasis) {
-                const uint4 a = S.basis[tid][0], b = S.basis[tid][1];
+                const uint4 a = S.basis[ri][0], b = S.basis[ri][1];
                 u32 o[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
                 const u32 y = sel8(o, h) & C;
                 if (y) {
                     wf_apply(S, o, h, C, half_word_times_T(S.r, y));
-                    S.basis[tid][0] = make_uint4(o[0], o[1], o[2], o[3]);
-                    S.basis[tid][1] = make_uint4(o[4], o[5], o[6], o[7]);
+                    S.basis[ri][0] = make_uint4(o[0], o[1], o[2], o[3]);
+                    S.basis[ri][1] = make_uint4(o[4], o[5], o[6], o[7]);
                 }
             }
-            pend = false;
         };
         while (h < 8 && nb < valid) {
             int ht = h;  // the half word of the next round
             if (pend && sel8(H, h) == 0xffffffffu && ++ht == 8) break;
             const u32 Ht = sel8(H, ht);
-            const u32 x = pend ? wf_half(S, v, h, ht, C, z) : sel8(v, ht);
-            const u32 d = mycol < 0 ? x & ~Ht : 0u;
-            const unsigned bal = __ballot_sync(0xffffffffu, d != 0);
+            u32 d = 0;
+            unsigned bal = 0;
             par ^= 1;
-            if (lane == 0) S.wcnt[par][warp] = __popc(bal);
+            if (holds) {
+                if (mycol < 0) d = (pend ? wf_half(S, v, h, ht, C, z) : sel8(v, ht)) & ~Ht;
+                bal = __ballot_sync(0xffffffffu, d != 0);
+                if (lane == 0) S.wcnt[par][rw] = __popc(bal);
+            }
             __syncthreads();
             const int wv = lane < NW ? S.wcnt[par][lane] : 0;
             const int total = __reduce_add_sync(0xffffffffu, wv);
             if (total == 0) {  // no unused row has data left in half word ht
-                take_in();
+                if (pend && holds) take_in();
+                pend = false;
                 h = ht + 1;
                 continue;
             }
-            int idx = __reduce_add_sync(0xffffffffu, lane < warp ? wv : 0) + __popc(bal & ((1u << lane) - 1));
+            int idx = __reduce_add_sync(0xffffffffu, lane < rw ? wv : 0) + __popc(bal & ((1u << lane) - 1));
             if (d == 0 || idx >= kHalfCand) idx = -1;
             if (idx >= 0) {
                 S.r.cand[idx] = d;
                 S.r.pcol[idx] = -1;
             }
             __syncthreads();
-            if (warp == NW - 1) {
+            if (warp == WF_SELECTOR) {
                 half_word_select(S.r, total < kHalfCand ? total : kHalfCand);
-            } else {
-                take_in();
+            } else if (holds) {
+                if (pend) take_in();
                 if (idx >= 0) {
                     S.cv[idx][0] = make_uint4(v[0], v[1], v[2], v[3]);
                     S.cv[idx][1] = make_uint4(v[4], v[5], v[6], v[7]);
@@ -320,8 +330,8 @@ window_factor_kernel(const u64 *__restrict__ M, i64 ld, i64 m, i64 n, i64 w, int
             C = S.r.C;
             // tables over the round's pivots: their original rows (without
             // the bits at C) and the rows of T
-            if (tid < 256) {
-                const int half = tid >> 7, g = (tid >> 4) & 7, e = tid & 15;
+            if (holds && ri < 256) {
+                const int half = ri >> 7, g = (ri >> 4) & 7, e = ri & 15;
                 uint4 a = make_uint4(0, 0, 0, 0);
 #pragma unroll
                 for (int b = 0; b < 4; ++b) {
@@ -337,7 +347,8 @@ window_factor_kernel(const u64 *__restrict__ M, i64 ld, i64 m, i64 n, i64 w, int
                 }
                 S.vt[half][g][e] = a;
             }
-            for (int e = WF_THREADS - 1 - tid; e < 128; e += WF_THREADS) half_word_tt(S.r, e);
+            if (!holds)
+                for (int e = 32 * (warp >> 2) + lane; e < 128; e += 96) half_word_tt(S.r, e);
             const int pc = idx >= 0 ? S.r.pcol[idx] : -1;
             __syncthreads();
             if (pc >= 0) {
@@ -347,7 +358,7 @@ window_factor_kernel(const u64 *__restrict__ M, i64 ld, i64 m, i64 n, i64 w, int
                 for (int q = 0; q < 8; ++q) v[q] = 0;
                 z = S.r.T[pc];
             } else {
-                const u32 y = x & C;
+                const u32 y = sel8(v, ht) & C;
                 z = y ? half_word_times_T(S.r, y) : 0u;
             }
             pend = true;
@@ -356,7 +367,7 @@ window_factor_kernel(const u64 *__restrict__ M, i64 ld, i64 m, i64 n, i64 w, int
 #pragma unroll
             for (int q = 0; q < 8; ++q) H[q] |= q == ht ? C : 0u;
         }
-        take_in();
+        if (pend && holds) take_in();
         if (mycol >= 0) {
             S.basis[mycol][0] = make_uint4(v[0], v[1], v[2], v[3]);
             S.basis[mycol][1] = make_uint4(v[4], v[5], v[6], v[7]);
