@@ -82,7 +82,8 @@ typedef enum {
                              64-column panels when a tuning field names k or the tile (k = 8 by default) */
     MELA_ELIM_M4RI_K4 = 3, /* the same panels with 4-bit tables (M4RI k = 4) */
     MELA_ELIM_FUSED = 4,   /* the whole elimination by one CTA in one launch */
-    MELA_ELIM_TC = 5       /* 256-column windows, trailing update on the tensor cores (tcgen05 kind::i8) */
+    MELA_ELIM_TC = 5       /* 256-column windows, trailing update on the tensor cores (tcgen05 kind::i8);
+                              where AUTO picks it for a small matrix the update goes by tables */
 } mela_elim_variant;
 
 /* Tuning fields of a variant argument.  A variant argument is a base

@@ -719,6 +719,7 @@ mela_status elim_device(int variant_arg, u64 *M, i64 ld, i64 m, i64 n, int rref,
                         cudaStream_t s)
 {
     Tuning tune{};
+    const bool chosen = MELA_VARIANT_BASE(variant_arg) == MELA_ELIM_AUTO;
     if (m > 0 && n > 0) variant_arg = resolve_elim_variant(variant_arg, M, ld, m, n, rref, s);
     if (!decode_elim_variant(variant_arg, &tune)) {
         set_error("elimination: bad variant argument 0x%x", variant_arg);
@@ -735,8 +736,13 @@ mela_status elim_device(int variant_arg, u64 *M, i64 ld, i64 m, i64 n, int rref,
     }
     if (variant == MELA_ELIM_FUSED)
         return launch_fused_elim(M, ld, m, n, d_rank, d_piv, d_prow, ws, ws_bytes, s);
-    // the Four-Russians form without tuning fields also goes by windows
-    const bool tables = variant_arg == MELA_ELIM_M4RI;
+    // The Four-Russians form without tuning fields also goes by windows.  Where
+    // AUTO picks the windows it leaves the update to the tables up to 40M cells:
+    // there the update hides behind the factorization either way, and the
+    // tables take fewer and shorter launches (rank 3000 x 5000 372 us, 409 on
+    // the tensor cores; RREF 4096 x 8192 603 / 656, 8192 x 8192 1230 / 1183).
+    const bool tables = variant_arg == MELA_ELIM_M4RI ||
+                        (chosen && variant == MELA_ELIM_TC && (double)m * (double)n <= 4e7);
     if (variant == MELA_ELIM_TC || tables)
         return elim_windows_device(M, ld, m, n, rref, tables, d_rank, d_piv, d_prow, ws, ws_bytes, s);
     ElimLayout L = elim_layout(m, n);
