@@ -42,11 +42,10 @@ __device__ __forceinline__ void half_word_select(HalfRound &S, int ncand)
     u32 hi = transpose32_warp(lane + 32 < ncand ? S.cand[lane + 32] : 0u);
     u32 ulo = ~0u, uhi = ~0u;    // unused rows
     u32 mlo = 0, mhi = 0;        // this column's pivot row
-    u32 xlo = __shfl_sync(0xffffffffu, lo, 0), xhi = __shfl_sync(0xffffffffu, hi, 0);
-#pragma unroll
-    for (int c = 0; c < 32; ++c) {
-        const u32 nlo = __shfl_sync(0xffffffffu, lo, (c + 1) & 31);
-        const u32 nhi = __shfl_sync(0xffffffffu, hi, (c + 1) & 31);
+    u32 xlo, xhi;                // the step's column
+    auto step = [&](int c, int next) {
+        const u32 nlo = __shfl_sync(0xffffffffu, lo, next);
+        const u32 nhi = __shfl_sync(0xffffffffu, hi, next);
         const u32 alo = xlo & ulo, ahi = xhi & uhi;
         const u32 plo = alo & (0u - alo), phi = alo ? 0u : ahi & (0u - ahi);
         const u32 rlo = xlo ^ plo, rhi = xhi ^ phi;
@@ -61,7 +60,11 @@ __device__ __forceinline__ void half_word_select(HalfRound &S, int ncand)
         const bool nhit = ((nlo & plo) | (nhi & phi)) != 0;
         xlo = nhit ? nlo ^ rlo : nlo;
         xhi = nhit ? nhi ^ rhi : nhi;
-    }
+    };
+    xlo = __shfl_sync(0xffffffffu, lo, 0);
+    xhi = __shfl_sync(0xffffffffu, hi, 0);
+#pragma unroll
+    for (int c = 0; c < 32; ++c) step(c, (c + 1) & 31);
     const u32 C = __ballot_sync(0xffffffffu, (mlo | mhi) != 0);
     const u32 wlo = transpose32_warp(lo), whi = transpose32_warp(hi);
     const int ci = mlo ? __ffs(mlo) - 1 : mhi ? 31 + __ffs(mhi) : -1;

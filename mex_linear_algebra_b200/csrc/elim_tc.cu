@@ -10,7 +10,7 @@
 //
 // One window of 256 columns (4 words) at a time:
 //   window_factor   one CTA.  Walks the list of active rows in chunks of 320
-//                   and brings the window part to reduced row echelon form
+//                   nonzero ones and brings the window part to reduced row echelon form
 //                   (lowest set bit leading), 32 columns at a time.  Every
 //                   basis vector carries its combination ("tag") over the rows
 //                   P_b that entered the basis, so R_window = tag * A[P, window].
@@ -88,6 +88,9 @@ struct WfSmem {
     uint4 vt[2][8][16];       // 4-bit tables of a round's pivot rows
     uint4 cv[kHalfCand][2];   // the candidates' vectors
     HalfRound r;
+    uint4 vrow[WF_ROWS][2];   // the chunk being gathered: vectors
+    int grow[WF_ROWS];        //   and rows
+    int cut;                  // first row of the block that did not fit
     int prow[WBITS];          // physical row of pivot column b
     int cnt;
     int wcnt[2][32];          // candidates per warp, alternating
@@ -183,7 +186,8 @@ __device__ __forceinline__ u32 wf_half(const WfSmem &S, const u32 (&v)[8], int h
 // the pivot columns found so far hold its combination over the pivot rows P_b
 // and elsewhere its data (a row with bit c set gets v ^= v_p without bit c, so
 // its bit c stays set and becomes the coefficient of P_c).  One CTA walks the
-// active rows in chunks of a row per thread; the columns go 32 at a time (half
+// active rows in chunks of a row per thread, leaving out the rows that are zero
+// modulo the basis so far (most rows of a sparse matrix); the columns go 32 at a time (half
 // words): up to 64 rows with data left there are eliminated by one warp
 // (half_word_select), and every row of the chunk then takes the round's pivots
 // in through 4-bit tables; rounds repeat until no unused row has data left in
@@ -193,7 +197,9 @@ __device__ __forceinline__ u32 wf_half(const WfSmem &S, const u32 (&v)[8], int h
 // Bound by the serial chain, not by throughput (one CTA): a round of up to 32
 // pivots costs about 2600 cycles in half_word_select, four barriers, the
 // tables and one half word of every row: about 29 us for a full window, against
-// 133 us when the rows are eliminated one pivot and one barrier at a time.
+// 133 us when the rows are eliminated one pivot and one barrier at a time
+// (rank of a 2000 x 4100 parity-check matrix 637 us, 976 with the zero rows in
+// the chunks).
 __global__ void __launch_bounds__(WF_THREADS, 1)
 window_factor_kernel(const u64 *__restrict__ M, i64 ld, i64 m, i64 n, i64 w, int *list, const unsigned char *live,
                      unsigned char *state, int *stamp, int wid, const WinState *prev, WinState *ws, long long *piv,
@@ -224,8 +230,7 @@ window_factor_kernel(const u64 *__restrict__ M, i64 ld, i64 m, i64 n, i64 w, int
     u32 H[8] = {};  // pivot columns so far (the same in every thread)
     int nb = 0;     // their number
     int walked = 0, par = 0;
-    for (int base = 0; base < na && nb < valid; base += WF_ROWS) {
-        walked = base + WF_ROWS < na ? base + WF_ROWS : na;
+    while (walked < na && nb < valid) {
         const bool older = nb > 0;  // basis vectors of earlier chunks
         u32 H0[8];
 #pragma unroll
@@ -244,32 +249,83 @@ window_factor_kernel(const u64 *__restrict__ M, i64 ld, i64 m, i64 n, i64 w, int
             }
             __syncthreads();
         }
-        const int k = base + ri;
-        int row = -1;
+        // the next rows that are not zero modulo the basis, up to WF_ROWS of
+        // them, from blocks of WF_ROWS list entries
+        int row = -1, filled = 0;
         u32 v[8] = {};
-        if (holds && k < na) {
-            row = L0[k];
+        for (;;) {
+            const int k = walked + ri;
+            int kr = -1;
+            u32 x[8] = {};
+            if (holds && k < na) {
+                kr = L0[k];
 #pragma unroll
-            for (int q = 0; q < WW; ++q)
-                if (q < wn) {
-                    const u64 x = M[(i64)row * ld + w + q];
-                    v[2 * q] = (u32)x;
-                    v[2 * q + 1] = (u32)(x >> 32);
+                for (int q = 0; q < WW; ++q)
+                    if (q < wn) {
+                        const u64 t = M[(i64)kr * ld + w + q];
+                        x[2 * q] = (u32)t;
+                        x[2 * q + 1] = (u32)(t >> 32);
+                    }
+            }
+            if (older) {
+                u32 y[8];
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    y[q] = x[q] & H0[q];
+                    x[q] &= ~H0[q];
                 }
-        }
-        if (older) {
-            u32 y[8];
 #pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                y[q] = v[q] & H0[q];
-                v[q] &= ~H0[q];
+                for (int g = 0; g < 64; ++g) {
+                    const int e = (int)((y[g >> 3] >> (4 * (g & 7))) & 15);
+                    if (e) xor8(x, S.tab[0][g][e], S.tab[1][g][e]);
+                }
             }
+            u32 any = 0;
 #pragma unroll
-            for (int g = 0; g < 64; ++g) {
-                const int e = (int)((y[g >> 3] >> (4 * (g & 7))) & 15);
-                if (e) xor8(v, S.tab[0][g][e], S.tab[1][g][e]);
+            for (int q = 0; q < 8; ++q) any |= x[q] & ~H0[q];
+            const unsigned bal = __ballot_sync(0xffffffffu, any != 0);
+            par ^= 1;
+            if (holds && lane == 0) S.wcnt[par][rw] = __popc(bal);
+            const int total = __syncthreads_count(any != 0);
+            const bool last = walked + WF_ROWS >= na;
+            if (filled == 0 && (last || 4 * total >= 3 * WF_ROWS)) {
+                // the block as it is: filling it up would not save a chunk
+                row = kr;
+#pragma unroll
+                for (int q = 0; q < 8; ++q) v[q] = x[q];
+                walked = last ? na : walked + WF_ROWS;
+                filled = total;
+                break;
+            }
+            const int wv = lane < rw && lane < NW ? S.wcnt[par][lane] : 0;
+            const int idx = filled + __reduce_add_sync(0xffffffffu, wv) + __popc(bal & ((1u << lane) - 1));
+            if (any && idx < WF_ROWS) {
+                S.vrow[idx][0] = make_uint4(x[0], x[1], x[2], x[3]);
+                S.vrow[idx][1] = make_uint4(x[4], x[5], x[6], x[7]);
+                S.grow[idx] = kr;
+            }
+            if (any && idx == WF_ROWS) S.cut = ri;
+            __syncthreads();
+            const bool over = filled + total > WF_ROWS;
+            walked = over ? walked + S.cut : last ? na : walked + WF_ROWS;
+            filled = over ? WF_ROWS : filled + total;
+            if (filled == WF_ROWS || walked >= na) {
+                if (ri < filled) {
+                    const uint4 a = S.vrow[ri][0], b = S.vrow[ri][1];
+                    v[0] = a.x;
+                    v[1] = a.y;
+                    v[2] = a.z;
+                    v[3] = a.w;
+                    v[4] = b.x;
+                    v[5] = b.y;
+                    v[6] = b.z;
+                    v[7] = b.w;
+                    row = S.grow[ri];
+                }
+                break;
             }
         }
+        if (filled == 0) break;  // only rows inside the span were left
         int mycol = -1;  // this row's pivot column
         // the last round, while its pivots are not in v yet: half word h,
         // columns C, combination z of this row

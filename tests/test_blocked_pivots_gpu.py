@@ -71,3 +71,10 @@ def test_update_tiles(cuda, form, m, n):
     one word."""
     P = gen.dense_packed(m, 0, m, n)
     check_all(P, m, n, form)
+
+
+@pytest.mark.parametrize("m,n,density", [(700, 260, 0.002), (1000, 600, 0.003), (1300, 520, 0.001), (2100, 300, 0.0006)])
+def test_chunks_of_nonzero_rows(cuda, m, n, density):
+    """Sparse matrices: chunks gathered from several blocks of the row list,
+    blocks that do not fit whole, lists that end inside a chunk."""
+    check_all(gen.sparse_packed(11, m, m, n, density), m, n, "m4ri")
