@@ -254,7 +254,7 @@ struct BigSmem {
     alignas(16) unsigned wmin[2][kRegWarps];  // per warp: its candidate pivot row
     int bits[64], srow[64];
     int slots[4];
-    u64 T[16][16][TW];  // nibble tables of the current chunk (TW words)
+    alignas(16) u64 T[16][16][TW];  // nibble tables of the current chunk (TW words)
     u64 pm;
     int p;
 };
@@ -643,57 +643,73 @@ __device__ void process_big_blocked(const BatchDevItem &it, const u64 *__restric
                 }
                 bar();
             }
-            // lane (h, xl) = (lane / TW, lane % TW) takes word x0 + xl of
-            // rows j0 + 4 h .. + 3 (32 / TW rows per warp instruction); the
-            // next rows' words are read while the current ones are combined
-            constexpr int RPW = 32 / TW;
-            const int kStep = nw * 4 * RPW;
-            const int xl = lane % TW, hsel = lane / TW;
+            // a lane takes words x and x + 1 (one 16-byte table read for both)
+            // of two rows, TW / 2 lanes a row: rows j0 + 2 h, j0 + 2 h + 1 of
+            // the warp's 2 RPW; the next rows' words are read while the
+            // current ones are combined
+            constexpr int LPR = TW / 2, RPW = 32 / LPR;
+            const int kStep = nw * 2 * RPW;
+            const int xl = 2 * (lane % LPR), hsel = lane / LPR;
             const int x = x0 + xl;
-            // rows jb .. jb + 3 (or list entries jb .. jb + 3): their indices,
+            const bool in0 = x < wc, in1 = x + 1 < wc;
+            auto combine = [&](u64 y, ulonglong2 &a) {
+#pragma unroll
+                for (int gi = 0; gi < 16; ++gi) {
+                    const ulonglong2 t = *reinterpret_cast<const ulonglong2 *>(&S.T[gi][(y >> (4 * gi)) & 15][xl]);
+                    a.x ^= t.x;
+                    a.y ^= t.y;
+                }
+            };
+            auto words_of_row = [&](int j) -> ulonglong2 {
+                const u64 *p = A + (size_t)j * wc + x;
+                return make_ulonglong2(in0 ? p[0] : 0ull, in1 ? p[1] : 0ull);
+            };
+            auto put = [&](int j, const ulonglong2 &a) {
+                u64 *p = A + (size_t)j * wc + x;
+                if (in0) p[0] = a.x;
+                if (in1) p[1] = a.y;
+            };
+            // rows jb, jb + 1 (or list entries jb, jb + 1): their indices,
             // coefficient words (0: skip) and matrix words
             const int nrows = ul ? nul : m;
-            auto fetch = [&](int jb, int (&jr)[4], u64 (&y)[4], u64 (&a)[4]) {
+            auto fetch = [&](int jb, int (&jr)[2], u64 (&y)[2], ulonglong2 (&a)[2]) {
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
+                for (int q = 0; q < 2; ++q) {
                     const int i = jb + q;
                     jr[q] = i < nrows ? (ul ? ul[i] : i) : -1;
                 }
 #pragma unroll
-                for (int q = 0; q < 4; ++q)
-                    y[q] = (jr[q] >= 0 && x < wc && (ul || active[jr[q]] != 2)) ? ysp[jr[q]] & pmask : 0ull;
+                for (int q = 0; q < 2; ++q)
+                    y[q] = (jr[q] >= 0 && in0 && (ul || active[jr[q]] != 2)) ? ysp[jr[q]] & pmask : 0ull;
 #pragma unroll
-                for (int q = 0; q < 4; ++q) a[q] = y[q] ? A[(size_t)jr[q] * wc + x] : 0ull;
+                for (int q = 0; q < 2; ++q) a[q] = y[q] ? words_of_row(jr[q]) : make_ulonglong2(0ull, 0ull);
             };
-            int jb = wq * 4 * RPW + 4 * hsel;
+            int jb = wq * 2 * RPW + 2 * hsel;
             if (ul) {
                 // listed rows (all to update): their words two steps ahead;
                 // coefficient words read from shared memory at use
-                auto load = [&](int j0, int (&jr)[4], u64 (&a)[4]) {
+                auto load = [&](int j0, int (&jr)[2], ulonglong2 (&a)[2]) {
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) jr[q] = (j0 + q < nul && x < wc) ? ul[j0 + q] : -1;
+                    for (int q = 0; q < 2; ++q) jr[q] = (j0 + q < nul && in0) ? ul[j0 + q] : -1;
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) a[q] = jr[q] >= 0 ? A[(size_t)jr[q] * wc + x] : 0ull;
+                    for (int q = 0; q < 2; ++q) a[q] = jr[q] >= 0 ? words_of_row(jr[q]) : make_ulonglong2(0ull, 0ull);
                 };
-                int j0r[4], j1r[4];
-                u64 a0[4], a1[4];
+                int j0r[2], j1r[2];
+                ulonglong2 a0[2], a1[2];
                 load(jb, j0r, a0);
                 load(jb + kStep, j1r, a1);
-                for (; jb - 4 * hsel < nul; jb += kStep) {
-                    int j2r[4];
-                    u64 a2[4];
+                for (; jb - 2 * hsel < nul; jb += kStep) {
+                    int j2r[2];
+                    ulonglong2 a2[2];
                     load(jb + 2 * kStep, j2r, a2);
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) {
+                    for (int q = 0; q < 2; ++q) {
                         if (j0r[q] < 0) continue;
-                        const u64 yq = ysp[j0r[q]] & pmask;
-                        u64 acc = 0;
-#pragma unroll
-                        for (int gi = 0; gi < 16; ++gi) acc ^= S.T[gi][(yq >> (4 * gi)) & 15][xl];
-                        A[(size_t)j0r[q] * wc + x] = a0[q] ^ acc;
+                        combine(ysp[j0r[q]] & pmask, a0[q]);
+                        put(j0r[q], a0[q]);
                     }
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) {
+                    for (int q = 0; q < 2; ++q) {
                         j0r[q] = j1r[q];
                         a0[q] = a1[q];
                         j1r[q] = j2r[q];
@@ -703,23 +719,23 @@ __device__ void process_big_blocked(const BatchDevItem &it, const u64 *__restric
                 bar();
                 continue;
             }
-            int jr[4];
-            u64 y[4], a[4];
+            int jr[2];
+            u64 y[2];
+            ulonglong2 a[2];
             fetch(jb, jr, y, a);
-            for (; jb - 4 * hsel < nrows; jb += kStep) {
-                int jn[4];
-                u64 yn[4], an[4];
+            for (; jb - 2 * hsel < nrows; jb += kStep) {
+                int jn[2];
+                u64 yn[2];
+                ulonglong2 an[2];
                 fetch(jb + kStep, jn, yn, an);
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
+                for (int q = 0; q < 2; ++q) {
                     if (!y[q]) continue;
-                    u64 acc = 0;
-#pragma unroll
-                    for (int gi = 0; gi < 16; ++gi) acc ^= S.T[gi][(y[q] >> (4 * gi)) & 15][xl];
-                    A[(size_t)jr[q] * wc + x] = a[q] ^ acc;
+                    combine(y[q], a[q]);
+                    put(jr[q], a[q]);
                 }
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
+                for (int q = 0; q < 2; ++q) {
                     jr[q] = jn[q];
                     y[q] = yn[q];
                     a[q] = an[q];
