@@ -257,6 +257,8 @@ struct BigSmem {
     alignas(16) u64 T[16][16][TW];  // nibble tables of the current chunk (TW words)
     u64 pm;
     int p;
+    int bycol;    // the panel's tags are indexed by pivot column (else by pivot)
+    HalfRound r;  // tables of one half word's pivots (warp_select)
 };
 // The big-matrix engine for a CTA of NT threads with SMEM bytes of shared
 // memory: TW words per update chunk (32, one per lane, for 512 threads; 16,
@@ -278,12 +280,12 @@ struct BigCfg {
 // v[i] for a lane-local index i < R (R <= 16) by a select tree: no local
 // memory and a dependence depth of four selects.
 template <int R>
-__device__ __forceinline__ u64 pick_reg(const u64 (&v)[R], int i)
+__device__ __forceinline__ u32 pick_reg(const u32 (&v)[R], int i)
 {
-    u64 a[8], b[4], c[2];
+    u32 a[8], b[4], c[2];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-        const u64 lo = 2 * j < R ? v[2 * j] : 0ull, hi = 2 * j + 1 < R ? v[2 * j + 1] : 0ull;
+        const u32 lo = 2 * j < R ? v[2 * j] : 0u, hi = 2 * j + 1 < R ? v[2 * j + 1] : 0u;
         a[j] = (i & 1) ? hi : lo;
     }
 #pragma unroll
@@ -293,115 +295,127 @@ __device__ __forceinline__ u64 pick_reg(const u64 (&v)[R], int i)
     return (i & 8) ? c[1] : c[0];
 }
 
-// Bit b of each of a lane's R words, as an R-bit mask (four independent
+// Bit b of each of a lane's R half words, as an R-bit mask (four independent
 // partial masks, so that the dependence chain stays short).
 template <int R>
-__device__ __forceinline__ u32 bit_mask(const u64 (&y)[R], int b)
+__device__ __forceinline__ u32 bit_mask(const u32 (&y)[R], int b)
 {
-    const int sh = b & 31;
     u32 h[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
-    for (int i = 0; i < R; ++i) {
-        const u32 half = (b & 32) ? (u32)(y[i] >> 32) : (u32)y[i];
-        h[i & 3] |= ((half >> sh) & 1u) << i;
-    }
+    for (int i = 0; i < R; ++i) h[i & 3] |= ((y[i] >> b) & 1u) << i;
     return (h[0] | h[1]) | (h[2] | h[3]);
 }
 
 // Pivot selection of one panel among its candidate rows (active rows with a
 // nonzero panel word; cnt <= 32 R) by one warp, no block barrier: lane l holds
-// candidates l + 32 i.  Per bit that some candidate holds (the OR of their
-// words: XORs create no other bit), the lowest unused candidate holding it
-// becomes pivot k and is XORed into every other candidate holding the bit.
-// A step's critical path is a ballot and a shuffle: which rows hold the next
-// bit is computed from the words before the XOR (the bit flips in the rows
-// that take the pivot where the pivot word has it), and the pivots' bits are
-// kept in registers and written out at the end.  The pivots' combination
-// tags (which other pivots' original rows make up each reduced pivot row)
-// come from a second elimination over the pivots alone, whose pivot rows are
-// known: p steps of two shuffles, no ballot.  Writes the pivots' bits, rows
-// and tags; returns the pivot count and the pivot mask.
+// candidates l + 32 i, their panel words in in-place form (basis.cuh).  The
+// columns go 32 at a time.  Per bit that some unused candidate holds (XORs
+// create no other bit), the lowest one holding it becomes the pivot and its
+// half word, without the bit, is XORed into every other candidate holding the
+// bit; the bit left standing there is the coefficient of that pivot row.  A
+// step's critical path is a ballot and a shuffle: which rows hold the next bit
+// is computed from the half words before the XOR (the bit flips in the rows
+// that take the pivot where the pivot has it).  After the 32 columns each
+// candidate's bits at the pivot columns name the original pivot rows it
+// contains, and its other half word takes theirs through 4-bit tables.  Against
+// 64-bit steps with a second elimination for the combinations: half the
+// instructions a step (SELNEW).  Writes the pivots' bits (ascending), rows and
+// tags (by pivot column: which original pivot rows make up each reduced one);
+// returns the pivot count and the pivot mask.
 template <int R>
-__device__ __forceinline__ int warp_select(const int *cand, int cnt, const u64 *ysnap, u64 *tag, int *bits,
-                                           int *srow, u64 *pm_out)
+__device__ __forceinline__ int warp_select(HalfRound &S, const int *cand, int cnt, const u64 *ysnap, u64 *tag,
+                                           int *bits, int *srow, u64 *pm_out)
 {
     const int lane = threadIdx.x & 31;
-    u64 y[R];
-    int pb[R];  // the bit a candidate became the pivot of, or -1
+    u32 w[R], o[R];  // the half word at work and the other one
+    int pb[R];       // the bit a candidate became the pivot of, or -1
     u32 unused = 0;
-    u64 orw = 0;
 #pragma unroll
     for (int i = 0; i < R; ++i) {
         const int c = lane + 32 * i;
-        y[i] = c < cnt ? ysnap[cand[c]] : 0ull;
+        const u64 y = c < cnt ? ysnap[cand[c]] : 0ull;
+        w[i] = (u32)y;
+        o[i] = (u32)(y >> 32);
         pb[i] = -1;
         unused |= (c < cnt ? 1u : 0u) << i;
-        orw |= y[i];
     }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) orw |= __shfl_xor_sync(0xffffffffu, orw, o);
-    int k = 0;
     u64 pmask = 0;
-    u64 rem = orw;
-    if (rem) {
-        int b = __ffsll((long long)rem) - 1;
-        u32 hold = bit_mask<R>(y, b);
-        while (true) {
-            const u64 rem_n = rem & (rem - 1);
-            const int bn = rem_n ? __ffsll((long long)rem_n) - 1 : 0;
-            u32 hold_n = bit_mask<R>(y, bn);
-            const u32 cm = hold & unused;
-            const u32 bal = __ballot_sync(0xffffffffu, cm != 0);
-            if (bal) {
-                const int src = __ffs((int)bal) - 1;
-                const int ib = __ffs((int)cm) - 1;  // meaningful in lane src
-                const u64 yp = __shfl_sync(0xffffffffu, pick_reg<R>(y, ib), src);
-                const u32 me = lane == src ? (1u << ib) : 0u;
-                const u32 hit = hold & ~me;  // every other candidate holding bit b
+#pragma unroll 1
+    for (int h = 0; h < 2; ++h) {
+        u32 orw = 0;
 #pragma unroll
-                for (int i = 0; i < R; ++i) {
-                    if ((hit >> i) & 1u) y[i] ^= yp;
-                    if ((me >> i) & 1u) pb[i] = b;
+        for (int i = 0; i < R; ++i) orw |= (unused >> i) & 1u ? w[i] : 0u;
+        u32 rem = __reduce_or_sync(0xffffffffu, orw);
+        u32 C = 0;
+        S.T[lane] = 0;
+        __syncwarp();
+        if (rem) {
+            int b = __ffs((int)rem) - 1;
+            u32 hold = bit_mask<R>(w, b);
+            while (true) {
+                const u32 rem_n = rem & (rem - 1);
+                const int bn = rem_n ? __ffs((int)rem_n) - 1 : 0;
+                u32 hold_n = bit_mask<R>(w, bn);
+                const u32 cm = hold & unused;
+                const u32 bal = __ballot_sync(0xffffffffu, cm != 0);
+                if (bal) {
+                    const int src = __ffs((int)bal) - 1;
+                    const int ib = __ffs((int)cm) - 1;  // meaningful in lane src
+                    const u32 yp = __shfl_sync(0xffffffffu, pick_reg<R>(w, ib), src) & ~(1u << b);
+                    const u32 me = lane == src ? (1u << ib) : 0u;
+                    const u32 hit = hold & ~me;  // every other candidate holding bit b
+#pragma unroll
+                    for (int i = 0; i < R; ++i) {
+                        w[i] ^= (hit >> i) & 1u ? yp : 0u;
+                        if ((me >> i) & 1u) pb[i] = 32 * h + b;
+                    }
+                    unused &= ~me;
+                    hold_n ^= ((yp >> bn) & 1u) ? hit : 0u;
+                    C |= 1u << b;
                 }
-                unused &= ~me;
-                hold_n ^= ((yp >> bn) & 1ull) ? hit : 0u;
-                pmask |= 1ull << b;
-                ++k;
+                if (!rem_n) break;
+                rem = rem_n;
+                b = bn;
+                hold = hold_n;
             }
-            if (!rem_n) break;
-            rem = rem_n;
-            b = bn;
-            hold = hold_n;
+        }
+        if (C) {  // uniform
+#pragma unroll
+            for (int i = 0; i < R; ++i)
+                if (pb[i] >= 32 * h && pb[i] < 32 * h + 32) {
+                    S.T[pb[i] - 32 * h] = o[i];
+                    o[i] = 0;
+                }
+            __syncwarp();
+#pragma unroll
+            for (int q = 0; q < 4; ++q) half_word_tt(S, lane + 32 * q);
+            __syncwarp();
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                const u32 z = w[i] & C;
+                if (z) o[i] ^= half_word_times_T(S, z);
+            }
+            __syncwarp();
+        }
+        pmask |= (u64)C << (32 * h);
+        // the halves change places; after the second one they are back
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const u32 t = w[i];
+            w[i] = o[i];
+            o[i] = t;
         }
     }
 #pragma unroll
     for (int i = 0; i < R; ++i)
         if (pb[i] >= 0) {
-            const int kk = __popcll(pmask & ((1ull << pb[i]) - 1));
+            const int kk = __popcll(pmask & ((1ull << pb[i]) - 1)), row = cand[lane + 32 * i];
             bits[kk] = pb[i];
-            srow[kk] = cand[lane + 32 * i];
+            srow[kk] = row;
+            tag[row] = ((u64)w[i] | ((u64)o[i] << 32)) & pmask;
         }
-    __syncwarp();
-    // tags: lane l holds pivots l and l + 32 (original panel words)
-    u64 v0 = lane < k ? ysnap[srow[lane]] : 0ull, v1 = lane + 32 < k ? ysnap[srow[lane + 32]] : 0ull;
-    u64 t0 = 0, t1 = 0;
-    for (int q = 0; q < k; ++q) {
-        const int bq = bits[q];
-        const u64 vq = __shfl_sync(0xffffffffu, q < 32 ? v0 : v1, q & 31);
-        const u64 tq = __shfl_sync(0xffffffffu, q < 32 ? t0 : t1, q & 31) ^ (1ull << q);
-        if (lane != q && ((v0 >> bq) & 1ull)) {
-            v0 ^= vq;
-            t0 ^= tq;
-        }
-        if (lane + 32 != q && ((v1 >> bq) & 1ull)) {
-            v1 ^= vq;
-            t1 ^= tq;
-        }
-    }
-    if (lane < k) tag[srow[lane]] = t0;
-    if (lane + 32 < k) tag[srow[lane + 32]] = t1;
     *pm_out = pmask;
-    return k;
+    return __popcll(pmask);
 }
 
 // Element i (0..3, per thread) of a register array, by a select tree.
@@ -593,18 +607,19 @@ __device__ void process_big_blocked(const BatchDevItem &it, const u64 *__restric
         u64 pmk;
         int kk;
         if (ncand <= 64)
-            kk = warp_select<2>(S.cand, ncand, ysp, tag, S.bits, S.srow, &pmk);
+            kk = warp_select<2>(S.r, S.cand, ncand, ysp, tag, S.bits, S.srow, &pmk);
         else if (ncand <= 128)
-            kk = warp_select<4>(S.cand, ncand, ysp, tag, S.bits, S.srow, &pmk);
+            kk = warp_select<4>(S.r, S.cand, ncand, ysp, tag, S.bits, S.srow, &pmk);
         else if (ncand <= 192)
-            kk = warp_select<6>(S.cand, ncand, ysp, tag, S.bits, S.srow, &pmk);
+            kk = warp_select<6>(S.r, S.cand, ncand, ysp, tag, S.bits, S.srow, &pmk);
         else if (ncand <= 256)
-            kk = warp_select<8>(S.cand, ncand, ysp, tag, S.bits, S.srow, &pmk);
+            kk = warp_select<8>(S.r, S.cand, ncand, ysp, tag, S.bits, S.srow, &pmk);
         else
-            kk = warp_select<12>(S.cand, ncand, ysp, tag, S.bits, S.srow, &pmk);
+            kk = warp_select<12>(S.r, S.cand, ncand, ysp, tag, S.bits, S.srow, &pmk);
         if (lane == 0) {
             S.p = kk;
             S.pm = pmk;
+            S.bycol = 1;
         }
     };
     // words [x_begin, wc) of every row that is not one of the panel's pivots
@@ -854,6 +869,7 @@ __device__ void process_big_blocked(const BatchDevItem &it, const u64 *__restric
                     if (tid == 0) {
                         S.p = k;
                         S.pm = pmask;
+                        S.bycol = 0;
                     }
                 }
                 __syncthreads();
@@ -863,6 +879,7 @@ __device__ void process_big_blocked(const BatchDevItem &it, const u64 *__restric
                 __syncthreads();
             } else {
                 // 1. panel words, pivot search for bit 0
+                if (tid == 0) S.bycol = 0;
                 if (tid < 3) S.slots[tid] = INT_MAX;
                 __syncthreads();
                 unsigned best = INT_MAX;
@@ -917,15 +934,17 @@ __device__ void process_big_blocked(const BatchDevItem &it, const u64 *__restric
         have_sel = false;
         const int p = k;
         if (p == 0) continue;
+        const bool bycol = S.bycol;
         for (int t = tid; t < p; t += NT) {
-            S.coef[t] = tag[S.srow[t]] ^ (1ull << t);
+            S.coef[t] = bycol ? tag[S.srow[t]] : tag[S.srow[t]] ^ (1ull << t);
             piv[r + t] = 64 * w + S.bits[t];
             prow[r + t] = S.srow[t];
             S.prev_srow[t] = S.srow[t];
         }
         const int rem = wc - w;
-        // 3. reduced pivot rows from the staged original rows (Rbuf row b:
-        // the reduced row of the pivot on bit b)
+        // 3. reduced pivot rows from the staged original rows (stage row i: the
+        // pivot row that bit i of a tag names; Rbuf row b: the reduced row of
+        // the pivot on bit b)
         __syncthreads();
         {
             constexpr int U = 8;
@@ -939,7 +958,8 @@ __device__ void process_big_blocked(const BatchDevItem &it, const u64 *__restric
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
                     const int e = e0 + u * NT;
-                    if (e < p * rem) stage[(size_t)(e / rem) * wc + w + e % rem] = v[u];
+                    if (e < p * rem)
+                        stage[(size_t)(bycol ? S.bits[e / rem] : e / rem) * wc + w + e % rem] = v[u];
                 }
             }
         }
