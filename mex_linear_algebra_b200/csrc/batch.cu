@@ -319,7 +319,8 @@ __device__ __forceinline__ u32 bit_mask(const u32 (&y)[R], int b)
 // candidate's bits at the pivot columns name the original pivot rows it
 // contains, and its other half word takes theirs through 4-bit tables.  Against
 // 64-bit steps with a second elimination for the combinations: half the
-// instructions a step (SELNEW).  Writes the pivots' bits (ascending), rows and
+// instructions a step (26K cycles a panel of a 1000-row parity-check matrix
+// beside the update, 38K before).  Writes the pivots' bits (ascending), rows and
 // tags (by pivot column: which original pivot rows make up each reduced one);
 // returns the pivot count and the pivot mask.
 template <int R>
@@ -565,8 +566,17 @@ __device__ void process_big_blocked(const BatchDevItem &it, const u64 *__restric
     const size_t pre_a_bytes = used;  // shared bytes before the matrix: free again for the null basis
     if (used + (size_t)m * wc * 8 <= kBigExtra) A = reinterpret_cast<u64 *>(extra + used);
 
+    // the matrix, eight words a thread in flight (one after the other the copy
+    // took 141K of a 1000-row matrix's 1.88M cycles)
     const u64 *src = in + it.in_off;
-    for (long long e = tid; e < (long long)m * wc; e += NT) A[e] = src[e];
+    for (int e0 = tid; e0 < m * wc; e0 += 8 * NT) {
+        u64 v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = e0 + u * NT < m * wc ? src[e0 + u * NT] : 0ull;
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            if (e0 + u * NT < m * wc) A[e0 + u * NT] = v[u];
+    }
     for (int j = tid; j < m; j += NT) active[j] = 1;
     __syncthreads();
 
@@ -942,6 +952,10 @@ __device__ void process_big_blocked(const BatchDevItem &it, const u64 *__restric
             S.prev_srow[t] = S.srow[t];
         }
         const int rem = wc - w;
+        // e / rem for e < 64 rem: (e + 1/2) / rem is at least 1 / (2 rem) from
+        // an integer, far beyond the product's rounding for rem <= 4096
+        const float inv = 1.0f / (float)rem;
+        auto row_of = [&](int e) { return rem <= 4096 ? (int)(((float)e + 0.5f) * inv) : e / rem; };
         // 3. reduced pivot rows from the staged original rows (stage row i: the
         // pivot row that bit i of a tag names; Rbuf row b: the reduced row of
         // the pivot on bit b)
@@ -952,25 +966,29 @@ __device__ void process_big_blocked(const BatchDevItem &it, const u64 *__restric
                 u64 v[U];
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
-                    const int e = e0 + u * NT;
-                    v[u] = e < p * rem ? A[(size_t)S.srow[e / rem] * wc + w + e % rem] : 0ull;
+                    const int e = e0 + u * NT, kk = row_of(e);
+                    v[u] = e < p * rem ? A[(size_t)S.srow[kk] * wc + w + (e - kk * rem)] : 0ull;
                 }
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
-                    const int e = e0 + u * NT;
-                    if (e < p * rem)
-                        stage[(size_t)(bycol ? S.bits[e / rem] : e / rem) * wc + w + e % rem] = v[u];
+                    const int e = e0 + u * NT, kk = row_of(e);
+                    if (e < p * rem) stage[(size_t)(bycol ? S.bits[kk] : kk) * wc + w + (e - kk * rem)] = v[u];
                 }
             }
         }
         __syncthreads();
         for (int e = tid; e < p * rem; e += NT) {
-            const int kk = e / rem, x = w + e % rem;
+            const int kk = row_of(e), x = w + (e - kk * rem);
+            const u64 *st = stage + x;
             u64 c = S.coef[kk], v = 0;
-            while (c) {
-                const int i = ctz64_(c);
-                c &= c - 1;
-                v ^= stage[(size_t)i * wc + x];
+            while (c) {  // four staged words in flight
+                u64 t[4] = {0ull, 0ull, 0ull, 0ull};
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    if (c) t[u] = st[(size_t)ctz64_(c) * wc];
+                    c &= c - 1;
+                }
+                v ^= (t[0] ^ t[1]) ^ (t[2] ^ t[3]);
             }
             Rbuf[(size_t)S.bits[kk] * wc + x] = v;
             A[(size_t)S.srow[kk] * wc + x] = v;
