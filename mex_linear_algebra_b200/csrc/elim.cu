@@ -840,7 +840,9 @@ NullLayout null_layout(i64 n, i64 rank)
     L.mask = off;    off += al256((size_t)wc * 8);
     L.before = off;  off += al256((size_t)wc * 8);
     L.mv = off;      off += al256((size_t)wc * 6 * 8);
-    L.x = off;       off += al256((size_t)(n - rank) * (size_t)ldx * 8);
+    // n - rank rows are used; room for n, so that a workspace for some rank
+    // also serves every smaller one
+    L.x = off;       off += al256((size_t)(n ? n : 1) * (size_t)ldx * 8);
     L.ldx = ldx;
     L.total = off;
     return L;

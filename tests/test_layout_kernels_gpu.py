@@ -78,3 +78,11 @@ def test_null_basis_edges(cuda, m, n, r):
         got = to_host(Zt)
         assert np.array_equal(got[:f, :-1], O.null_basis_packed(P, m, n))
         assert (Zt[f:] == -1).all() and (Zt[:, -1] == -1).all()
+
+
+def test_null_workspace_covers_smaller_ranks(cuda):
+    """A workspace sized for a rank serves every smaller rank."""
+    L = _lib.lib()
+    for n in (1, 64, 200, 1000, 4097):
+        sizes = [L.mela_null_workspace_size(n, r) for r in range(0, n + 1, max(1, n // 50))]
+        assert sizes == sorted(sizes)
