@@ -441,7 +441,8 @@ int32_t mela_costmodel_predict(int32_t op, int64_t m, int64_t n, int64_t p, doub
  * -1 without a model. */
 int32_t mela_costmodel_plan(int32_t op, int64_t m, int64_t n, int64_t p, int32_t *measure);
 /* The variant argument the calling thread's last AUTO call resolved to (-1
- * before any), and in *density the density it measured on the device for
+ * before any; MELA_GEMM_PLAIN for a host product small enough to be multiplied
+ * straight from its arrays, which asks no model), and in *density the density it measured on the device for
  * the choice, or a negative value when none was needed (mela_costmodel_plan). */
 int32_t mela_dispatch_last(double *density);
 /* The MELA_MLP_IN input features of a request. */

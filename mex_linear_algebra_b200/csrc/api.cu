@@ -936,6 +936,19 @@ static mela_status matmul_host(const mela_host_matrix *A, const mela_host_matrix
     cudaStream_t s;
     mela_status st = host_stream(&s);
     if (st != MELA_OK) return st;
+    const size_t ea = A->kind == MELA_KIND_DOUBLE ? 8 : 1, eb = B->kind == MELA_KIND_DOUBLE ? 8 : 1;
+    if (k > 0 && gemm_small_fits(m, k, n, ea, eb)) {
+        if (variant == MELA_GEMM_AUTO) remember_variant(MELA_GEMM_PLAIN, -1.0);  // AND and parity, untabled
+        const size_t ab = ((size_t)m * k * ea + 255) & ~(size_t)255, bb = ((size_t)k * n * eb + 255) & ~(size_t)255;
+        DevBuf all;
+        if ((st = all.alloc(ab + bb + (size_t)m * n, s)) != MELA_OK) return st;
+        unsigned char *dA = (unsigned char *)all.p, *dB = dA + ab, *dC = dB + bb;
+        MELA_CUDA_TRY(cudaMemcpyAsync(dA, A->data, (size_t)m * k * ea, cudaMemcpyHostToDevice, s));
+        MELA_CUDA_TRY(cudaMemcpyAsync(dB, B->data, (size_t)k * n * eb, cudaMemcpyHostToDevice, s));
+        t_upload_stats.direct_bytes += (int64_t)((size_t)m * k * ea + (size_t)k * n * eb);
+        if ((st = launch_gemm_small(A->kind, dA, B->kind, dB, dC, m, k, n, s)) != MELA_OK) return st;
+        return download_finish(C, dC, (size_t)m * n, s);
+    }
     const i64 lda = even_words(k), ldb = even_words(n), ldc = even_words(n);
     DevBuf pA, pB, pC, sA, sB, ws, outb;
     if ((st = pA.alloc((size_t)m * lda * 8, s)) != MELA_OK) return st;

@@ -204,7 +204,7 @@ thread_local int32_t t_last_variant = -1;
 thread_local double t_last_density = -1.0;
 }  // namespace
 
-static int32_t remember(int32_t v, double density)
+int32_t remember_variant(int32_t v, double density)
 {
     t_last_variant = v;
     t_last_density = density;
@@ -302,10 +302,10 @@ int32_t resolve_gemm_variant(int32_t variant, const u64 *A, i64 lda, i64 m, i64 
             // the FP4 form's f32 sums are exact below 2^24: past 2^23 terms use INT8
             if (MELA_VARIANT_BASE(v) == MELA_GEMM_TC_FP4 && k >= (1LL << 23))
                 v = MELA_GEMM_TC | (v & ~0xff);
-            return remember(v, t_last_density);
+            return remember_variant(v, t_last_density);
         }
     }
-    return remember(fixed_gemm_variant(m, k, n), -1.0);
+    return remember_variant(fixed_gemm_variant(m, k, n), -1.0);
 }
 
 int32_t fixed_gemm_variant(i64 m, i64 k, i64 n)
@@ -323,9 +323,9 @@ int32_t resolve_elim_variant(int32_t variant, const u64 *M, i64 ld, i64 m, i64 n
     if (costmodel_loaded() && m > 0 && n > 0) {
         const int c = choose_measuring(rref ? MELA_OP_NULL : MELA_OP_RANK, (double)m, (double)n, 0.0,
                                        (double)m * (double)n, M, ld, m, n, s);
-        if (c >= 0) return remember(config_variant(MELA_OP_RANK, c), t_last_density);
+        if (c >= 0) return remember_variant(config_variant(MELA_OP_RANK, c), t_last_density);
     }
-    return remember(fixed_elim_variant(m, n), -1.0);
+    return remember_variant(fixed_elim_variant(m, n), -1.0);
 }
 
 int32_t fixed_elim_variant(i64 m, i64 n)

@@ -50,6 +50,8 @@ bool decode_gemm_variant(int32_t v, Tuning *t);
 // Configurations of an op in the cost model's output order (dispatch.cu).
 int config_count(int op);
 int32_t config_variant(int op, int index);
+// Records what mela_dispatch_last reports, and returns v.
+int32_t remember_variant(int32_t v, double density);
 // AUTO -> a concrete variant argument: the installed model's choice for the
 // input's measured density, else the fixed rule.  Other variants pass through.
 int32_t resolve_gemm_variant(int32_t variant, const u64 *A, i64 lda, i64 m, i64 k, i64 n, cudaStream_t s);

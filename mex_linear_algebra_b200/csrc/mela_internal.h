@@ -53,6 +53,13 @@ mela_status make_u64_rows_map(CUtensorMap *map, const u64 *base, i64 rows, i64 w
 mela_status launch_gemm_m4ri(const u64 *A, i64 lda, const u64 *B, i64 ldb, u64 *C, i64 ldc,
                              i64 m, i64 k, i64 n, cudaStream_t s, int tile = 0);
 
+// Product of small arrays in MATLAB layout (column-major, element kinds and
+// sizes as given) in one launch: C (m x n logical).  fits: where it beats
+// packing (gemm_small.cu).
+bool gemm_small_fits(i64 m, i64 k, i64 n, size_t a_size, size_t b_size);
+mela_status launch_gemm_small(int kind_a, const void *A, int kind_b, const void *B, unsigned char *C, i64 m, i64 k,
+                              i64 n, cudaStream_t s);
+
 // Whole RREF of one matrix by one CTA in one launch: in shared memory where it
 // fits (elim_small.cu: up to 512 rows, 192 KB with its tables), else by the
 // batch engine for big matrices over the workspace (batch.cu).
