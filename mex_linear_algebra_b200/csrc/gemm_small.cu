@@ -73,14 +73,15 @@ gemm_small_kernel(const TA *__restrict__ A, const TB *__restrict__ B, unsigned c
 bool gemm_small_fits(i64 m, i64 k, i64 n, size_t a_size, size_t b_size)
 {
     if (m <= 0 || k <= 0 || n <= 0 || m > 4096 || n > 4096 || k > 32 * SP_KW) return false;
-    // Every block reads its rows of A and columns of B in full.  Up to 4 MiB of
-    // that and 256 bits of K it beats packing (200^3 logical 53 against 71 us,
-    // 512 x 256 x 512 89 against 108, 1000 x 64 x 1000 253 against 285); at 5
-    // to 8 MiB the two are level (200^3 double 90 against 91, 256^3 double 111
-    // and 111).  A longer K is a serial chain of loads in each block: 128 x 512
-    // x 128 double 121 against 110, 64 x 2000 x 64 156 against 95.
+    // Every block reads its rows of A and columns of B in full.  Up to 8 MiB of
+    // that and 256 bits of K it beats packing (200^3 logical 48 against 73 us,
+    // double 88 against 93; 256^3 double 110 against 115; 1000 x 64 x 1000
+    // logical 250 against 276); near 8 MiB the two draw level (1000 x 200 x 500
+    // logical 188 and 199).  A longer K is a serial chain of loads in each
+    // block: 128 x 512 x 128 double 121 against 110, 64 x 2000 x 64 156
+    // against 95.
     const i64 bi = (m + SP_T - 1) / SP_T, bj = (n + SP_T - 1) / SP_T;
-    return bi * bj * SP_T * k * (i64)(a_size + b_size) <= (i64)4 << 20;
+    return bi * bj * SP_T * k * (i64)(a_size + b_size) <= (i64)8 << 20;
 }
 
 mela_status launch_gemm_small(int kind_a, const void *A, int kind_b, const void *B, unsigned char *C, i64 m, i64 k,
