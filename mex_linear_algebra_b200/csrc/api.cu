@@ -353,6 +353,15 @@ mela_status gemm_device(int variant, const u64 *A, i64 lda, const u64 *B, i64 ld
                         i64 m, i64 k, i64 n, void *ws, size_t ws_bytes, cudaStream_t s)
 {
     if (m > 0 && n > 0 && k > 0) variant = resolve_gemm_variant(variant, A, lda, m, k, n, s);
+    if (m > 0 && n > 0 && k > 0) {
+        const GemmPlan p = plan_gemm(variant, m, k, n);
+        const bool fp4 = p.variant == MELA_GEMM_TC_FP4;
+        if ((fp4 || p.variant == MELA_GEMM_TC) && k < (1LL << 23) &&
+            gemm_strassen_fits(A, lda, B, ldb, C, ldc, m, k, n, fp4, p.tc_tile)) {
+            if (mela_status st = check_ws(p, ws, ws_bytes); st != MELA_OK) return st;
+            return launch_gemm_strassen(A, lda, B, ldb, C, ldc, m, k, n, ws, ws_bytes, fp4, s);
+        }
+    }
     mela_status st = gemm_prepare(variant, A, lda, B, ldb, m, k, n, ws, ws_bytes, s);
     if (st != MELA_OK) return st;
     return gemm_run(variant, A, lda, B, ldb, C, ldc, m, k, n, ws, ws_bytes, s);

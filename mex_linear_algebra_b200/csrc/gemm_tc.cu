@@ -254,7 +254,37 @@ struct PairCtl {
     u32 tmem;
     int abort;
 };
-constexpr int P_EPI_WARPS = 4;
+constexpr int P_EPI_WARPS = 8;                         // two per TMEM lane quarter, 128 columns each
+constexpr int P_THREADS = 64 + 32 * P_EPI_WARPS;
+
+// Up to two blocks of C (pitch ldc) that one product goes to.
+struct PairSum {
+    u64 *c[2];
+    i64 rows[2], words[2];  // 0: none
+    int add[2];             // XOR into the block instead of writing it
+};
+
+// Pins registers that an asynchronous TMEM load fills behind the wait for it.
+__device__ __forceinline__ void tie(u32 (&r)[32])
+{
+#pragma unroll
+    for (int j = 0; j < 32; ++j) asm volatile("" : "+r"(r[j]));
+}
+// The parities of 32 accumulators as one word, value j in bit j: four chains
+// of 8 funnel shifts, each of which moves a value's low bit in from the top.
+template <bool F4>
+__device__ __forceinline__ u32 low_bits(const u32 (&r)[32])
+{
+    u32 b[4] = {};
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const u32 x = r[8 * q + j];
+            b[q] = __funnelshift_r(b[q], F4 ? __float_as_uint(__uint_as_float(x) + 8388608.0f) : x, 1);
+        }
+    return __byte_perm(__byte_perm(b[0], b[1], 0x0073), __byte_perm(b[2], b[3], 0x0073), 0x5410);
+}
 }  // namespace
 
 // Persistent: cluster c computes tiles c, c + clusters, ... (grouped
@@ -262,10 +292,12 @@ constexpr int P_EPI_WARPS = 4;
 // so the producer fills the next tile's stages while the current tile's last
 // MMAs and its epilogue run; the MMA thread starts a tile once both CTAs'
 // epilogues have read the previous one out of TMEM.
-template <bool F4>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
+// SUM: the product is written or added (XOR) to the blocks of `out` instead.
+template <bool F4, bool SUM>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(P_THREADS, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                    u64 *__restrict__ C, i64 ldc, i64 m, i64 n, int tiles_m, int tiles_n, int kstages, u32 *err)
+                    u64 *__restrict__ C, i64 ldc, i64 m, i64 n, int tiles_m, int tiles_n, int kstages, u32 *err,
+                    const __grid_constant__ PairSum out)
 {
     constexpr u32 TMEM_COLS = F4 ? 512 : 256;
     extern __shared__ unsigned char smem_raw[];
@@ -312,7 +344,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     const u32 tmem = ctl->tmem;
     volatile int *abort_flag = &ctl->abort;
     if constexpr (F4) {
-        if (warp >= 2) {
+        if (warp >= 2 && warp < 6) {
             const u32 lane_base = (u32)((warp & 3) * 32) << 16;
             ptx::tmem_st_32x32b_x16(tmem + lane_base + SF_COL, 0x7F7F7F7Fu);
             ptx::tmem_st_32x32b_x16(tmem + lane_base + SF_COL + 16, 0x7F7F7F7Fu);
@@ -392,6 +424,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     } else {
         const int ew = warp & 3;  // TMEM lane quarter this warp may access
         const u32 acc_empty0 = ptx::mapa_shared(ptx::smem_u32(&ctl->acc_empty), 0);
+        const int side = (warp - 2) >> 2;  // its half of the tile's columns
         const i64 nw = words_of(n);
         int i = 0;
         for (int t = cid; t < ntiles; t += clusters, ++i) {
@@ -404,30 +437,45 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             int tm, tn;
             coords(t, tm, tn);
             const i64 row = (i64)tm * 256 + (i64)rank * 128 + ew * 32 + lane;
-            u32 bits[BN / 32];
+            // two chunks of 32 columns in registers: one on its way from TMEM
+            // while the other's bits are gathered (the tile's MMAs wait for
+            // this: 3.3K cycles a tile, 3.6K with four warps one chunk at a
+            // time; 16384 x 1024 x 16384 in 323K cycles against 338K)
+            u32 bits[4], r[2][32];
+            const u32 tcol = tmem + ((u32)(ew * 32) << 16) + (u32)(128 * side);
+            ptx::tmem_ld_32x32b_x32(tcol, r[0]);
 #pragma unroll
-            for (int c = 0; c < BN / 32; ++c) {
-                u32 r[32];
-                ptx::tmem_ld_32x32b_x32(tmem + ((u32)(ew * 32) << 16) + (u32)(c * 32), r);
+            for (int c = 0; c < 4; ++c) {
                 ptx::tmem_ld_wait();
-                u32 b = 0;
-#pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                    const u32 v = F4 ? __float_as_uint(__uint_as_float(r[j]) + 8388608.0f) : r[j];
-                    b |= (v & 1u) << j;
-                }
-                bits[c] = b;
+                tie(r[c & 1]);
+                if (c < 3) ptx::tmem_ld_32x32b_x32(tcol + (u32)(32 * (c + 1)), r[(c + 1) & 1]);
+                bits[c] = low_bits<F4>(r[c & 1]);
             }
             // this warp's TMEM reads are done: the next tile may overwrite them
             ptx::tc_fence_before();
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive_cluster(acc_empty0);
-            if (row < m) {
+            const i64 w0 = (i64)tn * (BN / 64) + 2 * side;
+            const u64 v[2] = {(u64)bits[0] | ((u64)bits[1] << 32), (u64)bits[2] | ((u64)bits[3] << 32)};
+            if constexpr (SUM) {
 #pragma unroll
-                for (int q = 0; q < BN / 64; ++q) {
-                    const i64 w = (i64)tn * (BN / 64) + q;
-                    if (w < nw) C[row * ldc + w] = (u64)bits[2 * q] | ((u64)bits[2 * q + 1] << 32);
+                for (int d = 0; d < 2; ++d) {
+                    u64 *c = out.c[d] + row * ldc + w0;
+                    const i64 left = row < out.rows[d] ? out.words[d] - w0 : 0;
+                    u64 old[2] = {};
+                    if (out.add[d]) {
+#pragma unroll
+                        for (int q = 0; q < 2; ++q)
+                            if (q < left) old[q] = c[q];
+                    }
+#pragma unroll
+                    for (int q = 0; q < 2; ++q)
+                        if (q < left) c[q] = old[q] ^ v[q];
                 }
+            } else if (row < m) {
+#pragma unroll
+                for (int q = 0; q < 2; ++q)
+                    if (w0 + q < nw) C[row * ldc + w0 + q] = v[q];
             }
         }
     }
@@ -522,6 +570,26 @@ static bool use_pairs(i64 mp, int tile)
     return !(e && e[0] == '0');
 }
 
+// The pair kernel over mp x np x kp expanded operands.
+template <bool SUM>
+static mela_status launch_pairs(const unsigned char *A8, const unsigned char *Bt8, i64 mp, i64 np, i64 kp, u64 *C,
+                                i64 ldc, i64 m, i64 n, bool fp4, const PairSum &out, cudaStream_t s)
+{
+    CUtensorMap ma, mb;
+    mela_status st = make_map(&ma, A8, mp, kp, 128);
+    if (st != MELA_OK) return st;
+    st = make_map(&mb, Bt8, np, kp, 128);
+    if (st != MELA_OK) return st;
+    const i64 tiles_m = mp / 256, tiles_n = np / BN, ntiles = tiles_m * tiles_n, clusters_max = sm_count() / 2;
+    const unsigned grid = (unsigned)(2 * (ntiles < clusters_max ? ntiles : clusters_max));
+    const auto kernel = fp4 ? gemm_tc_pair_kernel<true, SUM> : gemm_tc_pair_kernel<false, SUM>;
+    MELA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, P_SMEM_BYTES));
+    kernel<<<grid, P_THREADS, P_SMEM_BYTES, s>>>(ma, mb, C, ldc, m, n, (int)tiles_m, (int)tiles_n, (int)(kp / BK),
+                                           device_error_word(), out);
+    MELA_LAUNCH_CHECK("gemm_tc_pair_kernel");
+    return MELA_OK;
+}
+
 mela_status launch_gemm_tc(const unsigned char *A8, const unsigned char *Bt8, i64 mp, i64 np,
                            i64 kp, u64 *C, i64 ldc, i64 m, i64 n, cudaStream_t s, bool fp4, int tile)
 {
@@ -540,26 +608,7 @@ mela_status launch_gemm_tc(const unsigned char *A8, const unsigned char *Bt8, i6
         return MELA_ERR_UNSUPPORTED;
     }
     if (use_pairs(mp, tile)) {
-        CUtensorMap ma, mb;
-        mela_status st = make_map(&ma, A8, mp, kp, 128);
-        if (st != MELA_OK) return st;
-        st = make_map(&mb, Bt8, np, kp, 128);
-        if (st != MELA_OK) return st;
-        const i64 ntiles = (mp / 256) * tiles_n, clusters_max = sm_count() / 2;
-        const unsigned grid = (unsigned)(2 * (ntiles < clusters_max ? ntiles : clusters_max));
-        if (fp4) {
-            MELA_CUDA_TRY(cudaFuncSetAttribute(gemm_tc_pair_kernel<true>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, P_SMEM_BYTES));
-            gemm_tc_pair_kernel<true><<<grid, 192, P_SMEM_BYTES, s>>>(ma, mb, C, ldc, m, n, (int)(mp / 256),
-                                                                       (int)tiles_n, (int)kst, device_error_word());
-        } else {
-            MELA_CUDA_TRY(cudaFuncSetAttribute(gemm_tc_pair_kernel<false>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, P_SMEM_BYTES));
-            gemm_tc_pair_kernel<false><<<grid, 192, P_SMEM_BYTES, s>>>(ma, mb, C, ldc, m, n, (int)(mp / 256),
-                                                                        (int)tiles_n, (int)kst, device_error_word());
-        }
-        MELA_LAUNCH_CHECK("gemm_tc_pair_kernel");
-        return MELA_OK;
+        return launch_pairs<false>(A8, Bt8, mp, np, kp, C, ldc, m, n, fp4, PairSum{}, s);
     }
     CUtensorMap ma, mb;
     mela_status st = make_map(&ma, A8, mp, kp, BM);
@@ -585,6 +634,85 @@ mela_status launch_gemm_tc(const unsigned char *A8, const unsigned char *Bt8, i6
     kernel<<<grid, 192, SMEM_BYTES, s>>>(ma, mb, C, ldc, m, n, (int)tiles_m, (int)tiles_n, (int)kst, (int)per,
                                          device_error_word());
     MELA_LAUNCH_CHECK("gemm_tc_kernel");
+    return MELA_OK;
+}
+
+// ---------------------------------------------------------------- Strassen
+// Seven products of half-size blocks instead of eight (Strassen 1969; over
+// GF(2) every sign is +).  The sums of blocks cost no pass of their own: the
+// expansion reads both blocks of an operand and XORs them, and the epilogue
+// adds a product to each block of C that it belongs to.  Blocks are halves of
+// whole 256-bit tiles; the second ones are as short as the matrix leaves them
+// and count as zero past that.
+// Where it pays (device time, whole -> seven products): the seventh of the MMA
+// work saved has to cover 7/4 of the expansion and the worse efficiency of
+// products of half the K.  FP4: 32768^3 11.33 -> 9.97 ms (under the power cap
+// either way), 30001 x 27003 x 29999 7.85 -> 7.22, 27200^3 6.53 -> 6.24, 24576^3
+// 4.58 -> 4.59, 16384^3 1.39 -> 1.54; with K = 16384, 40000 x 16384 x 32768
+// 6.50 -> 6.59.  INT8, half the rate: 32768^3 20.9 -> 17.7 ms, 20480^3 4.87 ->
+// 4.66, 22000 x 16384 x 22300 4.56 -> 4.40, 16384^3 2.49 -> 2.50.
+constexpr i64 ST_MIN = 16384, ST_K_F4 = 20480;
+constexpr double ST_CELLS_F4 = 2e13, ST_CELLS_I8 = 8e12;
+
+bool gemm_strassen_fits(const u64 *A, i64 lda, const u64 *B, i64 ldb, const u64 *C, i64 ldc, i64 m, i64 k, i64 n,
+                        bool fp4, int tile)
+{
+    if (m < ST_MIN || k < (fp4 ? ST_K_F4 : ST_MIN) || n < ST_MIN || !use_pairs(256, tile)) return false;
+    if ((double)m * (double)k * (double)n < (fp4 ? ST_CELLS_F4 : ST_CELLS_I8)) return false;
+    // blocks of A and B are read after blocks of C are written
+    auto apart = [&](const u64 *x, i64 ldx, i64 rows, i64 cols) {
+        return x + (rows - 1) * ldx + words_of(cols) <= C || C + (m - 1) * ldc + words_of(n) <= x;
+    };
+    return apart(A, lda, m, k) && apart(B, ldb, k, n);
+}
+
+mela_status launch_gemm_strassen(const u64 *A, i64 lda, const u64 *B, i64 ldb, u64 *C, i64 ldc, i64 m, i64 k, i64 n,
+                                 void *ws, size_t ws_bytes, bool fp4, cudaStream_t s)
+{
+    auto half = [](i64 x) { return ((x + 1) / 2 + 255) / 256 * 256; };
+    const i64 mh = half(m), kh = half(k), nh = half(n), kp = fp4 ? kh / 2 : kh;
+    unsigned char *A8 = (unsigned char *)ws, *B8 = A8 + (size_t)mh * kp;
+    if ((uintptr_t)ws & 15) {
+        set_error("gemm_tc: operands must be 16-byte aligned");
+        return MELA_ERR_INVALID;
+    }
+    if ((size_t)(mh + nh) * kp > ws_bytes) {
+        set_error("gemm_strassen: workspace of %zu bytes needed, %zu given", (size_t)(mh + nh) * kp, ws_bytes);
+        return MELA_ERR_INVALID;
+    }
+    auto a = [&](int i, int j) {
+        return ExpandBlock{A + i * mh * lda + j * (kh / 64), i ? m - mh : mh, j ? k - kh : kh};
+    };
+    auto b = [&](int i, int j) {
+        return ExpandBlock{B + i * kh * ldb + j * (nh / 64), i ? k - kh : kh, j ? n - nh : nh};
+    };
+    const ExpandBlock none;
+    const struct {
+        ExpandBlock a[2], b[2];
+        int c[2], first[2];  // blocks of C (2 i + j, -1: none), and whether this product is the first there
+    } step[7] = {
+        {{a(0, 0), a(1, 1)}, {b(0, 0), b(1, 1)}, {0, 3}, {1, 1}},
+        {{a(1, 0), a(1, 1)}, {b(0, 0), none}, {2, 3}, {1, 0}},
+        {{a(0, 0), none}, {b(0, 1), b(1, 1)}, {1, 3}, {1, 0}},
+        {{a(1, 1), none}, {b(1, 0), b(0, 0)}, {0, 2}, {0, 0}},
+        {{a(0, 0), a(0, 1)}, {b(1, 1), none}, {0, 1}, {0, 0}},
+        {{a(1, 0), a(0, 0)}, {b(0, 0), b(0, 1)}, {3, -1}, {0, 0}},
+        {{a(0, 1), a(1, 1)}, {b(1, 0), b(1, 1)}, {0, -1}, {0, 0}},
+    };
+    for (const auto &p : step) {
+        mela_status st = launch_expand_sum(p.a, lda, mh, A8, p.b, ldb, nh, B8, kp, fp4, s);
+        if (st != MELA_OK) return st;
+        PairSum out{};
+        for (int d = 0; d < 2; ++d) {
+            if (p.c[d] < 0) continue;
+            const int i = p.c[d] >> 1, j = p.c[d] & 1;
+            out.c[d] = C + i * mh * ldc + j * (nh / 64);
+            out.rows[d] = i ? m - mh : mh;
+            out.words[d] = words_of(j ? n - nh : nh);
+            out.add[d] = !p.first[d];
+        }
+        if ((st = launch_pairs<true>(A8, B8, mh, nh, kp, nullptr, ldc, mh, nh, fp4, out, s)) != MELA_OK) return st;
+    }
     return MELA_OK;
 }
 

@@ -21,6 +21,15 @@ mela_status launch_pack_words(int kind, i64 m, i64 n, const void *in, u64 *out, 
 mela_status launch_unpack(const u64 *in, i64 ld, i64 m, i64 n, unsigned char *out, cudaStream_t s);
 mela_status launch_transpose(const u64 *in, i64 ld_in, i64 rows, i64 cols, u64 *out, i64 ld_out,
                              cudaStream_t s);
+// A block of a packed matrix (its pitch given beside it); rows = 0: empty.
+struct ExpandBlock {
+    const u64 *p = nullptr;
+    i64 rows = 0, cols = 0;
+};
+// Both operands as sums of two blocks, A[0] + A[1] (K in columns) and B[0] +
+// B[1] (K in rows), expanded to mp x kp and np x kp.
+mela_status launch_expand_sum(const ExpandBlock (&A)[2], i64 lda, i64 mp, unsigned char *A8, const ExpandBlock (&B)[2],
+                              i64 ldb, i64 np, unsigned char *B8, i64 kp, bool fp4, cudaStream_t s);
 // Tensor-core operands, both K-major with kp bytes per row (0/1 bytes, or e2m1
 // pairs when fp4), zero past the matrices' edges: A8 (mp rows) from the packed
 // m x k matrix A, B8 (np rows, a multiple of 256) from the columns of the packed
@@ -41,6 +50,13 @@ mela_status launch_gemm_plain(const u64 *A, i64 lda, const u64 *Bt, i64 ldbt, u6
 // 128 x 256 tile; 1 = always one CTA per tile; 2 = pairs where mp allows.
 mela_status launch_gemm_tc(const unsigned char *A8, const unsigned char *Bt8, i64 mp, i64 np,
                            i64 kp, u64 *C, i64 ldc, i64 m, i64 n, cudaStream_t s, bool fp4, int tile = 0);
+// One level of Strassen's algorithm over packed operands, the workspace (two
+// expanded quarter operands) at ws; fits: where it beats one product of the
+// whole, and C overlaps neither operand.
+bool gemm_strassen_fits(const u64 *A, i64 lda, const u64 *B, i64 ldb, const u64 *C, i64 ldc, i64 m, i64 k, i64 n,
+                        bool fp4, int tile);
+mela_status launch_gemm_strassen(const u64 *A, i64 lda, const u64 *B, i64 ldb, u64 *C, i64 ldc, i64 m, i64 k, i64 n,
+                                 void *ws, size_t ws_bytes, bool fp4, cudaStream_t s);
 // TMA map of a K-major byte matrix rows x kp (row pitch kp bytes): boxes of
 // 128 bytes x box_rows rows with 128-byte swizzle, as the tcgen05 kernels read them.
 mela_status make_u8_kmajor_map(CUtensorMap *map, const unsigned char *base, i64 rows, i64 kp, int box_rows);

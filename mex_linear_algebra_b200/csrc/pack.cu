@@ -236,8 +236,10 @@ __global__ void __launch_bounds__(256) transpose_kernel(const u64 *__restrict__ 
 // 64); zero outside rows x kbits.  One thread per 64-bit word -> 64 bytes.
 __device__ __forceinline__ u32 spread4(u32 nib) { return (nib * 0x00204081u) & 0x01010101u; }
 
-__device__ __forceinline__ void expand_u8(const u64 *__restrict__ in, i64 ld, i64 rows, i64 kbits, i64 rows_pad,
-                                          i64 kpad, unsigned char *__restrict__ out, i64 block, i64 blocks)
+template <bool SUM>
+__device__ __forceinline__ void expand_u8(const u64 *__restrict__ in, i64 ld, i64 rows, i64 kbits,
+                                          const ExpandBlock &in2, i64 rows_pad, i64 kpad,
+                                          unsigned char *__restrict__ out, i64 block, i64 blocks)
 {
     const i64 wpr = kpad >> 6;  // words per padded row
     const i64 total = rows_pad * wpr;
@@ -245,6 +247,7 @@ __device__ __forceinline__ void expand_u8(const u64 *__restrict__ in, i64 ld, i6
     for (i64 t = block * 256 + threadIdx.x; t < total; t += blocks * 256) {
         const i64 r = t / wpr, w = t - r * wpr;
         u64 v = (r < rows && w < wc) ? in[r * ld + w] : 0ull;
+        if (SUM && r < in2.rows && w < words_of(in2.cols)) v ^= in2.p[r * ld + w];
         uint4 *dst = reinterpret_cast<uint4 *>(out + r * kpad + w * 64);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -267,15 +270,18 @@ __device__ __forceinline__ u32 spread_even4(u32 v)  // bits 0,2,4,6 -> bit 0 of 
     return (v & 1u) | ((v & 4u) << 6) | ((v & 16u) << 12) | ((v & 64u) << 18);
 }
 
-__device__ __forceinline__ void expand_f4(const u64 *__restrict__ in, i64 ld, i64 rows, i64 kbits, i64 rows_pad,
-                                          i64 kpad_bytes, unsigned char *__restrict__ out, i64 block, i64 blocks)
+template <bool SUM>
+__device__ __forceinline__ void expand_f4(const u64 *__restrict__ in, i64 ld, i64 rows, i64 kbits,
+                                          const ExpandBlock &in2, i64 rows_pad, i64 kpad_bytes,
+                                          unsigned char *__restrict__ out, i64 block, i64 blocks)
 {
     const i64 wpr = kpad_bytes >> 5;  // 64-bit source words per padded row
     const i64 total = rows_pad * wpr;
     const i64 wc = words_of(kbits);
     for (i64 t = block * 256 + threadIdx.x; t < total; t += blocks * 256) {
         const i64 r = t / wpr, w = t - r * wpr;
-        const u64 v = (r < rows && w < wc) ? in[r * ld + w] : 0ull;
+        u64 v = (r < rows && w < wc) ? in[r * ld + w] : 0ull;
+        if (SUM && r < in2.rows && w < words_of(in2.cols)) v ^= in2.p[r * ld + w];
         u32 o[8];
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
@@ -296,8 +302,9 @@ __device__ __forceinline__ void expand_f4(const u64 *__restrict__ in, i64 ld, i6
 // warp reads 32 rows of 256 bits (a lane per row) and turns them into
 // 32-bit column slices by five rounds of shuffle butterflies; the output rows
 // are written in 16-byte pieces, contiguous along k.
-template <bool F4>
-__device__ __forceinline__ void expand_t(const u64 *__restrict__ in, i64 ld, i64 kbits, i64 cols, i64 kpad,
+template <bool F4, bool SUM>
+__device__ __forceinline__ void expand_t(const u64 *__restrict__ in, i64 ld, i64 kbits, i64 cols,
+                                         const ExpandBlock &in2, i64 kpad,
                                          unsigned char *__restrict__ out, i64 jb, i64 kb0, u32 (&U)[256][9])
 {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -313,6 +320,11 @@ __device__ __forceinline__ void expand_t(const u64 *__restrict__ in, i64 ld, i64
         if (k < kbits && c < cols) {
             v = in32[k * 2 * ld + (c >> 5)];
             if (cols - c < 32) v &= (1u << (cols - c)) - 1u;
+        }
+        if (SUM && k < in2.rows && c < in2.cols) {
+            u32 x = reinterpret_cast<const u32 *>(in2.p)[k * 2 * ld + (c >> 5)];
+            if (in2.cols - c < 32) x &= (1u << (in2.cols - c)) - 1u;
+            v ^= x;
         }
         a[g] = v;
     }
@@ -356,19 +368,21 @@ __device__ __forceinline__ void expand_t(const u64 *__restrict__ in, i64 ld, i64
 // be empty.  One launch instead of two: 2 us less per product of a few
 // thousand rows, where the expansion is launch-bound (2048 x 2048 x 1024: 11.3
 // us in all, 13.4 before).
-template <bool F4>
+// SUM: each operand is the sum of two blocks, A + A2 and B + B2 (A2, B2 may be
+// empty), of k rows or columns and zero past their own sizes.
+template <bool F4, bool SUM>
 __global__ void __launch_bounds__(256) expand_kernel(const u64 *__restrict__ A, i64 lda, i64 m, i64 mp,
                                                      unsigned char *__restrict__ A8, const u64 *__restrict__ B,
-                                                     i64 ldb, i64 n, unsigned char *__restrict__ B8, i64 k, i64 kp,
-                                                     i64 tb, i64 tj)
+                                                     i64 ldb, i64 n, unsigned char *__restrict__ B8, i64 ka, i64 kb,
+                                                     i64 kp, i64 tb, i64 tj, ExpandBlock A2, ExpandBlock B2)
 {
     __shared__ u32 U[256][9];
     if ((i64)blockIdx.x < tb)
-        expand_t<F4>(B, ldb, k, n, kp, B8, (i64)blockIdx.x % tj, (i64)blockIdx.x / tj, U);
+        expand_t<F4, SUM>(B, ldb, kb, n, B2, kp, B8, (i64)blockIdx.x % tj, (i64)blockIdx.x / tj, U);
     else if (F4)
-        expand_f4(A, lda, m, k, mp, kp, A8, (i64)blockIdx.x - tb, (i64)gridDim.x - tb);
+        expand_f4<SUM>(A, lda, m, ka, A2, mp, kp, A8, (i64)blockIdx.x - tb, (i64)gridDim.x - tb);
     else
-        expand_u8(A, lda, m, k, mp, kp, A8, (i64)blockIdx.x - tb, (i64)gridDim.x - tb);
+        expand_u8<SUM>(A, lda, m, ka, A2, mp, kp, A8, (i64)blockIdx.x - tb, (i64)gridDim.x - tb);
 }
 
 // ---------------------------------------------------------------- launchers
@@ -395,10 +409,22 @@ mela_status launch_expand(const u64 *A, i64 lda, i64 m, i64 mp, unsigned char *A
     const i64 tb = np > 0 ? tj * tk : 0;
     const i64 ta = mp > 0 ? grid_for(mp * (kp >> (fp4 ? 5 : 6)), 256) : 0;
     if (ta + tb == 0) return MELA_OK;
-    if (fp4)
-        expand_kernel<true><<<(unsigned)(ta + tb), 256, 0, s>>>(A, lda, m, mp, A8, B, ldb, n, B8, k, kp, tb, tj);
-    else
-        expand_kernel<false><<<(unsigned)(ta + tb), 256, 0, s>>>(A, lda, m, mp, A8, B, ldb, n, B8, k, kp, tb, tj);
+    const auto kernel = fp4 ? expand_kernel<true, false> : expand_kernel<false, false>;
+    kernel<<<(unsigned)(ta + tb), 256, 0, s>>>(A, lda, m, mp, A8, B, ldb, n, B8, k, k, kp, tb, tj, ExpandBlock{},
+                                               ExpandBlock{});
+    MELA_LAUNCH_CHECK("expand_kernel");
+    return MELA_OK;
+}
+
+mela_status launch_expand_sum(const ExpandBlock (&A)[2], i64 lda, i64 mp, unsigned char *A8, const ExpandBlock (&B)[2],
+                              i64 ldb, i64 np, unsigned char *B8, i64 kp, bool fp4, cudaStream_t s)
+{
+    const i64 kvals = fp4 ? 2 * kp : kp, tj = np / 256, tk = (kvals + 255) / 256;
+    if (mela_status st = check_grid_yz(tk, 1, "expand_t"); st != MELA_OK) return st;
+    const i64 tb = tj * tk, ta = grid_for(mp * (kp >> (fp4 ? 5 : 6)), 256);
+    const auto kernel = fp4 ? expand_kernel<true, true> : expand_kernel<false, true>;
+    kernel<<<(unsigned)(ta + tb), 256, 0, s>>>(A[0].p, lda, A[0].rows, mp, A8, B[0].p, ldb, B[0].cols, B8, A[0].cols,
+                                               B[0].rows, kp, tb, tj, A[1], B[1]);
     MELA_LAUNCH_CHECK("expand_kernel");
     return MELA_OK;
 }
