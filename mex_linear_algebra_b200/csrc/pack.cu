@@ -232,65 +232,96 @@ __global__ void __launch_bounds__(256) transpose_kernel(const u64 *__restrict__ 
 }
 
 // ---------------------------------------------------------------- expand to bytes
-// out[r][k] = bit k of packed row r, for r < rows_pad, k < kpad (multiple of
-// 64); zero outside rows x kbits.  One thread per 64-bit word -> 64 bytes.
 __device__ __forceinline__ u32 spread4(u32 nib) { return (nib * 0x00204081u) & 0x01010101u; }
-
-template <bool SUM>
-__device__ __forceinline__ void expand_u8(const u64 *__restrict__ in, i64 ld, i64 rows, i64 kbits,
-                                          const ExpandBlock &in2, i64 rows_pad, i64 kpad,
-                                          unsigned char *__restrict__ out, i64 block, i64 blocks)
+// 16 bits -> 16 bytes of 0/1.
+__device__ __forceinline__ uint4 bytes_16(u32 v)
 {
-    const i64 wpr = kpad >> 6;  // words per padded row
-    const i64 total = rows_pad * wpr;
-    const i64 wc = words_of(kbits);
-    for (i64 t = block * 256 + threadIdx.x; t < total; t += blocks * 256) {
-        const i64 r = t / wpr, w = t - r * wpr;
-        u64 v = (r < rows && w < wc) ? in[r * ld + w] : 0ull;
-        if (SUM && r < in2.rows && w < words_of(in2.cols)) v ^= in2.p[r * ld + w];
-        uint4 *dst = reinterpret_cast<uint4 *>(out + r * kpad + w * 64);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            u32 h = (u32)(v >> (16 * q));
-            uint4 o;
-            o.x = spread4(h & 15);
-            o.y = spread4((h >> 4) & 15);
-            o.z = spread4((h >> 8) & 15);
-            o.w = spread4((h >> 12) & 15);
-            dst[q] = o;
+    return make_uint4(spread4(v & 15), spread4((v >> 4) & 15), spread4((v >> 8) & 15), spread4((v >> 12) & 15));
+}
+// 8 bits at 1..8 of v -> bit 1 of 8 nibbles (e2m1 values 0x2 = 1.0, 0).
+__device__ __forceinline__ u32 e2m1_8(u32 v)
+{
+    v = (v | (v << 12)) & 0x001E001Eu;
+    v = (v | (v << 6)) & 0x06060606u;
+    return (v | (v << 3)) & 0x22222222u;
+}
+// 32 bits -> 32 e2m1 values, value j in nibble j & 1 of byte j / 2.
+__device__ __forceinline__ uint4 e2m1_32(u32 v)
+{
+    return make_uint4(e2m1_8((v << 1) & 0x1FEu), e2m1_8((v >> 7) & 0x1FEu), e2m1_8((v >> 15) & 0x1FEu),
+                      e2m1_8((v >> 23) & 0x1FEu));
+}
+
+// Rows of A: out (rows_pad x kpad bytes) = the values of bits 0 .. kpad's of
+// each packed row, zero outside rows x kbits (whole words; the matrix's bits
+// past its columns are zero).  A thread per 16 bytes, the lanes' pieces side by
+// side: bound by the writes (both operands of 32768^3: FP4 260 us, 5.2 TB/s,
+// against 368 with a word and a 64-bit division a thread; INT8 427 against 567;
+// of 2048 x 2048 x 1024 in FP4 3.1 against 4.5).  Row and piece advance by the
+// grid's step in both, so that only the step is divided out.
+template <bool F4, bool SUM>
+__device__ __forceinline__ void expand_rows(const u64 *__restrict__ in, i64 ld, i64 rows, i64 kbits,
+                                            const ExpandBlock &in2, i64 rows_pad, i64 kpad,
+                                            unsigned char *__restrict__ out, i64 block, i64 blocks)
+{
+    constexpr int PPW = F4 ? 2 : 4;  // pieces per packed word
+    const i64 ppr = kpad >> 4, total = rows_pad * ppr, step = blocks * 256;
+    const i64 pc = words_of(kbits) * PPW, pc2 = words_of(in2.cols) * PPW;
+    auto piece = [&](const u64 *p, i64 r, i64 q) -> u32 {
+        if (F4) return reinterpret_cast<const u32 *>(p)[r * 2 * ld + q];
+        return reinterpret_cast<const unsigned short *>(p)[r * 4 * ld + q];
+    };
+    i64 t = block * 256 + threadIdx.x, r, dr = 0;
+    if (total + step <= 0x7fffffff) {
+        r = (u32)t / (u32)ppr;
+        if (step < total) dr = (u32)step / (u32)ppr;
+    } else {
+        r = t / ppr;
+        dr = step / ppr;
+    }
+    i64 q = t - r * ppr;
+    const i64 dq = step - dr * ppr;
+    for (; t < total; t += step) {
+        u32 v = r < rows && q < pc ? piece(in, r, q) : 0u;
+        if (SUM && r < in2.rows && q < pc2) v ^= piece(in2.p, r, q);
+        *reinterpret_cast<uint4 *>(out + r * kpad + 16 * q) = F4 ? e2m1_32(v) : bytes_16(v);
+        r += dr;
+        q += dq;
+        if (q >= ppr) {
+            q -= ppr;
+            ++r;
         }
     }
 }
 
-// out (rows_pad x kpad_bytes, two e2m1 values per byte): value k of row r is
-// 1.0 (0x2) when bit k of packed row r is set, else 0; element 2j in the low
-// nibble of byte j.  One thread per 64-bit word -> 32 bytes.
-__device__ __forceinline__ u32 spread_even4(u32 v)  // bits 0,2,4,6 -> bit 0 of bytes 0..3
+// 256 bits of row k from column j0 (a multiple of 256), zero past rows and
+// cols: two 16-byte loads where the row's words are so aligned and all inside.
+__device__ __forceinline__ void load_256(const u64 *__restrict__ in, i64 ld, i64 k, i64 rows, i64 j0, i64 cols,
+                                         u32 (&a)[8])
 {
-    return (v & 1u) | ((v & 4u) << 6) | ((v & 16u) << 12) | ((v & 64u) << 18);
-}
-
-template <bool SUM>
-__device__ __forceinline__ void expand_f4(const u64 *__restrict__ in, i64 ld, i64 rows, i64 kbits,
-                                          const ExpandBlock &in2, i64 rows_pad, i64 kpad_bytes,
-                                          unsigned char *__restrict__ out, i64 block, i64 blocks)
-{
-    const i64 wpr = kpad_bytes >> 5;  // 64-bit source words per padded row
-    const i64 total = rows_pad * wpr;
-    const i64 wc = words_of(kbits);
-    for (i64 t = block * 256 + threadIdx.x; t < total; t += blocks * 256) {
-        const i64 r = t / wpr, w = t - r * wpr;
-        u64 v = (r < rows && w < wc) ? in[r * ld + w] : 0ull;
-        if (SUM && r < in2.rows && w < words_of(in2.cols)) v ^= in2.p[r * ld + w];
-        u32 o[8];
+    if (k < rows && j0 + 256 <= cols && !((ld & 1) | ((uintptr_t)in & 15))) {
+        const uint4 *src = reinterpret_cast<const uint4 *>(in + k * ld + (j0 >> 6));
+        const uint4 x = src[0], y = src[1];
+        a[0] = x.x;
+        a[1] = x.y;
+        a[2] = x.z;
+        a[3] = x.w;
+        a[4] = y.x;
+        a[5] = y.y;
+        a[6] = y.z;
+        a[7] = y.w;
+        return;
+    }
+    const u32 *in32 = reinterpret_cast<const u32 *>(in);
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const u32 x = (u32)(v >> (8 * q)) & 0xFFu;
-            o[q] = (spread_even4(x & 0x55u) << 1) | (spread_even4((x >> 1) & 0x55u) << 5);
+    for (int g = 0; g < 8; ++g) {
+        const i64 c = j0 + 32 * g;  // first column of word g
+        u32 v = 0;
+        if (k < rows && c < cols) {
+            v = in32[k * 2 * ld + (c >> 5)];
+            if (cols - c < 32) v &= (1u << (cols - c)) - 1u;
         }
-        uint4 *dst = reinterpret_cast<uint4 *>(out + r * kpad_bytes + w * 32);
-        dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
-        dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
+        a[g] = v;
     }
 }
 
@@ -310,23 +341,14 @@ __device__ __forceinline__ void expand_t(const u64 *__restrict__ in, i64 ld, i64
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const i64 j0 = jb * 256, k0 = kb0 * 256;
     // lane = row k0 + 32 warp + lane; a[g] = its 32 bits of columns j0 + 32 g ...
-    const u32 *in32 = reinterpret_cast<const u32 *>(in);
     const i64 k = k0 + 32 * warp + lane;
     u32 a[8];
+    load_256(in, ld, k, kbits, j0, cols, a);
+    if (SUM) {
+        u32 b[8];
+        load_256(in2.p, ld, k, in2.rows, j0, in2.cols, b);
 #pragma unroll
-    for (int g = 0; g < 8; ++g) {
-        const i64 c = j0 + 32 * g;  // first column of word g
-        u32 v = 0;
-        if (k < kbits && c < cols) {
-            v = in32[k * 2 * ld + (c >> 5)];
-            if (cols - c < 32) v &= (1u << (cols - c)) - 1u;
-        }
-        if (SUM && k < in2.rows && c < in2.cols) {
-            u32 x = reinterpret_cast<const u32 *>(in2.p)[k * 2 * ld + (c >> 5)];
-            if (in2.cols - c < 32) x &= (1u << (in2.cols - c)) - 1u;
-            v ^= x;
-        }
-        a[g] = v;
+        for (int g = 0; g < 8; ++g) a[g] ^= b[g];
     }
     // 32 x 32 bit transposes across the warp: afterwards lane l's a[g] holds,
     // at bit r, row k0 + 32 warp + r of column j0 + 32 g + l
@@ -341,14 +363,7 @@ __device__ __forceinline__ void expand_t(const u64 *__restrict__ in, i64 ld, i64
             const int j = e >> 3, q = e & 7;
             const i64 kb = (k0 + 32 * q) / 2;  // byte offset in the output row
             if (kb >= kpad) continue;
-            const u32 v = U[j][q];
-            u32 o[4];
-#pragma unroll
-            for (int h = 0; h < 4; ++h) {
-                const u32 x = (v >> (8 * h)) & 0xFFu;
-                o[h] = (spread_even4(x & 0x55u) << 1) | (spread_even4((x >> 1) & 0x55u) << 5);
-            }
-            *reinterpret_cast<uint4 *>(out + (j0 + j) * kpad + kb) = make_uint4(o[0], o[1], o[2], o[3]);
+            *reinterpret_cast<uint4 *>(out + (j0 + j) * kpad + kb) = e2m1_32(U[j][q]);
         }
     } else {
         // column j, k slice q (16 values): 16 bytes of 0/1
@@ -356,9 +371,7 @@ __device__ __forceinline__ void expand_t(const u64 *__restrict__ in, i64 ld, i64
             const int j = e >> 4, q = e & 15;
             const i64 kb = k0 + 16 * q;
             if (kb >= kpad) continue;
-            const u32 h = (U[j][q >> 1] >> (16 * (q & 1))) & 0xFFFFu;
-            *reinterpret_cast<uint4 *>(out + (j0 + j) * kpad + kb) =
-                make_uint4(spread4(h & 15), spread4((h >> 4) & 15), spread4((h >> 8) & 15), spread4((h >> 12) & 15));
+            *reinterpret_cast<uint4 *>(out + (j0 + j) * kpad + kb) = bytes_16(U[j][q >> 1] >> (16 * (q & 1)));
         }
     }
 }
@@ -367,7 +380,7 @@ __device__ __forceinline__ void expand_t(const u64 *__restrict__ in, i64 ld, i64
 // B's 256 x 256 tiles (tj tiles a row), the others A's rows.  Either part may
 // be empty.  One launch instead of two: 2 us less per product of a few
 // thousand rows, where the expansion is launch-bound (2048 x 2048 x 1024: 11.3
-// us in all, 13.4 before).
+// us for the product against 13.4).
 // SUM: each operand is the sum of two blocks, A + A2 and B + B2 (A2, B2 may be
 // empty), of k rows or columns and zero past their own sizes.
 template <bool F4, bool SUM>
@@ -379,10 +392,8 @@ __global__ void __launch_bounds__(256) expand_kernel(const u64 *__restrict__ A, 
     __shared__ u32 U[256][9];
     if ((i64)blockIdx.x < tb)
         expand_t<F4, SUM>(B, ldb, kb, n, B2, kp, B8, (i64)blockIdx.x % tj, (i64)blockIdx.x / tj, U);
-    else if (F4)
-        expand_f4<SUM>(A, lda, m, ka, A2, mp, kp, A8, (i64)blockIdx.x - tb, (i64)gridDim.x - tb);
     else
-        expand_u8<SUM>(A, lda, m, ka, A2, mp, kp, A8, (i64)blockIdx.x - tb, (i64)gridDim.x - tb);
+        expand_rows<F4, SUM>(A, lda, m, ka, A2, mp, kp, A8, (i64)blockIdx.x - tb, (i64)gridDim.x - tb);
 }
 
 // ---------------------------------------------------------------- launchers
@@ -407,7 +418,7 @@ mela_status launch_expand(const u64 *A, i64 lda, i64 m, i64 mp, unsigned char *A
     if (np > 0)
         if (mela_status st = check_grid_yz(tk, 1, "expand_t"); st != MELA_OK) return st;
     const i64 tb = np > 0 ? tj * tk : 0;
-    const i64 ta = mp > 0 ? grid_for(mp * (kp >> (fp4 ? 5 : 6)), 256) : 0;
+    const i64 ta = mp > 0 ? grid_for(mp * (kp >> 4), 256) : 0;
     if (ta + tb == 0) return MELA_OK;
     const auto kernel = fp4 ? expand_kernel<true, false> : expand_kernel<false, false>;
     kernel<<<(unsigned)(ta + tb), 256, 0, s>>>(A, lda, m, mp, A8, B, ldb, n, B8, k, k, kp, tb, tj, ExpandBlock{},
@@ -421,7 +432,7 @@ mela_status launch_expand_sum(const ExpandBlock (&A)[2], i64 lda, i64 mp, unsign
 {
     const i64 kvals = fp4 ? 2 * kp : kp, tj = np / 256, tk = (kvals + 255) / 256;
     if (mela_status st = check_grid_yz(tk, 1, "expand_t"); st != MELA_OK) return st;
-    const i64 tb = tj * tk, ta = grid_for(mp * (kp >> (fp4 ? 5 : 6)), 256);
+    const i64 tb = tj * tk, ta = grid_for(mp * (kp >> 4), 256);
     const auto kernel = fp4 ? expand_kernel<true, true> : expand_kernel<false, true>;
     kernel<<<(unsigned)(ta + tb), 256, 0, s>>>(A[0].p, lda, A[0].rows, mp, A8, B[0].p, ldb, B[0].cols, B8, A[0].cols,
                                                B[0].rows, kp, tb, tj, A[1], B[1]);
