@@ -188,20 +188,51 @@ Readback *readback()
 }
 }  // namespace
 
-mela_status finish(cudaStream_t s)
+// Waits for s; r holds the device error word by then (null: ask for it).
+static mela_status finish_words(cudaStream_t s, const Readback *r)
 {
-    Readback *r = readback();
-    const u32 *word = device_error_word();
-    const bool queued = r && word && cudaMemcpyAsync(&r->err, word, sizeof r->err, cudaMemcpyDeviceToHost, s) == cudaSuccess;
-    if (!queued) cudaGetLastError();
     MELA_CUDA_TRY(cudaStreamSynchronize(s));
-    if (queued && r->err == 0) return MELA_OK;
+    if (r && r->err == 0) return MELA_OK;
     u32 flags = 0;
     if (mela_device_error_flags(&flags, 1) == MELA_OK && (flags & kErrWaitTimeout)) {
         set_error("a bounded device-side wait timed out");
         return MELA_ERR_TIMEOUT;
     }
     return MELA_OK;
+}
+
+mela_status finish(cudaStream_t s)
+{
+    Readback *r = readback();
+    const u32 *word = device_error_word();
+    const bool queued = r && word && cudaMemcpyAsync(&r->err, word, sizeof r->err, cudaMemcpyDeviceToHost, s) == cudaSuccess;
+    if (!queued) cudaGetLastError();
+    return finish_words(s, queued ? r : nullptr);
+}
+
+bool posted(Posted *to)
+{
+    Readback *r = readback();
+    const u32 *word = device_error_word();
+    if (!r || !word) return false;
+    *to = Posted{&r->value, &r->err, word, r->small, kSmallBytes};
+    return true;
+}
+
+mela_status finish_posted(cudaStream_t s) { return finish_words(s, readback()); }
+
+void *posted_take()
+{
+    Readback *&slot = t_readback.dev[current_device()], *r = slot;
+    slot = nullptr;
+    return r;
+}
+
+void posted_give(void *words)
+{
+    Readback *&slot = t_readback.dev[current_device()];
+    if (slot) cudaFreeHost(slot);
+    slot = (Readback *)words;
 }
 
 mela_status read_value(long long *value, const long long *d, cudaStream_t s, bool last)

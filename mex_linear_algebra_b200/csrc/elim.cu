@@ -716,10 +716,10 @@ size_t elim_workspace(i64 m, i64 n)
 
 mela_status elim_device(int variant_arg, u64 *M, i64 ld, i64 m, i64 n, int rref, long long *d_rank,
                         long long *d_piv, long long *d_prow, void *ws, size_t ws_bytes,
-                        cudaStream_t s)
+                        cudaStream_t s, bool resolved)
 {
     Tuning tune{};
-    const bool chosen = MELA_VARIANT_BASE(variant_arg) == MELA_ELIM_AUTO;
+    const bool chosen = resolved || MELA_VARIANT_BASE(variant_arg) == MELA_ELIM_AUTO;
     if (m > 0 && n > 0) variant_arg = resolve_elim_variant(variant_arg, M, ld, m, n, rref, s);
     if (!decode_elim_variant(variant_arg, &tune)) {
         set_error("elimination: bad variant argument 0x%x", variant_arg);

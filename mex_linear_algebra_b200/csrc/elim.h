@@ -19,9 +19,10 @@ size_t elim_workspace(i64 m, i64 n);
 // Rank (rref = 0) or reduced row echelon form (rref = 1) of the packed m x n
 // matrix M, in place.  Writes the rank to d_rank, the pivot columns to d_piv
 // and the physical row of each RREF row to d_prow (both min(m,n) entries).
+// resolved: the caller has resolved AUTO to this variant.
 mela_status elim_device(int variant, u64 *M, i64 ld, i64 m, i64 n, int rref, long long *d_rank,
                         long long *d_piv, long long *d_prow, void *ws, size_t ws_bytes,
-                        cudaStream_t s);
+                        cudaStream_t s, bool resolved = false);
 
 // Forms by 256-column windows (elim_tc.cu), same contract as elim_device: the
 // trailing update on the tensor cores, or (tables) by Four-Russians tables.

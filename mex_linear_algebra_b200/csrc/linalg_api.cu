@@ -4,6 +4,7 @@
 // (pack, eliminate, extract the basis, unpack) and copy the result back.
 // Device entry points are stream-ordered on packed matrices.
 #include <algorithm>
+#include <cstring>
 
 #include "mela_common.cuh"
 #include "mela_internal.h"
@@ -14,17 +15,35 @@ namespace mela {
 
 static bool ok_kind(int k) { return k == MELA_KIND_LOGICAL || k == MELA_KIND_DOUBLE; }
 
+// Resolves *variant (chosen: it was AUTO) and says whether the result is the
+// single-CTA form in shared memory.
+static bool takes_small(int *variant, const u64 *P, i64 ld, i64 m, i64 n, int rref, cudaStream_t s, bool *chosen)
+{
+    if (m <= 0 || n <= 0 || !small_elim_fits(m, n)) return false;
+    *chosen = MELA_VARIANT_BASE(*variant) == MELA_ELIM_AUTO;
+    *variant = resolve_elim_variant(*variant, P, ld, m, n, rref, s);
+    return *variant == MELA_ELIM_FUSED;
+}
+
 // Rank of a packed device matrix (overwritten), read back to the host.
 mela_status rank_of_packed(u64 *P, i64 ld, i64 m, i64 n, int variant, cudaStream_t s, double *rank)
 {
     const i64 mn = m < n ? m : n;
-    DevBuf ws, out;
     mela_status st;
+    bool chosen = false;
+    Posted to;
+    if (takes_small(&variant, P, ld, m, n, 0, s, &chosen) && posted(&to)) {
+        if ((st = launch_small_post(P, ld, m, n, to, false, s)) != MELA_OK) return st;
+        if ((st = finish_posted(s)) != MELA_OK) return st;
+        *rank = (double)*to.value;
+        return MELA_OK;
+    }
+    DevBuf ws, out;
     const size_t wsb = elim_workspace(m, n);
     if ((st = ws.alloc(wsb, s)) != MELA_OK) return st;
     if ((st = out.alloc((size_t)(1 + 2 * mn) * 8, s)) != MELA_OK) return st;
     long long *d = (long long *)out.p;
-    st = elim_device(variant, P, ld, m, n, 0, d, d + 1, d + 1 + mn, ws.p, wsb, s);
+    st = elim_device(variant, P, ld, m, n, 0, d, d + 1, d + 1 + mn, ws.p, wsb, s, chosen);
     if (st != MELA_OK) return st;
     long long r = 0;
     if ((st = read_value(&r, d, s, true)) != MELA_OK) return st;
@@ -44,6 +63,23 @@ mela_status null_of_packed(u64 *P, i64 ld, i64 m, i64 n, int variant, mela_alloc
     }
     const i64 mn = m < n ? m : n;
     mela_status st;
+    bool chosen = false;
+    Posted to;
+    if (small_null_fits(m, n) && takes_small(&variant, P, ld, m, n, 1, s, &chosen) && posted(&to)) {
+        if ((st = launch_small_post(P, ld, m, n, to, true, s)) != MELA_OK) return st;
+        if ((st = finish_posted(s)) != MELA_OK) return st;
+        const i64 f = n - *to.value;
+        void *words = posted_take();
+        uint8_t *Z = alloc(ctx, n, f);
+        posted_give(words);
+        if (!Z && f > 0) {
+            set_error("output allocation failed");
+            return MELA_ERR_NOMEM;
+        }
+        if (nullity) *nullity = f;
+        if (f > 0) std::memcpy(Z, to.bytes, (size_t)f * n);
+        return MELA_OK;
+    }
     DevBuf ws, out;
     if ((st = out.alloc((size_t)(1 + 2 * (mn ? mn : 1)) * 8, s)) != MELA_OK) return st;
     long long *d = (long long *)out.p;
@@ -51,7 +87,7 @@ mela_status null_of_packed(u64 *P, i64 ld, i64 m, i64 n, int variant, mela_alloc
     if (m > 0) {
         const size_t wsb = elim_workspace(m, n);
         if ((st = ws.alloc(wsb, s)) != MELA_OK) return st;
-        st = elim_device(variant, P, ld, m, n, 1, d, d + 1, d + 1 + mn, ws.p, wsb, s);
+        st = elim_device(variant, P, ld, m, n, 1, d, d + 1, d + 1 + mn, ws.p, wsb, s, chosen);
         if (st != MELA_OK) return st;
         if ((st = read_value(&r, d, s, false)) != MELA_OK) return st;
     }

@@ -25,6 +25,14 @@ mela_status side_stream(cudaStream_t *s);
 // The calling thread's stream for capturing launch sequences into CUDA graphs
 // (a graph is captured there and launched on the caller's stream).
 mela_status capture_stream(cudaStream_t *s);
+// The calling thread's page-locked words for a kernel to write (false: there
+// are none), and the end of a call whose kernel has written them.
+bool posted(Posted *to);
+mela_status finish_posted(cudaStream_t s);
+// Out of the thread's hands around a caller's function that may call in here
+// again, and back.
+void *posted_take();
+void posted_give(void *words);
 // Synchronise `s` and turn a device-side wait timeout into MELA_ERR_TIMEOUT.
 mela_status finish(cudaStream_t s);
 // A device value read back to the host; last: this ends the call (finish).

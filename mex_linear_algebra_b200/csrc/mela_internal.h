@@ -82,6 +82,20 @@ mela_status launch_gemm_small(int kind_a, const void *A, int kind_b, const void 
 bool small_elim_fits(i64 m, i64 n);
 mela_status launch_small_elim(u64 *M, i64 ld, i64 m, i64 n, long long *d_rank, long long *d_piv,
                               long long *d_prow, cudaStream_t s);
+// The calling thread's page-locked words (api.cu: posted), which a kernel may
+// write itself: a value, the device error word (read at err_word) and bytes.
+struct Posted {
+    long long *value;
+    u32 *err;
+    const u32 *err_word;
+    unsigned char *bytes;
+    size_t bytes_size;
+};
+// The same elimination for a call that waits for the result: the rank and, for
+// a null space (of at most small_null_fits columns), the basis as logical
+// bytes, written to the caller's page-locked words.  M is left as it was.
+bool small_null_fits(i64 m, i64 n);
+mela_status launch_small_post(const u64 *M, i64 ld, i64 m, i64 n, const Posted &to, bool null_space, cudaStream_t s);
 size_t fused_workspace(i64 m, i64 n);
 mela_status launch_fused_elim(u64 *M, i64 ld, i64 m, i64 n, long long *d_rank, long long *d_piv,
                               long long *d_prow, void *ws, size_t ws_bytes, cudaStream_t s);
