@@ -167,6 +167,7 @@ struct Readback {
     u32 err;
     long long value;
     alignas(64) unsigned char small[kSmallBytes];
+    alignas(64) unsigned char in[24 << 10];
 };
 struct Readbacks {
     Readback *dev[kMaxDevices] = {};
@@ -215,7 +216,7 @@ bool posted(Posted *to)
     Readback *r = readback();
     const u32 *word = device_error_word();
     if (!r || !word) return false;
-    *to = Posted{&r->value, &r->err, word, r->small, kSmallBytes};
+    *to = Posted{&r->value, &r->err, word, r->small, r->in, kSmallBytes};
     return true;
 }
 
@@ -980,13 +981,35 @@ static mela_status matmul_host(const mela_host_matrix *A, const mela_host_matrix
     if (k > 0 && gemm_small_fits(m, k, n, ea, eb)) {
         if (variant == MELA_GEMM_AUTO) remember_variant(MELA_GEMM_PLAIN, -1.0);  // AND and parity, untabled
         const size_t ab = ((size_t)m * k * ea + 255) & ~(size_t)255, bb = ((size_t)k * n * eb + 255) & ~(size_t)255;
+        // The kernel writes up to 64 KB of result into the thread's page-locked
+        // words itself, where two copies and their start cost more than one
+        // GPU's scattered writes over the bus (64^3 43 -> 32 us a call, 200^3 52
+        // -> 47; 300 x 64 x 300, 90 KB, 51 -> 59).  Up to 24 KB of operands go
+        // up from there in one copy (100 x 120 x 80 34 -> 33 us, 16^3 38 -> 28;
+        // 64 x 200 x 64, 26 KB, 37 -> 41: the driver's own staging overlaps).
+        Posted to;
+        const bool post = (size_t)m * n <= ((size_t)64 << 10) && posted(&to);
         DevBuf all;
-        if ((st = all.alloc(ab + bb + (size_t)m * n, s)) != MELA_OK) return st;
-        unsigned char *dA = (unsigned char *)all.p, *dB = dA + ab, *dC = dB + bb;
-        MELA_CUDA_TRY(cudaMemcpyAsync(dA, A->data, (size_t)m * k * ea, cudaMemcpyHostToDevice, s));
-        MELA_CUDA_TRY(cudaMemcpyAsync(dB, B->data, (size_t)k * n * eb, cudaMemcpyHostToDevice, s));
+        if ((st = all.alloc(ab + bb + (post ? 0 : (size_t)m * n), s)) != MELA_OK) return st;
+        unsigned char *dA = (unsigned char *)all.p, *dB = dA + ab;
+        if (post && ab + bb <= ((size_t)24 << 10)) {
+            std::memcpy(to.in, A->data, (size_t)m * k * ea);
+            std::memcpy(to.in + ab, B->data, (size_t)k * n * eb);
+            MELA_CUDA_TRY(cudaMemcpyAsync(dA, to.in, ab + (size_t)k * n * eb, cudaMemcpyHostToDevice, s));
+        } else {
+            MELA_CUDA_TRY(cudaMemcpyAsync(dA, A->data, (size_t)m * k * ea, cudaMemcpyHostToDevice, s));
+            MELA_CUDA_TRY(cudaMemcpyAsync(dB, B->data, (size_t)k * n * eb, cudaMemcpyHostToDevice, s));
+        }
         t_upload_stats.direct_bytes += (int64_t)((size_t)m * k * ea + (size_t)k * n * eb);
-        if ((st = launch_gemm_small(A->kind, dA, B->kind, dB, dC, m, k, n, s)) != MELA_OK) return st;
+        if (post) {
+            st = launch_gemm_small(A->kind, dA, B->kind, dB, to.bytes, m, k, n, to.err_word, to.err, s);
+            if (st == MELA_OK) st = finish_posted(s);
+            if (st == MELA_OK) std::memcpy(C, to.bytes, (size_t)m * n);
+            return st;
+        }
+        unsigned char *dC = dB + bb;
+        st = launch_gemm_small(A->kind, dA, B->kind, dB, dC, m, k, n, nullptr, nullptr, s);
+        if (st != MELA_OK) return st;
         return download_finish(C, dC, (size_t)m * n, s);
     }
     const i64 lda = even_words(k), ldb = even_words(n), ldc = even_words(n);

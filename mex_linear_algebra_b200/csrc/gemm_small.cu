@@ -11,8 +11,8 @@
 // thread ANDs and XORs a row of A with four columns of B, the parity of the
 // final word giving the bit.
 // Bound by launch and load latency.  Whole gateway call, packed path -> this:
-// 16^3 52 -> 37 us, 64^3 62 -> 43, 100 x 120 x 80 logical 59 -> 43, double
-// 79 -> 62.
+// 16^3 52 -> 28 us, 64^3 62 -> 30, 100 x 120 x 80 logical 59 -> 33, double
+// 79 -> 55.
 #include "mela_common.cuh"
 #include "mela_internal.h"
 
@@ -33,13 +33,15 @@ __device__ __forceinline__ u32 bit_of(unsigned char x) { return x != 0; }
 
 template <typename TA, typename TB>
 __global__ void __launch_bounds__(256)
-gemm_small_kernel(const TA *__restrict__ A, const TB *__restrict__ B, unsigned char *__restrict__ C, int m, int k, int n)
+gemm_small_kernel(const TA *__restrict__ A, const TB *__restrict__ B, unsigned char *__restrict__ C, int m, int k, int n,
+                  const u32 *err, u32 *err_out)
 {
     __shared__ u32 As[SP_T][SP_KW + 1], Bs[SP_T][SP_KW + 1];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int i0 = (int)blockIdx.x * SP_T, j0 = (int)blockIdx.y * SP_T;
     const int i = i0 + lane;
     u32 acc[4] = {0, 0, 0, 0};
+    if (err_out && tid == 0 && blockIdx.x == 0 && blockIdx.y == 0) *err_out = *err;
     const int kw = (k + 31) >> 5;
     for (int q = warp; q < kw; q += 8) {
         const int c0 = 32 * q;
@@ -85,19 +87,19 @@ bool gemm_small_fits(i64 m, i64 k, i64 n, size_t a_size, size_t b_size)
 }
 
 mela_status launch_gemm_small(int kind_a, const void *A, int kind_b, const void *B, unsigned char *C, i64 m, i64 k,
-                              i64 n, cudaStream_t s)
+                              i64 n, const u32 *err, u32 *err_out, cudaStream_t s)
 {
     const dim3 grid((unsigned)((m + SP_T - 1) / SP_T), (unsigned)((n + SP_T - 1) / SP_T));
     const int mi = (int)m, ki = (int)k, ni = (int)n;
     const bool da = kind_a == MELA_KIND_DOUBLE, db = kind_b == MELA_KIND_DOUBLE;
     if (da && db)
-        gemm_small_kernel<<<grid, 256, 0, s>>>((const double *)A, (const double *)B, C, mi, ki, ni);
+        gemm_small_kernel<<<grid, 256, 0, s>>>((const double *)A, (const double *)B, C, mi, ki, ni, err, err_out);
     else if (da)
-        gemm_small_kernel<<<grid, 256, 0, s>>>((const double *)A, (const unsigned char *)B, C, mi, ki, ni);
+        gemm_small_kernel<<<grid, 256, 0, s>>>((const double *)A, (const unsigned char *)B, C, mi, ki, ni, err, err_out);
     else if (db)
-        gemm_small_kernel<<<grid, 256, 0, s>>>((const unsigned char *)A, (const double *)B, C, mi, ki, ni);
+        gemm_small_kernel<<<grid, 256, 0, s>>>((const unsigned char *)A, (const double *)B, C, mi, ki, ni, err, err_out);
     else
-        gemm_small_kernel<<<grid, 256, 0, s>>>((const unsigned char *)A, (const unsigned char *)B, C, mi, ki, ni);
+        gemm_small_kernel<<<grid, 256, 0, s>>>((const unsigned char *)A, (const unsigned char *)B, C, mi, ki, ni, err, err_out);
     MELA_LAUNCH_CHECK("gemm_small_kernel");
     return MELA_OK;
 }

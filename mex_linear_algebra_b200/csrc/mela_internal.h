@@ -70,11 +70,12 @@ mela_status launch_gemm_m4ri(const u64 *A, i64 lda, const u64 *B, i64 ldb, u64 *
                              i64 m, i64 k, i64 n, cudaStream_t s, int tile = 0);
 
 // Product of small arrays in MATLAB layout (column-major, element kinds and
-// sizes as given) in one launch: C (m x n logical).  fits: where it beats
-// packing (gemm_small.cu).
+// sizes as given) in one launch: C (m x n logical), and the device error word
+// copied to err_out where that is given.  fits: where it beats packing
+// (gemm_small.cu).
 bool gemm_small_fits(i64 m, i64 k, i64 n, size_t a_size, size_t b_size);
 mela_status launch_gemm_small(int kind_a, const void *A, int kind_b, const void *B, unsigned char *C, i64 m, i64 k,
-                              i64 n, cudaStream_t s);
+                              i64 n, const u32 *err, u32 *err_out, cudaStream_t s);
 
 // Whole RREF of one matrix by one CTA in one launch: in shared memory where it
 // fits (elim_small.cu: up to 512 rows, 192 KB with its tables), else by the
@@ -88,8 +89,8 @@ struct Posted {
     long long *value;
     u32 *err;
     const u32 *err_word;
-    unsigned char *bytes;
-    size_t bytes_size;
+    unsigned char *bytes, *in;  // results; inputs on their way up (24 KB)
+    size_t bytes_size;          // of the results
 };
 // The same elimination for a call that waits for the result: the rank and, for
 // a null space (of at most small_null_fits columns), the basis as logical
