@@ -603,11 +603,13 @@ static mela_status upload_and_pack_blocks(const mela_host_matrix *M, u64 *dP, i6
 }
 
 // Device bytes into the caller's (pageable) array, ending the call on s.
-// Large results come down through the staging slots, the parallel host copy
-// of one piece (which also takes the array's first-touch page faults)
-// overlapping the download of the next two: 9.4 MB into a fresh array took the
-// driver's own pageable copy 1.2-3 ms.  Small ones land in the thread's
-// page-locked words, so that the result and the error word need one wait.
+// Results come down through the staging slots, the host copy of one piece
+// (which also takes the array's first-touch page faults) overlapping the
+// download of the next two: 9.4 MB into a fresh array took the driver's own
+// pageable copy 1.2-3 ms, 0.5 MB 60 us more than this (700 x 300 x 700 149 us
+// the whole call, 212).  Below 1 MiB the calling thread copies by itself, sooner
+// than the copy threads are awake.  Small ones land in the thread's page-locked
+// words, so that the result and the error word need one wait.
 mela_status download_finish(void *dst, const void *src, size_t bytes, cudaStream_t s)
 {
     Readback *rb = readback();
@@ -617,13 +619,15 @@ mela_status download_finish(void *dst, const void *src, size_t bytes, cudaStream
         if (st == MELA_OK) std::memcpy(dst, rb->small, bytes);
         return st;
     }
-    if (bytes < ((size_t)1 << 20) || !staging_ready()) {
+    if (!staging_ready()) {
         MELA_CUDA_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s));
         return finish(s);
     }
     Staging &S = t_stage[current_device()];
+    const bool alone = bytes < ((size_t)1 << 20);
+    const size_t least = (size_t)(alone ? 128 : 512) << 10;
     size_t piece = (bytes / 4 + 0xffff) & ~(size_t)0xffff;
-    if (piece < ((size_t)512 << 10)) piece = (size_t)512 << 10;
+    if (piece < least) piece = least;
     if (piece > kStageBytes) piece = kStageBytes;
     const size_t pieces = (bytes + piece - 1) / piece;
     const int first = S.next;
@@ -640,7 +644,10 @@ mela_status download_finish(void *dst, const void *src, size_t bytes, cudaStream
         const int slot = (int)((first + c) % kStageSlots);
         const size_t off = c * piece, len = bytes - off < piece ? bytes - off : piece;
         MELA_CUDA_TRY(cudaEventSynchronize(S.read[slot]));
-        CopyPool::get().copy((char *)dst + off, S.slot[slot], len, false);
+        if (alone)
+            std::memcpy((char *)dst + off, S.slot[slot], len);
+        else
+            CopyPool::get().copy((char *)dst + off, S.slot[slot], len, false);
     }
     return finish(s);
 }
