@@ -344,7 +344,7 @@ typedef struct {
 } mela_batch_item;
 typedef struct mela_batch_plan mela_batch_plan;
 
-/* force_class: -1 = size-based (normal); 0/1/2 = run every item that fits
+/* force_class: -1 = by size and count (normal); 0/1/2 = run every item that fits
  * with the CTA / 128-thread / warp engine (for testing the engines). */
 mela_status mela_batch_plan_create(const mela_batch_item *items, int64_t count,
                                    int32_t force_class, mela_batch_plan **plan);

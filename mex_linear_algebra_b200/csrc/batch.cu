@@ -64,7 +64,6 @@ constexpr int kSmallBudget = kSmemTotal / (kThreads / 32);       // 13.75 KB
 // other's table updates and transposes
 constexpr int kBatchThreads = 256;
 constexpr int kSmallMaxRows = 192;  // largest m for the warp engine
-constexpr int kMidMaxRows = 240;    // the 128-thread engine below this m
 constexpr int kBatchSmem = kSmemTotal / (kThreads / kBatchThreads);
 
 __host__ __device__ inline size_t al8(size_t x) { return (x + 7) & ~(size_t)7; }
@@ -1550,6 +1549,47 @@ static mela_status plan_free(BatchPlanImpl *P)
     return MELA_OK;
 }
 
+// The size rule: matrices up to this many rows (0: none) go to the warp engine,
+// if they fit it, the others to the CTA engine.  A warp holds an eighth of a
+// CTA's slot for about 7.4 ns x m x n, the CTA engine the slot for about 5 us +
+// 0.148 us x (m + n): a warp does more per slot, but a late one keeps the launch
+// waiting while the other slots are empty.  So warps are taken where the slot
+// time they save, over all slots, passes half of the longest one's.  (Parity-check
+// matrices, packed, warps up to 192 rows and 128 threads up to 240 before ->
+// this: 4000 of m in [64, 1024] 5.66 -> 5.38 ms, all on CTAs; 500 in [64, 500] 0.60 ->
+// 0.29; 4000 in [150, 400] 2.16 -> 1.79; 200 in [64, 128] 0.25 -> 0.07; 4000 in
+// [64, 192], all on warps, 0.58 (CTAs 0.80).  The 128-thread engine is slower
+// than a CTA or a warp at every size now -- 4000 in [192, 240] 2.06 ms against
+// 1.36 -- and is left to the forced and learned policies.)
+static long long warp_rows_of(const mela_batch_item *h, long long count)
+{
+    constexpr int kSteps = 5;
+    const long long rows[kSteps] = {64, 96, 128, 160, kSmallMaxRows};
+    double saved[kSteps] = {}, longest[kSteps] = {};
+    for (long long i = 0; i < count; ++i) {
+        const long long m = h[i].m, n = h[i].n;
+        if (m <= 0 || n <= 0 || m > kSmallMaxRows || n > kSmallBudget * 8) continue;
+        if (aux_bytes((int)m, (int)n) + (size_t)m * smem_ld((int)n) * 8 > (size_t)kSmallBudget) continue;
+        const double warp = 0.0074 * (double)m * (double)n, cta = 5.0 + 0.148 * (double)(m + n);
+        for (int k = 0; k < kSteps; ++k)
+            if (m <= rows[k]) {
+                saved[k] += cta - warp / (kThreads / 32 / (kThreads / kBatchThreads));
+                longest[k] = std::max(longest[k], warp);
+            }
+    }
+    long long pick = 0;
+    double best = 0;
+    const double slots = (double)(kThreads / kBatchThreads) * (double)sm_count();
+    for (int k = 0; k < kSteps; ++k) {
+        const double gain = saved[k] / slots - 0.5 * longest[k];
+        if (gain > best) {
+            best = gain;
+            pick = rows[k];
+        }
+    }
+    return pick;
+}
+
 // Engine per matrix.  policy -1: by fit and size (the fixed rule below);
 // 0/1/2: that engine wherever the matrix fits its region; -2: the installed
 // cost model's cheapest engine among those the matrix fits, given its shape,
@@ -1572,6 +1612,7 @@ static mela_status plan_create(const mela_batch_item *h, long long count, int fo
         }
         mix /= (double)(count ? count : 1);
     }
+    const long long warp_rows = warp_rows_of(h, count);
     BatchPlanImpl *P = new BatchPlanImpl();
     P->count = (int)count;
     std::vector<BatchDevItem> items((size_t)count);
@@ -1592,14 +1633,7 @@ static mela_status plan_create(const mela_batch_item *h, long long count, int fo
         d.z_off = h[i].z_offset;
         const size_t aux = aux_bytes((int)m, (int)n);
         const size_t mat = (size_t)m * smem_ld((int)n) * 8;
-        // Class by fit and size: with two CTAs per SM the blocked CTA engine
-        // beats the 128-thread column engine from m = 240 up (parity-check
-        // matrices, n = 2m: 7% faster at m in [230, 300), 23% at [380, 460)),
-        // and the column engine beats a warp from m = 160 up.
-        int c;
-        if (aux + mat <= (size_t)kSmallBudget && m <= kSmallMaxRows) c = 2;
-        else if (aux + mat <= (size_t)kMidBudget && m < kMidMaxRows) c = 1;
-        else c = 0;
+        int c = aux + mat <= (size_t)kSmallBudget && m <= warp_rows ? 2 : 0;
         if (force_class >= 0 && force_class <= 2) {
             // a forced class must still fit its region; otherwise fall back to big
             const size_t budget = force_class == 2 ? kSmallBudget : force_class == 1 ? kMidBudget : kSmemTotal;
