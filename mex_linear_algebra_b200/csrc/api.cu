@@ -607,9 +607,12 @@ static mela_status upload_and_pack_blocks(const mela_host_matrix *M, u64 *dP, i6
 // (which also takes the array's first-touch page faults) overlapping the
 // download of the next two: 9.4 MB into a fresh array took the driver's own
 // pageable copy 1.2-3 ms, 0.5 MB 60 us more than this (700 x 300 x 700 149 us
-// the whole call, 212).  Below 1 MiB the calling thread copies by itself, sooner
-// than the copy threads are awake.  Small ones land in the thread's page-locked
-// words, so that the result and the error word need one wait.
+// the whole call, 212).  Below 8 MiB the calling thread copies by itself: in a
+// fresh array the page faults of several threads get in one another's way (whole
+// calls, result of 2.2 MB: 0.37 ms, 0.78 with the copy threads, 0.51 by the
+// driver; 4.5 MB 0.62, 1.24, 0.88; in an array in use 0.43 and 0.45 at 4.5 MB, at
+// 16 MB 1.2 and 0.6).  Small ones land in the thread's page-locked words, so that
+// the result and the error word need one wait.
 mela_status download_finish(void *dst, const void *src, size_t bytes, cudaStream_t s)
 {
     Readback *rb = readback();
@@ -624,11 +627,11 @@ mela_status download_finish(void *dst, const void *src, size_t bytes, cudaStream
         return finish(s);
     }
     Staging &S = t_stage[current_device()];
-    const bool alone = bytes < ((size_t)1 << 20);
-    const size_t least = (size_t)(alone ? 128 : 512) << 10;
+    const bool alone = bytes < ((size_t)8 << 20);
+    const size_t least = (size_t)(alone ? 128 : 512) << 10, most = alone ? (size_t)1 << 20 : kStageBytes;
     size_t piece = (bytes / 4 + 0xffff) & ~(size_t)0xffff;
     if (piece < least) piece = least;
-    if (piece > kStageBytes) piece = kStageBytes;
+    if (piece > most) piece = most;
     const size_t pieces = (bytes + piece - 1) / piece;
     const int first = S.next;
     size_t issued = 0;
