@@ -24,7 +24,8 @@
 // the matrix edges.  The table builders read their 8 rows from that tile.
 // Few blocks of C leave most of the chip idle (3001 x 1777: six), so K is then
 // split over gridDim.z: each CTA multiplies its slice of the stages and XORs
-// its block into C, which starts as zero -- GF(2) sums need no order.
+// its block into C, which starts as zero -- GF(2) sums need no order.  (Not
+// where C overlaps A or B.)
 // Where TMA cannot address B (a row pitch that is not a multiple of 16 bytes,
 // or an unaligned base) the rows are read with ordinary loads instead.
 #include "mela_common.cuh"
@@ -221,8 +222,12 @@ mela_status launch_gemm_m4ri(const u64 *A, i64 lda, const u64 *B, i64 ldb, u64 *
     // 4 stages (one word of A; a stage takes 2.3 us, the launch, first loads and
     // the atomic writes of a block about 6).  3001 x 2500 x 1777: 25.5 us in 20
     // slices, 367 us unsplit; 8192^3 in two 0.64 ms, 1.21 ms unsplit.
+    // A result over an operand stays in one slice: a block of C is then written
+    // after its CTA's last read (C over A is right up to 2048 columns, one block
+    // wide, C over B up to 512 rows), where slices would clear the operand first.
     const i64 nstages = (k + 15) / 16;
     i64 splits = std::min<i64>(sm_count() / (gx * gy), (nstages + 3) / 4);
+    if (!packed_apart(A, lda, m, k, C, ldc, m, n) || !packed_apart(B, ldb, k, n, C, ldc, m, n)) splits = 1;
     i64 per = nstages;
     if (splits > 1) {
         per = ((nstages + splits - 1) / splits + 3) / 4 * 4;

@@ -660,10 +660,7 @@ bool gemm_strassen_fits(const u64 *A, i64 lda, const u64 *B, i64 ldb, const u64 
     if (m < ST_MIN || k < (fp4 ? ST_K_F4 : ST_MIN) || n < ST_MIN || !use_pairs(256, tile)) return false;
     if ((double)m * (double)k * (double)n < (fp4 ? ST_CELLS_F4 : ST_CELLS_I8)) return false;
     // blocks of A and B are read after blocks of C are written
-    auto apart = [&](const u64 *x, i64 ldx, i64 rows, i64 cols) {
-        return x + (rows - 1) * ldx + words_of(cols) <= C || C + (m - 1) * ldc + words_of(n) <= x;
-    };
-    return apart(A, lda, m, k) && apart(B, ldb, k, n);
+    return packed_apart(A, lda, m, k, C, ldc, m, n) && packed_apart(B, ldb, k, n, C, ldc, m, n);
 }
 
 mela_status launch_gemm_strassen(const u64 *A, i64 lda, const u64 *B, i64 ldb, u64 *C, i64 ldc, i64 m, i64 k, i64 n,
