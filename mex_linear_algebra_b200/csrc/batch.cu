@@ -568,13 +568,14 @@ __device__ void process_big_blocked(const BatchDevItem &it, const u64 *__restric
     // the matrix, eight words a thread in flight (one after the other the copy
     // took 141K of a 1000-row matrix's 1.88M cycles)
     const u64 *src = in + it.in_off;
-    for (int e0 = tid; e0 < m * wc; e0 += 8 * NT) {
+    const long long words = (long long)m * wc;  // may pass 2^31 (16 GiB)
+    for (long long e0 = tid; e0 < words; e0 += 8 * NT) {
         u64 v[8];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) v[u] = e0 + u * NT < m * wc ? src[e0 + u * NT] : 0ull;
+        for (int u = 0; u < 8; ++u) v[u] = e0 + u * NT < words ? src[e0 + u * NT] : 0ull;
 #pragma unroll
         for (int u = 0; u < 8; ++u)
-            if (e0 + u * NT < m * wc) A[e0 + u * NT] = v[u];
+            if (e0 + u * NT < words) A[e0 + u * NT] = v[u];
     }
     for (int j = tid; j < m; j += NT) active[j] = 1;
     __syncthreads();
