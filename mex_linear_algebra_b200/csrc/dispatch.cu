@@ -7,6 +7,7 @@
 // variants ask the installed cost model for a configuration -- measuring
 // the input's density on the device first -- or, without a model, apply
 // the fixed rule.  Nothing here changes a result.
+#include <climits>
 #include <cmath>
 
 #include "mela_common.cuh"
@@ -220,9 +221,35 @@ int32_t remember_variant(int32_t v, double density)
 // smallest) is taken as it is.
 constexpr double kMeasureCostUs = 15.0;
 
+// Whether a configuration takes a request of this shape at all: the limits
+// that its launches check (rows, or K, along a grid's y dimension, the pivot
+// buffer of the plain elimination).  The model knows times only and would send
+// a product of 10M rows to the plain form, which refuses it.
+static bool config_takes(int op, int c, double m, double n, double p)
+{
+    constexpr double kGridY = 65535;
+    const int32_t v = config_variant(op, c);
+    Tuning t{};
+    if (op == MELA_OP_MATMUL) {  // m x n times n x p
+        if (!decode_gemm_variant(v, &t)) return false;
+        switch (t.base) {
+        case MELA_GEMM_PLAIN: return m <= 128 * kGridY && n <= 256 * kGridY;
+        case MELA_GEMM_M4RI: return m <= 512 * kGridY && n <= 0x7fffffff - 16;
+        default: return n <= 256 * kGridY && (m / 128 + 2) * (p / 256 + 1) < 2147483647.0;
+        }
+    }
+    if (!decode_elim_variant(v, &t)) return false;
+    switch (t.base) {
+    case MELA_ELIM_PLAIN: return n <= 64 * 25600;
+    case MELA_ELIM_FUSED: return m <= INT_MAX / 2 && n <= INT_MAX / 2;
+    case MELA_ELIM_TC: return n <= 2147483648.0;
+    default: return m <= (t.row_tile ? t.row_tile : 1024) * kGridY;
+    }
+}
+
 // Without the density: the configuration whose worst predicted loss over
 // the probed densities is smallest (index), and whether that loss exceeds
-// what measuring costs.  -1 without a model.
+// what measuring costs.  -1 without a model or a configuration for the shape.
 static int choose_unmeasured(int op, double m, double n, double p, double cells, bool *measure)
 {
     static const double probe[kCostProbes] = {0.001, 0.01, 0.1, 0.5};
@@ -231,13 +258,17 @@ static int choose_unmeasured(int op, double m, double n, double p, double cells,
     float y[kCostProbes][MELA_MLP_OUT];
     double best[kCostProbes];
     if (nc <= 0 || !costmodel_predict_densities(op, m, n, p, probe, 1, lc, y)) return -1;
+    bool takes[MELA_MLP_OUT];
+    for (int c = 0; c < nc; ++c) takes[c] = config_takes(op, c, m, n, p);
     for (int d = 0; d < kCostProbes; ++d) {
         best[d] = 1e300;
-        for (int c = 0; c < nc; ++c) best[d] = std::fmin(best[d], std::exp2((double)y[d][c]));
+        for (int c = 0; c < nc; ++c)
+            if (takes[c]) best[d] = std::fmin(best[d], std::exp2((double)y[d][c]));
     }
-    int pick = 0;
+    int pick = -1;
     double pick_loss = 1e300;
     for (int c = 0; c < nc; ++c) {
+        if (!takes[c]) continue;
         double loss = 0;
         for (int d = 0; d < kCostProbes; ++d) loss = std::fmax(loss, std::exp2((double)y[d][c]) - best[d]);
         if (loss < pick_loss) {
@@ -287,7 +318,12 @@ static int choose_measuring(int op, double m, double n, double p, double cells,
     if (pick < 0 || !measure) return pick;
     const double d = measure_density(M, ld, rows, cols, s);
     t_last_density = d;
-    return costmodel_choose(op, m, n, p, d, 1, std::log2(cells > 1 ? cells : 1));
+    float y[MELA_MLP_OUT];
+    if (!costmodel_predict(op, m, n, p, d, 1, std::log2(cells > 1 ? cells : 1), y)) return pick;
+    int best = pick;
+    for (int c = 0; c < config_count(op); ++c)
+        if (y[c] < y[best] && config_takes(op, c, m, n, p)) best = c;
+    return best;
 }
 
 // ---------------------------------------------------------------- choices
