@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("tile", [0, 1, 2])
 @pytest.mark.parametrize("m,k,n,over", [(512, 512, 512, "A"), (100, 65, 65, "A"), (2000, 2048, 2048, "A"),
-                                        (513, 300, 260, "A"), (512, 512, 512, "B"), (130, 65, 100, "B"),
+                                        (513, 300, 260, "A"), (512, 512, 512, "B"), (65, 130, 100, "B"),
                                         (500, 512, 3000, "B")])
 def test_result_over_an_operand(cuda, m, k, n, over, tile):
     A, B = O.rand_dense(7, 0, m, k), O.rand_dense(7, 1, k, n)
