@@ -324,13 +324,25 @@ static mela_status check_ws(const GemmPlan &p, void *ws, size_t ws_bytes)
     return MELA_OK;
 }
 
+// A product's form.  AUTO only takes one that the call's buffers allow: the
+// tensor-core forms read their expanded operands with 16-byte accesses, the
+// Four-Russians form needs no workspace at all.
+static int32_t form_of(int32_t variant, const u64 *A, i64 lda, i64 m, i64 k, i64 n, const void *ws, cudaStream_t s)
+{
+    const int32_t v = resolve_gemm_variant(variant, A, lda, m, k, n, s);
+    if (v == variant || ((uintptr_t)ws & 15) == 0) return v;
+    double density;
+    mela_dispatch_last(&density);
+    return remember_variant(MELA_GEMM_M4RI, density);
+}
+
 // Operand preparation: B transposed (plain and tensor-core forms) and the
 // 0/1 byte expansion of A and Bt (tensor-core form).
 mela_status gemm_prepare(int variant, const u64 *A, i64 lda, const u64 *B, i64 ldb, i64 m, i64 k,
                          i64 n, void *ws, size_t ws_bytes, cudaStream_t s)
 {
     if (m == 0 || n == 0 || k == 0) return MELA_OK;
-    variant = resolve_gemm_variant(variant, A, lda, m, k, n, s);
+    variant = form_of(variant, A, lda, m, k, n, ws, s);
     GemmPlan p = plan_gemm(variant, m, k, n);
     mela_status st = check_ws(p, ws, ws_bytes);
     if (st != MELA_OK) return st;
@@ -346,6 +358,10 @@ mela_status gemm_prepare(int variant, const u64 *A, i64 lda, const u64 *B, i64 l
             MELA_CUDA_TRY(cudaMemset2DAsync(b.Bt + words_of(k), (size_t)p.ldbt * 8, 0, 8, (size_t)n, s));
         }
     }
+    if ((p.variant == MELA_GEMM_TC || p.variant == MELA_GEMM_TC_FP4) && ((uintptr_t)ws & 15)) {
+        set_error("mela_dev_matmul: the tensor-core forms need a 16-byte aligned workspace");
+        return MELA_ERR_INVALID;
+    }
     if (p.variant == MELA_GEMM_TC || p.variant == MELA_GEMM_TC_FP4)
         return launch_expand(A, lda, m, p.mp, b.A8, B, ldb, n, p.np, b.B8, k, p.kp, p.variant == MELA_GEMM_TC_FP4, s);
     return MELA_OK;
@@ -360,7 +376,7 @@ mela_status gemm_run(int variant, const u64 *A, i64 lda, const u64 *B, i64 ldb, 
         MELA_CUDA_TRY(cudaMemset2DAsync(C, (size_t)ldc * 8, 0, (size_t)words_of(n) * 8, (size_t)m, s));
         return MELA_OK;
     }
-    variant = resolve_gemm_variant(variant, A, lda, m, k, n, s);
+    variant = form_of(variant, A, lda, m, k, n, ws, s);
     GemmPlan p = plan_gemm(variant, m, k, n);
     mela_status st = check_ws(p, ws, ws_bytes);
     if (st != MELA_OK) return st;
@@ -384,8 +400,17 @@ mela_status gemm_run(int variant, const u64 *A, i64 lda, const u64 *B, i64 ldb, 
 mela_status gemm_device(int variant, const u64 *A, i64 lda, const u64 *B, i64 ldb, u64 *C, i64 ldc,
                         i64 m, i64 k, i64 n, void *ws, size_t ws_bytes, cudaStream_t s)
 {
-    if (m > 0 && n > 0 && k > 0) variant = resolve_gemm_variant(variant, A, lda, m, k, n, s);
     if (m > 0 && n > 0 && k > 0) {
+        const bool chosen = MELA_VARIANT_BASE(variant) == MELA_GEMM_AUTO;
+        variant = form_of(variant, A, lda, m, k, n, ws, s);
+        if (chosen && ((uintptr_t)ws & 15) == 0 &&
+            !(packed_apart(A, lda, m, k, C, ldc, m, n) && packed_apart(B, ldb, k, n, C, ldc, m, n))) {
+            // a result over an operand: the forms that expand both operands
+            // before they write are right at every size
+            double density;
+            mela_dispatch_last(&density);
+            variant = remember_variant(k < (1LL << 23) ? MELA_GEMM_TC_FP4 : MELA_GEMM_TC, density);
+        }
         const GemmPlan p = plan_gemm(variant, m, k, n);
         const bool fp4 = p.variant == MELA_GEMM_TC_FP4;
         if ((fp4 || p.variant == MELA_GEMM_TC) && k < (1LL << 23) &&

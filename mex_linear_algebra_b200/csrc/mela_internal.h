@@ -38,11 +38,16 @@ mela_status launch_expand(const u64 *A, i64 lda, i64 m, i64 mp, unsigned char *A
                           i64 np, unsigned char *B8, i64 k, i64 kp, bool fp4, cudaStream_t s);
 
 // ---- products (packed, device)
-// The words of two packed matrices (pitch, rows, columns) lie apart: a product
-// that writes its result before it has read all of an operand needs that.
+// The words of two packed matrices (pitch, rows, columns) lie apart, one after
+// the other or as column blocks of one buffer: a product that writes its result
+// before it has read all of an operand needs that.
 inline bool packed_apart(const u64 *x, i64 ldx, i64 rx, i64 cx, const u64 *y, i64 ldy, i64 ry, i64 cy)
 {
-    return x + (rx - 1) * ldx + words_of(cx) <= y || y + (ry - 1) * ldy + words_of(cy) <= x;
+    const i64 wx = words_of(cx), wy = words_of(cy);
+    if (x + (rx - 1) * ldx + wx <= y || y + (ry - 1) * ldy + wy <= x) return true;
+    if (ldx != ldy) return false;
+    const i64 at = (y >= x ? y - x : ldx - 1 - (x - y - 1) % ldx) % ldx;  // y's first word in a row from x's
+    return at >= wx && at + wy <= ldx;
 }
 // Plain AND+popcount product: C (m x n) = A (m x k) * B (k x n), with the
 // transposed right operand Bt (n x k) already formed.
