@@ -725,7 +725,7 @@ mela_status elim_device(int variant_arg, u64 *M, i64 ld, i64 m, i64 n, int rref,
         set_error("elimination: bad variant argument 0x%x", variant_arg);
         return MELA_ERR_INVALID;
     }
-    const int variant = tune.base;
+    int variant = tune.base;
     if (m == 0 || n == 0) {
         MELA_CUDA_TRY(cudaMemsetAsync(d_rank, 0, sizeof(long long), s));
         return MELA_OK;
@@ -741,8 +741,16 @@ mela_status elim_device(int variant_arg, u64 *M, i64 ld, i64 m, i64 n, int rref,
     // there the update hides behind the factorization either way, and the
     // tables take fewer and shorter launches (rank 3000 x 5000 372 us, 409 on
     // the tensor cores; RREF 4096 x 8192 603 / 656, 8192 x 8192 1230 / 1183).
-    const bool tables = variant_arg == MELA_ELIM_M4RI ||
-                        (chosen && variant == MELA_ELIM_TC && (double)m * (double)n <= 4e7);
+    // The windows want a 16-byte aligned workspace, and more of it than the
+    // panels: a Four-Russians call that brings less takes panels, and so does
+    // AUTO on another alignment.
+    const bool aligned = ((uintptr_t)ws & 15) == 0;
+    const bool tables = (variant_arg == MELA_ELIM_M4RI && aligned && ws_bytes >= elim_tc_workspace(m, n)) ||
+                        (chosen && variant == MELA_ELIM_TC && aligned && (double)m * (double)n <= 4e7);
+    if (chosen && variant == MELA_ELIM_TC && !aligned) {
+        variant = MELA_ELIM_M4RI;
+        decode_elim_variant(variant, &tune);
+    }
     if (variant == MELA_ELIM_TC || tables)
         return elim_windows_device(M, ld, m, n, rref, tables, d_rank, d_piv, d_prow, ws, ws_bytes, s);
     ElimLayout L = elim_layout(m, n);
