@@ -25,6 +25,13 @@ static bool takes_small(int *variant, const u64 *P, i64 ld, i64 m, i64 n, int rr
     return *variant == MELA_ELIM_FUSED;
 }
 
+// The page-locked words out of the thread's hands while the caller's allocator
+// runs, which may call in here again or throw.
+struct PostedHold {
+    void *const words = posted_take();
+    ~PostedHold() { posted_give(words); }
+};
+
 // Rank of a packed device matrix (overwritten), read back to the host.
 mela_status rank_of_packed(u64 *P, i64 ld, i64 m, i64 n, int variant, cudaStream_t s, double *rank)
 {
@@ -69,9 +76,11 @@ mela_status null_of_packed(u64 *P, i64 ld, i64 m, i64 n, int variant, mela_alloc
         if ((st = launch_small_post(P, ld, m, n, to, true, s)) != MELA_OK) return st;
         if ((st = finish_posted(s)) != MELA_OK) return st;
         const i64 f = n - *to.value;
-        void *words = posted_take();
-        uint8_t *Z = alloc(ctx, n, f);
-        posted_give(words);
+        uint8_t *Z;
+        {
+            const PostedHold hold;
+            Z = alloc(ctx, n, f);
+        }
         if (!Z && f > 0) {
             set_error("output allocation failed");
             return MELA_ERR_NOMEM;
