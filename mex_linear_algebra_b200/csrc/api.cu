@@ -169,22 +169,54 @@ struct Readback {
     alignas(64) unsigned char small[kSmallBytes];
     alignas(64) unsigned char in[24 << 10];
 };
+// Sets not in use, kept for other threads: short-lived threads then neither
+// allocate (page-locking 280 KB takes 0.1 ms) nor free (which may wait for the
+// device).  At most kSpareReadbacks.
+constexpr size_t kSpareReadbacks = 32;
+std::mutex g_readback_mu;
+std::vector<Readback *> *g_readback_spare = nullptr;
+Readback *readback_new()
+{
+    {
+        std::lock_guard<std::mutex> g(g_readback_mu);
+        if (g_readback_spare && !g_readback_spare->empty()) {
+            Readback *r = g_readback_spare->back();
+            g_readback_spare->pop_back();
+            return r;
+        }
+    }
+    Readback *r = nullptr;
+    if (cudaHostAlloc((void **)&r, sizeof(Readback), cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return r;
+}
+void readback_spare(Readback *r)
+{
+    if (!r) return;
+    {
+        std::lock_guard<std::mutex> g(g_readback_mu);
+        if (!g_readback_spare) g_readback_spare = new std::vector<Readback *>();
+        if (g_readback_spare->size() < kSpareReadbacks) {
+            g_readback_spare->push_back(r);
+            return;
+        }
+    }
+    cudaFreeHost(r);
+}
 struct Readbacks {
     Readback *dev[kMaxDevices] = {};
     ~Readbacks()  // given back when the thread ends
     {
-        for (Readback *r : dev)
-            if (r) cudaFreeHost(r);
+        for (Readback *r : dev) readback_spare(r);
     }
 };
 thread_local Readbacks t_readback;
 Readback *readback()
 {
     Readback *&r = t_readback.dev[current_device()];
-    if (!r && cudaHostAlloc((void **)&r, sizeof(Readback), cudaHostAllocPortable) != cudaSuccess) {
-        cudaGetLastError();
-        r = nullptr;
-    }
+    if (!r) r = readback_new();
     return r;
 }
 }  // namespace
@@ -232,7 +264,7 @@ void *posted_take()
 void posted_give(void *words)
 {
     Readback *&slot = t_readback.dev[current_device()];
-    if (slot) cudaFreeHost(slot);
+    readback_spare(slot);
     slot = (Readback *)words;
 }
 
@@ -539,21 +571,120 @@ private:
     size_t job_bytes_ = 0;
 };
 
-// Page-locked staging slots of the calling thread (per device), taken in turn
-// across calls, uploads and downloads: a slot is refilled once the copy that
-// used it has completed.
+// Page-locked staging slots, taken in turn across calls, uploads and
+// downloads: a slot is refilled once the copy that used it has completed
+// (its event, which any thread can wait for).
 constexpr int kStageSlots = 3;
-constexpr size_t kStageBytes = (size_t)8 << 20;
+constexpr size_t kStageSmall = (size_t)1 << 20, kStageBytes = (size_t)8 << 20;  // the two sizes of a slot
 struct Staging {
     void *slot[kStageSlots] = {};
     cudaEvent_t read[kStageSlots] = {};  // the copy from or into the slot is done
     cudaEvent_t fence = nullptr;         // the device staging buffer is allocated
     int next = 0;                        // the next slot
-    bool ready = false;
-    bool failed = false;
+    size_t cap = 0;                      // bytes of a slot
 };
-// one set per device: events belong to the device they were created on
-thread_local Staging t_stage[kMaxDevices];
+// The sets of a device (events belong to it), shared by the host threads: a
+// call takes one for an upload or a download, so there are no more of them than
+// calls have ever been copying at once, at most kStageSets (384 MB); a copy
+// that finds none left goes by the driver.  The set used last is taken first.
+constexpr int kStageSets = 16;
+struct StagePool {
+    std::vector<Staging *> spare;
+    int made = 0;
+    bool asked[2] = {};   // a download has asked for slots of that size
+    bool failed = false;  // page-locked memory has run out
+};
+std::mutex g_stage_mu;
+StagePool *g_stage[kMaxDevices];
+
+// Slots of at least `bytes` for S, whose copies have ended.
+bool staging_grow(Staging &S, size_t bytes)
+{
+    for (int i = 0; i < kStageSlots; ++i) {
+        if (S.read[i]) cudaEventSynchronize(S.read[i]);
+        if (S.slot[i]) cudaFreeHost(S.slot[i]);
+        S.slot[i] = nullptr;
+    }
+    S.cap = 0;
+    bool ok = S.fence || cudaEventCreateWithFlags(&S.fence, cudaEventDisableTiming) == cudaSuccess;
+    for (int i = 0; ok && i < kStageSlots; ++i)
+        ok = (S.read[i] || cudaEventCreateWithFlags(&S.read[i], cudaEventDisableTiming) == cudaSuccess) &&
+             cudaHostAlloc(&S.slot[i], bytes, cudaHostAllocPortable) == cudaSuccess;
+    if (ok) {
+        S.cap = bytes;
+        return true;
+    }
+    cudaGetLastError();
+    for (int i = 0; i < kStageSlots; ++i) {
+        if (S.slot[i]) cudaFreeHost(S.slot[i]);
+        S.slot[i] = nullptr;
+    }
+    return false;
+}
+
+// A set for the life of this object; S is null where there is none.
+class StagingLease {
+public:
+    // Pieces of up to `want` bytes.  An upload always gets them; a download,
+    // which can also go by the driver or in smaller pieces, does not make the
+    // first call of a process pay for new slots (page-locking takes 0.5 ms a
+    // MB): they are made when it asks for the second time.
+    StagingLease(size_t want, bool download) : dev_(current_device())
+    {
+        const int size = want > kStageSmall;
+        const size_t bytes = size ? kStageBytes : kStageSmall;
+        bool grow = true;
+        {
+            std::lock_guard<std::mutex> g(g_stage_mu);
+            StagePool *&P = g_stage[dev_];
+            if (!P) P = new StagePool();
+            if (download) {
+                grow = P->asked[size];
+                P->asked[size] = true;
+            }
+            if (P->failed) grow = false;
+            if (!P->spare.empty()) {
+                size_t i = P->spare.size() - 1;
+                for (size_t j = i + 1; j-- > 0;)
+                    if (P->spare[j]->cap >= bytes) {
+                        i = j;
+                        break;
+                    }
+                S = P->spare[i];
+                P->spare.erase(P->spare.begin() + (long)i);
+            } else if (grow && P->made < kStageSets) {
+                S = new Staging();
+                ++P->made;
+            }
+        }
+        if (!S || S->cap >= bytes) return;
+        if (!grow && (S->cap == 0 || !download)) {
+            give_back();
+            return;
+        }
+        if (grow && !staging_grow(*S, bytes)) {
+            {
+                std::lock_guard<std::mutex> g(g_stage_mu);
+                g_stage[dev_]->failed = true;
+            }
+            give_back();
+        }
+    }
+    ~StagingLease() { give_back(); }
+    StagingLease(const StagingLease &) = delete;
+    StagingLease &operator=(const StagingLease &) = delete;
+    Staging *S = nullptr;
+
+private:
+    void give_back()
+    {
+        if (!S) return;
+        std::lock_guard<std::mutex> g(g_stage_mu);
+        g_stage[dev_]->spare.push_back(S);
+        S = nullptr;
+    }
+    int dev_;
+};
 thread_local mela_upload_stats t_upload_stats;
 
 double now_us()
@@ -561,27 +692,6 @@ double now_us()
     return std::chrono::duration<double, std::micro>(std::chrono::steady_clock::now().time_since_epoch()).count();
 }
 
-bool staging_ready()
-{
-    Staging &S = t_stage[current_device()];
-    if (S.ready) return true;
-    if (S.failed) return false;
-    for (int i = 0; i < kStageSlots; ++i) {
-        if (cudaHostAlloc(&S.slot[i], kStageBytes, cudaHostAllocPortable) != cudaSuccess ||
-            cudaEventCreateWithFlags(&S.read[i], cudaEventDisableTiming) != cudaSuccess) {
-            cudaGetLastError();
-            S.failed = true;
-            return false;
-        }
-    }
-    if (cudaEventCreateWithFlags(&S.fence, cudaEventDisableTiming) != cudaSuccess) {
-        cudaGetLastError();
-        S.failed = true;
-        return false;
-    }
-    S.ready = true;
-    return true;
-}
 }  // namespace
 
 // Column blocks of the MATLAB array go through the page-locked slots: the
@@ -589,7 +699,7 @@ bool staging_ready()
 // the upload stream, and each block is packed on s as soon as it has landed
 // (blocks are whole packed words: multiples of 64 columns).
 static mela_status upload_and_pack_blocks(const mela_host_matrix *M, u64 *dP, i64 ld, cudaStream_t s,
-                                          DevBuf &staging, i64 cols_per_block)
+                                          DevBuf &staging, i64 cols_per_block, Staging &S)
 {
     const i64 m = M->rows, n = M->cols;
     const size_t esz = M->kind == MELA_KIND_DOUBLE ? 8 : 1;
@@ -597,7 +707,6 @@ static mela_status upload_and_pack_blocks(const mela_host_matrix *M, u64 *dP, i6
     if (st != MELA_OK) return st;
     cudaStream_t sin = nullptr, sout = nullptr;
     if ((st = copy_streams(&sin, &sout)) != MELA_OK) return st;
-    Staging &S = t_stage[current_device()];
     // the device staging buffer comes from s's pool: uploads wait for it
     MELA_CUDA_TRY(cudaEventRecord(S.fence, s));
     MELA_CUDA_TRY(cudaStreamWaitEvent(sin, S.fence, 0));
@@ -647,16 +756,18 @@ mela_status download_finish(void *dst, const void *src, size_t bytes, cudaStream
         if (st == MELA_OK) std::memcpy(dst, rb->small, bytes);
         return st;
     }
-    if (!staging_ready()) {
-        MELA_CUDA_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s));
-        return finish(s);
-    }
-    Staging &S = t_stage[current_device()];
     const bool alone = bytes < ((size_t)8 << 20);
-    const size_t least = (size_t)(alone ? 128 : 512) << 10, most = alone ? (size_t)1 << 20 : kStageBytes;
+    const size_t least = (size_t)(alone ? 128 : 512) << 10, most = alone ? kStageSmall : kStageBytes;
     size_t piece = (bytes / 4 + 0xffff) & ~(size_t)0xffff;
     if (piece < least) piece = least;
     if (piece > most) piece = most;
+    StagingLease lease(piece, true);
+    if (!lease.S) {
+        MELA_CUDA_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s));
+        return finish(s);
+    }
+    Staging &S = *lease.S;
+    if (piece > S.cap) piece = S.cap;
     const size_t pieces = (bytes + piece - 1) / piece;
     const int first = S.next;
     size_t issued = 0;
@@ -697,8 +808,10 @@ mela_status upload_and_pack(const mela_host_matrix *M, u64 *dP, i64 ld, cudaStre
     const size_t quarter = bytes / 4 > ((size_t)1 << 20) ? bytes / 4 : (size_t)1 << 20;
     const i64 want = ((i64)(quarter / col_bytes) + 63) / 64 * 64;
     if (want >= 64 && want < cols_per_block) cols_per_block = want;
-    if (bytes >= ((size_t)2 << 20) && cols_per_block >= 64 && staging_ready())
-        return upload_and_pack_blocks(M, dP, ld, s, staging, cols_per_block);
+    if (bytes >= ((size_t)2 << 20) && cols_per_block >= 64) {
+        const StagingLease lease((size_t)cols_per_block * col_bytes, false);
+        if (lease.S) return upload_and_pack_blocks(M, dP, ld, s, staging, cols_per_block, *lease.S);
+    }
     mela_status st = staging.alloc(bytes, s);
     if (st != MELA_OK) return st;
     MELA_CUDA_TRY(cudaMemcpyAsync(staging.p, M->data, bytes, cudaMemcpyHostToDevice, s));
