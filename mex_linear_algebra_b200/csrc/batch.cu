@@ -276,6 +276,41 @@ struct BigCfg {
 };
 }  // namespace
 
+// Where a matrix and all of its elimination's storage lie in a CTA's shared
+// memory (byte offsets in `extra` bytes): the panel's storage from the start,
+// then the pivot lists and the matrix at the end; after the elimination the null
+// basis' index arrays and transposes take the place of the panel's storage and
+// the pivot lists.  fits: for 110 KB and n = 2m up to about m = 250.  A batch
+// whose CTA matrices all fit needs no scratch and runs the kernel compiled for
+// that: 200 matrices of m in [64, 128], n = 2m, plan created, used once and
+// destroyed 0.62 ms, 1.31 with scratch for 296 CTAs; 4000 of m in [192, 240]
+// 1.38 ms a run, 1.50 with the matrix alone in shared memory.
+struct ShmPlace {
+    int act_at, rows_at, ul_at, piv_at, mat_at, rt_at, q_at;
+    bool fits;
+};
+__host__ __device__ inline ShmPlace shm_place(int m, int n, int extra)
+{
+    const int wc = (n + 63) >> 6, mn = m < n ? m : n;
+    ShmPlace P;
+    P.act_at = 128 * wc * 8;
+    P.rows_at = P.act_at + ((m + 15) & ~15);
+    P.ul_at = P.rows_at + 24 * m;
+    const int panel = P.ul_at + ((4 * m + 15) & ~15);
+    P.mat_at = (extra - m * wc * 8) & ~15;
+    P.piv_at = P.mat_at - ((8 * mn + 15) & ~15);
+    const int idx = wc * 8 + (mn + 2 * n + wc + 1) * 4;
+    P.rt_at = (idx + 15) & ~15;
+    P.q_at = P.rt_at + n * ((mn + 127) >> 7) * 16;
+    P.fits = panel <= P.piv_at && idx <= P.piv_at && P.q_at + mn * ((n + 127) >> 7) * 16 <= P.mat_at;
+    return P;
+}
+// (shapes beyond these never fit, and below them nothing overflows)
+inline bool fits_shm(long long m, long long n, size_t extra)
+{
+    return m <= 16384 && n <= 16384 && shm_place((int)m, (int)n, (int)extra).fits;
+}
+
 // v[i] for a lane-local index i < R (R <= 16) by a select tree: no local
 // memory and a dependence depth of four selects.
 template <int R>
@@ -516,7 +551,8 @@ __device__ __forceinline__ TrWords<4> tr_words4(const u32 *p)
 //  * null basis: Zt = (Y)^T with Y row c = (R restricted to free columns)^T
 //    row p when c is pivot column p, the unit vector of its free index
 //    otherwise -- three 32x32 shuffle transposes, no per-bit gathers.
-template <int NT, int SMEM>
+// SHM: everything in shared memory (shm_place), no scratch.
+template <int NT, int SMEM, bool SHM>
 __device__ void process_big_blocked(const BatchDevItem &it, const u64 *__restrict__ in,
                                     u64 *__restrict__ zt, long long *ranks, int item,
                                     unsigned char *smem_raw, u64 *g, const FusedOut *fo = nullptr)
@@ -529,53 +565,74 @@ __device__ void process_big_blocked(const BatchDevItem &it, const u64 *__restric
     const int m = it.m, n = it.n, wc = (n + 63) >> 6, mn = m < n ? m : n;
     const int tid = threadIdx.x, lane = tid & 31;
     const BigLayout L = big_layout(m, n);
-    u64 *A = g + L.A;
-    int *piv = reinterpret_cast<int *>(g + L.ints);
-    int *prow = piv + mn;
+    unsigned char *extra = smem_raw + Cfg::kHead;
+    u64 *A, *stage, *ysnap0, *ysnap1, *tag;
+    unsigned char *active;
+    u32 *Rt, *Q;
+    int *piv, *prow, *ulist;
+    u64 *pm = g + L.pm;
+    bool r_in_smem = true;
+    size_t pre_a_bytes = 0;  // shared bytes before the matrix: free again for the null basis
+    if constexpr (SHM) {
+        const ShmPlace P = shm_place(m, n, (int)kBigExtra);
+        stage = reinterpret_cast<u64 *>(extra);
+        active = extra + P.act_at;
+        ysnap0 = reinterpret_cast<u64 *>(extra + P.rows_at);
+        ysnap1 = ysnap0 + m;
+        tag = ysnap1 + m;
+        ulist = reinterpret_cast<int *>(extra + P.ul_at);
+        piv = reinterpret_cast<int *>(extra + P.piv_at);
+        A = reinterpret_cast<u64 *>(extra + P.mat_at);
+        Rt = reinterpret_cast<u32 *>(extra + P.rt_at);
+        Q = reinterpret_cast<u32 *>(extra + P.q_at);
+    } else {
+        A = g + L.A;
+        piv = reinterpret_cast<int *>(g + L.ints);
+        Rt = reinterpret_cast<u32 *>(g + L.rt);
+        Q = reinterpret_cast<u32 *>(g + L.q);
+        const size_t rb_bytes = (size_t)64 * wc * 8, row_bytes = (size_t)m * 8;
+        r_in_smem = 2 * rb_bytes <= kBigExtra;
+        stage = r_in_smem ? reinterpret_cast<u64 *>(extra) : g + L.Rg;
+        size_t used = r_in_smem ? 2 * rb_bytes : 0;
+        // row states are read on every bit step: shared memory whenever possible
+        const size_t act_bytes = ((size_t)m + 15) & ~(size_t)15;
+        active = (used + act_bytes <= kBigExtra) ? extra + used : reinterpret_cast<unsigned char *>(g + L.active);
+        if (used + act_bytes <= kBigExtra) used += act_bytes;
+        const bool rows_in_smem = used + 3 * row_bytes <= kBigExtra;
+        ysnap0 = rows_in_smem ? reinterpret_cast<u64 *>(extra + used) : g + L.ysg;
+        ysnap1 = rows_in_smem ? ysnap0 + m : g + L.yvg;
+        tag = rows_in_smem ? ysnap1 + m : g + L.tagg;
+        if (rows_in_smem) used += 3 * row_bytes;
+        // the look-ahead's list of rows to update (row order), when it fits
+        const size_t ul_bytes = ((size_t)m * 4 + 15) & ~(size_t)15;
+        ulist = rows_in_smem && used + ul_bytes <= kBigExtra ? reinterpret_cast<int *>(extra + used) : nullptr;
+        if (ulist) used += ul_bytes;
+        // the matrix itself in shared memory too when it fits (at n = 2m: m up
+        // to about 420 with 110 KB, 650 with 220 KB), else in the CTA's
+        // L2-resident scratch
+        pre_a_bytes = used;
+        if (used + (size_t)m * wc * 8 <= kBigExtra) A = reinterpret_cast<u64 *>(extra + used);
+    }
+    u64 *Rbuf = stage + (size_t)64 * wc;
+    prow = piv + mn;
     int *fcol = prow + mn;
     int *cmap = fcol + n;
     int *pbase = cmap + n;
-    u64 *pm = g + L.pm;
-    u32 *Rt = reinterpret_cast<u32 *>(g + L.rt);
-    u32 *Q = reinterpret_cast<u32 *>(g + L.q);
-
-    unsigned char *extra = smem_raw + Cfg::kHead;
-    const size_t rb_bytes = (size_t)64 * wc * 8, row_bytes = (size_t)m * 8;
-    const bool r_in_smem = 2 * rb_bytes <= kBigExtra;
-    u64 *stage = r_in_smem ? reinterpret_cast<u64 *>(extra) : g + L.Rg;
-    u64 *Rbuf = stage + (size_t)64 * wc;
-    size_t used = r_in_smem ? 2 * rb_bytes : 0;
-    // row states are read on every bit step: shared memory whenever possible
-    const size_t act_bytes = ((size_t)m + 15) & ~(size_t)15;
-    unsigned char *active = (used + act_bytes <= kBigExtra) ? extra + used
-                                                           : reinterpret_cast<unsigned char *>(g + L.active);
-    if (used + act_bytes <= kBigExtra) used += act_bytes;
-    const bool rows_in_smem = used + 3 * row_bytes <= kBigExtra;
-    u64 *ysnap0 = rows_in_smem ? reinterpret_cast<u64 *>(extra + used) : g + L.ysg;
-    u64 *ysnap1 = rows_in_smem ? ysnap0 + m : g + L.yvg;
-    u64 *tag = rows_in_smem ? ysnap1 + m : g + L.tagg;
-    if (rows_in_smem) used += 3 * row_bytes;
-    // the look-ahead's list of rows to update (row order), when it fits
-    const size_t ul_bytes = ((size_t)m * 4 + 15) & ~(size_t)15;
-    int *ulist = rows_in_smem && used + ul_bytes <= kBigExtra ? reinterpret_cast<int *>(extra + used) : nullptr;
-    if (ulist) used += ul_bytes;
-    // the matrix itself in shared memory too when it fits (at n = 2m: m up
-    // to about 420 with 110 KB, 650 with 220 KB), else in the CTA's
-    // L2-resident scratch
-    const size_t pre_a_bytes = used;  // shared bytes before the matrix: free again for the null basis
-    if (used + (size_t)m * wc * 8 <= kBigExtra) A = reinterpret_cast<u64 *>(extra + used);
 
     // the matrix, eight words a thread in flight (one after the other the copy
     // took 141K of a 1000-row matrix's 1.88M cycles)
     const u64 *src = in + it.in_off;
-    const long long words = (long long)m * wc;  // may pass 2^31 (16 GiB)
-    for (long long e0 = tid; e0 < words; e0 += 8 * NT) {
-        u64 v[8];
+    const long long words = (long long)m * wc;  // may pass 2^31 (16 GiB): by 2^30
+    for (long long base = 0; base < words; base += 1 << 30) {
+        const int cnt = (int)min(words - base, 1LL << 30);
+        for (int e0 = tid; e0 < cnt; e0 += 8 * NT) {
+            u64 v[8];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) v[u] = e0 + u * NT < words ? src[e0 + u * NT] : 0ull;
+            for (int u = 0; u < 8; ++u) v[u] = e0 + u * NT < cnt ? src[base + e0 + u * NT] : 0ull;
 #pragma unroll
-        for (int u = 0; u < 8; ++u)
-            if (e0 + u * NT < words) A[e0 + u * NT] = v[u];
+            for (int u = 0; u < 8; ++u)
+                if (e0 + u * NT < cnt) A[base + e0 + u * NT] = v[u];
+        }
     }
     for (int j = tid; j < m; j += NT) active[j] = 1;
     __syncthreads();
@@ -1130,7 +1187,7 @@ __device__ void process_big_blocked(const BatchDevItem &it, const u64 *__restric
     // ---- null basis
     const int f = n - r;
     // its index arrays in the elimination's shared memory when they fit
-    if ((size_t)wc * 8 + ((size_t)r + 2 * (size_t)n + wc + 1) * 4 <= pre_a_bytes) {
+    if (SHM || (size_t)wc * 8 + ((size_t)r + 2 * (size_t)n + wc + 1) * 4 <= pre_a_bytes) {
         __syncthreads();
         u64 *pm_s = reinterpret_cast<u64 *>(extra);
         int *prow_s = reinterpret_cast<int *>(pm_s + wc);
@@ -1217,7 +1274,7 @@ __device__ void process_big_blocked(const BatchDevItem &it, const u64 *__restric
 // NT threads and SMEM bytes of shared memory per CTA, kThreads / NT CTAs per
 // SM: a big matrix takes a whole CTA, a medium one a 128-thread group with
 // kMidBudget bytes, a small one a warp with kSmallBudget bytes.
-template <int NT, int SMEM>
+template <int NT, int SMEM, bool SHM>
 __global__ void __launch_bounds__(NT, kThreads / NT)
 batch_kernel(const BatchDevItem *__restrict__ items, const int *__restrict__ order, int n_big,
              int n_mid, int n_small, int *counters, const u64 *__restrict__ in, u64 *__restrict__ zt,
@@ -1238,7 +1295,7 @@ batch_kernel(const BatchDevItem *__restrict__ items, const int *__restrict__ ord
         __syncthreads();
         if (k >= n_big) break;
         const int item = order[k];
-        process_big_blocked<NT, SMEM>(items[item], in, zt, ranks, item, smem, gmat);
+        process_big_blocked<NT, SMEM, SHM>(items[item], in, zt, ranks, item, smem, gmat);
     }
     // mid: groups of 128 threads, each with kMidBudget bytes of shared memory
     {
@@ -1466,7 +1523,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 fused_elim_kernel(BatchDevItem it, const u64 *__restrict__ in_compact, FusedOut fo, u64 *scratch)
 {
     extern __shared__ __align__(16) unsigned char smem[];
-    process_big_blocked<kThreads, kSmemTotal>(it, in_compact, nullptr, nullptr, 0, smem, scratch, &fo);
+    process_big_blocked<kThreads, kSmemTotal, false>(it, in_compact, nullptr, nullptr, 0, smem, scratch, &fo);
 }
 
 size_t fused_workspace(i64 m, i64 n)
@@ -1620,6 +1677,7 @@ static mela_status plan_create(const mela_batch_item *h, long long count, int fo
     std::vector<int> cls((size_t)count);
     std::vector<double> cost((size_t)count);
     long long max_big_words = 0;
+    bool shm = true;  // every CTA matrix fits in shared memory
     for (long long i = 0; i < count; ++i) {
         const long long m = h[i].m, n = h[i].n;
         if (m < 0 || n < 0 || m > INT_MAX / 2 || n > INT_MAX / 2 || h[i].in_offset < 0 || h[i].z_offset < 0) {
@@ -1651,6 +1709,7 @@ static mela_status plan_create(const mela_batch_item *h, long long count, int fo
         if (c == 0) {
             d.flags = 0;  // big matrices live in the CTA's global scratch
             max_big_words = std::max(max_big_words, big_scratch_words(m, n));
+            shm = shm && fits_shm(m, n, BigCfg<kBatchThreads, kBatchSmem>::kExtra);
         } else {
             d.flags = 1;
         }
@@ -1669,6 +1728,7 @@ static mela_status plan_create(const mela_batch_item *h, long long count, int fo
     P->n_mid = (int)P->class_count[1];
     P->n_small = (int)P->class_count[2];
     P->grid = (kThreads / kBatchThreads) * sm_count();
+    if (shm) max_big_words = 0;
     P->gscratch_words = max_big_words;
 
     // logical-input packing tiles
@@ -1723,7 +1783,9 @@ static mela_status enqueue(BatchPlanImpl *P, const u64 *in, u64 *zt, long long *
 {
     MELA_CUDA_TRY(cudaMemsetAsync(P->d_counters, 0, 4 * sizeof(int), s));
     if (P->count == 0) return MELA_OK;
-    batch_kernel<kBatchThreads, kBatchSmem><<<P->grid, kBatchThreads, kBatchSmem, s>>>(
+    const auto kernel = P->gscratch_words ? batch_kernel<kBatchThreads, kBatchSmem, false>
+                                          : batch_kernel<kBatchThreads, kBatchSmem, true>;
+    kernel<<<P->grid, kBatchThreads, kBatchSmem, s>>>(
         P->d_items, P->d_order, P->n_big, P->n_mid, P->n_small, P->d_counters, in, zt, ranks,
         P->d_gscratch, P->gscratch_words);
     MELA_LAUNCH_CHECK("batch_kernel");
@@ -1750,7 +1812,9 @@ static mela_status batch_attrs()
     int dev = 0;
     MELA_CUDA_TRY(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64 || done[dev]) return MELA_OK;
-    MELA_CUDA_TRY(cudaFuncSetAttribute(batch_kernel<kBatchThreads, kBatchSmem>,
+    MELA_CUDA_TRY(cudaFuncSetAttribute(batch_kernel<kBatchThreads, kBatchSmem, false>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, kBatchSmem));
+    MELA_CUDA_TRY(cudaFuncSetAttribute(batch_kernel<kBatchThreads, kBatchSmem, true>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, kBatchSmem));
     done[dev] = true;
     return MELA_OK;
