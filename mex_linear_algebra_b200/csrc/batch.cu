@@ -636,6 +636,14 @@ __device__ void process_big_blocked(const BatchDevItem &it, const u64 *__restric
     }
     for (int j = tid; j < m; j += NT) active[j] = 1;
     __syncthreads();
+    if (n & 63) {  // bits past the last column are no columns (the other engines never look at them)
+        const u64 past = ~0ull << (n & 63);
+        for (int j = tid; j < m; j += NT) {
+            u64 &v = A[(size_t)j * wc + wc - 1];
+            if (v & past) v &= ~past;
+        }
+        __syncthreads();
+    }
 
     // panel words of every row: one buffer for the current panel, the other
     // for the next panel's (look-ahead) or the per-bit path's working copy

@@ -83,9 +83,10 @@ elim_small_kernel(u64 *__restrict__ M, i64 ld, int m, int n, int lanes_log2, lon
     // P = 2^lanes_log2 lanes take a row's words together
     const int P = 1 << lanes_log2, part = tid & (P - 1), rows_per_pass = SM_THREADS >> lanes_log2;
 
+    const u64 last = n & 63 ? (1ull << (n & 63)) - 1 : ~0ull;  // bits past the last column are no columns
     for (int e = tid; e < m * wc; e += SM_THREADS) {
         const int j = e / wc, x = e - j * wc;
-        A[j * pitch + x] = M[(i64)j * ld + x];
+        A[j * pitch + x] = M[(i64)j * ld + x] & (x == wc - 1 ? last : ~0ull);
     }
     if (POST) S.prow_of[tid] = -1;
     bool used = tid >= m;  // row tid is a pivot row (or no row)
