@@ -752,7 +752,8 @@ mela_status elim_device(int variant_arg, u64 *M, i64 ld, i64 m, i64 n, int rref,
         decode_elim_variant(variant, &tune);
     }
     if (variant == MELA_ELIM_TC || tables)
-        return elim_windows_device(M, ld, m, n, rref, tables, d_rank, d_piv, d_prow, ws, ws_bytes, s);
+        return elim_windows_device(M, ld, m, n, rref, tables, variant_arg == MELA_ELIM_M4RI, d_rank, d_piv, d_prow, ws,
+                                   ws_bytes, s);
     ElimLayout L = elim_layout(m, n);
     if (ws_bytes < L.total || !ws) {
         set_error("elimination workspace of %zu bytes needed, %zu given", elim_workspace(m, n), ws_bytes);

@@ -27,7 +27,8 @@ mela_status elim_device(int variant, u64 *M, i64 ld, i64 m, i64 n, int rref, lon
 // Forms by 256-column windows (elim_tc.cu), same contract as elim_device: the
 // trailing update on the tensor cores, or (tables) by Four-Russians tables.
 size_t elim_tc_workspace(i64 m, i64 n);
-mela_status elim_windows_device(u64 *M, i64 ld, i64 m, i64 n, int rref, bool tables, long long *d_rank,
+// named: the caller asked for the Four-Russians form itself.
+mela_status elim_windows_device(u64 *M, i64 ld, i64 m, i64 n, int rref, bool tables, bool named, long long *d_rank,
                                 long long *d_piv, long long *d_prow, void *ws, size_t ws_bytes, cudaStream_t s);
 
 NullLayout null_layout(i64 n, i64 rank);

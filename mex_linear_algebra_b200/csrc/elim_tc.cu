@@ -1203,7 +1203,9 @@ size_t elim_tc_workspace(i64 m, i64 n) { return tc_layout(m, n).total; }
 
 namespace {
 // Captured eliminations, kept for the life of the process (at most
-// kMaxElimGraphs; further shapes or buffers run without a graph).
+// kMaxElimGraphs of calls that name the Four-Russians form and as many of the
+// others, so that neither keeps the other from being captured; further shapes
+// or buffers run without a graph).
 struct ElimGraphKey {
     int dev;
     const void *p[5];
@@ -1213,12 +1215,23 @@ struct ElimGraph {
     ElimGraphKey k;
     cudaGraphExec_t exec;
 };
+constexpr long long kElimTables = 2, kElimNamed = 4;  // bits of v[3]: update by tables, form named by the caller
 constexpr size_t kMaxElimGraphs = 16;
 constexpr size_t kMaxElimSeen = 64;
 std::mutex g_elim_graph_mu;
-std::vector<ElimGraph> *g_elim_graphs = nullptr;
-std::vector<ElimGraphKey> *g_elim_seen = nullptr;  // calls made once, without a graph
-size_t g_elim_seen_next = 0;                       // the oldest entry, replaced once the list is full
+struct ElimGraphs {
+    std::vector<ElimGraph> kept;
+    std::vector<ElimGraphKey> seen;  // calls made once, without a graph
+    size_t seen_next = 0;            // the oldest entry, replaced once the list is full
+};
+ElimGraphs *g_elim_graphs[2] = {};
+// of a call's kind (under g_elim_graph_mu)
+ElimGraphs &elim_graphs(const ElimGraphKey &k)
+{
+    ElimGraphs *&g = g_elim_graphs[(k.v[3] & kElimNamed) != 0];
+    if (!g) g = new ElimGraphs();
+    return *g;
+}
 
 bool elim_graphs_enabled()
 {
@@ -1229,8 +1242,7 @@ cudaGraphExec_t elim_graph_lookup(const ElimGraphKey &k)
 {
     if (!elim_graphs_enabled()) return nullptr;
     std::lock_guard<std::mutex> lk(g_elim_graph_mu);
-    if (!g_elim_graphs) return nullptr;
-    for (const ElimGraph &g : *g_elim_graphs)
+    for (const ElimGraph &g : elim_graphs(k).kept)
         if (std::memcmp(&g.k, &k, sizeof k) == 0) return g.exec;
     return nullptr;
 }
@@ -1246,29 +1258,28 @@ bool elim_graph_capturable(const ElimGraphKey &k, cudaStream_t s)
         return false;
     }
     std::lock_guard<std::mutex> lk(g_elim_graph_mu);
-    if (g_elim_graphs && g_elim_graphs->size() >= kMaxElimGraphs) return false;
-    if (!g_elim_seen) g_elim_seen = new std::vector<ElimGraphKey>();
-    for (const ElimGraphKey &q : *g_elim_seen)
+    ElimGraphs &G = elim_graphs(k);
+    if (G.kept.size() >= kMaxElimGraphs) return false;
+    for (const ElimGraphKey &q : G.seen)
         if (std::memcmp(&q, &k, sizeof k) == 0) return true;
     // remember the call; a full list forgets its oldest entry, so a stream of
     // one-off shapes never keeps a repeated call from being captured
-    if (g_elim_seen->size() < kMaxElimSeen) {
-        g_elim_seen->push_back(k);
+    if (G.seen.size() < kMaxElimSeen) {
+        G.seen.push_back(k);
     } else {
-        (*g_elim_seen)[g_elim_seen_next] = k;
-        g_elim_seen_next = (g_elim_seen_next + 1) % kMaxElimSeen;
+        G.seen[G.seen_next] = k;
+        G.seen_next = (G.seen_next + 1) % kMaxElimSeen;
     }
     return false;
 }
 void elim_graph_store(const ElimGraphKey &k, cudaGraphExec_t exec)
 {
     std::lock_guard<std::mutex> lk(g_elim_graph_mu);
-    if (!g_elim_graphs) g_elim_graphs = new std::vector<ElimGraph>();
-    g_elim_graphs->push_back(ElimGraph{k, exec});
+    elim_graphs(k).kept.push_back(ElimGraph{k, exec});
 }
 }  // namespace
 
-mela_status elim_windows_device(u64 *M, i64 ld, i64 m, i64 n, int rref, bool tables, long long *d_rank,
+mela_status elim_windows_device(u64 *M, i64 ld, i64 m, i64 n, int rref, bool tables, bool named, long long *d_rank,
                                 long long *d_piv, long long *d_prow, void *wsp, size_t ws_bytes, cudaStream_t s)
 {
     const TcLayout L = tc_layout(m, n);
@@ -1400,7 +1411,7 @@ mela_status elim_windows_device(u64 *M, i64 ld, i64 m, i64 n, int rref, bool tab
     key.v[0] = ld;
     key.v[1] = m;
     key.v[2] = n;
-    key.v[3] = rref + (tables ? 2 : 0);
+    key.v[3] = rref + (tables ? kElimTables : 0) + (named ? kElimNamed : 0);
     cudaGraphExec_t exec = elim_graph_lookup(key);
     cudaStream_t cap = nullptr;
     if (exec) {
