@@ -636,7 +636,9 @@ __device__ void process_big_blocked(const BatchDevItem &it, const u64 *__restric
     }
     for (int j = tid; j < m; j += NT) active[j] = 1;
     __syncthreads();
-    if (n & 63) {  // bits past the last column are no columns (the other engines never look at them)
+    // bits past the last column are no columns: the engines for small matrices
+    // never look at them, so they are cut where the matrix lies in shared memory
+    if ((n & 63) && (SHM || A != g + L.A)) {
         const u64 past = ~0ull << (n & 63);
         for (int j = tid; j < m; j += NT) {
             u64 &v = A[(size_t)j * wc + wc - 1];
