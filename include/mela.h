@@ -421,8 +421,13 @@ mela_status mela_mlp_gradient(const float *d_params, const float *d_X, const flo
 /* One Adam step (beta1 0.9, beta2 0.999, eps 1e-8); step counts from 1. */
 mela_status mela_mlp_adam_step(float *d_params, const float *d_grad, float *d_m1, float *d_m2,
                                int64_t step, float lr, void *stream);
-/* Install (or, with NULL, remove) the dispatch model from host memory. */
+/* Install (or, with NULL, remove) the dispatch model from host memory: one
+ * set of parameters for every request. */
 mela_status mela_costmodel_load(const float *h_params);
+/* Put back the model that the library loads with: one set for the ranges it
+ * was trained on (dimensions in [32, 8192], the left operand at most 8:1) and
+ * for batches, one for other requests.  None if it was built without. */
+void mela_costmodel_default(void);
 /* Configuration index the installed model picks for a request, or -1 when
  * none is installed (the dispatcher then uses its fixed rule).  Single calls
  * pass batch_count = 1 and batch_log2_cells = log2(m * n). */

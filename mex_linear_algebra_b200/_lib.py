@@ -115,6 +115,7 @@ SIGNATURES = {
     "mela_mlp_gradient": (_st, [_vp, _vp, _vp, _vp, _i64, C.c_float, _vp, _vp, _vp]),
     "mela_mlp_adam_step": (_st, [_vp, _vp, _vp, _vp, _i64, C.c_float, _vp]),
     "mela_costmodel_load": (_st, [_vp]),
+    "mela_costmodel_default": (None, []),
     "mela_costmodel_choose": (_i32, [_i32, _i64, _i64, _i64, C.c_double, _i64, C.c_double]),
     "mela_costmodel_features": (None, [_i32, _i64, _i64, _i64, C.c_double, _i64, C.c_double, _vp]),
     "mela_costmodel_config_count": (_i32, [_i32]),

@@ -13,7 +13,10 @@ is the judge of the model's regret.
 
 Requests: the mixed stream of rank, null-space and product requests (m, n,
 p log-uniform in [32, 8192], density log-uniform in [0.001, 0.5],
-``gen.mixed_stream``) and batch requests, half broad (``gen.batch_requests``)
+``gen.mixed_stream``), the same operations at any aspect ratio and down to
+single rows and columns (``gen.wide_requests``: what AUTO is asked outside the
+stream's ranges, where a model trained on the stream alone picked forms up to
+12 times slower than the best) and batch requests, half broad (``gen.batch_requests``)
 and half shaped like parity-check batches (``gen.batch_requests_sparse``):
 a batch of `count` m x n Bernoulli matrices; per-matrix time of each engine.
 
@@ -47,9 +50,10 @@ def _bernoulli(torch, seed, stream_id, m, n, density):
     return t
 
 
-def _time(torch, fn, reps, setup=None):
-    """Median of `reps` CUDA-event timings (us) after one untimed call; a
-    call slower than SLOW_US is timed once."""
+def _time(torch, fn, reps, setup=None, calls=1):
+    """Median of `reps` CUDA-event timings (us) of `calls` calls in a row,
+    per call, after one untimed call; a call slower than SLOW_US is timed
+    once."""
     if setup:
         setup()
     fn()
@@ -59,18 +63,22 @@ def _time(torch, fn, reps, setup=None):
             setup()
         e0, e1 = _events(torch)
         e0.record()
-        fn()
+        for _ in range(calls):
+            fn()
         e1.record()
         e1.synchronize()
-        ts.append(e0.elapsed_time(e1) * 1e3)
+        ts.append(e0.elapsed_time(e1) * 1e3 / calls)
         if ts[-1] > SLOW_US:
             break
     return float(np.median(ts))
 
 
-def time_matmul(torch, m, k, n, density, stream_id, reps=3, extra=None):
+def time_matmul(torch, m, k, n, density, stream_id, reps=3, extra=None, calls=1):
     """Every product configuration (and the `extra` variant arguments, e.g.
-    AUTO) on one request: (times by name, all results identical)."""
+    AUTO) on one request: (times by name, all results identical).  calls > 1
+    times that many products in a row: small ones are bound by the launches
+    (one to three by form), which the next call's overlap in a program but not
+    after an idle stream."""
     L = lib()
     s = torch.cuda.current_stream().cuda_stream
     A = _bernoulli(torch, SEED, 2 * stream_id, m, k, density)
@@ -86,7 +94,7 @@ def time_matmul(torch, m, k, n, density, stream_id, reps=3, extra=None):
         def run():
             check(L.mela_dev_matmul(v, A.data_ptr(), A.shape[1], B.data_ptr(), B.shape[1],
                                     C_.data_ptr(), wn, m, k, n, ws.data_ptr(), wsb, s))
-        times[name] = _time(torch, run, reps)
+        times[name] = _time(torch, run, reps, calls=calls)
         outs[name] = C_
         del ws
     agree = all(torch.equal(outs[x], outs["plain"]) for x in outs)
@@ -170,7 +178,7 @@ def time_request(req, reps=3, extra=None):
     op, m, n, p, d, sid = req["op"], req["m"], req["n"], req.get("p", 0), req["density"], req["stream"]
     out = dict(req)
     if op == "matmul":
-        times, agree = time_matmul(torch, m, n, p, d, sid, reps, extra)
+        times, agree = time_matmul(torch, m, n, p, d, sid, reps, extra, 1 if gen.in_stream(req) else 4)
     elif op == "batch":
         times, rule, agree = time_batch(torch, m, n, d, req["batch_count"], sid, reps)
         out["rule"] = rule
@@ -200,10 +208,12 @@ def stratified(reqs, count: int, bins: int = 12):
 
 
 def build_db(count: int, offset: int, reps: int = 3, max_cells: float = 7e7, batch_count: int = 0,
-             verbose: bool = False, out: str | None = None, budget_s: float = 0.0, window: int = 0):
+             verbose: bool = False, out: str | None = None, budget_s: float = 0.0, window: int = 0,
+             wide: int = 0):
     """Time `count` requests of the mixed stream from request `offset` on
     (requests above `max_cells` bits are skipped; the stream's largest,
-    8192 x 8192, is 6.7e7), then `batch_count` batch requests.  With `out`
+    8192 x 8192, is 6.7e7), then those of `wide` wide requests that lie outside
+    the stream's ranges, then `batch_count` batch requests.  With `out`
     the records so far are written there every 25 requests; with `budget_s`
     each part stops once it has used its share of that many seconds."""
     import torch
@@ -215,6 +225,8 @@ def build_db(count: int, offset: int, reps: int = 3, max_cells: float = 7e7, bat
     else:
         reqs = gen.mixed_stream(offset + count, SEED)[offset:]
     db = []
+    others = [r for r in gen.wide_requests(wide, SEED, offset) if not gen.in_stream(r)]
+    reqs = list(reqs) + others
     t0 = time.time()
 
     def save():
@@ -224,7 +236,7 @@ def build_db(count: int, offset: int, reps: int = 3, max_cells: float = 7e7, bat
     share = budget_s * (0.75 if batch_count else 1.0)
     for i, r in enumerate(reqs):
         cells = r["m"] * r["n"] + (r["n"] * r["p"] if r["op"] == "matmul" else 0)
-        if cells > max_cells:
+        if cells > max_cells and i < len(reqs) - len(others):
             continue
         db.append(time_request(r, reps))
         torch.cuda.empty_cache()
@@ -259,10 +271,11 @@ def main():
     ap.add_argument("--budget", type=float, default=0.0, help="seconds (0: no limit)")
     ap.add_argument("--window", type=int, default=0,
                     help="pick --count requests stratified by size from this many (0: consecutive)")
+    ap.add_argument("--wide", type=int, default=0, help="wide requests (any aspect ratio)")
     ap.add_argument("--out", default="autotune_db.json")
     a = ap.parse_args()
     db = build_db(a.count, a.offset, a.reps, batch_count=a.batches, verbose=True, out=a.out,
-                  budget_s=a.budget, window=a.window)
+                  budget_s=a.budget, window=a.window, wide=a.wide)
     print(f"{len(db)} records -> {a.out}; all configurations agree: {all(r['agree'] for r in db)}")
 
 

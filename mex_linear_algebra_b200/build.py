@@ -69,29 +69,29 @@ def _run(cmd):
     return r.stdout + r.stderr
 
 
-MODEL_JSON = os.path.join(PKG, "costmodel.json")
 MODEL_INC = os.path.join(OBJ, "costmodel_weights.inc")
 
 
 def write_model_weights() -> None:
-    """The trained cost model (costmodel.json) as a C initializer list that
-    mlp.cu compiles in as the library's default dispatch model.  Without a
-    model file of the network's size the include is empty and the library
-    starts on its fixed rule."""
+    """The trained cost models (costmodel.json, costmodel_wide.json) as C
+    initializer lists that mlp.cu compiles in as the library's default dispatch
+    model.  Without a model file of the network's size that part of the include
+    is left out; without the first the library starts on its fixed rule."""
     import json
     import re
-    params = []
-    if os.path.exists(MODEL_JSON):
-        with open(os.path.join(INCLUDE, "mela.h")) as f:
-            want = int(re.search(r"#define MELA_MLP_PARAMS (\d+)", f.read()).group(1))
-        with open(MODEL_JSON) as f:
-            p = json.load(f)["params"]
-        if len(p) == want:
-            params = p
-    text = "// generated from costmodel.json by build.py\n"
-    if params:
-        text += "#define MELA_DEFAULT_MODEL 1\n"
-        text += "static const float kDefaultModel[] = {\n"
+    with open(os.path.join(INCLUDE, "mela.h")) as f:
+        want = int(re.search(r"#define MELA_MLP_PARAMS (\d+)", f.read()).group(1))
+    text = "// generated from the cost model files by build.py\n"
+    for name, macro, array in (("costmodel.json", "MELA_DEFAULT_MODEL", "kDefaultModel"),
+                               ("costmodel_wide.json", "MELA_WIDE_MODEL", "kWideModel")):
+        path = os.path.join(PKG, name)
+        if not os.path.exists(path):
+            continue
+        with open(path) as f:
+            params = json.load(f)["params"]
+        if len(params) != want:
+            continue
+        text += f"#define {macro} 1\nstatic const float {array}[] = {{\n"
         text += ",\n".join(", ".join(f"{float(x)!r}f" for x in params[i:i + 8]) for i in range(0, len(params), 8))
         text += "\n};\n"
     old = open(MODEL_INC).read() if os.path.exists(MODEL_INC) else None

@@ -6,9 +6,10 @@ model predicts log2(microseconds) for each configuration of a request -- a
 variant with its tuning fields (Four-Russians k, tile), or for a matrix in a
 batched launch the engine that runs it; ``choose`` returns the configuration
 with the smallest prediction, and ``install`` hands the weights to the
-library's dispatcher (the library also installs costmodel.json by itself
-when it is built with one).  Without an installed model the library uses its
-fixed rule.
+library's dispatcher.  The library by itself installs what it is built with:
+costmodel.json for the ranges of the mixed request stream and for batches,
+costmodel_wide.json for other requests.  Without an installed model it uses
+its fixed rule.
 
 Inputs per request: shape, density, the op, and the batch mix (how many
 matrices share the launch and their mean log2(m*n); 1 and the request's own
@@ -29,6 +30,7 @@ from ._lib import check, lib
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 DEFAULT_MODEL = os.path.join(PKG, "costmodel.json")
+WIDE_MODEL = os.path.join(PKG, "costmodel_wide.json")  # outside the mixed stream's ranges
 OPS = {"rank": _lib.OP_RANK, "null": _lib.OP_NULL, "matmul": _lib.OP_MATMUL, "batch": _lib.OP_BATCH}
 
 # Configuration names in the model's output order (dispatch.cu lists the
@@ -98,7 +100,8 @@ def init_params(seed: int = 0) -> np.ndarray:
 
 
 def train(records, steps: int = 3000, lr: float = 3e-3, seed: int = 0, log_every: int = 0):
-    """Full-batch Adam on the GPU.  Returns (params float32, final loss)."""
+    """Full-batch Adam on the GPU, the step size falling to zero along a half
+    cosine.  Returns (params float32, final loss)."""
     import torch
     X, T, Mk = dataset(records)
     dev = torch.device("cuda")
@@ -116,7 +119,8 @@ def train(records, steps: int = 3000, lr: float = 3e-3, seed: int = 0, log_every
     for step in range(1, steps + 1):
         check(L.mela_mlp_gradient(P.data_ptr(), dX.data_ptr(), dT.data_ptr(), dM.data_ptr(), len(X),
                                   inv, G.data_ptr(), loss.data_ptr(), s))
-        check(L.mela_mlp_adam_step(P.data_ptr(), G.data_ptr(), m1.data_ptr(), m2.data_ptr(), step, lr, s))
+        rate = 0.5 * lr * (1.0 + math.cos(math.pi * (step - 1) / steps))
+        check(L.mela_mlp_adam_step(P.data_ptr(), G.data_ptr(), m1.data_ptr(), m2.data_ptr(), step, rate, s))
         if log_every and step % log_every == 0:
             print(f"step {step} loss {loss.item() * inv:.4f}")
     last = float(loss.item()) * inv
@@ -170,8 +174,9 @@ def predict_host(op: str, m: int, n: int, p: int, density: float, batch_count: i
 
 
 def install_default():
-    """Put back the model the library loads with (costmodel.json), if any."""
-    install(load() if os.path.exists(DEFAULT_MODEL) else None)
+    """Put back the model the library loads with (costmodel.json and
+    costmodel_wide.json as built), if any."""
+    lib().mela_costmodel_default()
 
 
 def choose(op: str, m: int, n: int, p: int, density: float, batch_count: int = 1,

@@ -159,16 +159,32 @@ __global__ void adam_kernel(float *__restrict__ params, const float *__restrict_
 // ---------------------------------------------------------------- host-side model
 // The dispatch copy of the trained parameters (host memory): single calls
 // evaluate the tiny network on the host to pick a variant before launching.
-// The model trained with the library (costmodel.json, compiled in by the
-// build) is installed when the library loads; mela_costmodel_load replaces
-// or removes it.
+// The library loads with two sets, compiled in by the build: one trained on the
+// mixed request stream and on batches (costmodel.json), and one for requests
+// outside that stream's ranges (costmodel_wide.json; the first one's choices
+// there cost up to 12 times the best: products with a short K, single rows and
+// columns).  One set for both fits neither as well.  mela_costmodel_load
+// replaces both by one, or removes them.
 #include "costmodel_weights.inc"
 // Installed weights: an immutable snapshot swapped under the mutex and read
 // through a shared pointer, so an evaluation neither copies the weights nor
 // holds the lock while it runs.
 struct CostModelWeights {
     float p[kParams];
+    bool has_wide = false;
+    float wide[kParams];  // for requests outside the mixed stream's ranges
 };
+// The mixed stream's ranges (gen.py: in_stream); batches have one set.
+static bool in_stream(int op, double m, double n, double p)
+{
+    if (op == MELA_OP_BATCH) return true;
+    const bool mn = m >= 32 && m <= 8192 && n >= 32 && n <= 8192 && m <= 8 * n && n <= 8 * m;
+    return mn && (op != MELA_OP_MATMUL || (p >= 32 && p <= 8192));
+}
+static const float *weights_for(const CostModelWeights &w, int op, double m, double n, double p)
+{
+    return w.has_wide && !in_stream(op, m, n, p) ? w.wide : w.p;
+}
 static std::mutex g_cm_mu;
 static std::shared_ptr<const CostModelWeights> g_cm;
 static std::atomic<unsigned> g_cm_generation{1};  // bumped on every install or removal
@@ -181,15 +197,27 @@ static std::shared_ptr<const CostModelWeights> current_model()
     return g_cm;
 }
 
+// The compiled-in model (null: the library was built without one).
+static std::shared_ptr<const CostModelWeights> default_model()
+{
 #ifdef MELA_DEFAULT_MODEL
-static_assert(sizeof kDefaultModel / sizeof kDefaultModel[0] == kParams, "compiled-in model size");
-static const bool g_cm_default = [] {
+    static_assert(sizeof kDefaultModel / sizeof kDefaultModel[0] == kParams, "compiled-in model size");
     auto w = std::make_shared<CostModelWeights>();
     std::memcpy(w->p, kDefaultModel, sizeof w->p);
-    g_cm = w;
+#ifdef MELA_WIDE_MODEL
+    static_assert(sizeof kWideModel / sizeof kWideModel[0] == kParams, "compiled-in model size");
+    std::memcpy(w->wide, kWideModel, sizeof w->wide);
+    w->has_wide = true;
+#endif
+    return w;
+#else
+    return nullptr;
+#endif
+}
+static const bool g_cm_default = [] {
+    g_cm = default_model();
     return true;
 }();
-#endif
 
 // The network on the host, layer by layer along contiguous weight rows.
 static void host_forward(const float *P, const float *x, float *y)
@@ -247,7 +275,7 @@ bool costmodel_predict(int op, double m, double n, double p, double density, dou
     if (!w) return false;
     float x[kIn], y[kOut];
     costmodel_features(op, m, n, p, density, batch_count, batch_log2_cells, x);
-    host_forward(w->p, x, y);
+    host_forward(weights_for(*w, op, m, n, p), x, y);
     const int nc = config_count(op);
     for (int o = 0; o < nc; ++o) y_out[o] = y[o];
     return true;
@@ -263,7 +291,7 @@ bool costmodel_predict_densities(int op, double m, double n, double p, const dou
     constexpr int NP = kCostProbes;
     const std::shared_ptr<const CostModelWeights> w = current_model();
     if (!w) return false;
-    const float *P = w->p;
+    const float *P = weights_for(*w, op, m, n, p);
     float x[kIn];
     costmodel_features(op, m, n, p, 0.5, batch_count, batch_log2_cells, x);
     float base[kH1];
@@ -380,6 +408,13 @@ extern "C" mela_status mela_costmodel_load(const float *h_params)
     g_cm = std::move(w);
     g_cm_generation.fetch_add(1, std::memory_order_acq_rel);
     return MELA_OK;
+}
+
+extern "C" void mela_costmodel_default(void)
+{
+    std::lock_guard<std::mutex> g(g_cm_mu);
+    g_cm = default_model();
+    g_cm_generation.fetch_add(1, std::memory_order_acq_rel);
 }
 
 extern "C" int32_t mela_costmodel_choose(int32_t op, int64_t m, int64_t n, int64_t p, double density,

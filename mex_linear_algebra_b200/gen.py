@@ -19,6 +19,9 @@ Configurations (seeds as in the benchmark definitions):
   words 3.. of the same stream.
 * mixed request stream -- ``mixed_stream``: m, n, p log-uniform in
   [32, 8192], density log-uniform in [0.001, 0.5], aspect ratio <= 8:1.
+* wide requests -- ``wide_requests``: rank, null-space and product requests of
+  any aspect ratio, from single rows and columns up (for training the
+  dispatch: a program's products can be 7000 x 40 by 40 x 16000).
 * batch requests -- ``batch_requests``: homogeneous batches for timing the
   batched engines: m log-uniform in [32, 1024], n = m * [1, 3], density
   log-uniform in [0.002, 0.5], 64 to 4096 matrices.
@@ -158,6 +161,40 @@ def mixed_stream(count: int = 50000, seed: int = 4):
     names = np.array(["rank", "null", "matmul"])[op]
     return [dict(op=str(names[i]), m=int(round(m[i])), n=int(round(n[i])), p=int(round(p[i])),
                  density=float(dens[i]), stream=i) for i in range(count)]
+
+
+def in_stream(r) -> bool:
+    """Whether a request lies in the mixed stream's ranges (mlp.cu: in_stream)."""
+    m, n = r["m"], r["n"]
+    return (32 <= m <= 8192 and 32 <= n <= 8192 and m <= 8 * n and n <= 8 * m and
+            (r["op"] != "matmul" or 32 <= r["p"] <= 8192))
+
+
+def wide_requests(count: int, seed: int = 4, offset: int = 0):
+    """Requests like mixed_stream's with every dimension log-uniform on its
+    own: products in [1, 32768] and at most 2^38 bit products, eliminations in
+    [1, 16384] and at most 2^25 bits; one request in four up to 2^20 (products)
+    or 2^17 (eliminations).  Word layout per request r: stream 1000000 + offset
+    + r, word 0 the op, 1 the density, then three words a try until the size
+    fits."""
+    out = []
+    for i in range(offset, offset + count):
+        w = words(seed, 1000000 + i, 0, 2 + 3 * 64).astype(np.float64) / 2.0 ** 64
+        op = ("rank", "null", "matmul")[int(w[0] * 3)]
+        big, prod = i % 4 == 0, op == "matmul"
+        hi = (20 if big else 15) if prod else (17 if big else 14)
+        for t in range(2, len(w) - 2, 3):
+            m, n, p = (int(round(2.0 ** (hi * x))) for x in w[t:t + 3])
+            if not prod:
+                p = 0
+            if m * n * p <= 1 << 38 and max(m * n, n * p, m * p) <= (1 << 31 if prod else 1 << 25):
+                break
+        else:
+            m = n = 64
+            p = 64 if prod else 0
+        out.append(dict(op=op, m=m, n=n, p=p, density=float(np.exp(np.log(0.001) + np.log(500.0) * w[1])),
+                        stream=300000 + i))
+    return out
 
 
 def batch_requests(count: int, seed: int = 4, offset: int = 0):

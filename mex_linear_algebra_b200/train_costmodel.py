@@ -3,6 +3,8 @@
     python -m mex_linear_algebra_b200.train_costmodel --train train.json --eval eval.json \
         --out mex_linear_algebra_b200/costmodel.json
 
+(and the same with a database of wide requests for costmodel_wide.json).
+
 Training runs on the GPU in the library's own kernels.  The report compares,
 on the evaluation records (every variant timed), the total time of the
 model's choices with the exhaustive best (regret) and with the fixed rule.
