@@ -34,6 +34,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 
 namespace mela {
 
@@ -61,7 +62,10 @@ __device__ __forceinline__ void gray_walk(u64 *Ts, int i0, u64 &val, const u64 (
 
 constexpr int M4_BTILE_WORDS = 16 * M4_CTA_WORDS;  // one stage's rows of B (4 KB)
 
-template <int WARPS, bool kTma>
+// kSplit: one slice of K of several (a variant of its own: with both ways to write
+// C in one kernel, a whole product took 2 to 6 us more, 28.3 against 22.1 us for
+// 9268 x 1 x 15331).
+template <int WARPS, bool kTma, bool kSplit>
 __global__ void __launch_bounds__(WARPS * 32, 1)
 gemm_m4ri_kernel(const u64 *__restrict__ A, i64 lda, const u64 *__restrict__ B, i64 ldb,
                  u64 *__restrict__ C, i64 ldc, i64 m, i64 k, i64 n, i64 stages_per_split,
@@ -87,8 +91,8 @@ gemm_m4ri_kernel(const u64 *__restrict__ A, i64 lda, const u64 *__restrict__ B, 
     for (int r = 0; r < M4_ROWS_PER_WARP; ++r) acc[r] = 0;
 
     // this CTA's stages: st0 .. nstages-1 (st0 a multiple of 4, whole words of A)
-    const i64 st0 = (i64)blockIdx.z * stages_per_split;
-    const i64 all = (k + 15) / 16, nstages = st0 + stages_per_split < all ? st0 + stages_per_split : all;
+    const i64 st0 = kSplit ? (i64)blockIdx.z * stages_per_split : 0;
+    const i64 all = (k + 15) / 16, nstages = kSplit && st0 + stages_per_split < all ? st0 + stages_per_split : all;
 
     // B: the 8 rows of this warp's strip in stage st, this lane's word
     auto load_b = [&](i64 st, u64 (&bv)[8]) {
@@ -187,10 +191,10 @@ gemm_m4ri_kernel(const u64 *__restrict__ A, i64 lda, const u64 *__restrict__ B, 
         for (int r = 0; r < M4_ROWS_PER_WARP; ++r) {
             const i64 row = row0 + r;
             if (row < m) {
-                if (gridDim.z == 1)
-                    C[row * ldc + cw] = acc[r];
-                else
+                if constexpr (kSplit)
                     atomicXor(&C[row * ldc + cw], acc[r]);
+                else
+                    C[row * ldc + cw] = acc[r];
             }
         }
     }
@@ -220,13 +224,15 @@ mela_status launch_gemm_m4ri(const u64 *A, i64 lda, const u64 *B, i64 ldb, u64 *
     u32 *err = device_error_word();
     // K slices: as many as one wave of CTAs takes (one per SM), each of at least
     // 4 stages (one word of A; a stage takes 2.3 us, the launch, first loads and
-    // the atomic writes of a block about 6).  3001 x 2500 x 1777: 25.5 us in 20
-    // slices, 367 us unsplit; 8192^3 in two 0.64 ms, 1.21 ms unsplit.
+    // the atomic writes of a block about 6), and none up to 6 stages, which the
+    // clearing of C costs again (922 x 80 x 1137 17.7 us whole, 18.7 in two; at
+    // K = 128 24.0 and 18.8).  3001 x 2500 x 1777: 25.5 us in 20 slices, 367 us
+    // unsplit; 8192^3 in two 0.64 ms, 1.21 ms unsplit.
     // A result over an operand stays in one slice: a block of C is then written
     // after its CTA's last read (C over A is right up to 2048 columns, one block
     // wide, C over B up to 512 rows), where slices would clear the operand first.
     const i64 nstages = (k + 15) / 16;
-    i64 splits = std::min<i64>(sm_count() / (gx * gy), (nstages + 3) / 4);
+    i64 splits = nstages > 6 ? std::min<i64>(sm_count() / (gx * gy), (nstages + 3) / 4) : 1;
     if (!packed_apart(A, lda, m, k, C, ldc, m, n) || !packed_apart(B, ldb, k, n, C, ldc, m, n)) splits = 1;
     i64 per = nstages;
     if (splits > 1) {
@@ -242,11 +248,13 @@ mela_status launch_gemm_m4ri(const u64 *A, i64 lda, const u64 *B, i64 ldb, u64 *
         kernel<<<grid, threads, smem, s>>>(A, lda, B, ldb, C, ldc, m, k, n, per, bmap, err);
         return MELA_OK;
     };
-    mela_status st;
-    if (tile == 1)
-        st = tma ? launch(gemm_m4ri_kernel<8, true>, 256) : launch(gemm_m4ri_kernel<8, false>, 256);
-    else
-        st = tma ? launch(gemm_m4ri_kernel<16, true>, 512) : launch(gemm_m4ri_kernel<16, false>, 512);
+    auto pick = [&](auto split) -> mela_status {
+        constexpr bool kSplit = decltype(split)::value;
+        if (tile == 1)
+            return tma ? launch(gemm_m4ri_kernel<8, true, kSplit>, 256) : launch(gemm_m4ri_kernel<8, false, kSplit>, 256);
+        return tma ? launch(gemm_m4ri_kernel<16, true, kSplit>, 512) : launch(gemm_m4ri_kernel<16, false, kSplit>, 512);
+    };
+    const mela_status st = splits > 1 ? pick(std::true_type{}) : pick(std::false_type{});
     if (st != MELA_OK) return st;
     MELA_LAUNCH_CHECK("gemm_m4ri_kernel");
     return MELA_OK;
