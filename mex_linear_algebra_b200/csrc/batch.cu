@@ -11,7 +11,7 @@
 //          (256 threads)    not fit, the CTA's L2-resident global scratch;
 //                           blocked by 64-column panels (process_big_blocked)
 //
-// (two CTAs per SM; the single-matrix fused mode runs the big engine in one
+// (two CTAs per SM; the single-matrix fused mode runs the column or the big engine in one
 // CTA of 512 threads with 220 KB)
 //
 // The host sorts the matrices into the three classes (largest first inside
@@ -99,7 +99,7 @@ __device__ __forceinline__ int ctz64b(u64 x) { return __ffsll((long long)x) - 1;
 template <int G>
 __device__ void process_matrix(const BatchDevItem &it, const u64 *__restrict__ in, u64 *__restrict__ zt,
                                long long *ranks, int item, unsigned char *region, u64 *gmat, int gtid,
-                               int bar_id)
+                               int bar_id, const FusedOut *fo = nullptr)
 {
     const int m = it.m, n = it.n, wc = (n + 63) >> 6, mn = m < n ? m : n;
     const bool in_smem = it.flags & 1;
@@ -164,6 +164,20 @@ __device__ void process_matrix(const BatchDevItem &it, const u64 *__restrict__ i
         }
         search(c + 1);
         group_sync(G, bar_id);
+    }
+    if (fo) {
+        // single-matrix mode: RREF rows back to the caller, pivot lists, rank
+        for (long long e = gtid; e < (long long)m * wc; e += G) {
+            const int rr = (int)(e / wc), x = (int)(e - (long long)rr * wc);
+            fo->M[(long long)rr * fo->ldm + x] = A[(size_t)rr * ld + x];
+        }
+        for (int t = gtid; t < r; t += G) {
+            fo->piv[t] = piv[t];
+            fo->prow[t] = prow[t];
+        }
+        if (gtid == 0) *fo->rank = r;
+        group_sync(G, bar_id);
+        return;
     }
     if (gtid == 0) ranks[item] = r;
 
@@ -1525,15 +1539,31 @@ __global__ void __launch_bounds__(256) batch_unpack_kernel(const BatchDevItem *_
 }
 
 // ---------------------------------------------------------------- single matrix
-// RREF of one matrix too large for shared memory (elim_small.cu) by one CTA in
-// one launch: the blocked engine over global scratch.  Reads the packed matrix
-// from a compact copy and writes the RREF rows over the caller's matrix (row
-// pitch ldm, any pitch >= ceil(n/64)).
+// RREF of one matrix that elim_small.cu does not take, by one CTA in one launch:
+// column by column in shared memory (flags 1), else by the blocked engine over
+// global scratch.  Reads the packed matrix from a compact copy and writes the
+// RREF rows over the caller's matrix (row pitch ldm, any pitch >= ceil(n/64)).
 __global__ void __launch_bounds__(kThreads, 1)
 fused_elim_kernel(BatchDevItem it, const u64 *__restrict__ in_compact, FusedOut fo, u64 *scratch)
 {
     extern __shared__ __align__(16) unsigned char smem[];
-    process_big_blocked<kThreads, kSmemTotal, false>(it, in_compact, nullptr, nullptr, 0, smem, scratch, &fo);
+    if (it.flags & 1)
+        process_matrix<kThreads>(it, in_compact, nullptr, nullptr, 0, smem, nullptr, threadIdx.x, 0, &fo);
+    else
+        process_big_blocked<kThreads, kSmemTotal, false>(it, in_compact, nullptr, nullptr, 0, smem, scratch, &fo);
+}
+
+// Where the column-by-column engine takes a matrix of more than 512 rows: the
+// blocked engine pays a panel's selection, reduced rows and barriers for every 64
+// columns however few there are, and holds a panel of up to 1024 rows in
+// registers.  (512 < m <= 1024, device time columns / blocked: 1000 x 16 33 / 51
+// us, x 32 49 / 54, 513 x 32 49 / 49, 1000 x 64 80 / 59; above: 6697 x 4 41 / 388,
+// 20000 x 8 111 / 1099, 2906 x 300 742 / 833, 2000 x 500 1011 / 1147, 1456 x 500
+// 809 / 812, 2000 x 800 1920 / 1894.)
+static bool columns_take(i64 m, i64 n)
+{
+    if (m > 32768 || n > (m > 1024 ? 480 : 24)) return false;
+    return aux_bytes((int)m, (int)n) + (size_t)m * smem_ld((int)n) * 8 <= (size_t)kSmemTotal;
 }
 
 size_t fused_workspace(i64 m, i64 n)
@@ -1566,6 +1596,7 @@ mela_status launch_fused_elim(u64 *M, i64 ld, i64 m, i64 n, long long *d_rank, l
     it.n = (int)n;
     it.in_off = 0;
     it.z_off = 0;
+    it.flags = columns_take(m, n) ? 1 : 0;
     FusedOut fo{M, ld, d_rank, d_piv, d_prow};
     MELA_CUDA_TRY(cudaFuncSetAttribute(fused_elim_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        kSmemTotal));
