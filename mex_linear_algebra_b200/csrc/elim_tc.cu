@@ -9,8 +9,8 @@
 // pivot t lives in physical row prow[t].
 //
 // One window of 256 columns (4 words) at a time:
-//   window_factor   one CTA.  Walks the list of active rows in chunks of 320
-//                   nonzero ones and brings the window part to reduced row echelon form
+//   window_factor   one CTA.  Walks the list of active rows in chunks of up to
+//                   320 nonzero ones and brings the window part to reduced row echelon form
 //                   (lowest set bit leading), 32 columns at a time.  Every
 //                   basis vector carries its combination ("tag") over the rows
 //                   P_b that entered the basis, so R_window = tag * A[P, window].
@@ -66,6 +66,7 @@ constexpr int WF_ROWS = 320;     // a chunk of rows; 320 random rows span 256 co
 constexpr int WF_WARPS = WF_ROWS / 32 + 3;
 constexpr int WF_THREADS = 32 * WF_WARPS;
 constexpr int WF_SELECTOR = 3;
+constexpr int WF_SPARSE = 32;  // set bits up to which a row is reduced bit by bit
 static_assert(WF_ROWS == 320, "ten row warps on three schedulers");
 
 // Everything that belongs to a pivot of a window is indexed by its column in
@@ -187,8 +188,8 @@ __device__ __forceinline__ u32 wf_half(const WfSmem &S, const u32 (&v)[8], int h
 // and elsewhere its data (a row with bit c set gets v ^= v_p without bit c, so
 // its bit c stays set and becomes the coefficient of P_c).  One CTA walks the
 // active rows in chunks of a row per thread, leaving out the rows that are zero
-// modulo the basis so far (most rows of a sparse matrix); the columns go 32 at a time (half
-// words): up to 64 rows with data left there are eliminated by one warp
+// modulo the basis so far (most rows of a sparse matrix; few-bit rows are reduced
+// bit by bit, others through tables); the columns go 32 at a time (half words): up to 64 rows with data left there are eliminated by one warp
 // (half_word_select), and every row of the chunk then takes the round's pivots
 // in through 4-bit tables; rounds repeat until no unused row has data left in
 // the half word.  Where a round fills its half word, the rows first bring only
@@ -229,7 +230,7 @@ window_factor_kernel(const u64 *__restrict__ M, i64 ld, i64 m, i64 n, i64 w, int
 
     u32 H[8] = {};  // pivot columns so far (the same in every thread)
     int nb = 0;     // their number
-    int walked = 0, par = 0;
+    int walked = 0, par = 0, chunks = 0;
     while (walked < na && nb < valid) {
         const bool older = nb > 0;  // basis vectors of earlier chunks
         u32 H0[8];
@@ -249,35 +250,53 @@ window_factor_kernel(const u64 *__restrict__ M, i64 ld, i64 m, i64 n, i64 w, int
             }
             __syncthreads();
         }
-        // the next rows that are not zero modulo the basis, up to WF_ROWS of
-        // them, from blocks of WF_ROWS list entries
+        // the next rows that are not zero modulo the basis, from blocks of
+        // WF_ROWS list entries, until there are enough of them to span the
+        // columns that are left: more with each chunk of the window, as the rows
+        // of a sparse matrix depend on one another.  (Always WF_ROWS of them
+        // walked all of a tall sparse matrix for its last columns: rank of
+        // 1000000 x 64 of density 0.001 3.46 ms, 0.17 this way, 100000 x 200 of
+        // 0.01 216 and 70 us; fewer from the start cost sparse square matrices
+        // chunks: 8192 x 1024 of 0.003 480 us with half of this, 376.)
+        const int goal = min(WF_ROWS, (4 << min(chunks, 6)) * (valid - nb) + 8);
+        ++chunks;
         int row = -1, filled = 0;
         u32 v[8] = {};
-        for (;;) {
-            const int k = walked + ri;
-            int kr = -1;
-            u32 x[8] = {};
-            if (holds && k < na) {
-                kr = L0[k];
+        auto words_of_row = [&](int r, u32 (&x)[8]) {
 #pragma unroll
-                for (int q = 0; q < WW; ++q)
-                    if (q < wn) {
-                        const u64 t = M[(i64)kr * ld + w + q];
-                        x[2 * q] = (u32)t;
-                        x[2 * q + 1] = (u32)(t >> 32);
-                    }
+            for (int q = 0; q < WW; ++q) {
+                const u64 t = r >= 0 && q < wn ? M[(i64)r * ld + w + q] : 0ull;
+                x[2 * q] = (u32)t;
+                x[2 * q + 1] = (u32)(t >> 32);
             }
+        };
+        int kr = holds && walked + ri < na ? L0[walked + ri] : -1;
+        u32 x[8];
+        words_of_row(kr, x);
+        for (;;) {
+            const int next = walked + WF_ROWS + ri, kn = holds && next < na ? L0[next] : -1;
             if (older) {
                 u32 y[8];
+                int bits = 0;
 #pragma unroll
                 for (int q = 0; q < 8; ++q) {
                     y[q] = x[q] & H0[q];
                     x[q] &= ~H0[q];
+                    bits += __popc(y[q]);
                 }
+                if (__reduce_max_sync(0xffffffffu, bits) <= WF_SPARSE) {  // (sparse rows: 64 table steps for a few bits)
 #pragma unroll
-                for (int g = 0; g < 64; ++g) {
-                    const int e = (int)((y[g >> 3] >> (4 * (g & 7))) & 15);
-                    if (e) xor8(x, S.tab[0][g][e], S.tab[1][g][e]);
+                    for (int q = 0; q < 8; ++q)
+                        for (u32 c = y[q]; c; c &= c - 1) {
+                            const uint4 *u = S.basis[32 * q + __ffs((int)c) - 1];
+                            xor8(x, u[0], u[1]);
+                        }
+                } else {
+#pragma unroll
+                    for (int g = 0; g < 64; ++g) {
+                        const int e = (int)((y[g >> 3] >> (4 * (g & 7))) & 15);
+                        if (e) xor8(x, S.tab[0][g][e], S.tab[1][g][e]);
+                    }
                 }
             }
             u32 any = 0;
@@ -288,7 +307,7 @@ window_factor_kernel(const u64 *__restrict__ M, i64 ld, i64 m, i64 n, i64 w, int
             if (holds && lane == 0) S.wcnt[par][rw] = __popc(bal);
             const int total = __syncthreads_count(any != 0);
             const bool last = walked + WF_ROWS >= na;
-            if (filled == 0 && (last || 4 * total >= 3 * WF_ROWS)) {
+            if (filled == 0 && (last || total >= goal || 4 * total >= 3 * WF_ROWS)) {
                 // the block as it is: filling it up would not save a chunk
                 row = kr;
 #pragma unroll
@@ -297,6 +316,8 @@ window_factor_kernel(const u64 *__restrict__ M, i64 ld, i64 m, i64 n, i64 w, int
                 filled = total;
                 break;
             }
+            u32 xn[8];  // on their way while this block is written out
+            words_of_row(kn, xn);
             const int wv = lane < rw && lane < NW ? S.wcnt[par][lane] : 0;
             const int idx = filled + __reduce_add_sync(0xffffffffu, wv) + __popc(bal & ((1u << lane) - 1));
             if (any && idx < WF_ROWS) {
@@ -309,7 +330,7 @@ window_factor_kernel(const u64 *__restrict__ M, i64 ld, i64 m, i64 n, i64 w, int
             const bool over = filled + total > WF_ROWS;
             walked = over ? walked + S.cut : last ? na : walked + WF_ROWS;
             filled = over ? WF_ROWS : filled + total;
-            if (filled == WF_ROWS || walked >= na) {
+            if (filled >= goal || walked >= na) {
                 if (ri < filled) {
                     const uint4 a = S.vrow[ri][0], b = S.vrow[ri][1];
                     v[0] = a.x;
@@ -324,6 +345,9 @@ window_factor_kernel(const u64 *__restrict__ M, i64 ld, i64 m, i64 n, i64 w, int
                 }
                 break;
             }
+            kr = kn;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) x[q] = xn[q];
         }
         if (filled == 0) break;  // only rows inside the span were left
         int mycol = -1;  // this row's pivot column
