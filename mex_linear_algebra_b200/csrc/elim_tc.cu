@@ -1382,6 +1382,7 @@ mela_status elim_windows_device(u64 *M, i64 ld, i64 m, i64 n, int rref, bool tab
                 MELA_CUDA_TRY(cudaStreamWaitEvent(sx, ev_join, 0));
                 forked = false;
             }
+            if (!rref && w + WW >= wc) break;  // a rank: no column is left to update
             window_near_kernel<<<near_blocks, 256, nr_smem, sx>>>(M, ld, m, wc, w, list, stamp, wid, rref, cur, ulist,
                                                                  X8, tables ? 0 : 1, live);
             MELA_CUDA_TRY(cudaEventRecord(ev_fork, sx));
