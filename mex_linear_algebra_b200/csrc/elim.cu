@@ -43,8 +43,6 @@
 namespace mela {
 
 // ---------------------------------------------------------------- helpers
-__device__ __forceinline__ int ctz64(u64 x) { return ctz64_(x); }
-
 // Panel bookkeeping shared by the blocked kernels (device memory); everything
 // of a pivot is indexed by its column in the panel.
 struct PanelState {
@@ -57,11 +55,17 @@ struct PanelState {
 };
 
 // ---------------------------------------------------------------- panel_select
-// Word 0 of every row: the first panel's words.
-__global__ void panel_words_kernel(const u64 *__restrict__ M, i64 ld, i64 m, u64 *__restrict__ y)
+// The state before the first panel: every row active, no pivots, word 0 of every
+// row (the first panel's words).  One launch instead of three fills and one.
+__global__ void panel_init_kernel(const u64 *__restrict__ M, i64 ld, i64 m, unsigned char *state, int *stamp,
+                                  PanelState *ps, u64 *__restrict__ y)
 {
-    for (i64 j = blockIdx.x * (i64)blockDim.x + threadIdx.x; j < m; j += (i64)gridDim.x * blockDim.x)
+    for (i64 j = blockIdx.x * (i64)blockDim.x + threadIdx.x; j < m; j += (i64)gridDim.x * blockDim.x) {
         y[j] = M[j * ld];
+        state[j] = 1;
+        stamp[j] = -1;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) ps->rank = 0;
 }
 
 namespace {
@@ -743,9 +747,13 @@ mela_status elim_device(int variant_arg, u64 *M, i64 ld, i64 m, i64 n, int rref,
     // the tensor cores; RREF 4096 x 8192 603 / 656, 8192 x 8192 1230 / 1183).
     // The windows want a 16-byte aligned workspace, and more of it than the
     // panels: a Four-Russians call that brings less takes panels, and so does
-    // AUTO on another alignment.
+    // AUTO on another alignment.  So does an RREF of one panel, where a window's
+    // launches and fork cost more (20 x 20 27 against 37 us a call, 5000 x 64 32
+    // against 38, 50000 x 64 32 against 56; a rank ends with the factorization,
+    // 16 us).
     const bool aligned = ((uintptr_t)ws & 15) == 0;
-    const bool tables = (variant_arg == MELA_ELIM_M4RI && aligned && ws_bytes >= elim_tc_workspace(m, n)) ||
+    const bool tables = (variant_arg == MELA_ELIM_M4RI && aligned && ws_bytes >= elim_tc_workspace(m, n) &&
+                         !(rref && n <= 64)) ||
                         (chosen && variant == MELA_ELIM_TC && aligned && (double)m * (double)n <= 4e7);
     if (chosen && variant == MELA_ELIM_TC && !aligned) {
         variant = MELA_ELIM_M4RI;
@@ -769,8 +777,8 @@ mela_status elim_device(int variant_arg, u64 *M, i64 ld, i64 m, i64 n, int rref,
     u64 *ysnap[2] = {(u64 *)(w + L.ysnap), (u64 *)(w + L.ysnap + al256((size_t)m * 8))};
     const i64 wc = words_of(n);
 
-    MELA_CUDA_TRY(cudaMemsetAsync(state, 1, (size_t)m, s));
     if (variant == MELA_ELIM_PLAIN) {
+        MELA_CUDA_TRY(cudaMemsetAsync(state, 1, (size_t)m, s));
         int init[3] = {INT_MAX, INT_MAX, INT_MAX};
         MELA_CUDA_TRY(cudaMemcpyAsync(cand, init, sizeof init, cudaMemcpyHostToDevice, s));
         MELA_CUDA_TRY(cudaMemsetAsync(gb, 0, sizeof(GridBar), s));
@@ -804,8 +812,6 @@ mela_status elim_device(int variant_arg, u64 *M, i64 ld, i64 m, i64 n, int rref,
         set_error("unknown elimination variant %d", variant);
         return MELA_ERR_INVALID;
     }
-    MELA_CUDA_TRY(cudaMemsetAsync(stamp, 0xff, (size_t)m * 4, s));
-    MELA_CUDA_TRY(cudaMemsetAsync(ps, 0, sizeof(PanelState), s));
     const PanelUpdateFn update = panel_update_for(tune.k);
     if (!update) {
         set_error("blocked elimination: M4RI k = %d (4 or 6..10 supported)", tune.k);
@@ -827,7 +833,7 @@ mela_status elim_device(int variant_arg, u64 *M, i64 ld, i64 m, i64 n, int rref,
     if (mela_status st = update(M, ld, m, wc, 0, ps, rbuf, state, stamp, 0, rref, nullptr, nullptr, 0, s, true);
         st != MELA_OK)
         return st;
-    panel_words_kernel<<<grid_cap(m, 256), 256, 0, s>>>(M, ld, m, ysnap[0]);
+    panel_init_kernel<<<grid_cap(m, 256), 256, 0, s>>>(M, ld, m, state, stamp, ps, ysnap[0]);
     for (i64 pw = 0; pw < wc; ++pw) {  // every word column is one panel
         const u64 *y = ysnap[pw & 1];
         panel_select_kernel<<<1, SEL_THREADS, 0, s>>>(y, m, n, pw, state, stamp, (int)pw, ps, d_piv, d_prow);
