@@ -106,6 +106,7 @@ panel_select_kernel(const u64 *__restrict__ y, i64 m, i64 n, i64 w, unsigned cha
     constexpr int NW = SEL_THREADS / 32;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int valid = n - 64 * w < 64 ? (int)(n - 64 * w) : 64;
+    const long long r0 = ps->rank;
     u64 H = 0;  // pivot columns so far
     int nb = 0, par = 0;
     for (i64 base = 0; base < m && nb < valid; base += SEL_THREADS) {
@@ -129,6 +130,7 @@ panel_select_kernel(const u64 *__restrict__ y, i64 m, i64 n, i64 w, unsigned cha
 #pragma unroll
             for (int g = 0; g < 16; ++g) v ^= S.tab[g][(yb >> (4 * g)) & 15];
         }
+        if (r0 >= m) break;  // every row is a pivot row
         int mycol = -1;
         for (int h = 0; h < 2 && nb < valid; ++h) {
             u32 Hh = (u32)(H >> (32 * h));
@@ -187,7 +189,6 @@ panel_select_kernel(const u64 *__restrict__ y, i64 m, i64 n, i64 w, unsigned cha
         if (mycol >= 0) S.basis[mycol] = v;
         __syncthreads();
     }
-    const long long r0 = ps->rank;
     __syncthreads();  // every thread has read the rank before it is advanced
     if (tid < 64) {
         int r = -1;
@@ -279,9 +280,10 @@ panel_update_kernel(u64 *__restrict__ M, i64 ld, i64 m, i64 wc, i64 w, const Pan
     const int tid = threadIdx.x;
     const i64 row0 = (i64)blockIdx.y * rt;
     // the next panel's words (word w + 1, in the first column tile) also go,
-    // packed, to ynext
+    // packed, to ynext, unless every row is a pivot row and none is looked at
+    // any more (55 x 5400, 84 panels behind the last pivot: 958 -> 780 us)
     if (p == 0) {
-        if (blockIdx.x == 0 && w + 1 < wc)
+        if (blockIdx.x == 0 && w + 1 < wc && ps->rank < m)
             for (i64 j = row0 + tid; j < row0 + rt && j < m; j += 256) ynext[j] = M[j * ld + w + 1];
         return;
     }
