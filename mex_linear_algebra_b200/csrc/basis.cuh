@@ -1,6 +1,7 @@
 // basis.cuh -- Gauss-Jordan elimination of a few rows over a 32-column half
 // word by one warp: the pivot search of the blocked eliminations (elim.cu,
-// elim_tc.cu).
+// elim_tc.cu) and of small matrices (elim_small.cu), and the tables of a round's
+// pivots, which the batch engine's selection (batch.cu) also uses.
 //
 // Rows are kept in in-place form: at the pivot columns found so far a row
 // holds its combination over the pivot rows (bit c: contains the original row

@@ -174,11 +174,12 @@ struct CostModelWeights {
     bool has_wide = false;
     float wide[kParams];  // for requests outside the mixed stream's ranges
 };
-// The mixed stream's ranges (gen.py: in_stream); batches have one set.
+// The mixed stream's ranges (gen.py: in_stream; 8:1 with room for its rounding);
+// batches have one set.
 static bool in_stream(int op, double m, double n, double p)
 {
     if (op == MELA_OP_BATCH) return true;
-    const bool mn = m >= 32 && m <= 8192 && n >= 32 && n <= 8192 && m <= 8 * n && n <= 8 * m;
+    const bool mn = m >= 32 && m <= 8192 && n >= 32 && n <= 8192 && m <= 8.2 * n && n <= 8.2 * m;
     return mn && (op != MELA_OP_MATMUL || (p >= 32 && p <= 8192));
 }
 static const float *weights_for(const CostModelWeights &w, int op, double m, double n, double p)
