@@ -149,7 +149,9 @@ mela_status mela_diag_wait_timeout(int32_t kind, uint64_t limit_ns, uint32_t *d_
  * inner dimension mismatch -> MELA_ERR_DIM, other classes -> MELA_ERR_TYPE. */
 mela_status mela_matmul_gf2(const mela_host_matrix *A, const mela_host_matrix *B,
                             uint8_t *C);
-/* Same result through the Four-Russians kernel (src/mela_matmul_m4ri.c). */
+/* Same result through the Four-Russians kernel (src/mela_matmul_m4ri.c);
+ * arrays small enough to be multiplied straight from their MATLAB layout (up
+ * to 256 bits of inner dimension) take that form in both functions. */
 mela_status mela_matmul_m4ri(const mela_host_matrix *A, const mela_host_matrix *B,
                              uint8_t *C);
 
@@ -266,7 +268,11 @@ size_t mela_matmul_workspace_size(int32_t variant, int64_t m, int64_t k, int64_t
 /* C = A*B mod 2 on packed device matrices (A m x k, B k x n, C m x n).
  * Replaces the product loops of src/mela_matmul_gf2.c:111-208 and
  * src/mela_matmul_m4ri.c:179-248.  `workspace` must hold
- * mela_matmul_workspace_size() bytes (may be NULL when that is 0). */
+ * mela_matmul_workspace_size() bytes (may be NULL when that is 0), 16-byte
+ * aligned for the tensor-core forms (AUTO takes another form where it is
+ * not).  dC may lie over dA or dB, row for row, with AUTO and the tensor-core
+ * forms; with MELA_GEMM_M4RI over dA up to 2048 columns of C and over dB up
+ * to 512 rows. */
 mela_status mela_dev_matmul(int32_t variant, const uint64_t *dA, int64_t lda,
                             const uint64_t *dB, int64_t ldb, uint64_t *dC, int64_t ldc,
                             int64_t m, int64_t k, int64_t n, void *workspace,
@@ -276,7 +282,9 @@ mela_status mela_dev_matmul(int32_t variant, const uint64_t *dA, int64_t lda,
  * separately: operand preparation into the workspace (B transposed; for the
  * tensor-core form also the 0/1 byte expansion of A and B^T), then the
  * product kernel over the prepared operands.  Same arguments and workspace
- * as mela_dev_matmul; run must follow prepare on the same stream. */
+ * as mela_dev_matmul; run must follow prepare on the same stream.  The two
+ * halves multiply the operands whole; mela_dev_matmul itself takes very large
+ * ones (27000 cubed and up) apart into seven products of half their size. */
 mela_status mela_dev_matmul_prepare(int32_t variant, const uint64_t *dA, int64_t lda,
                                     const uint64_t *dB, int64_t ldb, int64_t m, int64_t k,
                                     int64_t n, void *workspace, size_t workspace_bytes,
