@@ -83,7 +83,8 @@ typedef enum {
     MELA_ELIM_M4RI_K4 = 3, /* the same panels with 4-bit tables (M4RI k = 4) */
     MELA_ELIM_FUSED = 4,   /* the whole elimination by one CTA in one launch */
     MELA_ELIM_TC = 5       /* 256-column windows, trailing update on the tensor cores (tcgen05 kind::i8);
-                              where AUTO picks it for a small matrix the update goes by tables */
+                              where AUTO picks it for a small matrix the update goes by tables. An RREF of at
+                              most 64 columns takes one panel, here and by MELA_ELIM_M4RI */
 } mela_elim_variant;
 
 /* Tuning fields of a variant argument.  A variant argument is a base

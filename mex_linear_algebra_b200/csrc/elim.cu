@@ -749,19 +749,22 @@ mela_status elim_device(int variant_arg, u64 *M, i64 ld, i64 m, i64 n, int rref,
     // the tensor cores; RREF 4096 x 8192 603 / 656, 8192 x 8192 1230 / 1183).
     // The windows want a 16-byte aligned workspace, and more of it than the
     // panels: a Four-Russians call that brings less takes panels, and so does
-    // AUTO on another alignment.  So does an RREF of one panel, where a window's
-    // launches and fork cost more (20 x 20 27 against 37 us a call, 5000 x 64 32
-    // against 38, 50000 x 64 32 against 56; a rank ends with the factorization,
-    // 16 us).
-    const bool aligned = ((uintptr_t)ws & 15) == 0;
-    const bool tables = (variant_arg == MELA_ELIM_M4RI && aligned && ws_bytes >= elim_tc_workspace(m, n) &&
-                         !(rref && n <= 64)) ||
+    // AUTO on another alignment.
+    const bool aligned = ((uintptr_t)ws & 15) == 0, room = ws_bytes >= elim_tc_workspace(m, n);
+    // An RREF of one panel goes by it in either form: a window's launches and
+    // fork cost more (Four-Russians form 20 x 20 27 against 37 us a call, 5000 x
+    // 64 32 against 38, 50000 x 64 32 against 56; tensor-core form, ones at 0.5
+    // and 0.01: 100000 x 64 35 and 41 against 79 and 432, 3000000 x 16 152 and
+    // 145 against 1152 and 768; a rank ends with the factorization, 16 us).
+    // More rows than the panels take stay with the windows in the tensor-core
+    // form.
+    const bool one = rref && n <= 64;
+    const bool tables = (variant_arg == MELA_ELIM_M4RI && aligned && room && !one) ||
                         (chosen && variant == MELA_ELIM_TC && aligned && (double)m * (double)n <= 4e7);
-    if (chosen && variant == MELA_ELIM_TC && !aligned) {
+    if (variant == MELA_ELIM_TC && (aligned ? one && room && m <= 1024ll * 65535 : chosen)) {
         variant = MELA_ELIM_M4RI;
         decode_elim_variant(variant, &tune);
-    }
-    if (variant == MELA_ELIM_TC || tables)
+    } else if (variant == MELA_ELIM_TC || tables)
         return elim_windows_device(M, ld, m, n, rref, tables, variant_arg == MELA_ELIM_M4RI, d_rank, d_piv, d_prow, ws,
                                    ws_bytes, s);
     ElimLayout L = elim_layout(m, n);

@@ -1,4 +1,4 @@
-"""Four-Russians eliminations of one to five words of columns, where the RREF
+"""Four-Russians and window eliminations of one to five words of columns, where the RREF
 goes by panels up to one word: against the oracle."""
 import numpy as np
 import pytest
@@ -10,7 +10,7 @@ from mex_linear_algebra_b200 import _lib
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("form", ["M4RI", "M4RI_K4"])
+@pytest.mark.parametrize("form", ["M4RI", "M4RI_K4", "TC"])
 @pytest.mark.parametrize("m", [1, 2, 63, 300, 1025, 3000])
 @pytest.mark.parametrize("n", [1, 3, 63, 64, 65, 128, 256, 257])
 def test_few_columns(cuda, form, m, n):
